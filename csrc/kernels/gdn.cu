@@ -30,66 +30,154 @@ __device__ __forceinline__ float dsilu_f(float x) {
   return s * (1.f + x * (1.f - s));
 }
 
-// x [B, L, C] (row stride ldx), w [C, K], left [B, C, K-1] or null, y [B, L, C] contiguous.
-// One thread per (b, t, c); consecutive threads walk c, so every access is coalesced.
-__global__ void gdn_conv_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w,
-                                    const __nv_bfloat16* __restrict__ left, int B, int L, int C, int K, int act,
-                                    __nv_bfloat16* __restrict__ y) {
-  const long long n = static_cast<long long>(B) * L * C;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int c = static_cast<int>(i % C);
-    const long long bt = i / C;
-    const int t = static_cast<int>(bt % L), b = static_cast<int>(bt / L);
-    float acc = 0.f;
-    for (int j = 0; j < K; ++j) {
-      const int ts = t - (K - 1) + j;
-      float xv;
-      if (ts >= 0) xv = __bfloat162float(x[(static_cast<long long>(b) * L + ts) * ldx + c]);
-      else xv = left ? __bfloat162float(left[(static_cast<long long>(b) * C + c) * (K - 1) + (K - 1 + ts)]) : 0.f;
-      acc += __bfloat162float(w[c * K + j]) * xv;
+// Causal depthwise convolution, forward and backward.  x [B, L, C] (row stride ldx), w [C, K], left [B, C, K-1] or null,
+// y, dy, dx [B, L, C] contiguous.  Bound by memory: every input is wanted once and every output written once.  A thread
+// owns V neighbouring channels (V = 8: one 16-byte access a token) and walks `run` tokens with the last K - 1 inputs in
+// registers, so a token is read once and not once per tap; the K - 1 tokens in front of a run are the only ones read
+// twice.  [5119, 10240] channels, K = 4: forward 371 us with one element a thread, K reads a token and an index division
+// each, 93 us so (210 MB; what is left is the SiLU's arithmetic as much as the traffic); backward 1043 us, which also
+// formed every output K times, 135 us so (315 MB).  The taps are added in the same order as before, so the results are
+// the same bits.
+template <int V>
+__device__ __forceinline__ void conv_load(const __nv_bfloat16* p, float (&f)[V]) {
+  if constexpr (V == 8) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 t = __bfloat1622float2(h[e]);
+      f[2 * e] = t.x;
+      f[2 * e + 1] = t.y;
     }
-    // the eager form rounds the conv output to the activation dtype before the SiLU
-    acc = __bfloat162float(__float2bfloat16_rn(acc));
-    y[i] = __float2bfloat16_rn(act ? silu_f(acc) : acc);
+  } else {
+    f[0] = __bfloat162float(p[0]);
+  }
+}
+template <int V>
+__device__ __forceinline__ void conv_store(__nv_bfloat16* p, const float (&f)[V]) {
+  if constexpr (V == 8) {
+    uint4 u;
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+    *reinterpret_cast<uint4*>(p) = u;
+  } else {
+    p[0] = __float2bfloat16_rn(f[0]);
+  }
+}
+// channels c .. c+V-1 of x at token t of row b; the carried context where t < 0
+template <int K, int V>
+__device__ __forceinline__ void conv_input(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ left,
+                                           int b, int t, int c, int L, int C, float (&f)[V]) {
+  if (t >= 0) {
+    conv_load<V>(x + (static_cast<long long>(b) * L + t) * ldx + c, f);
+  } else {
+#pragma unroll
+    for (int e = 0; e < V; ++e)
+      f[e] = left ? __bfloat162float(left[(static_cast<long long>(b) * C + c + e) * (K - 1) + (K - 1 + t)]) : 0.f;
   }
 }
 
-// dx[b,t,c] = sum_j w[c,j] * dpre[b, t + K-1-j, c], dpre = dy * silu'(pre); pre is recomputed.
-__global__ void gdn_conv_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w,
-                                    const __nv_bfloat16* __restrict__ left, const __nv_bfloat16* __restrict__ dy,
-                                    int B, int L, int C, int K, int act, __nv_bfloat16* __restrict__ dx) {
-  const long long n = static_cast<long long>(B) * L * C;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int c = static_cast<int>(i % C);
-    const long long bt = i / C;
-    const int t = static_cast<int>(bt % L), b = static_cast<int>(bt / L);
-    float wv[kMaxConvK];
-    for (int j = 0; j < K; ++j) wv[j] = __bfloat162float(w[c * K + j]);
-    // inputs x[t-(K-1) .. t+(K-1)] cover every output this input feeds
-    float xin[2 * kMaxConvK - 1];
-    for (int o = 0; o < 2 * K - 1; ++o) {
-      const int ts = t - (K - 1) + o;
-      if (ts >= L) xin[o] = 0.f;
-      else if (ts >= 0) xin[o] = __bfloat162float(x[(static_cast<long long>(b) * L + ts) * ldx + c]);
-      else xin[o] = left ? __bfloat162float(left[(static_cast<long long>(b) * C + c) * (K - 1) + (K - 1 + ts)]) : 0.f;
+template <int K, int V>
+__global__ void __launch_bounds__(128)
+gdn_conv_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w,
+                    const __nv_bfloat16* __restrict__ left, int L, int C, int runs, int run, int act, __nv_bfloat16* __restrict__ y) {
+  const int c = (blockIdx.y * 128 + threadIdx.x) * V;
+  if (c >= C) return;
+  const int b = blockIdx.x / runs, t0 = (blockIdx.x - b * runs) * run, t1 = min(L, t0 + run);
+  float wv[K][V], win[K][V];            // win[j]: the input that tap j meets
+#pragma unroll
+  for (int j = 0; j < K; ++j)
+#pragma unroll
+    for (int e = 0; e < V; ++e) wv[j][e] = __bfloat162float(w[(c + e) * K + j]);
+#pragma unroll
+  for (int j = 1; j < K; ++j) conv_input<K, V>(x, ldx, left, b, t0 - K + j, c, L, C, win[j]);
+#pragma unroll 4
+  for (int t = t0; t < t1; ++t) {
+#pragma unroll
+    for (int j = 0; j + 1 < K; ++j)
+#pragma unroll
+      for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
+    conv_load<V>(x + (static_cast<long long>(b) * L + t) * ldx + c, win[K - 1]);
+    float o[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      float acc = 0.f;
+#pragma unroll
+      for (int j = 0; j < K; ++j) acc += wv[j][e] * win[j][e];
+      // the eager form rounds the conv output to the activation dtype before the SiLU
+      acc = __bfloat162float(__float2bfloat16_rn(acc));
+      o[e] = act ? silu_f(acc) : acc;
     }
-    float acc = 0.f;
-    for (int j = 0; j < K; ++j) {
-      const int to = t + (K - 1) - j;       // output position that reads x[t] through tap j
-      if (to >= L) continue;
-      float d = __bfloat162float(dy[(static_cast<long long>(b) * L + to) * C + c]);
-      if (act) {
-        float pre = 0.f;
-        for (int jj = 0; jj < K; ++jj) pre += wv[jj] * xin[(to - t) + jj];
-        pre = __bfloat162float(__float2bfloat16_rn(pre));
-        d *= dsilu_f(pre);
-      }
-      acc += wv[j] * d;
-    }
-    dx[i] = __float2bfloat16_rn(acc);
+    conv_store<V>(y + (static_cast<long long>(b) * L + t) * C + c, o);
   }
+}
+
+// dx[b,t,c] = sum_j w[c,j] * dpre[b, t + K-1-j, c], dpre = dy * silu'(pre); pre is recomputed, once for each output.
+template <int K, int V>
+__global__ void __launch_bounds__(128)
+gdn_conv_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w,
+                    const __nv_bfloat16* __restrict__ left, const __nv_bfloat16* __restrict__ dy, int L, int C, int runs, int run,
+                    int act, __nv_bfloat16* __restrict__ dx) {
+  const int c = (blockIdx.y * 128 + threadIdx.x) * V;
+  if (c >= C) return;
+  const int b = blockIdx.x / runs, t0 = (blockIdx.x - b * runs) * run, t1 = min(L, t0 + run);
+  float wv[K][V], win[K][V], d[K][V];   // d[j]: the gradient that tap j passes on, that of output t + K - 1 - j
+#pragma unroll
+  for (int j = 0; j < K; ++j)
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      wv[j][e] = __bfloat162float(w[(c + e) * K + j]);
+      d[j][e] = 0.f;
+    }
+#pragma unroll
+  for (int j = 1; j < K; ++j) conv_input<K, V>(x, ldx, left, b, t0 - K + j, c, L, C, win[j]);
+#pragma unroll 4
+  for (int to = t0; to < t1 + K - 1; ++to) {
+#pragma unroll
+    for (int j = K - 1; j > 0; --j)
+#pragma unroll
+      for (int e = 0; e < V; ++e) d[j][e] = d[j - 1][e];
+    if (to < L) {
+#pragma unroll
+      for (int j = 0; j + 1 < K; ++j)
+#pragma unroll
+        for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
+      conv_load<V>(x + (static_cast<long long>(b) * L + to) * ldx + c, win[K - 1]);
+      conv_load<V>(dy + (static_cast<long long>(b) * L + to) * C + c, d[0]);
+      if (act) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          float pre = 0.f;
+#pragma unroll
+          for (int j = 0; j < K; ++j) pre += wv[j][e] * win[j][e];
+          d[0][e] *= dsilu_f(__bfloat162float(__float2bfloat16_rn(pre)));
+        }
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < V; ++e) d[0][e] = 0.f;
+    }
+    const int t = to - (K - 1);
+    if (t >= t0) {
+      float o[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        o[e] = 0.f;
+#pragma unroll
+        for (int j = 0; j < K; ++j) o[e] += wv[j][e] * d[j][e];
+      }
+      conv_store<V>(dx + (static_cast<long long>(b) * L + t) * C + c, o);
+    }
+  }
+}
+
+// Tokens per thread: long runs re-read less context (K - 1 tokens a run); a short input takes shorter ones until the
+// chip has about 2048 threads an SM.
+int conv_run(long long rows_of_tokens, int L, int C, int V) {
+  int run = 32;
+  while (run > 4 && rows_of_tokens * ((L + run - 1) / run) * (C / V) < 148LL * 2048) run /= 2;
+  return run;
 }
 
 // One token: y[b,c] = act(sum_j w[c,j] * ctx[j]), ctx = [state[b,c,:], x[b,c]]; state shifts left.
@@ -542,33 +630,54 @@ gdn_chunk_fwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* _
 
 }  // namespace
 
+namespace {
+
+// 16-byte accesses want whole groups of eight channels on 16-byte boundaries; anything else goes channel by channel.
+bool conv_vec(int C, long long ldx, const void* x, const void* y, const void* z) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z);
+  return C % 8 == 0 && ldx % 8 == 0 && at % 16 == 0;
+}
+
+template <int K>
+void conv_launch(bool bwd, const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, const __nv_bfloat16* left,
+                 const __nv_bfloat16* dy, int B, int L, int C, int act, __nv_bfloat16* out, cudaStream_t stream) {
+  const bool vec = conv_vec(C, ldx, x, out, dy);
+  const int V = vec ? 8 : 1, run = conv_run(B, L, C, V), runs = (L + run - 1) / run;
+  const dim3 grid(B * runs, (C / V + 127) / 128);
+  if (!bwd && vec) gdn_conv_fwd_kernel<K, 8><<<grid, 128, 0, stream>>>(x, ldx, w, left, L, C, runs, run, act, out);
+  else if (!bwd) gdn_conv_fwd_kernel<K, 1><<<grid, 128, 0, stream>>>(x, ldx, w, left, L, C, runs, run, act, out);
+  else if (vec) gdn_conv_bwd_kernel<K, 8><<<grid, 128, 0, stream>>>(x, ldx, w, left, dy, L, C, runs, run, act, out);
+  else gdn_conv_bwd_kernel<K, 1><<<grid, 128, 0, stream>>>(x, ldx, w, left, dy, L, C, runs, run, act, out);
+}
+
+const char* conv_any(bool bwd, const void* x, long long ldx, const void* w, const void* left, const void* dy, int B, int L, int C,
+                     int K, bool act, void* out, cudaStream_t stream) {
+  if (K < 1 || K > kMaxConvK) return "gdn_conv: kernel width 1..8";
+  if (static_cast<long long>(B) * L * C == 0) return nullptr;
+  const auto* xp = static_cast<const __nv_bfloat16*>(x);
+  const auto* wp = static_cast<const __nv_bfloat16*>(w);
+  const auto* lp = static_cast<const __nv_bfloat16*>(left);
+  const auto* dp = static_cast<const __nv_bfloat16*>(dy);
+  auto* op = static_cast<__nv_bfloat16*>(out);
+  switch (K) {
+#define FERRL_CONV(KV) case KV: conv_launch<KV>(bwd, xp, ldx, wp, lp, dp, B, L, C, act ? 1 : 0, op, stream); break
+    FERRL_CONV(1); FERRL_CONV(2); FERRL_CONV(3); FERRL_CONV(4); FERRL_CONV(5); FERRL_CONV(6); FERRL_CONV(7); FERRL_CONV(8);
+#undef FERRL_CONV
+  }
+  count_launch();
+  return cudaGetLastError() == cudaSuccess ? nullptr : (bwd ? "gdn_conv_bwd launch failed" : "gdn_conv_fwd launch failed");
+}
+
+}  // namespace
+
 const char* gdn_conv_fwd(const void* x, long long ldx, const void* w, const void* left, int B, int L, int C, int K,
                          bool act, void* y, cudaStream_t stream) {
-  if (K < 1 || K > kMaxConvK) return "gdn_conv: kernel width 1..8";
-  const long long n = static_cast<long long>(B) * L * C;
-  if (n == 0) return nullptr;
-  const int blocks = static_cast<int>(std::min<long long>((n + 255) / 256, 148 * 32));
-  gdn_conv_fwd_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), ldx,
-                                                  static_cast<const __nv_bfloat16*>(w),
-                                                  static_cast<const __nv_bfloat16*>(left), B, L, C, K, act ? 1 : 0,
-                                                  static_cast<__nv_bfloat16*>(y));
-  count_launch();
-  return cudaGetLastError() == cudaSuccess ? nullptr : "gdn_conv_fwd launch failed";
+  return conv_any(false, x, ldx, w, left, nullptr, B, L, C, K, act, y, stream);
 }
 
 const char* gdn_conv_bwd(const void* x, long long ldx, const void* w, const void* left, const void* dy, int B, int L,
                          int C, int K, bool act, void* dx, cudaStream_t stream) {
-  if (K < 1 || K > kMaxConvK) return "gdn_conv: kernel width 1..8";
-  const long long n = static_cast<long long>(B) * L * C;
-  if (n == 0) return nullptr;
-  const int blocks = static_cast<int>(std::min<long long>((n + 255) / 256, 148 * 32));
-  gdn_conv_bwd_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), ldx,
-                                                  static_cast<const __nv_bfloat16*>(w),
-                                                  static_cast<const __nv_bfloat16*>(left),
-                                                  static_cast<const __nv_bfloat16*>(dy), B, L, C, K, act ? 1 : 0,
-                                                  static_cast<__nv_bfloat16*>(dx));
-  count_launch();
-  return cudaGetLastError() == cudaSuccess ? nullptr : "gdn_conv_bwd launch failed";
+  return conv_any(true, x, ldx, w, left, dy, B, L, C, K, act, dx, stream);
 }
 
 const char* gdn_conv_step(const void* x, long long ldx, const void* w, void* state, int B, int C, int K, bool act,

@@ -1,0 +1,31 @@
+"""Causal convolution kernels at the edges of their runs of tokens and groups of channels, against float64 autograd."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,L,C,K,wide,left", [
+    (2, 31, 64, 4, 96, True), (1, 32, 64, 4, 64, False), (3, 33, 2048, 4, 2056, True),    # around a run of 32 tokens, strided rows
+    (2, 129, 24, 3, 24, True), (1, 5, 8, 8, 16, True), (2, 70, 16, 1, 16, False),          # few channels, widest and narrowest kernel
+    (1, 1, 8, 4, 8, True), (2, 37, 100, 4, 108, True), (2, 9, 20, 2, 21, False),           # one token; no whole groups of eight
+])
+def test_conv_at_run_and_group_edges(B, L, C, K, wide, left):
+    from ferrl_b200.ops import cuda as Cc
+    g = torch.Generator(device="cuda").manual_seed(L * C + K)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    x, w, dy = rnd(B, L, wide)[..., :C], rnd(C, K), rnd(B, L, C)
+    ctx = rnd(B, C, K - 1) if left else None
+    xr = x.double().requires_grad_()
+    pad = torch.cat([(ctx if left else x.new_zeros(B, C, K - 1)).double(), xr.transpose(1, 2)], -1)
+    pre = sum(w.double()[:, j, None] * pad[..., j:j + L] for j in range(K)).transpose(1, 2)
+    # the kernel rounds `pre` to bf16 once (2^-9 of it) and silu' is at most 1.1, silu'' at most 0.5; outputs are rounded once
+    for act in (False, True):
+        ref = torch.nn.functional.silu(pre) if act else pre
+        y = Cc.lib().gdn_conv_fwd(x, w, ctx, act)
+        assert bool(((y.double() - ref).abs() <= 2 ** -8 * ref.abs() + 1.2 * 2 ** -8 * pre.abs() + 1e-6).all())
+        (dref,) = torch.autograd.grad(ref, xr, dy.double(), retain_graph=True)
+        scale = sum(w.double()[:, j].abs() * torch.nn.functional.pad((dy.double().abs() * (1.1 + 0.5 * pre.detach().abs() if act else 1)),
+                                                                    (0, 0, 0, K - 1))[:, K - 1 - j:K - 1 - j + L] for j in range(K))
+        dx = Cc.lib().gdn_conv_bwd(x, w, ctx, dy, act)
+        assert bool(((dx.double() - dref).abs() <= 2 ** -8 * dref.abs() + 2 ** -8 * scale + 1e-6).all())
