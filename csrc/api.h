@@ -19,6 +19,7 @@ struct GluAct { int act; float alpha, limit; };
 struct GemmArgs {
   const void* A; const void* B; const void* A2; const void* B2;  // bf16, K-major
   long long lda, ldb, lda2, ldb2;                                 // row strides in elements
+  int b_mn;                                                       // B and B2 are [K, N] / [K2, N] (grouped: [experts * K, N]), N contiguous
   int M, N, K, K2;
   void* out; long long ldo; bool out_f32;
   const void* residual; long long ldr;                            // optional bf16 [M, ldr]

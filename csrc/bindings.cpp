@@ -281,6 +281,36 @@ Tensor gemm(const Tensor& A, const Tensor& B, const optional<Tensor>& A2, const 
   return out;
 }
 
+// A [M,K] @ B [K,N] (+ A2 [M,K2] @ B2 [K2,N]) with B and B2 as they lie in memory: the input gradient of a projection
+// reads its [N,K] weight without a transposed copy.  Rules of choice as in gemm().
+Tensor gemm_nn(const Tensor& A, const Tensor& B, const optional<Tensor>& A2, const optional<Tensor>& B2) {
+  TORCH_CHECK(A.is_cuda() && B.is_cuda() && A.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16 && A.dim() == 2 &&
+                  B.dim() == 2 && A.size(1) == B.size(0) && A.stride(1) == 1 && B.stride(1) == 1, "gemm_nn: A [M,K], B [K,N] bf16");
+  c10::cuda::CUDAGuard guard(A.device());
+  ferrl::GemmArgs a{};
+  a.A = A.data_ptr(); a.B = B.data_ptr(); a.lda = A.stride(0); a.ldb = B.stride(0);
+  a.M = A.size(0); a.N = B.size(1); a.K = A.size(1); a.b_mn = 1;
+  if (A2.has_value() && A2->defined()) {
+    TORCH_CHECK(B2.has_value() && B2->defined() && A2->scalar_type() == at::kBFloat16 && B2->scalar_type() == at::kBFloat16 &&
+                    A2->dim() == 2 && B2->dim() == 2 && A2->size(0) == a.M && B2->size(1) == a.N && A2->size(1) == B2->size(0) &&
+                    A2->stride(1) == 1 && B2->stride(1) == 1, "gemm_nn: side operands A2 [M,K2], B2 [K2,N] bf16");
+    a.A2 = A2->data_ptr(); a.B2 = B2->data_ptr(); a.lda2 = A2->stride(0); a.ldb2 = B2->stride(0); a.K2 = A2->size(1);
+  }
+  Tensor out = out_empty({a.M, a.N}, A.options());
+  a.out = out.data_ptr(); a.ldo = a.N;
+  a.status = status_word(); a.num_sms = num_sms();
+  if (a.M >= 1024 && a.N >= 512) {
+    a.two_cta = 256;
+  } else {
+    int bn = 0, split = 1, cluster = 1;
+    ferrl::gemm_plan(a.M, a.N, a.K, a.K2, a.num_sms, &bn, &split, &cluster, nullptr);
+    a.force_bn = bn == 176 ? 256 : bn < 64 ? 64 : bn;
+    if (cluster > 1) a.cluster_k = cluster;
+  }
+  FERRL_CHECK(ferrl::gemm_bf16(a, stream()));
+  return out;
+}
+
 // act(x Wg^T) * (x Wu^T) in one kernel: W holds the gate and up rows interleaved in groups of 16
 // (8 gate rows, then the 8 up rows of the same features); returns [M, N/2].
 Tensor gemm_glu(const Tensor& A, const Tensor& B, int64_t act, bool static_b, double alpha, double limit) {
@@ -701,14 +731,15 @@ Tensor moe_gather(const Tensor& x, const Tensor& token_of, const optional<Tensor
 }
 
 // ys[rows, N] = xs[rows, K] x W[e(row)]^T with W [E, N, K]; rows sorted by expert in 128-row segments
-Tensor moe_grouped_gemm(const Tensor& xs, const Tensor& W, const Tensor& tile_expert, const optional<Tensor>& out_buf) {
+// `nn`: W is [E,K,N] instead (the weight of the forward pass read by the backward one; K a multiple of 64).
+Tensor moe_grouped_gemm(const Tensor& xs, const Tensor& W, const Tensor& tile_expert, const optional<Tensor>& out_buf, bool nn) {
   TORCH_CHECK(xs.is_cuda() && xs.scalar_type() == at::kBFloat16 && W.scalar_type() == at::kBFloat16, "moe_grouped_gemm: bf16");
-  TORCH_CHECK(xs.dim() == 2 && W.dim() == 3 && W.is_contiguous() && xs.is_contiguous() && xs.size(1) == W.size(2), "moe_grouped_gemm: xs [R,K], W [E,N,K]");
+  TORCH_CHECK(xs.dim() == 2 && W.dim() == 3 && W.is_contiguous() && xs.is_contiguous() && xs.size(1) == W.size(nn ? 1 : 2), "moe_grouped_gemm: xs [R,K], W [E,N,K]");
   TORCH_CHECK(xs.size(0) % 128 == 0 && tile_expert.numel() * 128 >= xs.size(0) && tile_expert.scalar_type() == at::kInt, "moe_grouped_gemm: rows in 128-row tiles with one expert id each");
   c10::cuda::CUDAGuard guard(xs.device());
   ferrl::GemmArgs a{};
   a.A = xs.data_ptr(); a.B = W.data_ptr(); a.lda = xs.stride(0); a.ldb = W.size(2);
-  a.M = xs.size(0); a.N = W.size(1); a.K = xs.size(1);
+  a.M = xs.size(0); a.N = W.size(nn ? 2 : 1); a.K = xs.size(1); a.b_mn = nn;
   a.tile_expert = tile_expert.data_ptr<int>(); a.n_experts = W.size(0);
   // rows of unused tiles are never written: start from zeros so padding stays finite downstream
   Tensor out;
@@ -1840,6 +1871,7 @@ void add_launches(int64_t n) { ferrl::count_launch(static_cast<int>(n)); }
 }  // namespace
 
 TORCH_LIBRARY(ferrl_b200, m) {
+  m.def("gemm_nn(Tensor a, Tensor b, Tensor? a2=None, Tensor? b2=None) -> Tensor", &gemm_nn);
   m.def("gemm(Tensor A, Tensor B, Tensor? A2, Tensor? B2, Tensor? residual, bool out_f32, int force_bn, int force_split, int two_cta=0, Tensor? debug=None, int cluster_k=0, int stream_k=0, bool static_b=False) -> Tensor", &gemm);  // two_cta: 0 auto, -1 never, 128/256 forced
   m.def("decode_gemm(Tensor A, Tensor B, Tensor? residual=None, int glu_act=-1, int max_clusters=0, bool static_b=False, Tensor? debug=None) -> Tensor", &decode_gemm);
   m.def("set_decode_gemm(bool on) -> ()", &set_decode_gemm);
@@ -1860,7 +1892,7 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("moe_route(Tensor logits, int k, bool renorm, int score=0) -> (Tensor, Tensor, Tensor, Tensor)", &moe_route);
   m.def("moe_plan(Tensor idx, Tensor counts) -> (Tensor, Tensor, Tensor, Tensor)", &moe_plan);
   m.def("moe_gather(Tensor x, Tensor token_of, Tensor? pair_w, Tensor row_of) -> Tensor", &moe_gather);
-  m.def("moe_grouped_gemm(Tensor xs, Tensor W, Tensor tile_expert, Tensor(a!)? out=None) -> Tensor(a!)", &moe_grouped_gemm);
+  m.def("moe_grouped_gemm(Tensor xs, Tensor W, Tensor tile_expert, Tensor(a!)? out=None, bool nn=False) -> Tensor(a!)", &moe_grouped_gemm);
   m.def("ep_dispatch(Tensor x, Tensor idx, Tensor? pair_w, Tensor counts, int[] counts_all, int[] xs, int[] flags, int rank, int world, int epoch, float limit_s, int cap_rows, Tensor(a!) dest_row, Tensor(b!) tile_expert, Tensor(c!) local_rows, bool reuse_plan, Tensor(d!) abort_word) -> ()", &ep_dispatch);
   m.def("ep_combine(int[] ys, Tensor idx, Tensor dest_row, Tensor? w, int H, int E_local, int[] flags, int rank, int world, int epoch, float limit_s, Tensor(a!)? keep_rows, Tensor(b!) abort_word) -> Tensor", &ep_combine);
   m.def("moe_combine(Tensor ys, Tensor row_of, Tensor? w, int T, int k) -> Tensor", &moe_combine);

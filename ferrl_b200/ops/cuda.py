@@ -61,6 +61,12 @@ def gemm(a, b, a2=None, b2=None, residual=None, out_f32=False, force_bn=0, force
                       bool(static_b))
 
 
+def gemm_nn(a, b, a2=None, b2=None):
+    """``a [M,K] @ b [K,N] (+ a2 [M,K2] @ b2 [K2,N])``: the second operands are read as they lie, so the input gradient of
+    a projection needs no transposed copy of its ``[N,K]`` weight.  ``N`` and ``K`` multiples of 8."""
+    return lib().gemm_nn(a, b, a2, b2)
+
+
 def gemm_glu(x, w_interleaved, act="silu"):
     """``act(x Wg^T) * (x Wu^T)`` with ``w_interleaved`` ``[2F, K]`` holding gate and up rows in groups of
     16 (8 gate, 8 up): the GLU runs in the GEMM epilogue (``[..., F]`` out, no ``[..., 2F]`` round trip)."""
@@ -137,13 +143,13 @@ class _LoraLinear(torch.autograd.Function):
         dx = da = db = None
         u = None
         if a_stack is not None:
-            u = gemm(dy2, b16.t().contiguous())                                # [M, R] = dy @ B
+            u = gemm_nn(dy2, b16)                                              # [M, R] = dy @ B
         if ctx.x_grad:
-            wt_ = wt if wt is not None else w.t().contiguous()
-            if u is not None:
-                dx = gemm(dy2, wt_, u, a16.t().contiguous())
+            # a resident transpose is read K-major like every forward operand (0 to 4 % faster); else the weight as it lies
+            if wt is None:
+                dx = gemm_nn(dy2, w, u, a16)
             else:
-                dx = gemm(dy2, wt_)
+                dx = gemm(dy2, wt, u, None if u is None else a16.t().contiguous())
             dx = dx.view(ctx.x_shape)
         if a_stack is not None:
             R = a_stack.shape[0]
@@ -879,6 +885,15 @@ def moe_route(logits_f32, k, renorm=True, score="softmax"):
     return _MoeRoute.apply(logits_f32, int(k), bool(renorm), score)
 
 
+def _grouped_input_grad(dy, w, wt, tile_expert):
+    """``dy_e @ w_e`` per expert for frozen ``w`` ``[E,N,K]``, read as it lies where the kernel can (``N`` a multiple of
+    64: a k-block must not reach into the next expert); ``wt`` is the optional resident transpose."""
+    out = dy.new_empty(dy.shape[0], w.shape[2])
+    if wt is None and w.shape[1] % 64 == 0:
+        return lib().moe_grouped_gemm(dy, w, tile_expert, out, True)
+    return lib().moe_grouped_gemm(dy, w.transpose(1, 2).contiguous() if wt is None else wt, tile_expert, out)
+
+
 class _MoeExperts(torch.autograd.Function):
     """Routed frozen experts: plan -> gather -> grouped GEMM -> SwiGLU -> grouped GEMM -> combine,
     with no host synchronisation; gradients flow to the tokens and to the routing scores.  The routing weights
@@ -891,15 +906,12 @@ class _MoeExperts(torch.autograd.Function):
         sc = scores.float().contiguous()
         row_of, token_of, tile_expert, _ = L.moe_plan(idx.contiguous(), counts)
         xs = L.moe_gather(x.contiguous(), token_of, sc if weight_input else None, row_of)
-        # rows of unused tiles are never written and never read back (the combine reads routed rows only); the
-        # zero fill of the outputs is kept for training, where the padded rows are saved for the backward pass
-        train = any(ctx.needs_input_grad)
-        o1 = None if train else torch.empty(xs.shape[0], gate_up.shape[1], dtype=xs.dtype, device=xs.device)
-        gu = L.moe_grouped_gemm(xs, gate_up, tile_expert, o1)
+        # rows of unused tiles are never written and never read back: the combine and the score gradient read routed rows
+        # only, the grouped products skip those tiles in both directions
+        gu = L.moe_grouped_gemm(xs, gate_up, tile_expert, xs.new_empty(xs.shape[0], gate_up.shape[1]))
         del xs
         h = L.glu_fwd(gu, act)
-        o2 = None if train else torch.empty(h.shape[0], down.shape[1], dtype=h.dtype, device=h.device)
-        ys = L.moe_grouped_gemm(h, down, tile_expert, o2)
+        ys = L.moe_grouped_gemm(h, down, tile_expert, h.new_empty(h.shape[0], down.shape[1]))
         del h
         out = L.moe_combine(ys, row_of, None if weight_input else sc, T, k)
         # kept rows: the outputs for the gradient of output weights, the tokens for that of input weights
@@ -918,15 +930,11 @@ class _MoeExperts(torch.autograd.Function):
         if not ctx.weight_input:
             dsc = L.moe_pair_dot(dout, ys, row_of, ctx.k).to(ctx.score_dtype)
         dys = L.moe_gather(dout, token_of, None if ctx.weight_input else sc.view(-1), row_of)
-        if down_t is None:
-            down_t = down.transpose(1, 2).contiguous()
-        dh = L.moe_grouped_gemm(dys, down_t, tile_expert)
+        dh = _grouped_input_grad(dys, down, down_t, tile_expert)
         del dys
         dgu = L.glu_bwd(gu, dh, ctx.act)
         del dh
-        if gate_up_t is None:
-            gate_up_t = gate_up.transpose(1, 2).contiguous()
-        dxs = L.moe_grouped_gemm(dgu, gate_up_t, tile_expert)
+        dxs = _grouped_input_grad(dgu, gate_up, gate_up_t, tile_expert)
         if ctx.weight_input:
             dsc = L.moe_pair_dot(ys.contiguous(), dxs, row_of, ctx.k).to(ctx.score_dtype)     # <token, d(weighted token)>
         dx = L.moe_combine(dxs, row_of, sc if ctx.weight_input else None, T, ctx.k)
@@ -983,13 +991,12 @@ class _LogprobGather(torch.autograd.Function):
         temperature, softcap = ctx.meta
         N, V = h.shape[0], head_w.shape[0]
         chunk = max(256, min(N, (LOGPROB_CHUNK_BYTES // (2 * V)) // 256 * 256)) if N else 1
-        wt = head_wt if head_wt is not None else head_w.t().contiguous()
         dh = torch.empty_like(h)
         coef = (-dlp).contiguous().float()
         for s in range(0, N, chunk):
             dl = lib().logprob_head_dlogits(h[s:s + chunk], head_w, t[s:s + chunk], lse[s:s + chunk], coef[s:s + chunk],
                                             temperature, softcap, 0)
-            dh[s:s + chunk] = gemm(dl, wt)
+            dh[s:s + chunk] = gemm_nn(dl, head_w) if head_wt is None else gemm(dl, head_wt)
             del dl
         return dh, None, None, None, None, None
 
