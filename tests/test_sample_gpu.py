@@ -1,0 +1,62 @@
+"""Sampler kernel where its slices, clusters, counters, segments and key ranges have edges, against a host restatement of its
+fixed-point arithmetic."""
+import numpy as np
+import pytest
+import torch
+
+from ferrl_b200.sampler import uniforms_for_rows
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,V,dtype,std,top_p,T,pad", [
+    (1, 1, torch.bfloat16, 1.0, 0.9, 1.0, 0), (3, 7, torch.float32, 1.0, 0.5, 0.7, 0),         # less than a group
+    (2, 8191, torch.bfloat16, 2.0, 0.95, 1.0, 1), (2, 8192, torch.float32, 3.0, 0.8, 1.2, 4),   # one CTA; ragged and strided rows
+    (1, 65537, torch.bfloat16, 2.5, 0.95, 1.0, 0), (5, 50257, torch.float32, 2.5, 0.9, 1.0, 3),  # clusters with a short last slice
+    (130, 151936, torch.bfloat16, 2.5, 0.95, 1.0, 0), (4, 262144, torch.float32, 2.5, None, 0.7, 0),
+    (4, 32000, torch.bfloat16, 0.0, 0.3, 1.0, 0), (4, 32000, torch.bfloat16, 40.0, 0.999, 1.0, 0),   # all equal; almost all mass on one
+    (2, 9000, torch.bfloat16, 0.01, 0.5, 1.0, 0), (2, 9000, torch.float32, 1e-3, 0.5, 1.0, 0),       # the cut around zero: widest key range
+    (2, 20000, torch.bfloat16, 300.0, 0.9, 100.0, 0), (2, 20000, torch.bfloat16, 1e-4, 0.9, 1.0, 0),  # values without a counter: large, small
+    (1, 1400000, torch.bfloat16, 2.0, 0.9, 1.0, 0),                                                  # slices of many elements
+])
+def test_draws_match_the_fixed_point_oracle(rows, V, dtype, std, top_p, T, pad):
+    from ferrl_b200.ops import cuda as Cc
+    g = torch.Generator(device="cuda").manual_seed(rows * V)
+    x = (torch.randn(rows, V + pad, generator=g, device="cuda") * std + (std == 0)).to(dtype)[:, :V]
+    if V > 100:
+        x[:, 5:50] = float("-inf")                                           # masked vocabulary entries
+    ids = torch.randint(0, 1 << 40, (rows,), generator=g, device="cuda")
+    u = uniforms_for_rows(11, ids.cpu(), 3).double().numpy()
+    tok, lp = (t.cpu().numpy() for t in Cc.sample_top_p(x, 11, ids, 3, T, top_p, None))
+    xs = x.double().cpu().numpy()
+    for r in range(rows):
+        # the device's exponential and its 2^-40 truncation move every mass by 1e-5 of it (arguments down to -90), which
+        # moves the cut and the drawn point by as much of the whole; lp additionally rounds a float32 logarithm
+        e = np.exp((xs[r] - xs[r].max()) / T)
+        keep = np.ones(V, bool)
+        eps = 2e-5
+        if top_p is not None:
+            order = np.argsort(-e, kind="stable")
+            cum = e[order].cumsum()
+            at = lambda p: e[order[min(V - 1, int(np.searchsorted(cum, p * cum[-1])))]]  # noqa: E731
+            lo, hi = at(min(1.0, top_p + eps)), at(top_p - eps)
+            assert e[tok[r]] >= lo * (1 - eps)
+            keep = e >= lo * (1 - eps)
+            surely = (e >= hi * (1 + eps)) | ((e == hi) & (lo == hi))
+        else:
+            surely = keep
+        slack = e[keep & ~surely].sum() + eps * e.sum()
+        before, mass = e[:tok[r]][surely[:tok[r]]].sum(), e[surely].sum()
+        assert u[r] * mass >= before - slack and u[r] * mass <= before + e[tok[r]] + slack
+        assert abs(lp[r] - np.log(e[tok[r]] / mass)) <= 2e-5 + 2 * slack / mass
+    again = Cc.sample_top_p(x.clone(), 11, ids, 3, T, top_p, None)
+    assert np.array_equal(again[0].cpu().numpy(), tok) and np.array_equal(again[1].cpu().numpy(), lp)
+
+
+def test_rows_without_mass_give_a_valid_token():
+    from ferrl_b200.ops import cuda as Cc
+    x = torch.full((3, 20000), float("-inf"), device="cuda", dtype=torch.bfloat16)
+    x[1, 777] = float("inf")
+    x[2] = float("nan")
+    tok, lp = Cc.sample_top_p(x, 1, torch.arange(3, device="cuda"), 0, 1.0, 0.9, None)
+    assert tok.tolist() == [0, 777, 0] and bool((lp <= 0).all())
