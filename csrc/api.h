@@ -378,7 +378,8 @@ const char* gdn_conv_step(const void* x, long long ldx, const void* w, void* sta
 const char* gdn_chunk_fwd(const void* q, const void* k, const void* v, long long q_bs, long long q_ts, long long k_bs,
                           long long k_ts, long long v_bs, long long v_ts, const float* g, const float* beta,
                           const float* S0, float* S_out, void* out, int B, int T, int Hk, int Hv, int KD, int VD,
-                          bool l2norm, float eps, cudaStream_t stream);
+                          bool l2norm, float eps, void* workspace, cudaStream_t stream);
+size_t gdn_chunk_workspace(int B, int T, int Hv);      // bytes that gdn_chunk_fwd takes
 // Optional gate inputs straight from the input projection (decode): a, b bf16 [B, Hv] with row strides lda, ldb,
 // A_log and dt_bias fp32 [Hv]; the kernel then forms g = -exp(A_log) softplus(a + dt_bias) and beta = sigmoid(b)
 // itself and ignores `g` / `beta`.

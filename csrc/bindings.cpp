@@ -649,8 +649,16 @@ std::vector<Tensor> gdn_tc_bwd(const Tensor& q, const Tensor& k, const Tensor& v
   return {dq, dk, dv, dbeta, dG, dS0};
 }
 
-std::tuple<Tensor, Tensor> gdn_chunk_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g,
+std::tuple<Tensor, Tensor> gdn_chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g,
                                          const Tensor& beta, const optional<Tensor>& S0, bool l2norm, double eps) {
+  // rows are read in 16-byte pieces: views that start or step elsewhere are copied
+  auto rows16 = [](const Tensor& t) {
+    const bool ok = t.dim() != 4 || !t.is_cuda() || (reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && t.stride(0) % 8 == 0 && t.stride(1) % 8 == 0);
+    return ok ? t : t.clone(at::MemoryFormat::Contiguous);
+  };
+  TORCH_CHECK(q_.is_cuda() && k_.is_cuda() && v_.is_cuda(), "gdn_chunk_fwd: bf16 [B,T,H,D]");
+  c10::cuda::CUDAGuard guard(q_.device());
+  const Tensor q = rows16(q_), k = rows16(k_), v = rows16(v_);
   TORCH_CHECK(q.is_cuda() && q.scalar_type() == at::kBFloat16 && k.scalar_type() == at::kBFloat16 &&
                   v.scalar_type() == at::kBFloat16 && q.dim() == 4 && k.dim() == 4 && v.dim() == 4, "gdn_chunk_fwd: bf16 [B,T,H,D]");
   const int64_t B = q.size(0), T = q.size(1), Hk = q.size(2), KD = q.size(3), Hv = v.size(2), VD = v.size(3);
@@ -658,20 +666,21 @@ std::tuple<Tensor, Tensor> gdn_chunk_fwd(const Tensor& q, const Tensor& k, const
   TORCH_CHECK(packed(q) && packed(k) && packed(v), "gdn_chunk_fwd: heads must be packed in the last two dims");
   TORCH_CHECK(g.scalar_type() == at::kFloat && beta.scalar_type() == at::kFloat && g.is_contiguous() && beta.is_contiguous() &&
                   g.numel() == B * T * Hv && beta.numel() == B * T * Hv, "gdn_chunk_fwd: g,beta f32 [B,T,Hv]");
-  c10::cuda::CUDAGuard guard(q.device());
   const float* s0 = nullptr;
   Tensor s0c;
   if (S0.has_value() && S0->defined()) {
     s0c = S0->to(at::kFloat).contiguous();
     TORCH_CHECK(s0c.numel() == B * Hv * KD * VD, "gdn_chunk_fwd: state [B,Hv,KD,VD]");
+    if (reinterpret_cast<uintptr_t>(s0c.data_ptr()) % 8) s0c = s0c.clone();
     s0 = s0c.data_ptr<float>();
   }
   Tensor out = out_empty({B, T, Hv, VD}, q.options());
   Tensor S = out_empty({B, Hv, KD, VD}, q.options().dtype(at::kFloat));
+  Tensor ws = at::empty({static_cast<int64_t>(ferrl::gdn_chunk_workspace(B, T, Hv))}, q.options().dtype(at::kByte));
   FERRL_CHECK(ferrl::gdn_chunk_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), q.stride(1), k.stride(0),
                                    k.stride(1), v.stride(0), v.stride(1), g.data_ptr<float>(), beta.data_ptr<float>(), s0,
                                    S.data_ptr<float>(), out.data_ptr(), B, T, Hk, Hv, KD, VD, l2norm,
-                                   static_cast<float>(eps), stream()));
+                                   static_cast<float>(eps), ws.data_ptr(), stream()));
   return {out, S};
 }
 

@@ -310,7 +310,7 @@ class Qwen35Layer(nn.Module):
             g = g * valid[:, :, None]
         S0 = None if state is None else state[1]
         if fast and not decode and not torch.is_grad_enabled() and self.kd == 128 and self.vd == 128:
-            # grad-free scoring and prefill: the whole chunked scan is one kernel with the state in shared memory
+            # grad-free scoring and prefill: chunk factors in parallel, then the scan with the state in registers
             from ..ops import cuda as C
             res = C.gdn_chunk_fwd(q, k, v, g, beta, S0, True, 1e-6)
             if res is not None:
