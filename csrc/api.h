@@ -97,13 +97,14 @@ int decode_gemm_groups(int K);
 const char* decode_gemm(const DecodeGemmArgs& a, cudaStream_t stream);
 
 // ---- norms / rope ----
-const char* rmsnorm(int dtype, const void* x, const void* res, const void* w, const void* gate, void* y, void* h_out,
-                    long long rows, int H, float eps, bool zero_centered, cudaStream_t s);
+// gate row r at (r / gate_per) * gate_ld + (r % gate_per) * H
+const char* rmsnorm(int dtype, const void* x, const void* res, const void* w, const void* gate, int gate_per, long long gate_ld,
+                    void* y, void* h_out, long long rows, int H, float eps, bool zero_centered, cudaStream_t s);
 const char* rmsnorm_bwd(int dtype, const void* x, const void* w, const void* dy, void* dx, long long rows, int H,
                         float eps, bool zero_centered, cudaStream_t s);
 // gated form y = rmsnorm(x) * w * silu(gate): gradients of x and gate for a frozen weight
-const char* rmsnorm_gated_bwd(int dtype, const void* x, const void* gate, const void* w, const void* dy, void* dx,
-                              void* dg, long long rows, int H, float eps, cudaStream_t s);
+const char* rmsnorm_gated_bwd(int dtype, const void* x, const void* gate, int gate_per, long long gate_ld, const void* w,
+                              const void* dy, void* dx, void* dg, long long rows, int H, float eps, cudaStream_t s);
 struct QkNormRopeArgs {
   int dtype; bool backward;
   const void* q_in; long long ld_q;                     // [n_tok, Hq*D] rows with token stride ld_q (may be a view

@@ -873,6 +873,19 @@ Tensor moe_pair_dot(const Tensor& dy, const Tensor& ys, const Tensor& row_of, in
   return dw;
 }
 
+// rows of a gate: contiguous, or [n, per, H] whose heads are packed in rows of a wider matrix
+struct GateRows {
+  int per = 1;
+  long long ld = 0;
+};
+GateRows gate_rows(const Tensor& gate, const Tensor& x, const char* what) {
+  TORCH_CHECK(gate.is_cuda() && gate.sizes() == x.sizes() && gate.scalar_type() == x.scalar_type(), what);
+  const int64_t H = x.size(-1);
+  if (gate.is_contiguous()) return {1, H};
+  TORCH_CHECK(gate.dim() == 3 && gate.stride(2) == 1 && gate.stride(1) == H, what);
+  return {static_cast<int>(gate.size(1)), gate.stride(0)};
+}
+
 std::tuple<Tensor, Tensor> rmsnorm(const Tensor& x, const optional<Tensor>& res, const optional<Tensor>& w,
                                    const optional<Tensor>& gate, double eps, bool zc) {
   TORCH_CHECK(x.is_cuda() && x.is_contiguous(), "rmsnorm: contiguous CUDA tensor required");
@@ -886,8 +899,9 @@ std::tuple<Tensor, Tensor> rmsnorm(const Tensor& x, const optional<Tensor>& res,
     h = out_empty_like(x);
   }
   if (w.has_value() && w->defined()) TORCH_CHECK(w->scalar_type() == x.scalar_type() && w->numel() == H && w->is_contiguous(), "rmsnorm: weight");
-  if (gate.has_value() && gate->defined()) TORCH_CHECK(gate->is_contiguous() && gate->sizes() == x.sizes() && gate->scalar_type() == x.scalar_type(), "rmsnorm: gate");
-  FERRL_CHECK(ferrl::rmsnorm(dt(x), x.data_ptr(), optr(res), optr(w), optr(gate), y.data_ptr(),
+  GateRows gr;
+  if (gate.has_value() && gate->defined()) gr = gate_rows(*gate, x, "rmsnorm: gate");
+  FERRL_CHECK(ferrl::rmsnorm(dt(x), x.data_ptr(), optr(res), optr(w), optr(gate), gr.per, gr.ld, y.data_ptr(),
                              h.defined() ? h.data_ptr() : nullptr, rows, H, static_cast<float>(eps), zc, stream()));
   return {y, h.defined() ? h : Tensor()};
 }
@@ -904,14 +918,14 @@ Tensor rmsnorm_bwd(const Tensor& x, const optional<Tensor>& w, const Tensor& dy,
 }
 
 std::tuple<Tensor, Tensor> rmsnorm_gated_bwd(const Tensor& x, const Tensor& gate, const Tensor& w, const Tensor& dy, double eps) {
-  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && gate.is_contiguous() && dy.is_contiguous() && w.is_contiguous() &&
-                  dy.sizes() == x.sizes() && gate.sizes() == x.sizes() && dy.scalar_type() == x.scalar_type() &&
-                  gate.scalar_type() == x.scalar_type() && w.scalar_type() == x.scalar_type() && w.numel() == x.size(-1),
+  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && dy.is_contiguous() && w.is_contiguous() &&
+                  dy.sizes() == x.sizes() && dy.scalar_type() == x.scalar_type() && w.scalar_type() == x.scalar_type() && w.numel() == x.size(-1),
               "rmsnorm_gated_bwd: x, gate, dy of one shape and dtype, w [H]");
   c10::cuda::CUDAGuard guard(x.device());
   const int H = x.size(-1);
   Tensor dx = out_empty_like(x), dg = out_empty_like(x);
-  FERRL_CHECK(ferrl::rmsnorm_gated_bwd(dt(x), x.data_ptr(), gate.data_ptr(), w.data_ptr(), dy.data_ptr(), dx.data_ptr(),
+  const GateRows gr = gate_rows(gate, x, "rmsnorm_gated_bwd: gate");
+  FERRL_CHECK(ferrl::rmsnorm_gated_bwd(dt(x), x.data_ptr(), gate.data_ptr(), gr.per, gr.ld, w.data_ptr(), dy.data_ptr(), dx.data_ptr(),
                                        dg.data_ptr(), x.numel() / H, H, static_cast<float>(eps), stream()));
   return {dx, dg};
 }

@@ -24,8 +24,8 @@ namespace {
 
 template <typename T>
 __global__ void rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ res, const T* __restrict__ w,
-                               const T* __restrict__ gate, T* __restrict__ y, T* __restrict__ h_out, int H, float eps,
-                               int zero_centered) {
+                               const T* __restrict__ gate, int gate_per, long long gate_ld, T* __restrict__ y,
+                               T* __restrict__ h_out, int H, float eps, int zero_centered) {
   pdl_trigger();   // a dependent GEMM may start streaming its weights while this kernel runs
   pdl_wait();      // launched as a programmatic dependent itself: nothing is read before the predecessor is done
   __shared__ float red[32];
@@ -47,6 +47,7 @@ __global__ void rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ re
   float tot = block_sum(ss, red);
   float rstd = rsqrtf(tot / H + eps);
   const T* src = rr ? h_out + row * H : xr;
+  const long long gate_row = gate ? row / gate_per * gate_ld + row % gate_per * H : 0;
   for (int i = threadIdx.x; i < H; i += blockDim.x) {
     float v = to_f(src[i]) * rstd;
     if (w) {
@@ -54,7 +55,7 @@ __global__ void rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ re
       v *= zero_centered ? (1.f + wv) : wv;
     }
     if (gate) {
-      float g = to_f(gate[row * H + i]);
+      float g = to_f(gate[gate_row + i]);
       v *= g / (1.f + __expf(-g));
     }
     y[row * H + i] = from_f<T>(v);
@@ -113,8 +114,8 @@ __device__ __forceinline__ uint4 pack8f(const float* f) {
 
 __global__ void rmsnorm_vec_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                                    const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ gate,
-                                   __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out, int H, float eps,
-                                   int zero_centered) {
+                                   int gate_per, long long gate_ld, __nv_bfloat16* __restrict__ y,
+                                   __nv_bfloat16* __restrict__ h_out, int H, float eps, int zero_centered) {
   pdl_trigger();   // a dependent GEMM may start streaming its weights while this kernel runs
   pdl_wait();      // launched as a programmatic dependent itself: nothing is read before the predecessor is done
   __shared__ float red[32];
@@ -156,7 +157,7 @@ __global__ void rmsnorm_vec_kernel(const __nv_bfloat16* __restrict__ x, const __
       }
       if (gate) {
         float g[8];
-        unpack8(reinterpret_cast<const uint4*>(gate + row * H)[c], g);
+        unpack8(reinterpret_cast<const uint4*>(gate + row / gate_per * gate_ld + row % gate_per * H)[c], g);
 #pragma unroll
         for (int e = 0; e < 8; ++e) o[e] *= g[e] / (1.f + __expf(-g[e]));
       }
@@ -206,6 +207,143 @@ __global__ void rmsnorm_bwd_vec_kernel(const __nv_bfloat16* __restrict__ x, cons
     }
   }
 }
+
+// Rows of at most 256 entries (heads): LPR lanes hold a row, one 16-byte chunk each, and a CTA has 256 / LPR rows.  With a
+// CTA of 64 threads to a row of 128 the launch of 393024 CTAs bounded the pass: gated, 8188 x 48 rows, 403 -> 99 us (the
+// bytes take 46 us), and 34 us for the contiguous copy of the gate that it no longer needs.
+// `gate` may be a column range of a wider matrix: row r lies at (r / gate_per) * gate_ld + (r % gate_per) * H.
+template <int LPR>
+__device__ __forceinline__ float lanes_sum(float v) {
+#pragma unroll
+  for (int o = LPR / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ long long gate_at(long long row, int H, int gate_per, long long gate_ld) {
+  const long long t = row / gate_per;
+  return t * gate_ld + (row - t * gate_per) * H;
+}
+
+template <int LPR>
+__global__ void __launch_bounds__(256)
+rmsnorm_head_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
+                    const __nv_bfloat16* __restrict__ gate, int gate_per, long long gate_ld, __nv_bfloat16* __restrict__ y,
+                    __nv_bfloat16* __restrict__ h_out, long long rows, int H, float eps, int zero_centered) {
+  pdl_trigger();
+  pdl_wait();
+  const int c = threadIdx.x % LPR;
+  const long long row = static_cast<long long>(blockIdx.x) * (256 / LPR) + threadIdx.x / LPR;
+  const bool on = row < rows && c < H / 8;
+  float v[8] = {}, g[8] = {}, wv[8] = {};
+  if (on) {
+    unpack8(reinterpret_cast<const uint4*>(x + row * H)[c], v);
+    if (gate) unpack8(reinterpret_cast<const uint4*>(gate + gate_at(row, H, gate_per, gate_ld))[c], g);
+    if (w) unpack8(reinterpret_cast<const uint4*>(w)[c], wv);
+    if (res) {
+      float r[8];
+      unpack8(reinterpret_cast<const uint4*>(res + row * H)[c], r);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] += r[e];
+      const uint4 hv = pack8f(v);          // the norm sees exactly what the residual stream holds
+      reinterpret_cast<uint4*>(h_out + row * H)[c] = hv;
+      unpack8(hv, v);
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) ss += v[e] * v[e];
+  const float rstd = rsqrtf(lanes_sum<LPR>(ss) / H + eps);
+  if (!on) return;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    v[e] *= rstd;
+    if (w) v[e] *= zero_centered ? (1.f + wv[e]) : wv[e];
+    if (gate) v[e] *= g[e] / (1.f + __expf(-g[e]));
+  }
+  reinterpret_cast<uint4*>(y + row * H)[c] = pack8f(v);
+}
+
+template <int LPR>
+__global__ void __launch_bounds__(256)
+rmsnorm_head_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ dy,
+                        __nv_bfloat16* __restrict__ dx, long long rows, int H, float eps, int zero_centered) {
+  const int c = threadIdx.x % LPR;
+  const long long row = static_cast<long long>(blockIdx.x) * (256 / LPR) + threadIdx.x / LPR;
+  const bool on = row < rows && c < H / 8;
+  float v[8] = {}, gw[8] = {}, ss = 0.f, dot = 0.f;
+  if (on) {
+    float wv[8];
+    unpack8(reinterpret_cast<const uint4*>(x + row * H)[c], v);
+    unpack8(reinterpret_cast<const uint4*>(dy + row * H)[c], gw);
+    if (w) unpack8(reinterpret_cast<const uint4*>(w)[c], wv);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float ww = w ? wv[e] : 1.f;
+      if (zero_centered) ww += 1.f;
+      gw[e] *= ww;
+      ss += v[e] * v[e];
+      dot += v[e] * gw[e];
+    }
+  }
+  ss = lanes_sum<LPR>(ss);
+  dot = lanes_sum<LPR>(dot);
+  if (!on) return;
+  const float rstd = rsqrtf(ss / H + eps), cc = dot * rstd * rstd / H;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) v[e] = rstd * (gw[e] - v[e] * cc);
+  reinterpret_cast<uint4*>(dx + row * H)[c] = pack8f(v);
+}
+
+// y = x * rstd * w * silu(g) with a frozen w: see rmsnorm_gated_bwd_kernel
+template <int LPR>
+__global__ void __launch_bounds__(256)
+rmsnorm_gated_head_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate, int gate_per, long long gate_ld,
+                              const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx,
+                              __nv_bfloat16* __restrict__ dg, long long rows, int H, float eps) {
+  const int c = threadIdx.x % LPR;
+  const long long row = static_cast<long long>(blockIdx.x) * (256 / LPR) + threadIdx.x / LPR;
+  const bool on = row < rows && c < H / 8;
+  float v[8] = {}, g[8] = {}, d[8] = {}, sg[8], ss = 0.f, dot = 0.f;
+  if (on) {
+    float wv[8];
+    unpack8(reinterpret_cast<const uint4*>(x + row * H)[c], v);
+    unpack8(reinterpret_cast<const uint4*>(gate + gate_at(row, H, gate_per, gate_ld))[c], g);
+    unpack8(reinterpret_cast<const uint4*>(dy + row * H)[c], d);
+    unpack8(reinterpret_cast<const uint4*>(w)[c], wv);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      d[e] *= wv[e];
+      sg[e] = 1.f / (1.f + __expf(-g[e]));
+      ss += v[e] * v[e];
+      dot += v[e] * d[e] * g[e] * sg[e];
+    }
+  }
+  ss = lanes_sum<LPR>(ss);
+  dot = lanes_sum<LPR>(dot);
+  if (!on) return;
+  const float rstd = rsqrtf(ss / H + eps), cc = dot * rstd * rstd / H;
+  float o[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    o[e] = rstd * (d[e] * g[e] * sg[e] - v[e] * cc);
+    g[e] = d[e] * v[e] * rstd * sg[e] * (1.f + g[e] * (1.f - sg[e]));
+  }
+  reinterpret_cast<uint4*>(dx + row * H)[c] = pack8f(o);
+  reinterpret_cast<uint4*>(dg + row * H)[c] = pack8f(g);
+}
+
+// lanes of a row of H <= 256 entries
+static inline int head_lanes(int H) { return H <= 32 ? 4 : H <= 64 ? 8 : H <= 128 ? 16 : 32; }
+static inline unsigned head_blocks(long long rows, int H) {
+  const int per = 256 / head_lanes(H);
+  return static_cast<unsigned>((rows + per - 1) / per);
+}
+#define FERRL_HEAD(H, CALL)          \
+  switch (head_lanes(H)) {           \
+    case 4: CALL(4); break;          \
+    case 8: CALL(8); break;          \
+    case 16: CALL(16); break;        \
+    default: CALL(32); break;        \
+  }
 
 static inline bool vec_ok(int H, const void* a, const void* b, const void* c, const void* d, const void* e, const void* f) {
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
@@ -480,29 +618,37 @@ __global__ void kv_append_kernel(const T* __restrict__ k, const T* __restrict__ 
 }  // namespace
 
 template <typename T>
-static const char* rmsnorm_t(const void* x, const void* res, const void* w, const void* gate, void* y, void* h_out,
-                             long long rows, int H, float eps, bool zc, cudaStream_t s) {
+static const char* rmsnorm_t(const void* x, const void* res, const void* w, const void* gate, int gate_per, long long gate_ld, void* y,
+                             void* h_out, long long rows, int H, float eps, bool zc, cudaStream_t s) {
   if (rows == 0) return nullptr;
-  if (sizeof(T) == 2 && vec_ok(H, x, res, w, gate, y, h_out)) {
+  if (sizeof(T) == 2 && (!gate || gate_ld % 8 == 0) && vec_ok(H, x, res, w, gate, y, h_out)) {
     using B = __nv_bfloat16;
-    launch_pdl(rmsnorm_vec_kernel, dim3(static_cast<unsigned>(rows)), dim3(vec_threads(H)), 0, s,
-               static_cast<const B*>(x), static_cast<const B*>(res), static_cast<const B*>(w), static_cast<const B*>(gate),
-               static_cast<B*>(y), static_cast<B*>(h_out), H, eps, zc ? 1 : 0);
+    const B *xb = static_cast<const B*>(x), *rb = static_cast<const B*>(res), *wb = static_cast<const B*>(w), *gb = static_cast<const B*>(gate);
+    if (H <= 256) {
+#define FERRL_CALL(L)                                                                                                        \
+  launch_pdl(rmsnorm_head_kernel<L>, dim3(head_blocks(rows, H)), dim3(256), 0, s, xb, rb, wb, gb, gate_per, gate_ld, static_cast<B*>(y), \
+             static_cast<B*>(h_out), rows, H, eps, zc ? 1 : 0)
+      FERRL_HEAD(H, FERRL_CALL)
+#undef FERRL_CALL
+    } else {
+      launch_pdl(rmsnorm_vec_kernel, dim3(static_cast<unsigned>(rows)), dim3(vec_threads(H)), 0, s, xb, rb, wb, gb, gate_per, gate_ld,
+                 static_cast<B*>(y), static_cast<B*>(h_out), H, eps, zc ? 1 : 0);
+    }
     count_launch();
     return cudaGetLastError() == cudaSuccess ? nullptr : "rmsnorm launch failed";
   }
   int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
   rmsnorm_kernel<T><<<static_cast<unsigned>(rows), threads, 0, s>>>(
-      static_cast<const T*>(x), static_cast<const T*>(res), static_cast<const T*>(w), static_cast<const T*>(gate),
+      static_cast<const T*>(x), static_cast<const T*>(res), static_cast<const T*>(w), static_cast<const T*>(gate), gate_per, gate_ld,
       static_cast<T*>(y), static_cast<T*>(h_out), H, eps, zc ? 1 : 0);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? nullptr : "rmsnorm launch failed";
 }
 
-const char* rmsnorm(int dtype, const void* x, const void* res, const void* w, const void* gate, void* y, void* h_out,
-                    long long rows, int H, float eps, bool zero_centered, cudaStream_t s) {
-  return dtype == kF32 ? rmsnorm_t<float>(x, res, w, gate, y, h_out, rows, H, eps, zero_centered, s)
-                       : rmsnorm_t<__nv_bfloat16>(x, res, w, gate, y, h_out, rows, H, eps, zero_centered, s);
+const char* rmsnorm(int dtype, const void* x, const void* res, const void* w, const void* gate, int gate_per, long long gate_ld, void* y,
+                    void* h_out, long long rows, int H, float eps, bool zero_centered, cudaStream_t s) {
+  return dtype == kF32 ? rmsnorm_t<float>(x, res, w, gate, gate_per, gate_ld, y, h_out, rows, H, eps, zero_centered, s)
+                       : rmsnorm_t<__nv_bfloat16>(x, res, w, gate, gate_per, gate_ld, y, h_out, rows, H, eps, zero_centered, s);
 }
 
 template <typename T>
@@ -511,9 +657,14 @@ static const char* rmsnorm_bwd_t(const void* x, const void* w, const void* dy, v
   if (rows == 0) return nullptr;
   if (sizeof(T) == 2 && vec_ok(H, x, w, dy, dx, nullptr, nullptr)) {
     using B = __nv_bfloat16;
-    rmsnorm_bwd_vec_kernel<<<static_cast<unsigned>(rows), vec_threads(H), 0, s>>>(
-        static_cast<const B*>(x), static_cast<const B*>(w), static_cast<const B*>(dy), static_cast<B*>(dx), H, eps,
-        zc ? 1 : 0);
+    const B *xb = static_cast<const B*>(x), *wb = static_cast<const B*>(w), *db = static_cast<const B*>(dy);
+    if (H <= 256) {
+#define FERRL_CALL(L) rmsnorm_head_bwd_kernel<L><<<head_blocks(rows, H), 256, 0, s>>>(xb, wb, db, static_cast<B*>(dx), rows, H, eps, zc ? 1 : 0)
+      FERRL_HEAD(H, FERRL_CALL)
+#undef FERRL_CALL
+    } else {
+      rmsnorm_bwd_vec_kernel<<<static_cast<unsigned>(rows), vec_threads(H), 0, s>>>(xb, wb, db, static_cast<B*>(dx), H, eps, zc ? 1 : 0);
+    }
     count_launch();
     return cudaGetLastError() == cudaSuccess ? nullptr : "rmsnorm_bwd launch failed";
   }
@@ -535,14 +686,14 @@ const char* rmsnorm_bwd(int dtype, const void* x, const void* w, const void* dy,
 //   a_i = dy_i w_i silu(g_i);  dx_i = rstd (a_i - x_i rstd^2 mean_j(a_j x_j));  dg_i = dy_i x_i rstd w_i silu'(g_i)
 // One warp per row (rows are GatedDeltaNet value heads, H = 128), several rows per CTA.
 template <typename T>
-__global__ void rmsnorm_gated_bwd_kernel(const T* __restrict__ x, const T* __restrict__ gate, const T* __restrict__ w,
+__global__ void rmsnorm_gated_bwd_kernel(const T* __restrict__ x, const T* __restrict__ gate, int gate_per, long long gate_ld, const T* __restrict__ w,
                                          const T* __restrict__ dy, T* __restrict__ dx, T* __restrict__ dg, long long rows,
                                          int H, float eps) {
   const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
   const T* xr = x + row * H;
-  const T* gr = gate + row * H;
+  const T* gr = gate + gate_at(row, H, gate_per, gate_ld);
   const T* yr = dy + row * H;
   float ss = 0.f, dot = 0.f;
   for (int i = lane; i < H; i += 32) {
@@ -564,21 +715,32 @@ __global__ void rmsnorm_gated_bwd_kernel(const T* __restrict__ x, const T* __res
 }
 
 template <typename T>
-static const char* rmsnorm_gated_bwd_t(const void* x, const void* gate, const void* w, const void* dy, void* dx, void* dg,
-                                       long long rows, int H, float eps, cudaStream_t s) {
+static const char* rmsnorm_gated_bwd_t(const void* x, const void* gate, int gate_per, long long gate_ld, const void* w, const void* dy,
+                                       void* dx, void* dg, long long rows, int H, float eps, cudaStream_t s) {
   if (rows == 0) return nullptr;
+  if (sizeof(T) == 2 && H <= 256 && gate_ld % 8 == 0 && vec_ok(H, x, gate, w, dy, dx, dg)) {
+    using B = __nv_bfloat16;
+#define FERRL_CALL(L)                                                                                                        \
+  rmsnorm_gated_head_bwd_kernel<L><<<head_blocks(rows, H), 256, 0, s>>>(                                                     \
+      static_cast<const B*>(x), static_cast<const B*>(gate), gate_per, gate_ld, static_cast<const B*>(w), static_cast<const B*>(dy), \
+      static_cast<B*>(dx), static_cast<B*>(dg), rows, H, eps)
+    FERRL_HEAD(H, FERRL_CALL)
+#undef FERRL_CALL
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? nullptr : "rmsnorm_gated_bwd launch failed";
+  }
   const int warps = 8;
   rmsnorm_gated_bwd_kernel<T><<<static_cast<unsigned>((rows + warps - 1) / warps), warps * 32, 0, s>>>(
-      static_cast<const T*>(x), static_cast<const T*>(gate), static_cast<const T*>(w), static_cast<const T*>(dy),
+      static_cast<const T*>(x), static_cast<const T*>(gate), gate_per, gate_ld, static_cast<const T*>(w), static_cast<const T*>(dy),
       static_cast<T*>(dx), static_cast<T*>(dg), rows, H, eps);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? nullptr : "rmsnorm_gated_bwd launch failed";
 }
 
-const char* rmsnorm_gated_bwd(int dtype, const void* x, const void* gate, const void* w, const void* dy, void* dx,
-                              void* dg, long long rows, int H, float eps, cudaStream_t s) {
-  return dtype == kF32 ? rmsnorm_gated_bwd_t<float>(x, gate, w, dy, dx, dg, rows, H, eps, s)
-                       : rmsnorm_gated_bwd_t<__nv_bfloat16>(x, gate, w, dy, dx, dg, rows, H, eps, s);
+const char* rmsnorm_gated_bwd(int dtype, const void* x, const void* gate, int gate_per, long long gate_ld, const void* w,
+                              const void* dy, void* dx, void* dg, long long rows, int H, float eps, cudaStream_t s) {
+  return dtype == kF32 ? rmsnorm_gated_bwd_t<float>(x, gate, gate_per, gate_ld, w, dy, dx, dg, rows, H, eps, s)
+                       : rmsnorm_gated_bwd_t<__nv_bfloat16>(x, gate, gate_per, gate_ld, w, dy, dx, dg, rows, H, eps, s);
 }
 
 template <typename T, bool BWD>

@@ -277,7 +277,7 @@ class Qwen35Layer(nn.Module):
                 g = -self.A_log.float().exp() * F.softplus(a[:, 0].float() + self.dt_bias.float())
                 core = C.gdn_decode_step(y[:, :self.key_dim], y[:, self.key_dim:2 * self.key_dim], y[:, 2 * self.key_dim:],
                                          g, beta, state[1], True, 1e-6)
-            core = ops.rmsnorm_gated(core.reshape(-1, self.vd), z.reshape(-1, self.vd), self.gdn_norm, self.eps)
+            core = ops.rmsnorm_gated(core.reshape(-1, self.vh, self.vd), z.reshape(-1, self.vh, self.vd), self.gdn_norm, self.eps)
             return f(self.out, core.reshape(B, S_, self.value_dim)), (state[0], state[1])
         y = None
         if fast:
@@ -315,7 +315,7 @@ class Qwen35Layer(nn.Module):
             res = C.gdn_chunk_fwd(q, k, v, g, beta, S0, True, 1e-6)
             if res is not None:
                 core, S1 = res
-                core = ops.rmsnorm_gated(core.reshape(-1, self.vd), z.reshape(-1, self.vd), self.gdn_norm, self.eps)
+                core = ops.rmsnorm_gated(core.reshape(-1, self.vh, self.vd), z.reshape(-1, self.vh, self.vd), self.gdn_norm, self.eps)
                 return f(self.out, core.reshape(B, S_, self.value_dim)), (new_left, S1)
         if fast and not decode and self.kd == 128 and self.vd == 128:
             # training: tensor-core chunk kernels with a hand-written backward
@@ -323,7 +323,7 @@ class Qwen35Layer(nn.Module):
             res = C.gdn_chunk_tc(q, k, v, g, beta, S0, 1e-6)
             if res is not None:
                 core, S1 = res
-                core = ops.rmsnorm_gated(core.reshape(-1, self.vd), z.reshape(-1, self.vd), self.gdn_norm, self.eps)
+                core = ops.rmsnorm_gated(core.reshape(-1, self.vh, self.vd), z.reshape(-1, self.vh, self.vd), self.gdn_norm, self.eps)
                 return f(self.out, core.reshape(B, S_, self.value_dim)), (new_left, S1)
         rep = self.vh // self.kh
         if rep > 1:
@@ -332,7 +332,7 @@ class Qwen35Layer(nn.Module):
             core, S1 = G.gated_delta_rule_recurrent(q, k, v, g, beta, S0, use_qk_l2norm=True)
         else:
             core, S1 = G.gated_delta_rule_chunked(q, k, v, g, beta, S0, use_qk_l2norm=True)
-        core = ops.rmsnorm_gated(core.reshape(-1, self.vd), z.reshape(-1, self.vd), self.gdn_norm, self.eps)
+        core = ops.rmsnorm_gated(core.reshape(-1, self.vh, self.vd), z.reshape(-1, self.vh, self.vd), self.gdn_norm, self.eps)
         return f(self.out, core.reshape(B, S_, self.value_dim)), (new_left, S1)
 
     def _ffn(self, x, merged):

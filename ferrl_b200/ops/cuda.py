@@ -388,9 +388,12 @@ def rmsnorm_gated(x, gate, weight, eps):
     if weight.requires_grad or gate.dtype != x.dtype:
         return eager.rmsnorm_gated(x, gate, weight, eps)
     w = weight.to(x.dtype).contiguous()
+    # heads [n, per, H] packed in the columns of a wider matrix are read where they lie
+    if not (gate.dim() == 3 and gate.stride(2) == 1 and gate.stride(1) == gate.shape[2]):
+        gate = gate.contiguous()
     if torch.is_grad_enabled() and (x.requires_grad or gate.requires_grad):
-        return _RmsNormGated.apply(x.contiguous(), gate.contiguous(), w, eps)
-    y, _ = lib().rmsnorm(x.contiguous(), None, w, gate.contiguous(), eps, False)
+        return _RmsNormGated.apply(x.contiguous(), gate, w, eps)
+    y, _ = lib().rmsnorm(x.contiguous(), None, w, gate, eps, False)
     return y
 
 
