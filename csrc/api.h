@@ -36,6 +36,7 @@ struct GemmArgs {
   int stream_k; float* sk_ws; unsigned int* sk_flags; int sk_max_ctas; unsigned long long* sk_debug;
   // grouped mode: B is [n_experts * N, K]; tile_expert[m tile] = expert (or -1: skip the tile)
   const int* tile_expert; int n_experts;
+  const int* tile_token;      // optional [M]: token of each row, -1 behind the tokens of a segment (blocks of 16 rows without one are skipped)
   // fused GEMM -> all-reduce over the symmetric heap (ar_world > 1): see tcgen05_gemm.cu
   int ar_world, ar_rank; int ar_max_tiles; unsigned long long ar_limit_ns;
   long long ar_stage_elems, ar_out_elems;                         // capacity of the symmetric staging / output buffers (bf16 elements)
@@ -130,8 +131,10 @@ const char* kv_append(int dtype, const void* k, const void* v, long long ldv, vo
                       int batch, int smax, int HD, cudaStream_t s);
 
 // ---- misc ----
+// token_of: optional [rows]; forward rows in blocks of 16 that begin with -1 are left unwritten (16-bit)
 const char* glu(int dtype, bool backward, const void* gu, const void* dout, void* out, long long rows, int F, GluAct act,
-                cudaStream_t s);
+                cudaStream_t s,
+                const int* token_of = nullptr);
 const char* embedding(int dtype, const long long* ids, const void* table, void* out, long long n_tok, int H,
                       long long vocab, float scale, cudaStream_t s);
 const char* lora_merge(int dtype, const void* w, const float* a, const float* b, void* out, int O, int I, int R,
@@ -363,7 +366,7 @@ const char* moe_combine_any(int dtype, const void* ys, const int* row_of, const 
 const char* moe_plan(const int* idx, const int* counts, int n_pairs, int k, int E, int max_rows, int* row_of,
                      int* token_of, int* tile_expert, int* seg_start, cudaStream_t stream);
 const char* moe_gather(const void* x, long long ldx, const int* token_of, const float* pair_w, const int* row_of,
-                       int n_pairs, float* row_scale, int rows, int H, void* xs, cudaStream_t stream);
+                       int n_pairs, float* row_scale, int rows, int H, void* xs, bool sparse, cudaStream_t stream);
 const char* moe_combine(const void* ys, const int* row_of, const float* w, int T, int k, int H, void* out,
                         cudaStream_t stream);
 const char* moe_pair_dot(const void* dy, const void* ys, const int* row_of, int n_pairs, int k, int H, float* dw,

@@ -684,7 +684,7 @@ std::tuple<Tensor, Tensor> gdn_chunk_fwd(const Tensor& q_, const Tensor& k_, con
   return {out, S};
 }
 
-Tensor glu_fwd(const Tensor& gu, int64_t act, double alpha = 0.0, double limit = 0.0);
+Tensor glu_fwd(const Tensor& gu, int64_t act, double alpha = 0.0, double limit = 0.0, const optional<Tensor>& token_of = {});
 
 // ---------------------------------------------------------------- mixture of experts
 // logits [T, E] fp32 -> (probs [T,E] f32, scores [T,k] f32, idx [T,k] i32, counts [E] i32)
@@ -721,8 +721,9 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> moe_plan(const Tensor& idx, const Ten
   return {row_of, token_of, tile_expert, seg_start};
 }
 
-// xs[row] = (pair_w ? pair_w[pair of row] : 1) * x[token_of[row]]; padding rows are zero
-Tensor moe_gather(const Tensor& x, const Tensor& token_of, const optional<Tensor>& pair_w, const Tensor& row_of) {
+// xs[row] = (pair_w ? pair_w[pair of row] : 1) * x[token_of[row]]; padding rows are zero, or with `sparse` not written where a
+// block of 16 rows has no token (readers skip those blocks)
+Tensor moe_gather(const Tensor& x, const Tensor& token_of, const optional<Tensor>& pair_w, const Tensor& row_of, bool sparse) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1, "moe_gather: bf16 [T,H]");
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t rows = token_of.size(0), H = x.size(1);
@@ -735,13 +736,14 @@ Tensor moe_gather(const Tensor& x, const Tensor& token_of, const optional<Tensor
     pw = pair_w->data_ptr<float>();
   }
   FERRL_CHECK(ferrl::moe_gather(x.data_ptr(), x.stride(0), token_of.data_ptr<int>(), pw, row_of.data_ptr<int>(),
-                                row_of.numel(), pw ? row_scale.data_ptr<float>() : nullptr, rows, H, xs.data_ptr(), stream()));
+                                row_of.numel(), pw ? row_scale.data_ptr<float>() : nullptr, rows, H, xs.data_ptr(), sparse, stream()));
   return xs;
 }
 
 // ys[rows, N] = xs[rows, K] x W[e(row)]^T with W [E, N, K]; rows sorted by expert in 128-row segments
 // `nn`: W is [E,K,N] instead (the weight of the forward pass read by the backward one; K a multiple of 64).
-Tensor moe_grouped_gemm(const Tensor& xs, const Tensor& W, const Tensor& tile_expert, const optional<Tensor>& out_buf, bool nn) {
+Tensor moe_grouped_gemm(const Tensor& xs, const Tensor& W, const Tensor& tile_expert, const optional<Tensor>& out_buf, bool nn,
+                        const optional<Tensor>& token_of) {
   TORCH_CHECK(xs.is_cuda() && xs.scalar_type() == at::kBFloat16 && W.scalar_type() == at::kBFloat16, "moe_grouped_gemm: bf16");
   TORCH_CHECK(xs.dim() == 2 && W.dim() == 3 && W.is_contiguous() && xs.is_contiguous() && xs.size(1) == W.size(nn ? 1 : 2), "moe_grouped_gemm: xs [R,K], W [E,N,K]");
   TORCH_CHECK(xs.size(0) % 128 == 0 && tile_expert.numel() * 128 >= xs.size(0) && tile_expert.scalar_type() == at::kInt, "moe_grouped_gemm: rows in 128-row tiles with one expert id each");
@@ -750,6 +752,10 @@ Tensor moe_grouped_gemm(const Tensor& xs, const Tensor& W, const Tensor& tile_ex
   a.A = xs.data_ptr(); a.B = W.data_ptr(); a.lda = xs.stride(0); a.ldb = W.size(2);
   a.M = xs.size(0); a.N = W.size(nn ? 2 : 1); a.K = xs.size(1); a.b_mn = nn;
   a.tile_expert = tile_expert.data_ptr<int>(); a.n_experts = W.size(0);
+  if (token_of.has_value() && token_of->defined()) {
+    TORCH_CHECK(token_of->is_cuda() && token_of->scalar_type() == at::kInt && token_of->is_contiguous() && token_of->numel() >= xs.size(0), "moe_grouped_gemm: token of each row, i32");
+    a.tile_token = token_of->data_ptr<int>();
+  }
   // rows of unused tiles are never written: start from zeros so padding stays finite downstream
   Tensor out;
   if (out_buf.has_value() && out_buf->defined()) {
@@ -1037,14 +1043,20 @@ static ferrl::GluAct glu_act(int64_t act, double alpha, double limit) {
   return ferrl::GluAct{static_cast<int>(act), static_cast<float>(alpha), static_cast<float>(limit)};
 }
 
-Tensor glu_fwd(const Tensor& gu, int64_t act, double alpha, double limit) {
+// `token_of` [rows] i32: blocks of 16 rows that begin with -1 are left unwritten
+Tensor glu_fwd(const Tensor& gu, int64_t act, double alpha, double limit, const optional<Tensor>& token_of) {
   TORCH_CHECK(gu.is_cuda() && gu.is_contiguous(), "glu: contiguous CUDA tensor");
   c10::cuda::CUDAGuard guard(gu.device());
   const int F = gu.size(-1) / 2;
   auto sizes = gu.sizes().vec();
   sizes.back() = F;
   Tensor out = out_empty(sizes, gu.options());
-  FERRL_CHECK(ferrl::glu(dt(gu), false, gu.data_ptr(), nullptr, out.data_ptr(), gu.numel() / (2 * F), F, glu_act(act, alpha, limit), stream()));
+  const int* tok = nullptr;
+  if (token_of.has_value() && token_of->defined()) {
+    TORCH_CHECK(token_of->is_cuda() && token_of->scalar_type() == at::kInt && token_of->is_contiguous() && token_of->numel() * 2 * F >= gu.numel(), "glu: token of each row, i32");
+    tok = token_of->data_ptr<int>();
+  }
+  FERRL_CHECK(ferrl::glu(dt(gu), false, gu.data_ptr(), nullptr, out.data_ptr(), gu.numel() / (2 * F), F, glu_act(act, alpha, limit), stream(), tok));
   return out;
 }
 
@@ -1914,8 +1926,8 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("gdn_decode_step(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor(a!) S, bool l2norm, float eps) -> Tensor", &gdn_decode_step);
   m.def("moe_route(Tensor logits, int k, bool renorm, int score=0) -> (Tensor, Tensor, Tensor, Tensor)", &moe_route);
   m.def("moe_plan(Tensor idx, Tensor counts) -> (Tensor, Tensor, Tensor, Tensor)", &moe_plan);
-  m.def("moe_gather(Tensor x, Tensor token_of, Tensor? pair_w, Tensor row_of) -> Tensor", &moe_gather);
-  m.def("moe_grouped_gemm(Tensor xs, Tensor W, Tensor tile_expert, Tensor(a!)? out=None, bool nn=False) -> Tensor(a!)", &moe_grouped_gemm);
+  m.def("moe_gather(Tensor x, Tensor token_of, Tensor? pair_w, Tensor row_of, bool sparse=False) -> Tensor", &moe_gather);
+  m.def("moe_grouped_gemm(Tensor xs, Tensor W, Tensor tile_expert, Tensor(a!)? out=None, bool nn=False, Tensor? token_of=None) -> Tensor(a!)", &moe_grouped_gemm);
   m.def("ep_dispatch(Tensor x, Tensor idx, Tensor? pair_w, Tensor counts, int[] counts_all, int[] xs, int[] flags, int rank, int world, int epoch, float limit_s, int cap_rows, Tensor(a!) dest_row, Tensor(b!) tile_expert, Tensor(c!) local_rows, bool reuse_plan, Tensor(d!) abort_word) -> ()", &ep_dispatch);
   m.def("ep_combine(int[] ys, Tensor idx, Tensor dest_row, Tensor? w, int H, int E_local, int[] flags, int rank, int world, int epoch, float limit_s, Tensor(a!)? keep_rows, Tensor(b!) abort_word) -> Tensor", &ep_combine);
   m.def("moe_combine(Tensor ys, Tensor row_of, Tensor? w, int T, int k) -> Tensor", &moe_combine);
@@ -1928,7 +1940,7 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("qk_norm_rope_bwd(Tensor q, Tensor k, Tensor? qw, Tensor? kw, Tensor cos, Tensor sin, Tensor pos, int pos_div, float eps, bool zc, Tensor dq, Tensor dk, Tensor(a!) dq_in, Tensor(b!) dk_in) -> ()", &qk_norm_rope_bwd);
   m.def("kv_append(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor kv_len) -> ()", &kv_append);
   m.def("kv_append_paged(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor kv_len, Tensor table) -> ()", &kv_append_paged);
-  m.def("glu_fwd(Tensor gu, int act, float alpha=0.0, float limit=0.0) -> Tensor", &glu_fwd);
+  m.def("glu_fwd(Tensor gu, int act, float alpha=0.0, float limit=0.0, Tensor? token_of=None) -> Tensor", &glu_fwd);
   m.def("glu_bwd(Tensor gu, Tensor dout, int act, float alpha=0.0, float limit=0.0) -> Tensor", &glu_bwd);
   m.def("embedding(Tensor ids, Tensor table, float scale) -> Tensor", &embedding);
   m.def("lora_merge(Tensor w, Tensor a, Tensor b) -> Tensor", &lora_merge);

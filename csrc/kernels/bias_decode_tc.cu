@@ -121,7 +121,6 @@ bias_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   const int split = blockIdx.x, g = blockIdx.y / head_tiles, h0 = (blockIdx.y % head_tiles) * NH, b = blockIdx.z;
   const int nh = min(NH, rep - h0), hq0 = g * rep + h0, D = a.D;
   const int n_blocks = (geo.na + 1) / 2;        // 128-entry blocks of a key
-  pdl_trigger();
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     mbar_init(&s_full[0], 1);
@@ -147,6 +146,7 @@ bias_decode_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();                                // after the allocation: a dependent may hold tensor memory while it waits
   pdl_wait();                                   // positions, queries and the token's key come from the predecessors
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tO = tmem_base, tS = tmem_base + n_blocks * NH;           // S^T buffers at tS and tS + NH

@@ -91,7 +91,6 @@ latent_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = blockIdx.x, hb = blockIdx.y * NH, b = blockIdx.z;
   const int n_blocks = (g.na_lat + 1) / 2;      // 128-entry blocks of the latent
-  pdl_trigger();
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     mbar_init(&s_full[0], 1);
@@ -113,6 +112,7 @@ latent_decode_tc_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();                                // after the allocation: a dependent may hold tensor memory while it waits
   pdl_wait();                                   // counts, queries and the newest cache rows come from the predecessors
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tO = tmem_base, tS = tmem_base + n_blocks * NH;           // S^T buffers at tS and tS + NH

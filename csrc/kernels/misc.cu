@@ -64,7 +64,7 @@ __global__ void glu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ out, lo
 }
 // bf16 vector forms: 8 elements per thread per step, 16-byte loads and stores; F % 8 == 0
 __global__ void glu_fwd_vec_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long rows,
-                                   int F, GluAct act) {
+                                   int F, GluAct act, const int* __restrict__ token_of) {
   pdl_trigger();   // a dependent GEMM may start streaming its weights while this kernel runs
   pdl_wait();      // launched as a programmatic dependent itself: nothing is read before the predecessor is done
   const int chunks = F / 8;
@@ -73,6 +73,7 @@ __global__ void glu_fwd_vec_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bf
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long r = i / chunks;
     const int c = static_cast<int>(i - r * chunks);
+    if (token_of && token_of[r & ~15LL] < 0) continue;       // padding behind an expert's tokens
     const uint4 gv = *reinterpret_cast<const uint4*>(gu + r * 2 * F + c * 8);
     const uint4 uv = *reinterpret_cast<const uint4*>(gu + r * 2 * F + F + c * 8);
     const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&gv);
@@ -306,7 +307,7 @@ inline unsigned grid_for(long long n, int threads) {
 }  // namespace
 
 const char* glu(int dtype, bool backward, const void* gu, const void* dout, void* out, long long rows, int F, GluAct act,
-                cudaStream_t s) {
+                cudaStream_t s, const int* token_of) {
   if (rows * F == 0) return nullptr;
   unsigned grid = grid_for(rows * F, 256);
   if (dtype == kF32) {
@@ -323,7 +324,7 @@ const char* glu(int dtype, bool backward, const void* gu, const void* dout, void
       glu_bwd_vec_kernel<<<vgrid, 256, 0, s>>>(static_cast<const B*>(gu), static_cast<const B*>(dout), static_cast<B*>(out),
                                                rows, F, act);
     else
-      launch_pdl(glu_fwd_vec_kernel, dim3(vgrid), dim3(256), 0, s, static_cast<const B*>(gu), static_cast<B*>(out), rows, F, act);
+      launch_pdl(glu_fwd_vec_kernel, dim3(vgrid), dim3(256), 0, s, static_cast<const B*>(gu), static_cast<B*>(out), rows, F, act, token_of);
   } else {
     using B = __nv_bfloat16;
     if (backward)

@@ -145,16 +145,17 @@ __global__ void moe_plan_kernel(const int* __restrict__ idx, const int* __restri
 }
 
 // xs[row, :] = (w ? w[pair_of_row] : 1) * x[token_of[row], :]; H % 8 == 0.  pair scale is looked up
-// through row_of's inverse, passed as `row_scale` [rows] (or null).
+// through row_of's inverse, passed as `row_scale` [rows] (or null).  `sparse`: blocks of 16 rows without a token stay unwritten.
 __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const int* __restrict__ token_of,
                                   const float* __restrict__ row_scale, int rows, int H,
-                                  __nv_bfloat16* __restrict__ xs) {
+                                  __nv_bfloat16* __restrict__ xs, int sparse) {
   const int chunks = H / 8;
   const long long n = static_cast<long long>(rows) * chunks;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int r = static_cast<int>(i / chunks), c = static_cast<int>(i % chunks);
     const int t = token_of[r];
+    if (sparse && t < 0 && token_of[r & ~15] < 0) continue;
     uint4 o = make_uint4(0, 0, 0, 0);
     if (t >= 0) {
       o = *reinterpret_cast<const uint4*>(x + static_cast<long long>(t) * ldx + c * 8);
@@ -364,7 +365,7 @@ const char* moe_plan(const int* idx, const int* counts, int n_pairs, int k, int 
 }
 
 const char* moe_gather(const void* x, long long ldx, const int* token_of, const float* pair_w, const int* row_of,
-                       int n_pairs, float* row_scale, int rows, int H, void* xs, cudaStream_t stream) {
+                       int n_pairs, float* row_scale, int rows, int H, void* xs, bool sparse, cudaStream_t stream) {
   if (H % 8) return "moe_gather: H % 8";
   if (pair_w) {
     moe_row_scale_kernel<<<(n_pairs + 255) / 256, 256, 0, stream>>>(pair_w, row_of, n_pairs, row_scale);
@@ -373,7 +374,7 @@ const char* moe_gather(const void* x, long long ldx, const int* token_of, const 
   const long long n = static_cast<long long>(rows) * (H / 8);
   const int blocks = static_cast<int>(std::min<long long>((n + 255) / 256, 148 * 16));
   moe_gather_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), ldx, token_of,
-                                                pair_w ? row_scale : nullptr, rows, H, static_cast<__nv_bfloat16*>(xs));
+                                                pair_w ? row_scale : nullptr, rows, H, static_cast<__nv_bfloat16*>(xs), sparse ? 1 : 0);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? nullptr : "moe_gather launch failed";
 }

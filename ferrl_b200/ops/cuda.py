@@ -888,13 +888,13 @@ def moe_route(logits_f32, k, renorm=True, score="softmax"):
     return _MoeRoute.apply(logits_f32, int(k), bool(renorm), score)
 
 
-def _grouped_input_grad(dy, w, wt, tile_expert):
+def _grouped_input_grad(dy, w, wt, tile_expert, tok=None):
     """``dy_e @ w_e`` per expert for frozen ``w`` ``[E,N,K]``, read as it lies where the kernel can (``N`` a multiple of
     64: a k-block must not reach into the next expert); ``wt`` is the optional resident transpose."""
     out = dy.new_empty(dy.shape[0], w.shape[2])
     if wt is None and w.shape[1] % 64 == 0:
-        return lib().moe_grouped_gemm(dy, w, tile_expert, out, True)
-    return lib().moe_grouped_gemm(dy, w.transpose(1, 2).contiguous() if wt is None else wt, tile_expert, out)
+        return lib().moe_grouped_gemm(dy, w, tile_expert, out, True, tok)
+    return lib().moe_grouped_gemm(dy, w.transpose(1, 2).contiguous() if wt is None else wt, tile_expert, out, token_of=tok)
 
 
 class _MoeExperts(torch.autograd.Function):
@@ -908,18 +908,21 @@ class _MoeExperts(torch.autograd.Function):
         T, k = idx.shape
         sc = scores.float().contiguous()
         row_of, token_of, tile_expert, _ = L.moe_plan(idx.contiguous(), counts)
-        xs = L.moe_gather(x.contiguous(), token_of, sc if weight_input else None, row_of)
+        # Few rows an expert: a tile of 128 rows is mostly padding, and only its blocks of 16 rows with a token are moved
+        # (128 experts, 8 rows each, 2048 wide: both products 268 -> 219 us, activation 6.5 -> 4.1 us).  Full tiles load in one box.
+        tok = token_of if token_of.shape[0] > 2 * T * k else None
+        xs = L.moe_gather(x.contiguous(), token_of, sc if weight_input else None, row_of, tok is not None)
         # rows of unused tiles are never written and never read back: the combine and the score gradient read routed rows
         # only, the grouped products skip those tiles in both directions
-        gu = L.moe_grouped_gemm(xs, gate_up, tile_expert, xs.new_empty(xs.shape[0], gate_up.shape[1]))
+        gu = L.moe_grouped_gemm(xs, gate_up, tile_expert, xs.new_empty(xs.shape[0], gate_up.shape[1]), token_of=tok)
         del xs
-        h = L.glu_fwd(gu, act)
-        ys = L.moe_grouped_gemm(h, down, tile_expert, h.new_empty(h.shape[0], down.shape[1]))
+        h = L.glu_fwd(gu, act, token_of=tok)
+        ys = L.moe_grouped_gemm(h, down, tile_expert, h.new_empty(h.shape[0], down.shape[1]), token_of=tok)
         del h
         out = L.moe_combine(ys, row_of, None if weight_input else sc, T, k)
         # kept rows: the outputs for the gradient of output weights, the tokens for that of input weights
         ctx.save_for_backward(gu, x if weight_input else ys, sc, row_of, token_of, tile_expert, gate_up, down, gate_up_t, down_t)
-        ctx.act, ctx.k, ctx.weight_input = act, k, weight_input
+        ctx.act, ctx.k, ctx.weight_input, ctx.sparse = act, k, weight_input, tok is not None
         ctx.score_dtype = scores.dtype
         return out
 
@@ -932,12 +935,13 @@ class _MoeExperts(torch.autograd.Function):
         dsc = None
         if not ctx.weight_input:
             dsc = L.moe_pair_dot(dout, ys, row_of, ctx.k).to(ctx.score_dtype)
-        dys = L.moe_gather(dout, token_of, None if ctx.weight_input else sc.view(-1), row_of)
-        dh = _grouped_input_grad(dys, down, down_t, tile_expert)
+        tok = token_of if ctx.sparse else None
+        dys = L.moe_gather(dout, token_of, None if ctx.weight_input else sc.view(-1), row_of, ctx.sparse)
+        dh = _grouped_input_grad(dys, down, down_t, tile_expert, tok)
         del dys
         dgu = L.glu_bwd(gu, dh, ctx.act)
         del dh
-        dxs = _grouped_input_grad(dgu, gate_up, gate_up_t, tile_expert)
+        dxs = _grouped_input_grad(dgu, gate_up, gate_up_t, tile_expert, tok)
         if ctx.weight_input:
             dsc = L.moe_pair_dot(ys.contiguous(), dxs, row_of, ctx.k).to(ctx.score_dtype)     # <token, d(weighted token)>
         dx = L.moe_combine(dxs, row_of, sc if ctx.weight_input else None, T, ctx.k)

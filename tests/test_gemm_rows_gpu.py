@@ -1,0 +1,70 @@
+"""Projections of few rows (decode) and experts with few rows: boxes, blocks and rings that are cut to the rows at hand."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rnd(gen, *s, std=1.0):
+    return (torch.randn(*s, generator=gen, device="cuda") * std).bfloat16()
+
+
+def _close(y, ref, scale):
+    # 32-bit sums of K products, each off by 2^-24 of it per step at most, and one rounding to 16 bits
+    assert bool(((y.double() - ref).abs() <= 2 ** -8 * ref.abs() + 2e-5 * scale).all())
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 31, 33, 64, 65, 127, 128, 129, 200])
+@pytest.mark.parametrize("N,K", [(1536, 1024), (64, 72), (272, 520), (4096, 2048)])
+def test_few_rows(M, N, K):
+    from ferrl_b200.ops import cuda as C
+    gen = torch.Generator(device="cuda").manual_seed(M * N + K)
+    a, b, r = _rnd(gen, M, K), _rnd(gen, N, K, std=K ** -0.5), _rnd(gen, M, N)
+    ref, scale = a.double() @ b.double().T, (a.double().abs() @ b.double().abs().T)
+    for y in (C.gemm(a, b), C.gemm(a, b, static_b=True)):
+        _close(y, ref, scale)
+    _close(C.gemm(a, b, residual=r, static_b=True), ref + r.double(), scale)
+    for bn, cl in ((64, 2), (64, 4), (128, 2), (128, 4), (128, 8), (256, 2)):
+        if N >= bn and K >= 64 * cl:
+            _close(C.gemm(a, b, force_bn=bn, cluster_k=cl), ref, scale)
+            _close(C.gemm(a, b, residual=r, force_bn=bn, cluster_k=cl, static_b=True), ref + r.double(), scale)
+    for bn in (32, 64, 128, 256):
+        _close(C.gemm(a, b, force_bn=bn), ref, scale)
+
+
+def test_chain_of_dependent_launches():
+    """Kernels that start beside their predecessors (short rings leave room) give what they give one by one."""
+    from ferrl_b200.ops import cuda as C
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    ws = [_rnd(gen, n, k, std=k ** -0.5) for n, k in ((1536, 1024), (1024, 1536), (6144, 1024), (1024, 6144), (2048, 1024), (1024, 2048)) * 4]
+    for M in (1, 8, 64):
+        x = _rnd(gen, M, 1024)
+        one = x
+        for w in ws:
+            one = C.gemm(one, w)
+            torch.cuda.synchronize()
+        for _ in range(5):
+            y = x
+            for w in ws:
+                y = C.gemm(y, w, static_b=True)
+            assert torch.equal(y, one)
+
+
+@pytest.mark.parametrize("T,E,k,H,I", [(1, 8, 2, 64, 64), (33, 16, 4, 256, 128), (128, 128, 8, 512, 192), (140, 2, 1, 128, 64), (48, 3, 3, 128, 320)])
+def test_experts_with_few_rows(T, E, k, H, I):
+    from ferrl_b200.models import moe as M
+    from ferrl_b200.ops import cuda as C
+    gen = torch.Generator(device="cuda").manual_seed(T * E)
+    x, gu, dn = _rnd(gen, T, H), _rnd(gen, E, 2 * I, H, std=H ** -0.5), _rnd(gen, E, H, I, std=I ** -0.5)
+    logits = torch.randn(T, E, generator=gen, device="cuda") + 2 * torch.arange(E, device="cuda").float().cos()
+    torch.full((64 << 20,), float("nan"), device="cuda")                  # what padding rows find in memory
+    scores, idx, counts, _ = C.moe_route(logits, k, True)
+    xs = x.clone().requires_grad_()
+    y = C.moe_experts(xs, scores, idx, counts, gu, dn)
+    dy = _rnd(gen, T, H)
+    y.backward(dy)
+    xr = x.double().requires_grad_()
+    yr = M.moe_experts(xr, idx.long(), scores.double(), gu.double(), dn.double())
+    yr.backward(dy.double())
+    # bf16 activations between the products: 2^-9 of each, through two or three roundings
+    assert float((y - yr).norm() / yr.norm()) < 0.01 and float((xs.grad - xr.grad).norm() / xr.grad.norm()) < 0.015
