@@ -384,6 +384,14 @@ const char* gdn_chunk_fwd(const void* q, const void* k, const void* v, long long
                           const float* S0, float* S_out, void* out, int B, int T, int Hk, int Hv, int KD, int VD,
                           bool l2norm, float eps, void* workspace, cudaStream_t stream);
 size_t gdn_chunk_workspace(int B, int T, int Hv);      // bytes that gdn_chunk_fwd takes
+// 16-bit activations <-> the 32-bit whole chunks of the training kernels (Tp = T rounded up to 64; heads packed, 8-byte aligned)
+const char* gdn_pack(const void* q, long long q_bs, long long q_ts, const void* k, long long k_bs, long long k_ts, const void* v,
+                     long long v_bs, long long v_ts, const float* g, const float* beta, int B, int T, int Tp, int Hk, int Hv, float eps,
+                     float* qf, float* kf, float* vf, float* gp, float* bp, cudaStream_t s);
+const char* gdn_pad(const void* x, long long bs, long long ts, int B, int T, int Tp, int H, float* out, cudaStream_t s);
+const char* gdn_unpack_bwd(const void* q, long long q_bs, long long q_ts, const void* k, long long k_bs, long long k_ts, const float* dqf,
+                           const float* dkf, const float* dvf, const float* dG, const float* dbp, int B, int T, int Tp, int Hk, int Hv,
+                           float eps, void* dq, void* dk, void* dv, float* dg, float* dbeta, cudaStream_t s);
 // Optional gate inputs straight from the input projection (decode): a, b bf16 [B, Hv] with row strides lda, ldb,
 // A_log and dt_bias fp32 [Hv]; the kernel then forms g = -exp(A_log) softplus(a + dt_bias) and beta = sigmoid(b)
 // itself and ignores `g` / `beta`.

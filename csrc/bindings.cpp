@@ -649,6 +649,56 @@ std::vector<Tensor> gdn_tc_bwd(const Tensor& q, const Tensor& k, const Tensor& v
   return {dq, dk, dv, dbeta, dG, dS0};
 }
 
+// [B, T, H, 128] bf16 with packed heads whose rows start on 8 bytes
+void gdn_rows_check(const Tensor& t, const char* what) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.dim() == 4 && t.size(3) == 128 && t.stride(3) == 1 &&
+                  (t.size(2) == 1 || t.stride(2) == 128) && t.stride(0) % 4 == 0 && t.stride(1) % 4 == 0 &&
+                  reinterpret_cast<uintptr_t>(t.data_ptr()) % 8 == 0, what);
+}
+
+// -> qf, kf [B,Tp,Hk,128], vf [B,Tp,Hv,128], g, beta [B,Tp,Hv] f32, Tp = T rounded up to whole chunks
+std::vector<Tensor> gdn_pack(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, double eps) {
+  gdn_rows_check(q, "gdn_pack: q bf16 [B,T,Hk,128]"); gdn_rows_check(k, "gdn_pack: k"); gdn_rows_check(v, "gdn_pack: v");
+  gdn_tc_check(g, "g"); gdn_tc_check(beta, "beta");
+  const int64_t B = q.size(0), T = q.size(1), Hk = q.size(2), Hv = v.size(2), Tp = (T + 63) / 64 * 64;
+  TORCH_CHECK(k.sizes() == q.sizes() && v.size(0) == B && v.size(1) == T && g.numel() == B * T * Hv && beta.numel() == B * T * Hv, "gdn_pack: shapes");
+  c10::cuda::CUDAGuard guard(q.device());
+  auto opt = g.options();
+  Tensor qf = out_empty({B, Tp, Hk, 128}, opt), kf = out_empty({B, Tp, Hk, 128}, opt), vf = out_empty({B, Tp, Hv, 128}, opt);
+  Tensor gp = out_empty({B, Tp, Hv}, opt), bp = out_empty({B, Tp, Hv}, opt);
+  FERRL_CHECK(ferrl::gdn_pack(q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), k.stride(1), v.data_ptr(), v.stride(0),
+                              v.stride(1), g.data_ptr<float>(), beta.data_ptr<float>(), B, T, Tp, Hk, Hv, static_cast<float>(eps),
+                              qf.data_ptr<float>(), kf.data_ptr<float>(), vf.data_ptr<float>(), gp.data_ptr<float>(), bp.data_ptr<float>(), stream()));
+  return {qf, kf, vf, gp, bp};
+}
+
+Tensor gdn_pad(const Tensor& x) {
+  gdn_rows_check(x, "gdn_pad: bf16 [B,T,H,128]");
+  const int64_t B = x.size(0), T = x.size(1), H = x.size(2), Tp = (T + 63) / 64 * 64;
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = out_empty({B, Tp, H, 128}, x.options().dtype(at::kFloat));
+  FERRL_CHECK(ferrl::gdn_pad(x.data_ptr(), x.stride(0), x.stride(1), B, T, Tp, H, out.data_ptr<float>(), stream()));
+  return out;
+}
+
+// gradients of gdn_tc_bwd (dq, dk per value head, [B,Tp,..]) -> dq, dk [B,T,Hk,128], dv [B,T,Hv,128] bf16, dg, dbeta [B,T,Hv]
+std::vector<Tensor> gdn_unpack_bwd(const Tensor& q, const Tensor& k, const Tensor& dqf, const Tensor& dkf, const Tensor& dvf, const Tensor& dG,
+                                   const Tensor& dbp, double eps) {
+  gdn_rows_check(q, "gdn_unpack_bwd: q"); gdn_rows_check(k, "gdn_unpack_bwd: k");
+  gdn_tc_check(dqf, "dq"); gdn_tc_check(dkf, "dk"); gdn_tc_check(dvf, "dv"); gdn_tc_check(dG, "dG"); gdn_tc_check(dbp, "dbeta");
+  const int64_t B = q.size(0), T = q.size(1), Hk = q.size(2), Hv = dvf.size(2), Tp = dvf.size(1);
+  TORCH_CHECK(k.sizes() == q.sizes() && Tp % 64 == 0 && Tp >= T && Hv % Hk == 0 && dvf.size(0) == B && dqf.sizes() == dvf.sizes() &&
+                  dkf.sizes() == dvf.sizes() && dG.numel() == B * Tp * Hv && dbp.numel() == B * Tp * Hv, "gdn_unpack_bwd: shapes");
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor dq = out_empty({B, T, Hk, 128}, q.options()), dk = out_empty({B, T, Hk, 128}, q.options()), dv = out_empty({B, T, Hv, 128}, q.options());
+  Tensor dg = out_empty({B, T, Hv}, dG.options()), dbeta = out_empty({B, T, Hv}, dG.options());
+  FERRL_CHECK(ferrl::gdn_unpack_bwd(q.data_ptr(), q.stride(0), q.stride(1), k.data_ptr(), k.stride(0), k.stride(1), dqf.data_ptr<float>(),
+                                    dkf.data_ptr<float>(), dvf.data_ptr<float>(), dG.data_ptr<float>(), dbp.data_ptr<float>(), B, T, Tp, Hk, Hv,
+                                    static_cast<float>(eps), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dg.data_ptr<float>(),
+                                    dbeta.data_ptr<float>(), stream()));
+  return {dq, dk, dv, dg, dbeta};
+}
+
 std::tuple<Tensor, Tensor> gdn_chunk_fwd(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g,
                                          const Tensor& beta, const optional<Tensor>& S0, bool l2norm, double eps) {
   // rows are read in 16-byte pieces: views that start or step elsewhere are copied
@@ -1916,6 +1966,9 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("gdn_conv_fwd(Tensor x, Tensor w, Tensor? left, bool act) -> Tensor", &gdn_conv_fwd);
   m.def("gdn_conv_bwd(Tensor x, Tensor w, Tensor? left, Tensor dy, bool act) -> Tensor", &gdn_conv_bwd);
   m.def("gdn_conv_step(Tensor x, Tensor w, Tensor(a!) state, bool act) -> Tensor", &gdn_conv_step);
+  m.def("gdn_pack(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, float eps) -> Tensor[]", &gdn_pack);
+  m.def("gdn_pad(Tensor x) -> Tensor", &gdn_pad);
+  m.def("gdn_unpack_bwd(Tensor q, Tensor k, Tensor dqf, Tensor dkf, Tensor dvf, Tensor dG, Tensor dbeta, float eps) -> Tensor[]", &gdn_unpack_bwd);
   m.def("gdn_chunk_fwd(Tensor q, Tensor k, Tensor v, Tensor g, Tensor beta, Tensor? S0, bool l2norm, float eps) -> (Tensor, Tensor)", &gdn_chunk_fwd);
   m.def("set_canary(bool on) -> ()", &set_canary);
   m.def("check_canaries() -> int", &check_canaries);

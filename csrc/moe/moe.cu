@@ -149,22 +149,23 @@ __global__ void moe_plan_kernel(const int* __restrict__ idx, const int* __restri
 __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const int* __restrict__ token_of,
                                   const float* __restrict__ row_scale, int rows, int H,
                                   __nv_bfloat16* __restrict__ xs, int sparse) {
-  const int chunks = H / 8;
-  const long long n = static_cast<long long>(rows) * chunks;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int r = static_cast<int>(i / chunks), c = static_cast<int>(i % chunks);
-    const int t = token_of[r];
-    if (sparse && t < 0 && token_of[r & ~15] < 0) continue;
+  // a warp per row: the token is read once, and rows to skip end there (17280 rows of which 1024 hold a token: 13.3 -> 4.9 us;
+  // 65408 rows, 49136 tokens, 2048 wide: 61 -> 50 us)
+  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  const int t = token_of[r];
+  if (sparse && t < 0 && token_of[r & ~15] < 0) return;
+  const float s = row_scale && t >= 0 ? row_scale[r] : 1.f;
+#pragma unroll 4
+  for (int c = lane; c < H / 8; c += 32) {
     uint4 o = make_uint4(0, 0, 0, 0);
     if (t >= 0) {
       o = *reinterpret_cast<const uint4*>(x + static_cast<long long>(t) * ldx + c * 8);
       if (row_scale) {
-        const float s = row_scale[r];
         __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          float2 f = __bfloat1622float2(h[e]);
+          const float2 f = __bfloat1622float2(h[e]);
           h[e] = __floats2bfloat162_rn(f.x * s, f.y * s);
         }
       }
@@ -371,9 +372,8 @@ const char* moe_gather(const void* x, long long ldx, const int* token_of, const 
     moe_row_scale_kernel<<<(n_pairs + 255) / 256, 256, 0, stream>>>(pair_w, row_of, n_pairs, row_scale);
     count_launch();
   }
-  const long long n = static_cast<long long>(rows) * (H / 8);
-  const int blocks = static_cast<int>(std::min<long long>((n + 255) / 256, 148 * 16));
-  moe_gather_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), ldx, token_of,
+  if (rows == 0) return nullptr;
+  moe_gather_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), ldx, token_of,
                                                 pair_w ? row_scale : nullptr, rows, H, static_cast<__nv_bfloat16*>(xs), sparse ? 1 : 0);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? nullptr : "moe_gather launch failed";

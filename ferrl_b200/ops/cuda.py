@@ -821,6 +821,38 @@ class _GdnTc(torch.autograd.Function):
         return dq, dk, dv, dg, dbeta, (dS0 if ctx.needs_input_grad[5] else None)
 
 
+def _gdn_rows(t):
+    """Heads packed in rows that start on 8 bytes, read where they lie."""
+    ok = t.stride(3) == 1 and (t.shape[2] == 1 or t.stride(2) == 128) and t.stride(0) % 4 == 0 and t.stride(1) % 4 == 0
+    return t if ok and t.data_ptr() % 8 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
+class _GdnTc16(torch.autograd.Function):
+    """``_GdnTc`` between 16-bit activations: normalisation, padding and their derivatives are one pass each."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, beta, S0, eps):
+        L = lib()
+        q, k, v = _gdn_rows(q), _gdn_rows(k), _gdn_rows(v)
+        qf, kf, vf, gp, bp = L.gdn_pack(q, k, v, g, beta, eps)
+        out, S1, *saved = L.gdn_tc_fwd(qf, kf, vf, gp, bp, S0)
+        if any(ctx.needs_input_grad):
+            ctx.save_for_backward(q, k, qf, kf, vf, bp, *saved)
+            ctx.eps = eps
+        ctx.set_materialize_grads(False)
+        return out[:, :q.shape[1]].to(v.dtype), S1
+
+    @staticmethod
+    def backward(ctx, dO, dS1):
+        L = lib()
+        q, k, qf, kf, vf, bp, Gc, gl, Tm, Wn, Kd, Vn, Sin = ctx.saved_tensors
+        dO = torch.zeros_like(vf) if dO is None else L.gdn_pad(_gdn_rows(dO))
+        dqf, dkf, dvf, dbp, dG, dS0 = L.gdn_tc_bwd(qf, kf, vf, bp, Gc, gl, Tm, Wn, Kd, Vn, Sin, dO,
+                                                   None if dS1 is None else dS1.contiguous())
+        dq, dk, dv, dg, dbeta = L.gdn_unpack_bwd(q, k, dqf, dkf, dvf, dG, dbp, ctx.eps)
+        return dq, dk, dv, dg, dbeta, (dS0 if ctx.needs_input_grad[5] else None), None
+
+
 def gdn_chunk_tc(q, k, v, g, beta, S0=None, eps=1e-6):
     """Chunked gated delta rule on the tensor cores with autograd: ``q,k`` ``[B,T,Hk,128]`` (raw; they are
     L2-normalised here and q is scaled by 1/sqrt(128)), ``v`` ``[B,T,Hv,128]``, ``g,beta`` ``[B,T,Hv]``, ``S0``
@@ -828,6 +860,9 @@ def gdn_chunk_tc(q, k, v, g, beta, S0=None, eps=1e-6):
     kernels' domain (head dims other than 128)."""
     if q.shape[-1] != 128 or v.shape[-1] != 128 or v.shape[2] % q.shape[2]:
         return None
+    if _bf16(q) and _bf16(k) and _bf16(v):
+        return _GdnTc16.apply(q, k, v, g.float().contiguous(), beta.float().contiguous(),
+                              None if S0 is None else S0.float().contiguous(), float(eps))
     T = q.shape[1]
     qf = eager.l2norm(q.float(), eps) * (128 ** -0.5)
     kf = eager.l2norm(k.float(), eps)
