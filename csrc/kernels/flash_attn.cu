@@ -253,13 +253,13 @@ __global__ void flash_delta_kernel(FlashArgs a) {
   if (lane == 0) a.delta[(static_cast<long long>(b) * a.Hq + h) * a.Sq + i] = s;
 }
 
-// dK/dV: CTA owns 64 keys of one kv head. DSPLIT warps groups split the head dim of the accumulators.
-template <int D, int DSPLIT>
-__global__ void __launch_bounds__(128 * DSPLIT) flash_bwd_dkv_kernel(FlashArgs a) {
+// dK/dV: CTA owns 64 keys of one kv head.
+template <int D>
+__global__ void __launch_bounds__(128) flash_bwd_dkv_kernel(FlashArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int TILE = 64 * D * 2;
-  constexpr int THREADS = 128 * DSPLIT;
-  constexpr int DW = D / DSPLIT;  // accumulator width per warp
+  constexpr int THREADS = 128;
+  constexpr int DW = D;  // accumulator width per warp
   uint8_t* sK = smem;
   uint8_t* sV = smem + TILE;
   uint8_t* sQ = smem + 2 * TILE;
@@ -269,8 +269,7 @@ __global__ void __launch_bounds__(128 * DSPLIT) flash_bwd_dkv_kernel(FlashArgs a
   const int n0 = blockIdx.x * BKV, hk = blockIdx.y, b = blockIdx.z;
   const int rep = a.Hq / a.Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int kw = warp & 3, dh = warp >> 2;
-  const int k0 = kw * 16, d0 = dh * DW;
+  const int k0 = warp * 16, d0 = 0;
   const __nv_bfloat16* kb = static_cast<const __nv_bfloat16*>(a.k) + b * a.k_bs + hk * D;
   const __nv_bfloat16* vb = static_cast<const __nv_bfloat16*>(a.v) + b * a.v_bs + hk * D;
   load_tile<D, THREADS>(sK, kb, a.k_ts, n0, a.Sk);
@@ -500,15 +499,278 @@ const char* fwd_d(const FlashArgs& a, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? nullptr : "flash_fwd launch failed";
 }
 
-template <int D, int DSPLIT>
+// ---- backward for head dim 256.  Eight warps form the score tiles once (16 rows x 32 columns each) and pass them on as
+// 16-bit operand fragments through shared memory; for the products with them a warp then has 32 rows and 64 of the 256
+// columns, so a fragment of the streamed tiles serves two row tiles.  The next pair of streamed tiles loads meanwhile.
+// What bounds it is reading fragments from shared memory (0.45 reads of 512 bytes per product).  With every warp forming
+// whole score rows (twice over) behind unhidden loads: 5119 tokens, 24 query and 4 key heads, causal 8.44 -> 6.27 ms, 4 x 1535
+// tokens, 16 and 2 heads 2.36 -> 1.72 ms.
+// Every sum keeps its order, so the results are the same bits.
+constexpr int kD256 = 256;
+constexpr int kTile256 = 64 * kD256 * 2;
+constexpr int kFrag256 = 4 * 4 * 32 * 16;         // fragments of a [64, 64] tile
+
+__global__ void __launch_bounds__(256) flash_bwd256_dkv_kernel(FlashArgs a) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  constexpr int D = kD256, TILE = kTile256;
+  uint8_t *sK = smem, *sV = smem + TILE, *sStream = smem + 2 * TILE;        // then Q, dO of two buffers
+  uint4* sP = reinterpret_cast<uint4*>(smem + 6 * TILE);                    // [4 key tiles][4 query tiles][32]
+  uint4* sS = sP + kFrag256 / 16;
+  float* sLse = reinterpret_cast<float*>(smem + 6 * TILE + 2 * kFrag256);   // [2][64]
+  float* sDel = sLse + 128;
+  const int n0 = blockIdx.x * BKV, hk = blockIdx.y, b = blockIdx.z;
+  const int rep = a.Hq / a.Hkv;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int kw = warp & 3, qh = warp >> 2;        // score tile: keys 16 kw.., queries 32 qh..
+  const int kp = warp & 1, d0 = (warp >> 1) * 64; // products: keys 32 kp.., columns d0..
+  load_tile<D, 256>(sK, static_cast<const __nv_bfloat16*>(a.k) + b * a.k_bs + hk * D, a.k_ts, n0, a.Sk);
+  load_tile<D, 256>(sV, static_cast<const __nv_bfloat16*>(a.v) + b * a.v_bs + hk * D, a.v_ts, n0, a.Sk);
+  cp_commit();
+
+  float dk[2][8][4], dv[2][8][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dk[i][j][e] = dv[i][j][e] = 0.f;
+  const float c = a.scale * LOG2E;
+  // query rows that can see this key block: pos_i >= n0 (causal) and pos_i < n0 + 64 + window - 1
+  const int i_lo = a.causal ? max(0, n0 - a.q_offset) : 0;
+  const int i_hi = a.window > 0 ? min(a.Sq, n0 + BKV + a.window - 1 - a.q_offset) : a.Sq;
+  const int ib0 = i_lo / BQ, nb = max(0, (i_hi + BQ - 1) / BQ - ib0), n_it = nb * rep;
+  const int key0 = n0 + kw * 16 + g, key1 = key0 + 8;
+  auto fetch = [&](int it) {
+    const int r = it / nb, ib = ib0 + it - r * nb, h = hk * rep + r, buf = it & 1;
+    uint8_t* q = sStream + buf * 2 * TILE;
+    load_tile<D, 256>(q, static_cast<const __nv_bfloat16*>(a.q) + b * a.q_bs + h * D, a.q_ts, ib * BQ, a.Sq);
+    load_tile<D, 256>(q + TILE, static_cast<const __nv_bfloat16*>(a.d_o) + b * a.do_bs + h * D, a.do_ts, ib * BQ, a.Sq);
+    cp_commit();
+    if (threadIdx.x < 64) {
+      const int i = ib * BQ + threadIdx.x;
+      const long long at = (static_cast<long long>(b) * a.Hq + h) * a.Sq + i;
+      sLse[buf * 64 + threadIdx.x] = i < a.Sq ? a.lse[at] * LOG2E : INFINITY;
+      sDel[buf * 64 + threadIdx.x] = i < a.Sq ? a.delta[at] : 0.f;
+    }
+  };
+  if (n_it > 0) fetch(0);
+  for (int it = 0; it < n_it; ++it) {
+    const int ib = ib0 + it % nb, buf = it & 1;
+    const uint8_t *sQ = sStream + buf * 2 * TILE, *sdO = sQ + TILE;
+    cp_wait<0>();
+    __syncthreads();      // this iteration's tiles are here, the last one's readers are done
+    if (it + 1 < n_it) fetch(it + 1);
+    float st[4][4] = {}, dpt[4][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+      uint32_t ak[4], av[4];
+      load_a<D>(sK, kw * 16, kk, ak);
+      load_a<D>(sV, kw * 16, kk, av);
+#pragma unroll
+      for (int np = 0; np < 2; ++np) {
+        uint32_t bq[4], bd[4];
+        load_b_nk<D>(sQ, qh * 32 + np * 16, kk, bq);
+        load_b_nk<D>(sdO, qh * 32 + np * 16, kk, bd);
+        mma16816(st[2 * np], ak, bq[0], bq[1]);
+        mma16816(st[2 * np + 1], ak, bq[2], bq[3]);
+        mma16816(dpt[2 * np], av, bd[0], bd[1]);
+        mma16816(dpt[2 * np + 1], av, bd[2], bd[3]);
+      }
+    }
+#pragma unroll
+    for (int np = 0; np < 2; ++np) {
+      uint32_t pf[4], df[4];
+#pragma unroll
+      for (int hn = 0; hn < 2; ++hn) {
+        float p[4], ds[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int il = qh * 32 + (2 * np + hn) * 8 + 2 * t + (e & 1), i = ib * BQ + il;
+          const bool ok = i < a.Sq && allowed(a.q_offset + i, e < 2 ? key0 : key1, a.Sk, a.causal, a.window);
+          p[e] = ok ? exp2f(st[2 * np + hn][e] * c - sLse[buf * 64 + il]) : 0.f;
+          ds[e] = p[e] * (dpt[2 * np + hn][e] - sDel[buf * 64 + il]);
+        }
+        pf[2 * hn] = pack_bf16(p[0], p[1]);
+        pf[2 * hn + 1] = pack_bf16(p[2], p[3]);
+        df[2 * hn] = pack_bf16(ds[0], ds[1]);
+        df[2 * hn + 1] = pack_bf16(ds[2], ds[3]);
+      }
+      const int at = (kw * 4 + qh * 2 + np) * 32 + lane;
+      sP[at] = make_uint4(pf[0], pf[1], pf[2], pf[3]);
+      sS[at] = make_uint4(df[0], df[1], df[2], df[3]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k2 = 0; k2 < 4; ++k2) {
+      uint4 pf[2], df[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        pf[i] = sP[((kp * 2 + i) * 4 + k2) * 32 + lane];
+        df[i] = sS[((kp * 2 + i) * 4 + k2) * 32 + lane];
+      }
+#pragma unroll
+      for (int dp = 0; dp < 4; ++dp) {
+        uint32_t bo[4], bq[4];
+        load_b_kn<D>(sdO, k2 * 16, d0 + dp * 16, bo);
+        load_b_kn<D>(sQ, k2 * 16, d0 + dp * 16, bq);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          mma16816(dv[i][2 * dp], &pf[i].x, bo[0], bo[1]);
+          mma16816(dv[i][2 * dp + 1], &pf[i].x, bo[2], bo[3]);
+          mma16816(dk[i][2 * dp], &df[i].x, bq[0], bq[1]);
+          mma16816(dk[i][2 * dp + 1], &df[i].x, bq[2], bq[3]);
+        }
+      }
+    }
+  }
+  cp_wait<0>();
+  __nv_bfloat16* dkb = static_cast<__nv_bfloat16*>(a.dk) + b * a.dk_bs + hk * D + d0;
+  __nv_bfloat16* dvb = static_cast<__nv_bfloat16*>(a.dv) + b * a.dv_bs + hk * D + d0;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int key = n0 + kp * 32 + i * 16 + g + r * 8;
+      if (key >= a.Sk) continue;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        *reinterpret_cast<uint32_t*>(dkb + static_cast<long long>(key) * a.dk_ts + j * 8 + 2 * t) =
+            pack_bf16(dk[i][j][2 * r] * a.scale, dk[i][j][2 * r + 1] * a.scale);
+        *reinterpret_cast<uint32_t*>(dvb + static_cast<long long>(key) * a.dv_ts + j * 8 + 2 * t) = pack_bf16(dv[i][j][2 * r], dv[i][j][2 * r + 1]);
+      }
+    }
+}
+
+__global__ void __launch_bounds__(256) flash_bwd256_dq_kernel(FlashArgs a) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  constexpr int D = kD256, TILE = kTile256;
+  uint8_t *sQ = smem, *sdO = smem + TILE, *sStream = smem + 2 * TILE;       // then K, V of two buffers
+  uint4* sS = reinterpret_cast<uint4*>(smem + 6 * TILE);                    // [4 row tiles][4 key tiles][32]
+  const int m0 = blockIdx.x * BQ, h = blockIdx.y, b = blockIdx.z;
+  const int hk = h / (a.Hq / a.Hkv);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int rw = warp & 3, jh = warp >> 2;        // score tile: rows 16 rw.., keys 32 jh..
+  const int rp = warp & 1, d0 = (warp >> 1) * 64; // product: rows 32 rp.., columns d0..
+  load_tile<D, 256>(sQ, static_cast<const __nv_bfloat16*>(a.q) + b * a.q_bs + h * D, a.q_ts, m0, a.Sq);
+  load_tile<D, 256>(sdO, static_cast<const __nv_bfloat16*>(a.d_o) + b * a.do_bs + h * D, a.do_ts, m0, a.Sq);
+  cp_commit();
+  const int row0 = m0 + rw * 16 + g, row1 = row0 + 8;
+  const float* lse = a.lse + (static_cast<long long>(b) * a.Hq + h) * a.Sq;
+  const float* del = a.delta + (static_cast<long long>(b) * a.Hq + h) * a.Sq;
+  const float lse0 = row0 < a.Sq ? lse[row0] * LOG2E : INFINITY, lse1 = row1 < a.Sq ? lse[row1] * LOG2E : INFINITY;
+  const float del0 = row0 < a.Sq ? del[row0] : 0.f, del1 = row1 < a.Sq ? del[row1] : 0.f;
+  const float c = a.scale * LOG2E;
+  float dq[2][8][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dq[i][j][e] = 0.f;
+  const int j_hi = a.causal ? min(a.Sk, a.q_offset + m0 + BQ) : a.Sk;
+  const int j_lo = a.window > 0 ? max(0, a.q_offset + m0 - a.window + 1) : 0;
+  const int jb0 = j_lo / BKV, jb1 = (j_hi + BKV - 1) / BKV;
+  auto fetch = [&](int jb) {
+    uint8_t* k = sStream + ((jb - jb0) & 1) * 2 * TILE;
+    load_tile<D, 256>(k, static_cast<const __nv_bfloat16*>(a.k) + b * a.k_bs + hk * D, a.k_ts, jb * BKV, a.Sk);
+    load_tile<D, 256>(k + TILE, static_cast<const __nv_bfloat16*>(a.v) + b * a.v_bs + hk * D, a.v_ts, jb * BKV, a.Sk);
+    cp_commit();
+  };
+  if (jb0 < jb1) fetch(jb0);
+  for (int jb = jb0; jb < jb1; ++jb) {
+    const uint8_t *sK = sStream + ((jb - jb0) & 1) * 2 * TILE, *sV = sK + TILE;
+    cp_wait<0>();
+    __syncthreads();
+    if (jb + 1 < jb1) fetch(jb + 1);
+    float s[4][4] = {}, dp[4][4] = {};
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+      uint32_t aq[4], ad[4];
+      load_a<D>(sQ, rw * 16, kk, aq);
+      load_a<D>(sdO, rw * 16, kk, ad);
+#pragma unroll
+      for (int np = 0; np < 2; ++np) {
+        uint32_t bk[4], bv[4];
+        load_b_nk<D>(sK, jh * 32 + np * 16, kk, bk);
+        load_b_nk<D>(sV, jh * 32 + np * 16, kk, bv);
+        mma16816(s[2 * np], aq, bk[0], bk[1]);
+        mma16816(s[2 * np + 1], aq, bk[2], bk[3]);
+        mma16816(dp[2 * np], ad, bv[0], bv[1]);
+        mma16816(dp[2 * np + 1], ad, bv[2], bv[3]);
+      }
+    }
+#pragma unroll
+    for (int np = 0; np < 2; ++np) {
+      uint32_t df[4];
+#pragma unroll
+      for (int hn = 0; hn < 2; ++hn) {
+        float ds[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int j = jb * BKV + jh * 32 + (2 * np + hn) * 8 + 2 * t + (e & 1), row = e < 2 ? row0 : row1;
+          const bool ok = row < a.Sq && allowed(a.q_offset + row, j, a.Sk, a.causal, a.window);
+          const float p = ok ? exp2f(s[2 * np + hn][e] * c - (e < 2 ? lse0 : lse1)) : 0.f;
+          ds[e] = p * (dp[2 * np + hn][e] - (e < 2 ? del0 : del1));
+        }
+        df[2 * hn] = pack_bf16(ds[0], ds[1]);
+        df[2 * hn + 1] = pack_bf16(ds[2], ds[3]);
+      }
+      sS[(rw * 4 + jh * 2 + np) * 32 + lane] = make_uint4(df[0], df[1], df[2], df[3]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k2 = 0; k2 < 4; ++k2) {
+      uint4 df[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) df[i] = sS[((rp * 2 + i) * 4 + k2) * 32 + lane];
+#pragma unroll
+      for (int dd = 0; dd < 4; ++dd) {
+        uint32_t bk[4];
+        load_b_kn<D>(sK, k2 * 16, d0 + dd * 16, bk);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          mma16816(dq[i][2 * dd], &df[i].x, bk[0], bk[1]);
+          mma16816(dq[i][2 * dd + 1], &df[i].x, bk[2], bk[3]);
+        }
+      }
+    }
+  }
+  cp_wait<0>();
+  __nv_bfloat16* dqb = static_cast<__nv_bfloat16*>(a.dq) + b * a.dq_bs + h * D + d0;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int row = m0 + rp * 32 + i * 16 + g + r * 8;
+      if (row >= a.Sq) continue;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<uint32_t*>(dqb + static_cast<long long>(row) * a.dq_ts + j * 8 + 2 * t) =
+            pack_bf16(dq[i][j][2 * r] * a.scale, dq[i][j][2 * r + 1] * a.scale);
+    }
+}
+
+const char* bwd_256(const FlashArgs& a, cudaStream_t s) {
+  const long long warps = static_cast<long long>(a.B) * a.Sq * a.Hq;
+  flash_delta_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, s>>>(a);
+  constexpr size_t smem = 6 * kTile256 + 2 * kFrag256 + 4 * 64 * sizeof(float), smem2 = 6 * kTile256 + kFrag256;
+  if (const char* e = set_smem(flash_bwd256_dkv_kernel, smem)) return e;
+  if (const char* e = set_smem(flash_bwd256_dq_kernel, smem2)) return e;
+  flash_bwd256_dkv_kernel<<<dim3((a.Sk + BKV - 1) / BKV, a.Hkv, a.B), 256, smem, s>>>(a);
+  flash_bwd256_dq_kernel<<<dim3((a.Sq + BQ - 1) / BQ, a.Hq, a.B), 256, smem2, s>>>(a);
+  count_launch(3);
+  return cudaGetLastError() == cudaSuccess ? nullptr : "flash_bwd launch failed";
+}
+
+template <int D>
 const char* bwd_d(const FlashArgs& a, cudaStream_t s) {
   long long warps = static_cast<long long>(a.B) * a.Sq * a.Hq;
   flash_delta_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, s>>>(a);
   count_launch();
   size_t smem = 4 * 64 * D * 2 + 512;
-  if (const char* e = set_smem(flash_bwd_dkv_kernel<D, DSPLIT>, smem)) return e;
+  if (const char* e = set_smem(flash_bwd_dkv_kernel<D>, smem)) return e;
   dim3 gkv((a.Sk + BKV - 1) / BKV, a.Hkv, a.B);
-  flash_bwd_dkv_kernel<D, DSPLIT><<<gkv, 128 * DSPLIT, smem, s>>>(a);
+  flash_bwd_dkv_kernel<D><<<gkv, 128, smem, s>>>(a);
   count_launch();
   size_t smem2 = 4 * 64 * D * 2;
   if (const char* e = set_smem(flash_bwd_dq_kernel<D>, smem2)) return e;
@@ -545,9 +807,9 @@ const char* flash_bwd(const FlashArgs& a, cudaStream_t s) {
   if (a.B == 0 || a.Sq == 0) return nullptr;
   if (const char* e = check(a)) return e;
   switch (a.D) {
-    case 64: return bwd_d<64, 1>(a, s);
-    case 128: return bwd_d<128, 1>(a, s);
-    case 256: return bwd_d<256, 2>(a, s);
+    case 64: return bwd_d<64>(a, s);
+    case 128: return bwd_d<128>(a, s);
+    case 256: return bwd_256(a, s);
     default: return "flash: head_dim must be 64, 128 or 256";
   }
 }
