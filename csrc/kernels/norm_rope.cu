@@ -464,10 +464,14 @@ __global__ void qk_norm_rope_kernel(const T* __restrict__ q_in, long long ld_q, 
   }
 }
 
-// bf16 vector form for D = 32*EPL (128 or 256): one warp per (token, head), EPL consecutive
-// channels per lane in one 8- or 16-byte access, rotation partners fetched with a warp shuffle
+// bf16 vector form for D = LPH*EPL (128 or 256): LPH lanes hold a head, EPL consecutive channels each in one 8- or
+// 16-byte access, and a warp takes U times 32/LPH heads of one token; rotation partners are fetched with a warp shuffle
 // (partner lane = lane +- half/EPL).  Same arithmetic and rounding points as the kernel above.
-template <int EPL, bool BWD>
+// What bounds it is instructions per entry: with a head of 128 to a warp (four entries a lane) shuffles, sums and the
+// angles, loaded again for each head, were most of them.
+// 8192 tokens x 40 heads of 128: forward 126 -> 74 us; 11384 tokens: 141 -> 91 us, backward 180 -> 157 us (the
+// bytes take 36 and 54 us).
+template <int EPL, bool BWD, int LPH, int U>
 __global__ void qk_norm_rope_vec_kernel(const __nv_bfloat16* __restrict__ q_in, long long ld_q,
                                         const __nv_bfloat16* __restrict__ k_in, long long ld_k, long long ld_dq,
                                         long long ld_dk, const __nv_bfloat16* __restrict__ qw,
@@ -482,20 +486,16 @@ __global__ void qk_norm_rope_vec_kernel(const __nv_bfloat16* __restrict__ q_in, 
                                         int smax) {
   pdl_trigger();
   pdl_wait();      // may be launched as a programmatic dependent: nothing is read before the predecessor is done
-  constexpr int D = 32 * EPL;
+  constexpr int D = LPH * EPL, HP = 32 / LPH;
   const long long wid = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const int heads = Hq + Hkv;
-  if (wid >= n_tok * heads) return;          // warp-uniform
-  const long long tok = wid / heads;
-  const int hh = static_cast<int>(wid % heads);
-  const bool is_q = hh < Hq;
-  const int h = is_q ? hh : hh - Hq;
-  const __nv_bfloat16* src = (is_q ? q_in + tok * ld_q : k_in + tok * ld_k) + h * D + lane * EPL;
-  const __nv_bfloat16* wv = is_q ? qw : kw;
-  const long long p = pos ? pos[tok / pos_div] : static_cast<long long>(pos32[tok / pos_div]);
+  const int heads = Hq + Hkv, groups = (heads + U * HP - 1) / (U * HP);
+  if (wid >= n_tok * groups) return;         // warp-uniform
+  const long long tok = wid / groups;
+  const int li = lane % LPH;                                     // place in the head
+  const int h0 = static_cast<int>(wid - tok * groups) * (U * HP) + lane / LPH;
   const int rot = 2 * half;
-  const int i0 = lane * EPL;
+  const int i0 = li * EPL;
   const int shift = half / EPL;                                  // lanes between rotation partners
   const bool in_rot = i0 < rot, lower = i0 < half;
   const int partner = in_rot ? (lower ? lane + shift : lane - shift) : lane;
@@ -522,24 +522,22 @@ __global__ void qk_norm_rope_vec_kernel(const __nv_bfloat16* __restrict__ q_in, 
     }
   };
 
-  float x[EPL], w[EPL], c[EPL], sn[EPL];
-  load(src, x);
-  float ss = 0.f;
+  float x[U][EPL] = {}, g[BWD ? U : 1][EPL] = {}, c[EPL], sn[EPL];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int hh = h0 + u * HP;
+    const bool is_q = hh < Hq;
+    const int h = is_q ? hh : hh - Hq;
+    if (hh < heads) {
+      load((is_q ? q_in + tok * ld_q : k_in + tok * ld_k) + h * D + i0, x[u]);
+      if (BWD) load((is_q ? dq + (tok * Hq + h) * D : dk + (tok * Hkv + h) * D) + i0, g[u]);
+    }
+  }
+  const long long p = pos ? pos[tok / pos_div] : static_cast<long long>(pos32[tok / pos_div]);
 #pragma unroll
   for (int e = 0; e < EPL; ++e) {
-    ss += x[e] * x[e];
-    w[e] = 1.f;
     c[e] = 1.f;
     sn[e] = 0.f;
-  }
-  float rstd = 1.f;
-  if (wv) {
-    load(wv + i0, w);
-    if (zero_centered) {
-#pragma unroll
-      for (int e = 0; e < EPL; ++e) w[e] += 1.f;
-    }
-    rstd = rsqrtf(warp_sum(ss) / D + eps);
   }
   if (in_rot) {
     const int f0 = lower ? i0 : i0 - half;
@@ -549,53 +547,78 @@ __global__ void qk_norm_rope_vec_kernel(const __nv_bfloat16* __restrict__ q_in, 
       sn[e] = sin_t[p * half + f0 + e];
     }
   }
-  if (!BWD) {
-    float v[EPL], o[EPL];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int hh = h0 + u * HP;
+    const bool on = hh < heads;
+    const bool is_q = hh < Hq;
+    const int h = is_q ? hh : hh - Hq;
+    const __nv_bfloat16* wv = is_q ? qw : kw;
+    float w[EPL], ss = 0.f;
 #pragma unroll
     for (int e = 0; e < EPL; ++e) {
-      v[e] = x[e] * rstd * w[e];
-      // the unfused form rounds the normalised value to bf16 before rotating it
-      if (in_rot) v[e] = __bfloat162float(__float2bfloat16_rn(v[e]));
+      ss += x[u][e] * x[u][e];
+      w[e] = 1.f;
     }
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-      const float u = __shfl_sync(0xffffffffu, v[e], partner);
-      o[e] = in_rot ? (lower ? v[e] * c[e] - u * sn[e] : v[e] * c[e] + u * sn[e]) : v[e];
-    }
-    if (!is_q && kc) {
-      // decode: the key goes to its cache row, and the value row of the same head is copied along
-      const int t = kv_len[tok];
-      const long long slot = table ? static_cast<long long>(table[tok * bt_stride + t / page]) * page + t % page
-                                   : tok * smax + t;
-      const long long off = (slot * Hkv + h) * D + i0;
-      store(kc + off, o);
-      float vv[EPL];
-      load(v_in + tok * ld_v + h * D + i0, vv);
-      store(vc + off, vv);
-    } else {
-      store((is_q ? q_out + (tok * Hq + h) * D : k_out + (tok * Hkv + h) * D) + i0, o);
-    }
-  } else {
-    float g[EPL], dn[EPL];
-    load((is_q ? dq + (tok * Hq + h) * D : dk + (tok * Hkv + h) * D) + i0, g);
-    float dot = 0.f;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-      const float gj = __shfl_sync(0xffffffffu, g[e], partner);
-      dn[e] = in_rot ? (lower ? g[e] * c[e] + gj * sn[e] : g[e] * c[e] - gj * sn[e]) : g[e];
-      dot += x[e] * w[e] * dn[e];
-    }
-    __nv_bfloat16* dst = (is_q ? q_out + tok * ld_dq : k_out + tok * ld_dk) + h * D + i0;
-    float o[EPL];
+    ss = lanes_sum<LPH>(ss);                 // every lane takes part, whatever its head
+    float rstd = 1.f;
     if (wv) {
-      const float c2 = warp_sum(dot) * rstd * rstd / D;
+      load(wv + i0, w);
+      if (zero_centered) {
 #pragma unroll
-      for (int e = 0; e < EPL; ++e) o[e] = rstd * (w[e] * dn[e] - x[e] * c2);
-    } else {
-#pragma unroll
-      for (int e = 0; e < EPL; ++e) o[e] = dn[e];
+        for (int e = 0; e < EPL; ++e) w[e] += 1.f;
+      }
+      rstd = rsqrtf(ss / D + eps);
     }
-    store(dst, o);
+    if (!BWD) {
+      float v[EPL], o[EPL];
+#pragma unroll
+      for (int e = 0; e < EPL; ++e) {
+        v[e] = x[u][e] * rstd * w[e];
+        // the unfused form rounds the normalised value to bf16 before rotating it
+        if (in_rot) v[e] = __bfloat162float(__float2bfloat16_rn(v[e]));
+      }
+#pragma unroll
+      for (int e = 0; e < EPL; ++e) {
+        const float y = __shfl_sync(0xffffffffu, v[e], partner);
+        o[e] = in_rot ? (lower ? v[e] * c[e] - y * sn[e] : v[e] * c[e] + y * sn[e]) : v[e];
+      }
+      if (!on) continue;
+      if (!is_q && kc) {
+        // decode: the key goes to its cache row, and the value row of the same head is copied along
+        const int t = kv_len[tok];
+        const long long slot = table ? static_cast<long long>(table[tok * bt_stride + t / page]) * page + t % page
+                                     : tok * smax + t;
+        const long long off = (slot * Hkv + h) * D + i0;
+        store(kc + off, o);
+        float vv[EPL];
+        load(v_in + tok * ld_v + h * D + i0, vv);
+        store(vc + off, vv);
+      } else {
+        store((is_q ? q_out + (tok * Hq + h) * D : k_out + (tok * Hkv + h) * D) + i0, o);
+      }
+    } else {
+      float dn[EPL];
+      float dot = 0.f;
+#pragma unroll
+      for (int e = 0; e < EPL; ++e) {
+        const float gj = __shfl_sync(0xffffffffu, g[u][e], partner);
+        dn[e] = in_rot ? (lower ? g[u][e] * c[e] + gj * sn[e] : g[u][e] * c[e] - gj * sn[e]) : g[u][e];
+        dot += x[u][e] * w[e] * dn[e];
+      }
+      __nv_bfloat16* dst = (is_q ? q_out + tok * ld_dq : k_out + tok * ld_dk) + h * D + i0;
+      float o[EPL];
+      dot = lanes_sum<LPH>(dot);
+      if (wv) {
+        const float c2 = dot * rstd * rstd / D;
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) o[e] = rstd * (w[e] * dn[e] - x[u][e] * c2);
+      } else {
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) o[e] = dn[e];
+      }
+      if (on) store(dst, o);
+    }
   }
 }
 
@@ -758,14 +781,25 @@ static const char* qknr_t(const QkNormRopeArgs& a, cudaStream_t s) {
                     (!a.kc || (!BWD && al(a.kc, epl) && al(a.vc, epl) && al(a.v_in, a.ld_v) && a.kv_len));
     if (ok) {
       using B = __nv_bfloat16;
-#define FERRL_QKV(EPLV)                                                                                             \
-  launch_pdl(qk_norm_rope_vec_kernel<EPLV, BWD>, dim3(static_cast<unsigned>(blocks)), dim3(wpb * 32), 0, s,          \
+      // many heads a warp where that still leaves every SM its 64 warps, one (a decode step's few tokens) where not;
+      // heads of 128 in 16-byte pieces, where addresses and the rotated width allow it
+      auto wide = [](const void* p, long long ld) { return (reinterpret_cast<uintptr_t>(p) % 16) == 0 && (ld % 8) == 0; };
+      const bool eight = a.half % 8 == 0 && wide(a.q_in, a.ld_q) && wide(a.k_in, a.ld_k) && wide(a.q_out, BWD ? a.ld_dq : 8) &&
+                         wide(a.k_out, BWD ? a.ld_dk : 8) && wide(a.qw, 8) && wide(a.kw, 8) && wide(a.dq, 8) && wide(a.dk, 8) &&
+                         (!a.kc || (wide(a.kc, 8) && wide(a.vc, 8) && wide(a.v_in, a.ld_v)));
+      const int per = units < 148LL * 64 * 4 || !eight ? 1 : a.D == 128 ? 8 : 4;
+      blocks = (a.n_tok * ((a.Hq + a.Hkv + per - 1) / per) + wpb - 1) / wpb;
+#define FERRL_QKV(EPLV, LPH, U)                                                                                     \
+  launch_pdl(qk_norm_rope_vec_kernel<EPLV, BWD, LPH, U>, dim3(static_cast<unsigned>(blocks)), dim3(wpb * 32), 0, s,       \
       static_cast<const B*>(a.q_in), a.ld_q, static_cast<const B*>(a.k_in), a.ld_k, a.ld_dq, a.ld_dk,               \
       static_cast<const B*>(a.qw), static_cast<const B*>(a.kw), a.cos_t, a.sin_t, a.pos64, a.pos32, a.pos_div,      \
       static_cast<B*>(a.q_out), static_cast<B*>(a.k_out), static_cast<const B*>(a.dq), static_cast<const B*>(a.dk), \
       a.n_tok, a.Hq, a.Hkv, a.half, a.eps, a.zero_centered ? 1 : 0, static_cast<B*>(a.kc), static_cast<B*>(a.vc),      \
       static_cast<const B*>(a.v_in), a.ld_v, a.kv_len, a.table, a.bt_stride, a.page, a.smax)
-      if (epl == 4) FERRL_QKV(4); else FERRL_QKV(8);
+      if (per == 8) FERRL_QKV(8, 16, 4);
+      else if (per == 4) FERRL_QKV(8, 32, 4);
+      else if (epl == 4) FERRL_QKV(4, 32, 1);
+      else FERRL_QKV(8, 32, 1);
 #undef FERRL_QKV
       count_launch();
       return cudaGetLastError() == cudaSuccess ? nullptr : "qk_norm_rope launch failed";
