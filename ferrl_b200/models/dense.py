@@ -120,7 +120,8 @@ class DenseLayer(nn.Module):
         return out
 
     # full-sequence forward (training / scoring / prefill)
-    def forward(self, h, positions, cos, sin, comm: Comm, merged: bool = False, kv_out=None):
+    def forward(self, h, positions, cos, sin, comm: Comm, merged: bool = False, kv_out=None, pick=None):
+        """``pick`` = (rows, positions): past the attention only these tokens go on; returns ``[1, n, H]``."""
         B, S, _ = h.shape
         lin = (lambda m, x: m.forward_merged(x)) if merged else (lambda m, x: m(x))
         x = ops.rmsnorm(h, self.input_norm, self.eps)
@@ -135,7 +136,10 @@ class DenseLayer(nn.Module):
             kv_out[0][:, :S].copy_(k)
             kv_out[1][:, :S].copy_(v)
         a = ops.attention(q, k, v, scale=self.scale, causal=True, softmax_fp32=True)
-        o = self.o.forward_reduce(a.reshape(B, S, self.hq * self.D), comm, merged)
+        a = a.reshape(B, S, self.hq * self.D)
+        if pick is not None:
+            a, h = a[pick].unsqueeze(0), h[pick].unsqueeze(0)
+        o = self.o.forward_reduce(a, comm, merged)
         x, h = ops.add_rmsnorm(o, h, self.post_norm, self.eps)
         x = copy_to_tp(x, comm)
         mid = self.gate_up.forward_merged_glu(x, self.act) if merged else ops.swiglu(self.gate_up(x), self.act)
@@ -259,6 +263,11 @@ def _decode_fused_ok(layers, h, comm) -> bool:
                                                                                             "gelu_tanh"):
             return False
     return True
+
+
+def _wanted(P, lens, at, device):
+    """Places whose logits a prefill returns: every prompt's last token, or ``at``."""
+    return (torch.arange(P, device=device), (lens - 1).to(device).long()) if at is None else at
 
 
 def ops_cache_write(k_cache, v_cache, k, v, kv_len):
@@ -388,7 +397,9 @@ class DenseGradModel(nn.Module):
 
     # ------------------------------------------------------------- forward
     def forward_hidden(self, ids: torch.Tensor, comm: Optional[Comm] = None, merged: bool = False,
-                       kv_out=None, detached: bool = False) -> torch.Tensor:
+                       kv_out=None, detached: bool = False, pick=None) -> torch.Tensor:
+        """``pick`` (with ``kv_out``) = (rows, positions): only these tokens' hidden states ``[n, H]`` are wanted, so
+        the last layer projects and transforms no others."""
         comm = comm or SoloComm()
         B, S = ids.shape
         if S > self.cos.shape[0]:
@@ -412,9 +423,10 @@ class DenseGradModel(nn.Module):
                 fn = (lambda x, layer=layer: layer(x, positions, self.cos, self.sin, comm, merged, None))
                 h = remat_segment(fn, h, layer.adapter_params() if not self.full_ft else list(layer.parameters()), None)
             else:
-                h = layer(h, positions, self.cos, self.sin, comm, merged, kv)
+                last = pick if i == len(self.layers) - 1 else None
+                h = layer(h, positions, self.cos, self.sin, comm, merged, kv, last)
         del cot
-        return h
+        return h if pick is None else h.squeeze(0)
 
     def forward(self, ids: torch.Tensor, comm: Optional[Comm] = None) -> torch.Tensor:
         """Full-position logits ``[B, S, V]`` in float32 (oracle/test surface)."""
@@ -484,13 +496,12 @@ class DenseCachedDecoder:
         tmp = [(torch.empty(P, L, self.k[0].shape[2], self.k[0].shape[3], dtype=m.dtype, device=ids.device),
                 torch.empty(P, L, self.k[0].shape[2], self.k[0].shape[3], dtype=m.dtype, device=ids.device))
                for _ in m.layers]
-        h = m.forward_hidden(ids, self.comm, merged=True, kv_out=tmp, detached=True)
+        h = m.forward_hidden(ids, self.comm, merged=True, kv_out=tmp, detached=True, pick=_wanted(P, lens, at, ids.device))
         for i in range(len(m.layers)):
             self.k[i][rows, :L] = tmp[i][0]
             self.v[i][rows, :L] = tmp[i][1]
         self.kv_len[rows] = lens.to(torch.int32)
-        last = h[(torch.arange(P, device=ids.device), (lens - 1).long()) if at is None else at]
-        last = ops.rmsnorm(last, m.final_norm, m.spec.rms_norm_eps)
+        last = ops.rmsnorm(h, m.final_norm, m.spec.rms_norm_eps)
         return ops.lora_linear(last, m.head_weight(), None, None).float()
 
     @torch.no_grad()
@@ -603,7 +614,7 @@ class DensePagedDecoder(DenseCachedDecoder):
         hkv, D = self.k[0].shape[2], self.k[0].shape[3]
         tmp = [(torch.empty(P, L, hkv, D, dtype=m.dtype, device=dev), torch.empty(P, L, hkv, D, dtype=m.dtype, device=dev))
                for _ in m.layers]
-        h = m.forward_hidden(ids, self.comm, merged=True, kv_out=tmp, detached=True)
+        h = m.forward_hidden(ids, self.comm, merged=True, kv_out=tmp, detached=True, pick=_wanted(P, lens, at, ids.device))
         ppr = self.pages_per_row
         full = (lens // page).to(torch.int64)                                  # shared (full) pages per prompt
         # block table: shared page ids first, then the row's private pages
@@ -624,8 +635,7 @@ class DensePagedDecoder(DenseCachedDecoder):
                 tail = torch.gather(src, 1, tail_idx[:, :, None, None].expand(P, page, hkv, D))
                 pool[first_private] = tail.repeat_interleave(G, dim=0)
         self.kv_len.copy_(lens.to(torch.int32).repeat_interleave(G))
-        last = h[(torch.arange(P, device=dev), (lens - 1).long()) if at is None else at]
-        last = ops.rmsnorm(last, m.final_norm, m.spec.rms_norm_eps)
+        last = ops.rmsnorm(h, m.final_norm, m.spec.rms_norm_eps)
         return ops.lora_linear(last, m.head_weight(), None, None).float()
 
     @torch.no_grad()

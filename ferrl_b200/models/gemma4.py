@@ -34,7 +34,7 @@ from .. import ops
 from ..comm import Comm, SoloComm
 from ..parallel.tp import TensorParallelPlan, copy_to_tp
 from ..remat import remat_segment
-from .dense import ops_cache_write
+from .dense import _wanted, ops_cache_write
 from .lora import BaseQuantization, DenseLoraTargets, FusedLoraLinear, LoraSpec, Shard
 
 
@@ -188,7 +188,8 @@ class Gemma4Layer(nn.Module):
         q, k = ops.qk_norm_rope(q, k, self.q_norm, self.k_norm, self.eps, cos, sin, positions)
         return q, k, v
 
-    def attn_half(self, h, positions, cos, sin, comm, merged=False, kv_out=None):
+    def attn_half(self, h, positions, cos, sin, comm, merged=False, kv_out=None, pick=None):
+        """``pick`` = (rows, positions): past the attention only these tokens go on; returns ``[1, n, H]``."""
         B, S, _ = h.shape
         lin = (lambda m, z: m.forward_merged(z)) if merged else (lambda m, z: m(z))
         x = copy_to_tp(ops.rmsnorm(h, self.input_norm, self.eps), comm)
@@ -199,7 +200,10 @@ class Gemma4Layer(nn.Module):
         a = ops.attention(q, k, v, scale=1.0, causal=True, window=self.window, softmax_fp32=True)
         # row-parallel projection and its tensor-parallel sum: one fused GEMM -> all-reduce kernel where a
         # reducer is registered for ``comm`` (the residual joins after the post-norm, so none rides along)
-        o = self.o.forward_reduce(a.reshape(B, S, self.hq * self.D), comm, merged)
+        a = a.reshape(B, S, self.hq * self.D)
+        if pick is not None:
+            a, h = a[pick].unsqueeze(0), h[pick].unsqueeze(0)
+        o = self.o.forward_reduce(a, comm, merged)
         return h + ops.rmsnorm(o, self.post_attn_norm, self.eps)
 
     # ---- sequence-sharded forms: ``hs`` holds this rank's block of the flattened [B * S, H] token rows
@@ -323,7 +327,9 @@ class Gemma4GradModel(nn.Module):
                 p.init_adapters(g)
         self.refresh_head()
 
-    def forward_hidden(self, ids, comm: Optional[Comm] = None, merged=False, kv_out=None, detached=False):
+    def forward_hidden(self, ids, comm: Optional[Comm] = None, merged=False, kv_out=None, detached=False, pick=None):
+        """``pick`` (with ``kv_out``) = (rows, positions): only these tokens' hidden states ``[n, H]`` are wanted, so
+        the last layer projects and transforms no others."""
         comm = comm or SoloComm()
         B, S = ids.shape
         positions = torch.arange(S, device=ids.device)
@@ -349,9 +355,10 @@ class Gemma4GradModel(nn.Module):
                 h = remat_segment(lambda x, l=layer, c=cos, s=sin: l.attn_half(x, positions, c, s, comm, merged), h, params)
                 h = remat_segment(lambda x, l=layer: l.mlp_half(x, comm, merged), h, params)
             else:
-                h = layer.attn_half(h, positions, cos, sin, comm, merged, None if kv_out is None else kv_out[i])
+                last = pick if i == len(self.layers) - 1 else None
+                h = layer.attn_half(h, positions, cos, sin, comm, merged, None if kv_out is None else kv_out[i], last)
                 h = layer.mlp_half(h, comm, merged)
-        return h
+        return h if pick is None else h.squeeze(0)
 
     def _softcap(self, logits):
         c = self.spec.final_logit_softcapping
@@ -413,7 +420,7 @@ class Gemma4CachedDecoder:
         rows = torch.arange(P, device=ids.device) if rows is None else rows
         tmp = [(torch.empty(P, L, l.hkv, l.D, dtype=m.dtype, device=ids.device),
                 torch.empty(P, L, l.hkv, l.D, dtype=m.dtype, device=ids.device)) for l in m.layers]
-        h = m.forward_hidden(ids, self.comm, merged=True, kv_out=tmp, detached=True)
+        h = m.forward_hidden(ids, self.comm, merged=True, kv_out=tmp, detached=True, pick=_wanted(P, lens, at, ids.device))
         lens64 = lens.to(ids.device).long()
         for i, n in enumerate(self.slots):
             if n >= L:
@@ -427,8 +434,7 @@ class Gemma4CachedDecoder:
             self.k[i][rows] = torch.gather(tmp[i][0], 1, gi)
             self.v[i][rows] = torch.gather(tmp[i][1], 1, gi)
         self.kv_len[rows] = lens.to(torch.int32)
-        last = h[(torch.arange(P, device=ids.device), (lens - 1).long()) if at is None else at]
-        last = ops.rmsnorm(last, m.final_norm, m.spec.rms_norm_eps)
+        last = ops.rmsnorm(h, m.final_norm, m.spec.rms_norm_eps)
         return m._softcap(ops.lora_linear(last, m.embed, None, None).float())
 
     @torch.no_grad()
