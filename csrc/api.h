@@ -97,6 +97,18 @@ bool decode_gemm_supported(int M, int N, int K, bool glu);
 int decode_gemm_groups(int K);
 const char* decode_gemm(const DecodeGemmArgs& a, cudaStream_t stream);
 
+// ---- adapters of a fused projection ----
+constexpr int kMaxLoraParts = 8;
+struct LoraParts {
+  const float *A[kMaxLoraParts], *B[kMaxLoraParts];       // [r, K], [rows, r]
+  int start[kMaxLoraParts], rows[kMaxLoraParts];          // rows of the projection's output
+  long long off[kMaxLoraParts];                           // lora_unpack: where each part's gradient lies in `out`
+  int n, r, Rp, K, N;                                     // Rp: n * r rounded up to 8
+  float scale;
+};
+const char* lora_pack(const LoraParts& p, void* a16, void* b16, cudaStream_t s);                         // -> [Rp, K], [N, Rp] bf16
+const char* lora_unpack(const float* dbt, long long ld, const LoraParts& p, float* out, cudaStream_t s);
+
 // ---- norms / rope ----
 // gate row r at (r / gate_per) * gate_ld + (r % gate_per) * H
 const char* rmsnorm(int dtype, const void* x, const void* res, const void* w, const void* gate, int gate_per, long long gate_ld,

@@ -929,6 +929,45 @@ Tensor moe_pair_dot(const Tensor& dy, const Tensor& ys, const Tensor& row_of, in
   return dw;
 }
 
+// adapters A_j [r,K], B_j [rows_j,r] f32 of the parts of a projection -> (A [Rp,K], scale * B [N,Rp]) bf16, Rp = n r rounded up to 8
+std::tuple<Tensor, Tensor> lora_pack(const std::vector<Tensor>& A, const std::vector<Tensor>& B, std::vector<int64_t> starts, int64_t N, double scale) {
+  TORCH_CHECK(!A.empty() && A.size() == B.size() && A.size() == starts.size() && A.size() <= ferrl::kMaxLoraParts, "lora_pack: 1 to 8 parts");
+  ferrl::LoraParts p{};
+  p.n = static_cast<int>(A.size()); p.r = static_cast<int>(A[0].size(0)); p.K = static_cast<int>(A[0].size(1)); p.N = static_cast<int>(N);
+  p.Rp = (p.n * p.r + 7) / 8 * 8; p.scale = static_cast<float>(scale);
+  for (int j = 0; j < p.n; ++j) {
+    TORCH_CHECK(A[j].is_cuda() && B[j].is_cuda() && A[j].scalar_type() == at::kFloat && B[j].scalar_type() == at::kFloat && A[j].is_contiguous() &&
+                    B[j].is_contiguous() && A[j].dim() == 2 && B[j].dim() == 2 && A[j].size(0) == p.r && A[j].size(1) == p.K && B[j].size(1) == p.r &&
+                    starts[j] >= 0 && starts[j] + B[j].size(0) <= N, "lora_pack: contiguous f32 A [r,K], B [rows,r] inside the output");
+    p.A[j] = A[j].data_ptr<float>(); p.B[j] = B[j].data_ptr<float>();
+    p.start[j] = static_cast<int>(starts[j]); p.rows[j] = static_cast<int>(B[j].size(0));
+  }
+  c10::cuda::CUDAGuard guard(A[0].device());
+  Tensor a16 = out_empty({p.Rp, p.K}, A[0].options().dtype(at::kBFloat16)), b16 = out_empty({N, p.Rp}, A[0].options().dtype(at::kBFloat16));
+  FERRL_CHECK(ferrl::lora_pack(p, a16.data_ptr(), b16.data_ptr(), stream()));
+  return {a16, b16};
+}
+
+// dbt [>= n r, N] f32, the transposed gradient of lora_pack's second result before the scale -> dB_j [rows_j,r]
+std::vector<Tensor> lora_unpack(const Tensor& dbt, std::vector<int64_t> starts, std::vector<int64_t> rows, int64_t r, double scale) {
+  TORCH_CHECK(dbt.is_cuda() && dbt.scalar_type() == at::kFloat && dbt.dim() == 2 && dbt.stride(1) == 1 && starts.size() == rows.size() &&
+                  starts.size() <= ferrl::kMaxLoraParts && dbt.size(0) >= static_cast<int64_t>(starts.size()) * r, "lora_unpack: f32 [R,N]");
+  ferrl::LoraParts p{};
+  p.n = static_cast<int>(starts.size()); p.r = static_cast<int>(r); p.scale = static_cast<float>(scale);
+  long long at = 0;
+  for (int j = 0; j < p.n; ++j) {
+    TORCH_CHECK(starts[j] >= 0 && rows[j] >= 0 && starts[j] + rows[j] <= dbt.size(1), "lora_unpack: parts inside the output");
+    p.start[j] = static_cast<int>(starts[j]); p.rows[j] = static_cast<int>(rows[j]); p.off[j] = at;
+    at += (rows[j] * r + 63) / 64 * 64;                   // every part starts on 256 bytes
+  }
+  c10::cuda::CUDAGuard guard(dbt.device());
+  Tensor out = out_empty({at}, dbt.options());
+  FERRL_CHECK(ferrl::lora_unpack(dbt.data_ptr<float>(), dbt.stride(0), p, out.data_ptr<float>(), stream()));
+  std::vector<Tensor> parts;
+  for (int j = 0; j < p.n; ++j) parts.push_back(out.narrow(0, p.off[j], rows[j] * r).view({rows[j], r}));
+  return parts;
+}
+
 // rows of a gate: contiguous, or [n, per, H] whose heads are packed in rows of a wider matrix
 struct GateRows {
   int per = 1;
@@ -1987,6 +2026,8 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("moe_pair_dot(Tensor dy, Tensor ys, Tensor row_of, int k) -> Tensor", &moe_pair_dot);
   m.def("kernel_status() -> int", &kernel_status);
   m.def("reset_status() -> ()", &reset_status);
+  m.def("lora_pack(Tensor[] A, Tensor[] B, int[] starts, int N, float scale) -> (Tensor, Tensor)", &lora_pack);
+  m.def("lora_unpack(Tensor dbt, int[] starts, int[] rows, int r, float scale) -> Tensor[]", &lora_unpack);
   m.def("rmsnorm(Tensor x, Tensor? res, Tensor? w, Tensor? gate, float eps, bool zc) -> (Tensor, Tensor)", &rmsnorm);
   m.def("rmsnorm_bwd(Tensor x, Tensor? w, Tensor dy, float eps, bool zc) -> Tensor", &rmsnorm_bwd);
   m.def("qk_norm_rope_fwd(Tensor q, Tensor k, Tensor? qw, Tensor? kw, Tensor cos, Tensor sin, Tensor pos, int pos_div, float eps, bool zc) -> (Tensor, Tensor)", &qk_norm_rope_fwd);

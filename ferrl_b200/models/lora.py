@@ -283,6 +283,12 @@ class FusedLoraLinear(nn.Module):
 
     # --------------------------------------------------------------- forward
     def forward(self, x: torch.Tensor, residual=None) -> torch.Tensor:
+        if self.bias is None and self.shard is None and self.enabled and self.has_adapters() and ops.native(x):
+            from ..ops import cuda as _c
+            starts = [sum(self.out_sizes[:i]) for i in self.adapted_idx]
+            y = _c.lora_linear_parts(x, self.weight, self.weight_t, list(self.lora_A), list(self.lora_B), starts, self.scale, residual)
+            if y is not None:
+                return y
         a, b = self._stacks()
         return ops.lora_linear(x, self.weight, a, b, wt=self.weight_t, bias=self.bias, residual=residual)
 

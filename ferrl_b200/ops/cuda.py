@@ -160,6 +160,48 @@ class _LoraLinear(torch.autograd.Function):
         return dx, None, None, da, db, (dy if getattr(ctx, "res_grad", False) else None)
 
 
+class _LoraLinearParts(torch.autograd.Function):
+    """``_LoraLinear`` from the adapters themselves (``A_j`` ``[r, K]``, ``B_j`` ``[rows_j, r]``, float32): the stacked
+    operands are made, and their gradients taken apart, in one launch each."""
+
+    @staticmethod
+    def forward(ctx, x, w, wt, residual, starts, scale, n, *adapters):
+        a16, b16 = lib().lora_pack(adapters[:n], adapters[n:], starts, w.shape[0], scale)
+        x2 = x.reshape(-1, x.shape[-1])
+        if x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
+            x2 = x2.contiguous()
+        t = gemm(x2, a16)
+        res2 = None
+        if residual is not None:
+            res2 = residual.reshape(-1, w.shape[0])
+            if res2.stride(-1) != 1:
+                res2 = res2.contiguous()
+        y = gemm(x2, w, t, b16, res2)
+        ctx.save_for_backward(x2, w, wt, t, a16, b16)
+        ctx.x_shape, ctx.x_grad, ctx.res_grad = x.shape, x.requires_grad, residual is not None and residual.requires_grad
+        ctx.parts = (starts, [b.shape[0] for b in adapters[n:]], adapters[0].shape[0], scale, n)
+        return y.view(*x.shape[:-1], w.shape[0])
+
+    @staticmethod
+    def backward(ctx, dy):
+        x2, w, wt, t, a16, b16 = ctx.saved_tensors
+        starts, rows, r, scale, n = ctx.parts
+        dy2 = dy.reshape(-1, w.shape[0])
+        if not dy2.is_contiguous():
+            dy2 = dy2.contiguous()
+        u = gemm_nn(dy2, b16)
+        dx = None
+        if ctx.x_grad:
+            dx = (gemm_nn(dy2, w, u, a16) if wt is None else gemm(dy2, wt, u, a16.t().contiguous())).view(ctx.x_shape)
+        need = ctx.needs_input_grad[7:]
+        grads = [None] * (2 * n)
+        if any(need[:n]):
+            grads[:n] = _lora_grad(u, x2)[:n * r].split(r)
+        if any(need[n:]):
+            grads[n:] = lib().lora_unpack(_lora_grad(t, dy2), starts, rows, r, scale)
+        return (dx, None, None, dy if ctx.res_grad else None, None, None, None, *(g if on else None for g, on in zip(grads, need)))
+
+
 class _LoraLinearReduce(torch.autograd.Function):
     """Row-parallel projection whose tensor-parallel sum happens inside the GEMM kernel.
     Backward is the local one: the cotangent of an all-reduced value is already replicated."""
@@ -316,6 +358,17 @@ def lora_linear(x, w, a_stack, b_stack, wt=None, bias=None, residual=None):
     if residual is not None and residual.dtype != torch.bfloat16:
         return residual + _LoraLinear.apply(x, w, wt, a_stack, b_stack)
     return _LoraLinear.apply(x, w, wt, a_stack, b_stack, residual)
+
+
+def lora_linear_parts(x, w, wt, A, B, starts, scale, residual=None):
+    """``lora_linear`` with the adapters ``A``, ``B`` of the output's parts, which begin at rows ``starts``; ``None``
+    outside the kernels' domain."""
+    fits = _bf16(x) and _bf16(w) and not w.requires_grad and x.shape[-1] % 8 == 0 and 0 < len(A) <= 8
+    if not fits or (residual is not None and residual.dtype != torch.bfloat16):
+        return None
+    if any(p.dtype != torch.float32 or p.device != x.device or not p.is_contiguous() for p in (*A, *B)):
+        return None
+    return _LoraLinearParts.apply(x, w, wt, residual, starts, float(scale), len(A), *A, *B)
 
 
 def lora_merge(w, a_stack, b_stack):
