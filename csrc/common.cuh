@@ -93,6 +93,12 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
 }
 #endif
 
+// A GEMM that holds all 512 columns of an SM's tensor memory leaves less than kTmemSmemFloor of the kSmSmem bytes of shared
+// memory that two CTAs can share, and the split-k GEMM takes at least that much: its CTAs are not placed where they would
+// sit in their allocation until the running kernel ends.
+constexpr int kSmSmem = 226 * 1024;
+constexpr int kTmemSmemFloor = 36 * 1024;
+
 // cudaFuncSetAttribute values are per device: a flag that remembers "already set" must be kept per
 // device too, or a process that drives a second GPU launches there without the opt-in.  This is a
 // once-per-(call site, device) guard; devices beyond kMaxDevices simply set the attribute every time.

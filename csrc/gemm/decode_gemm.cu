@@ -67,6 +67,7 @@ static_assert(DG_LAND_OFF >= 0 && DG_LAND_OFF % 1024 == 0, "landing zone must st
 constexpr int DG_LAND_STAGE = DG_LAND_OFF / DG_B_BYTES;   // first ring stage that the landing zone overlaps (>= DG_STAGES: none)
 constexpr int DG_TMEM_COLS = 512;       // 256 columns of activations + two 64-column accumulators
 constexpr int DG_ACC_COL = DG_RES * 32; // first accumulator column
+static_assert(DG_SMEM + kTmemSmemFloor > kSmSmem, "a kernel with tensor memory of its own must not fit beside 512 columns");
 
 struct DgParams {
   int M, N, K;
@@ -211,7 +212,6 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const int my_tiles = c < p.n_tiles ? (p.n_tiles - c + p.C - 1) / p.C : 0;
   const bool work = kb_cnt > 0 && my_tiles > 0;  // a rank without k-blocks only contributes zeros to the exchange
 
-  if (threadIdx.x == 0) pdl_trigger();
   if (threadIdx.x == 0) {
     for (int i = 0; i < DG_STAGES; ++i) {
       mbar_init(&full[i], 1);
@@ -240,6 +240,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (threadIdx.x == 0) pdl_trigger();           // after the allocation: a dependent may hold tensor memory while it waits
   // Peers signal into this CTA's barriers: every CTA of the cluster must have initialised them before
   // the first exchange.  Arrive now; each role waits where it first needs it.
   dg_cluster_arrive();
