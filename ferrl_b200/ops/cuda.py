@@ -437,12 +437,20 @@ class _RmsNormGated(torch.autograd.Function):
         return dx, dg, None, None
 
 
+def _gate_in_place(gate):
+    """Heads ``[n, per, H]`` packed in the columns of a wider matrix are read where they lie.  Rows of 16-byte pieces have to
+    start on 16 bytes: from another pitch or place the kernel would go entry by entry, which costs more than a copy."""
+    H = gate.shape[-1]
+    if not (gate.dim() == 3 and gate.stride(2) == 1 and gate.stride(1) == H):
+        return False
+    return gate.dtype != torch.bfloat16 or H % 8 != 0 or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0)
+
+
 def rmsnorm_gated(x, gate, weight, eps):
     if weight.requires_grad or gate.dtype != x.dtype:
         return eager.rmsnorm_gated(x, gate, weight, eps)
     w = weight.to(x.dtype).contiguous()
-    # heads [n, per, H] packed in the columns of a wider matrix are read where they lie
-    if not (gate.dim() == 3 and gate.stride(2) == 1 and gate.stride(1) == gate.shape[2]):
+    if not _gate_in_place(gate):
         gate = gate.contiguous()
     if torch.is_grad_enabled() and (x.requires_grad or gate.requires_grad):
         return _RmsNormGated.apply(x.contiguous(), gate, w, eps)

@@ -8,6 +8,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("n,per,H,wide,off", [
     (1, 1, 8, 8, 0), (5, 13, 24, 400, 8), (64, 1, 32, 32, 0), (9, 7, 40, 283, 3), (3, 33, 64, 2200, 16),
     (257, 3, 128, 640, 128), (2, 48, 128, 6150, 6), (17, 2, 136, 300, 8), (31, 4, 256, 1024, 0), (2, 2, 264, 600, 8),
+    (6, 3, 100, 391, 3),
 ])
 def test_short_rows(n, per, H, wide, off):
     from ferrl_b200.ops import cuda as C, eager
