@@ -74,8 +74,11 @@ struct GemmArgs {
 };
 // number of partial rows ss_out needs for a call that would run with tile width bn and cluster size (1: none)
 inline int gemm_ss_parts(int N, int bn, int cluster) { return ((N + bn - 1) / bn) * (cluster > 1 ? cluster : 1); }
+// tile width, k-split over memory and k-split over a cluster that a call should take, of the forms that it does not refuse
+enum GemmRefuse { kNoPartials = 1, kNoCluster = 2, kNo32 = 4, kNo176 = 8 };
+constexpr int kStoredRows = kNo32 | kNo176;      // what B stored [K, N] refuses
 void gemm_plan(int M, int N, int K, int K2, int num_sms, int* bn_out, int* split_out, int* cluster_out,
-               double* est_out = nullptr);
+               double* est_out = nullptr, int refuse = 0);
 const char* gemm_bf16(const GemmArgs& a, cudaStream_t stream);
 int gemm_pick_bn(int M, int N, int num_sms);
 

@@ -311,6 +311,13 @@ Tensor gemm_nn(const Tensor& A, const Tensor& B, const optional<Tensor>& A2, con
   return out;
 }
 
+// -> [tile width, k-split over memory, k-split over a cluster]
+std::vector<int64_t> gemm_plan(int64_t M, int64_t N, int64_t K, int64_t K2, int64_t sms, bool nn) {
+  int bn = 0, split = 1, cluster = 1;
+  ferrl::gemm_plan(M, N, K, K2, sms, &bn, &split, &cluster, nullptr, nn ? ferrl::kStoredRows : 0);
+  return {bn, split, cluster};
+}
+
 // act(x Wg^T) * (x Wu^T) in one kernel: W holds the gate and up rows interleaved in groups of 16
 // (8 gate rows, then the 8 up rows of the same features); returns [M, N/2].
 Tensor gemm_glu(const Tensor& A, const Tensor& B, int64_t act, bool static_b, double alpha, double limit) {
@@ -331,9 +338,8 @@ Tensor gemm_glu(const Tensor& A, const Tensor& B, int64_t act, bool static_b, do
   a.glu_alpha = alpha; a.glu_limit = limit;
   a.pdl = (static_b && a.M <= 256) ? 1 : 0;
   int bn = 0, split = 1, cluster = 1;
-  ferrl::gemm_plan(a.M, a.N, a.K, 0, a.num_sms, &bn, &split, &cluster, nullptr);
-  if (split > 1 || cluster > 1 || bn == 32) bn = 128;      // the epilogue needs whole tiles in one CTA
-  a.force_bn = bn;
+  ferrl::gemm_plan(a.M, a.N, a.K, 0, a.num_sms, &bn, &split, &cluster, nullptr, ferrl::kNoPartials | ferrl::kNoCluster | ferrl::kNo32);
+  a.force_bn = bn;                                         // the epilogue needs whole tiles in one CTA
   if (a.M == 0) return out;
   FERRL_CHECK(ferrl::gemm_bf16(a, stream()));
   return out;
@@ -372,11 +378,8 @@ std::tuple<Tensor, Tensor> gemm_norm(const Tensor& A, const Tensor& B, const opt
     a.ss_inv_k = 1.0f / static_cast<float>(a.K); a.ss_eps = static_cast<float>(eps);
   }
   int bn = 0, split = 1, cluster = 1;
-  ferrl::gemm_plan(a.M, a.N, a.K, 0, a.num_sms, &bn, &split, &cluster, nullptr);
-  if (glu_act >= 0 || cluster <= 1) {
-    if (split > 1 || cluster > 1 || bn == 32) bn = 128;      // whole tiles in one CTA
-    cluster = 1;
-  }
+  ferrl::gemm_plan(a.M, a.N, a.K, 0, a.num_sms, &bn, &split, &cluster, nullptr,
+                   ferrl::kNoPartials | ferrl::kNo32 | (glu_act >= 0 ? ferrl::kNoCluster : 0));      // with GLU whole tiles in one CTA
   a.force_bn = bn;
   a.cluster_k = cluster > 1 ? cluster : 0;
   Tensor ss_out;
@@ -1995,6 +1998,7 @@ void add_launches(int64_t n) { ferrl::count_launch(static_cast<int>(n)); }
 }  // namespace
 
 TORCH_LIBRARY(ferrl_b200, m) {
+  m.def("gemm_plan(int M, int N, int K, int K2=0, int sms=148, bool nn=False) -> int[]", &gemm_plan);
   m.def("gemm_nn(Tensor a, Tensor b, Tensor? a2=None, Tensor? b2=None) -> Tensor", &gemm_nn);
   m.def("gemm(Tensor A, Tensor B, Tensor? A2, Tensor? B2, Tensor? residual, bool out_f32, int force_bn, int force_split, int two_cta=0, Tensor? debug=None, int cluster_k=0, int stream_k=0, bool static_b=False) -> Tensor", &gemm);  // two_cta: 0 auto, -1 never, 128/256 forced
   m.def("decode_gemm(Tensor A, Tensor B, Tensor? residual=None, int glu_act=-1, int max_clusters=0, bool static_b=False, Tensor? debug=None) -> Tensor", &decode_gemm);

@@ -32,6 +32,36 @@ def test_few_rows(M, N, K):
         _close(C.gemm(a, b, force_bn=bn), ref, scale)
 
 
+@pytest.mark.no_canary
+@pytest.mark.parametrize("M,N,K", [(100, 768, 64), (16, 1024, 256), (1, 64, 131072), (128, 96, 32768), (64, 64, 12288), (256, 256, 32768), (48, 2048, 32768),
+                                   (64, 1536, 1024), (16, 5120, 5120), (128, 24576, 4096), (128, 16, 17408), (300, 128, 1024), (1500, 96, 1024), (1000, 16, 17408)])
+def test_planned_form_is_near_the_fastest(M, N, K):
+    """Forms differ up to five times; the plan's model is within 12 % of the fastest over all but one shape in twenty, which the
+    bound doubles, plus a microsecond of noise."""
+    from ferrl_b200.ops import cuda as C
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    a, ws = _rnd(gen, M, K), [_rnd(gen, N, K, std=K ** -0.5) for _ in range(max(3, min(16, (160 << 20) // (N * K * 2))))]
+
+    def us(**form):
+        for _ in range(2):
+            [C.gemm(a, w, **form) for w in ws]
+        g, ts = torch.cuda.CUDAGraph(), []
+        with torch.cuda.graph(g):
+            [C.gemm(a, w, **form) for w in ws]
+        for _ in range(7):
+            x, y = torch.cuda.Event(True), torch.cuda.Event(True)
+            x.record()
+            g.replay()
+            y.record()
+            torch.cuda.synchronize()
+            ts.append(x.elapsed_time(y) * 1e3 / len(ws))
+        return sorted(ts)[3]
+    forms = [dict(force_bn=bn) for bn in (32, 64, 128, 256) if bn <= 64 or N > bn // 2]
+    forms += [dict(force_bn=bn, cluster_k=cl) for bn, cl in ((64, 2), (64, 4), (128, 2), (128, 4), (128, 8), (256, 2)) if (bn == 64 or N > bn // 2) and K >= 64 * cl]
+    forms += [dict(force_bn=bn, force_split=sp) for bn in (64, 128, 256) for sp in (4, 8, 16) if M <= 256 and N > bn // 2 and K >= 256 * sp]
+    assert us() <= 1.25 * min(us(**f) for f in forms) + 1.0
+
+
 def test_chain_of_dependent_launches():
     """Kernels that start beside their predecessors (short rings leave room) give what they give one by one."""
     from ferrl_b200.ops import cuda as C
