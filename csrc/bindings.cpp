@@ -282,7 +282,7 @@ Tensor gemm(const Tensor& A, const Tensor& B, const optional<Tensor>& A2, const 
 }
 
 // A [M,K] @ B [K,N] (+ A2 [M,K2] @ B2 [K2,N]) with B and B2 as they lie in memory: the input gradient of a projection
-// reads its [N,K] weight without a transposed copy.  Rules of choice as in gemm().
+// reads its [N,K] weight without a transposed copy.  Rules of choice as in gemm(), among the forms that take B so.
 Tensor gemm_nn(const Tensor& A, const Tensor& B, const optional<Tensor>& A2, const optional<Tensor>& B2) {
   TORCH_CHECK(A.is_cuda() && B.is_cuda() && A.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16 && A.dim() == 2 &&
                   B.dim() == 2 && A.size(1) == B.size(0) && A.stride(1) == 1 && B.stride(1) == 1, "gemm_nn: A [M,K], B [K,N] bf16");
@@ -299,13 +299,19 @@ Tensor gemm_nn(const Tensor& A, const Tensor& B, const optional<Tensor>& A2, con
   Tensor out = out_empty({a.M, a.N}, A.options());
   a.out = out.data_ptr(); a.ldo = a.N;
   a.status = status_word(); a.num_sms = num_sms();
+  Tensor partial;
   if (a.M >= 1024 && a.N >= 512) {
     a.two_cta = 256;
   } else {
     int bn = 0, split = 1, cluster = 1;
-    ferrl::gemm_plan(a.M, a.N, a.K, a.K2, a.num_sms, &bn, &split, &cluster, nullptr);
-    a.force_bn = bn == 176 ? 256 : bn < 64 ? 64 : bn;
+    ferrl::gemm_plan(a.M, a.N, a.K, a.K2, a.num_sms, &bn, &split, &cluster, nullptr, ferrl::kStoredRows);
+    a.force_bn = bn;
     if (cluster > 1) a.cluster_k = cluster;
+    if (split > 1) {
+      partial = out_empty({split, a.M, a.N}, A.options().dtype(at::kFloat));
+      a.partial = partial.data_ptr<float>();
+      a.split_k = split;
+    }
   }
   FERRL_CHECK(ferrl::gemm_bf16(a, stream()));
   return out;
