@@ -74,7 +74,7 @@ gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
   float* A = reinterpret_cast<float*>(sm8 + 2 * GC * GD * 2);
   float* Ts = A + GC * LA;
   float *Gs = Ts + GC * LT, *Gl = Gs + GC, *kn = Gl + GC, *qn = kn + GC, *bs = qn + GC;
-  const int ci = blockIdx.x, hv = blockIdx.y, b = blockIdx.z;
+  const int ci = blockIdx.x % a.n, bh = blockIdx.x / a.n, b = bh / a.Hv, hv = bh % a.Hv;
   const int hk = hv / (a.Hv / a.Hk), t0 = (a.c0 + ci) * GC, n = min(GC, a.T - t0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int e = tid; e < 2 * GC * 16; e += NTH) {
@@ -131,7 +131,7 @@ gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
     }
   }
   __syncthreads();                           // kn, qn
-  const long long co = (static_cast<long long>(b) * a.Hv + hv) * a.n + ci;
+  const long long co = static_cast<long long>(bh) * a.n + ci;
   __nv_bfloat16* pc = a.pieces + co * 6 * PIECE;
 #pragma unroll
   for (int j = 0; j < 4; ++j)
@@ -456,7 +456,7 @@ const char* gdn_chunk_fwd(const void* q, const void* k, const void* v, long long
     a.n = std::min(round, chunks - c0);
     a.vec = reinterpret_cast<float*>(a.pieces + static_cast<long long>(B) * Hv * a.n * 6 * PIECE);
     const float* from = c0 == 0 ? S0 : S_out;
-    gdn_chunk_prep_kernel<<<dim3(a.n, Hv, B), NTH, kPrepSmem, stream>>>(a, l2norm ? 1 : 0, eps);
+    gdn_chunk_prep_kernel<<<a.n * B * Hv, NTH, kPrepSmem, stream>>>(a, l2norm ? 1 : 0, eps);
     if (narrow) gdn_chunk_scan_kernel<32><<<B * Hv * 4, NTH, scan_smem<32>(), stream>>>(a, from, S_out, static_cast<__nv_bfloat16*>(out));
     else gdn_chunk_scan_kernel<64><<<B * Hv * 2, NTH, scan_smem<64>(), stream>>>(a, from, S_out, static_cast<__nv_bfloat16*>(out));
     count_launch(2);

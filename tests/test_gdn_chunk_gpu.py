@@ -45,3 +45,16 @@ def test_chunks_match_the_recurrence(B, T, Hk, Hv, state, l2norm, wide):
     assert bool(((o - ro).abs() <= 2 ** -8 * ro.abs() + 2e-5 * ro.abs().max()).all())
     again = Cc.gdn_chunk_fwd(q, k, v, g, beta, S0, l2norm, 1e-6)
     assert torch.equal(again[0], o) and torch.equal(again[1], S)
+
+
+def test_more_rows_than_a_grid_has_in_its_last_dimension():
+    from ferrl_b200.ops import cuda as Cc
+    B = 65536
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(B, 1, 1, 128, generator=gen, device="cuda").bfloat16() for _ in range(3))
+    g, beta = -torch.rand(B, 1, 1, generator=gen, device="cuda"), torch.rand(B, 1, 1, generator=gen, device="cuda")
+    o, S = Cc.gdn_chunk_fwd(q, k, v, g, beta, None, True, 1e-6)
+    for at in (slice(0, 3), slice(B - 3, B)):
+        ro, rS = recurrence(q[at], k[at], v[at], g[at], beta[at], None, True)
+        assert float((S[at] - rS).norm() / rS.norm()) < 5e-6
+        assert bool(((o[at] - ro).abs() <= 2 ** -8 * ro.abs() + 2e-5 * ro.abs().max()).all())
