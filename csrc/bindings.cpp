@@ -735,7 +735,7 @@ std::tuple<Tensor, Tensor> gdn_chunk_fwd(const Tensor& q_, const Tensor& k_, con
   }
   Tensor out = out_empty({B, T, Hv, VD}, q.options());
   Tensor S = out_empty({B, Hv, KD, VD}, q.options().dtype(at::kFloat));
-  Tensor ws = at::empty({static_cast<int64_t>(ferrl::gdn_chunk_workspace(B, T, Hv))}, q.options().dtype(at::kByte));
+  Tensor ws = out_empty({static_cast<int64_t>(ferrl::gdn_chunk_workspace(B, T, Hv))}, q.options().dtype(at::kByte));
   FERRL_CHECK(ferrl::gdn_chunk_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), q.stride(1), k.stride(0),
                                    k.stride(1), v.stride(0), v.stride(1), g.data_ptr<float>(), beta.data_ptr<float>(), s0,
                                    S.data_ptr<float>(), out.data_ptr(), B, T, Hk, Hv, KD, VD, l2norm,

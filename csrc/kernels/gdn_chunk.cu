@@ -20,7 +20,7 @@
 // One CTA per head with everything in 32-bit multiply-adds was bound by them and by its serial chain, on 48 SMs for 48
 // heads: 5119 tokens x 48 heads 5057 -> 722 us, 4 x 2047 x 48 4053 -> 958 us, 1024 x 16 966 -> 95 us.  The state is now
 // 1.1e-7 to 1.8e-7 off float64 (2-norm), 1.7e-7 to 6.9e-7 before.  What bounds the scan is issuing the warp-level products
-// and their fragments (five barriers a chunk, 9 us a chunk for 64 columns); 16-bit pieces of a third the size would halve it and
+// and their fragments (four barriers a chunk, 9 us a chunk for 64 columns); 16-bit pieces of a third the size would halve it and
 // lose the last eight bits of every sum.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -423,8 +423,8 @@ constexpr size_t kChunkBytes = 6 * PIECE * 2 + VEC * GC * sizeof(float);      //
 
 }  // namespace
 
-// Chunks of every row that go through the two kernels together: 256 MB of pieces (at least one chunk); a longer sequence
-// takes several rounds, the state carried between them.
+// Chunks of every row that go through the two kernels together: 256 MB of pieces, or one chunk of every row and head (50 KB each)
+// where that is more; a longer sequence takes several rounds, the state carried between them.
 static int chunk_round(int B, int T, int Hv) {
   const long long chunks = (T + GC - 1) / GC, heads = std::max(1LL, static_cast<long long>(B) * Hv);
   return static_cast<int>(std::max(1LL, std::min(chunks, (256LL << 20) / (heads * static_cast<long long>(kChunkBytes)))));

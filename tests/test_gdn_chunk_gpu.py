@@ -58,3 +58,14 @@ def test_more_rows_than_a_grid_has_in_its_last_dimension():
         ro, rS = recurrence(q[at], k[at], v[at], g[at], beta[at], None, True)
         assert float((S[at] - rS).norm() / rS.norm()) < 5e-6
         assert bool(((o[at] - ro).abs() <= 2 ** -8 * ro.abs() + 2e-5 * ro.abs().max()).all())
+
+
+def test_scratch_is_guarded():
+    """Canary mode keeps every buffer that kernels write until it is checked: the chunk factors' scratch is one of them."""
+    from ferrl_b200.ops import cuda as Cc
+    q, k, v = (torch.randn(1, 640, 4, 128, device="cuda").bfloat16() for _ in range(3))
+    g, beta = -torch.rand(1, 640, 4, device="cuda"), torch.rand(1, 640, 4, device="cuda")
+    before = torch.cuda.memory_allocated()
+    out = Cc.gdn_chunk_fwd(q, k, v, g, beta, None, True, 1e-6)
+    pieces = 10 * 4 * 6 * 64 * 64 * 2                                          # ten chunks of four heads, six 16-bit pieces each
+    assert torch.cuda.memory_allocated() - before >= pieces + sum(t.numel() * t.element_size() for t in out)
