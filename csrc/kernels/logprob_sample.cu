@@ -162,6 +162,7 @@ constexpr int SRES = 3;        // CTAs on an SM
 constexpr int SCL = 8;         // CTAs of a cluster at most
 constexpr int SEG = 8;         // segments of the general cut
 constexpr int BINS = 256;      // bins of a refinement
+constexpr int AHEAD = 4;       // groups of a lane in flight in the last walk
 constexpr int KLO = (127 - 9) << 7, KN = 18 * 128;   // 16-bit magnitudes from 2^-9 to 2^9: first pattern, how many
 constexpr int KPT = 2 * KN / ST;                     // counters of a thread
 constexpr int TINY = 1024;     // values below 2^-9 that a CTA lists
@@ -186,7 +187,7 @@ static_assert(KPT * ST == 2 * KN && KPT * (ST / 2) == KN, "a thread's counters h
 // 128 rows of 151936 bf16 logits, top-p 0.95: 171 -> 68 us (one CTA of 1024 threads per row, three shared atomics per
 // element and digit before; shared atomics still bound it, 17 cycles a warp, the bytes would take 6 us; without counters,
 // by the general path, 270 us).  float32: 339 -> 168 us.  One row of 151936: 168 -> 27 us.
-template <typename T, bool VEC>
+template <typename T, bool VEC, bool CUT>
 __global__ void __launch_bounds__(ST, SRES)
 sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* __restrict__ global_rows,
                    uint64_t seed, const int* __restrict__ draw_dev, int draw_host, long long* __restrict__ tok_out,
@@ -242,9 +243,10 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
   auto plus = [](u64 a, u64 b) { return a + b; };
 
   unsigned int *counts_top = counts + KN - 1, *counts_mid = counts + KN;    // of -2^-9 and 2^-9
+  constexpr bool counted = K16 && CUT;      // without a cut the sum of the masses is all that is wanted
 
-  // 1. the row's maximum, and for 16-bit logits the counts of its values
-  if (K16) {
+  // 1. the row's maximum, and for 16-bit logits that are cut the counts of their values
+  if (counted) {
     for (int i = tid; i < 2 * KN; i += ST) counts[i] = 0;
     if (tid == 0) n_tiny = large = 0;
     __syncthreads();
@@ -260,7 +262,7 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (gb + u * ST < G) {
-        if (!K16) {
+        if (!counted) {
           const T* e = reinterpret_cast<const T*>(&raw[u]);
 #pragma unroll
           for (int k = 0; k < EPT; ++k) m = fmaxf(m, to_f(e[k]));
@@ -291,8 +293,8 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
         }
       }
   }
-  if (K16) m = fmaxf(__low2float(m2), __high2float(m2));
-  if (K16 && big) large = 1;
+  if (counted) m = fmaxf(__low2float(m2), __high2float(m2));
+  if (counted && big) large = 1;
   m = block_max(m, red);
   if (tid == 0) row_max = m;
   cluster.sync();
@@ -320,13 +322,12 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
   };
   const int gpw = ((G + SW - 1) / SW + 31) / 32 * 32;                      // groups of a warp, in vocabulary order
   const int w0 = min(G, warp * gpw), w1 = min(G, w0 + gpw);
-  const bool nucleus = top_p > 0.f && top_p < 1.f;
 
   unsigned int thresh_key = 0;              // keep everything
   u64 Z = 0, kept_mass = 0;
   u64 mine = 0;                             // kept mass of this CTA
-  bool general = !K16;
-  if (K16) {
+  bool general = !counted;
+  if (counted) {
     // a thread's KPT counters hold neighbouring values, highest first over the threads
     auto slot = [&](int i) { return 2 * KN - 1 - (tid * KPT + i); };
     auto value = [&](int s) {
@@ -386,24 +387,21 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
       const u64 parts = lane < CL ? *cluster.map_shared_rank(&segs[0], lane) : 0;
       const u64 small = warp_total(lane < CL ? *cluster.map_shared_rank(&segs[1], lane) : 0);
       Z = warp_total(parts) + small;
-      kept_mass = Z;
-      if (nucleus) {
-        const u64 target = static_cast<u64>(static_cast<double>(Z) * static_cast<double>(top_p));
-        u64 cum = warp_total(lane < rank ? parts : 0) + incl - sum;
-        if (cum + sum + small >= target)
-          for (int i = i0; i < i1; ++i) {
-            const u64 c = cum + (p0 + i >= KN ? small : 0), f = mass_at(i);      // the small values lie before the negative ones
-            if (c < target && c + f >= target) {                                // in one thread of the cluster at most
-              sel_u64[0] = c + f;
-              sel_u32 = key_of(value(2 * KN - 1 - p0 - i), 0.f);
-            }
-            cum += f;
+      const u64 target = static_cast<u64>(static_cast<double>(Z) * static_cast<double>(top_p));
+      u64 cum = warp_total(lane < rank ? parts : 0) + incl - sum;
+      if (cum + sum + small >= target)
+        for (int i = i0; i < i1; ++i) {
+          const u64 c = cum + (p0 + i >= KN ? small : 0), f = mass_at(i);        // the small values lie before the negative ones
+          if (c < target && c + f >= target) {                                  // in one thread of the cluster at most
+            sel_u64[0] = c + f;
+            sel_u32 = key_of(value(2 * KN - 1 - p0 - i), 0.f);
           }
-        cluster.sync();
-        thresh_key = gather(&sel_u32, [](unsigned int a, unsigned int b) { return max(a, b); });
-        kept_mass = gather(&sel_u64[0], [](u64 a, u64 b) { return max(a, b); });
-        general = thresh_key == 0;                       // among the small values (or nothing at all to cut)
-      }
+          cum += f;
+        }
+      cluster.sync();
+      thresh_key = gather(&sel_u32, [](unsigned int a, unsigned int b) { return max(a, b); });
+      kept_mass = gather(&sel_u64[0], [](u64 a, u64 b) { return max(a, b); });
+      general = thresh_key == 0;                         // among the small values (or nothing at all to cut)
       if (!general) {
 #pragma unroll
         for (int i = 0; i < KPT; ++i) {
@@ -425,32 +423,44 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
     }
   }
   if (general) {
-    // 2. masses by segment (all in the first one where nothing is cut)
+    // 2. masses by segment, of a row that is not cut by warp
+    if (CUT) {
 #pragma unroll
-    for (int s = 0; s < SEG; ++s) priv[s * ST + tid] = 0;
-    for (int g = w0 + lane; g < w1; g += 32) {
-      float v[EPT];
-      group(g, v);
-      if (nucleus) {
+      for (int s = 0; s < SEG; ++s) priv[s * ST + tid] = 0;
+      for (int g = w0 + lane; g < w1; g += 32) {
+        float v[EPT];
+        group(g, v);
 #pragma unroll
         for (int k = 0; k < EPT; ++k) {
           const float e = e_val(v[k]);
           priv[seg_of(v[k], e) * ST + tid] += fix_of(e);
         }
-      } else {
-        u64 part = 0;
-#pragma unroll
-        for (int k = 0; k < EPT; ++k) part += fix_of(e_val(v[k]));
-        priv[tid] += part;
       }
-    }
-    __syncthreads();
-    for (int s = warp; s < SEG; s += SW) {
-      u64 t = 0;
+      __syncthreads();
+      for (int s = warp; s < SEG; s += SW) {
+        u64 t = 0;
 #pragma unroll
-      for (int i = 0; i < ST / 32; ++i) t += priv[s * ST + i * 32 + lane];
+        for (int i = 0; i < ST / 32; ++i) t += priv[s * ST + i * 32 + lane];
+        t = warp_total(t);
+        if (lane == 0) segs[s] = t;
+      }
+    } else {
+      u64 t = 0;
+#pragma unroll 4
+      for (int g = w0 + lane; g < w1; g += 32) {
+        float v[EPT];
+        group(g, v);
+#pragma unroll
+        for (int k = 0; k < EPT; ++k) t += fix_of(e_val(v[k]));
+      }
       t = warp_total(t);
-      if (lane == 0) segs[s] = t;
+      if (lane == 0) wmass[warp] = t;
+      __syncthreads();
+      if (tid < SEG) {
+        t = 0;
+        for (int w = 0; w < SW; ++w) t += tid == 0 ? wmass[w] : 0;
+        segs[tid] = t;
+      }
     }
     if (tid < 2) range_sh[tid] = tid == 0 ? 0xFFFFFFFFu : 0u;
     cluster.sync();
@@ -464,7 +474,7 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
         const u64 p = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += p;
       }
-      if (nucleus) {
+      if (CUT) {
         target = static_cast<u64>(static_cast<double>(Z) * static_cast<double>(top_p));
         const unsigned int hit = __ballot_sync(0xffffffffu, t > 0 && incl >= target);
         cut = hit ? __ffs(hit) - 1 : SEG;
@@ -623,40 +633,47 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
     return t;
   };
   float v[EPT];
-  {
+  if (CUT) {                            // those of a row that is not cut are known
     u64 t = 0;
+#pragma unroll 4
     for (int g = w0 + lane; g < w1; g += 32) t += group_mass(g, v);
     t = warp_total(t);
     if (lane == 0) wmass[warp] = t;
+    __syncthreads();
   }
-  __syncthreads();
   for (int w = 0; w < warp; ++w) before += wmass[w];
   if (point < before || point >= before + wmass[warp]) return;
-  for (int gb = w0; gb < w1; gb += 32) {    // one warp is left; a step is 32 neighbouring groups
-    const u64 t = gb + lane < w1 ? group_mass(gb + lane, v) : 0;
-    u64 incl = t;
-    for (int o = 1; o < 32; o <<= 1) {
-      const u64 p = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += p;
-    }
-    const unsigned int hit = __ballot_sync(0xffffffffu, before + incl > point);
-    if (hit) {
-      if (lane == __ffs(hit) - 1) {
-        u64 cum = before + incl - t;
-        int pick = -1;
+  for (int gb = w0; gb < w1; gb += 32 * AHEAD) {       // one warp is left; a step is 32 neighbouring groups, AHEAD of them loaded at a time
+    u64 t[AHEAD];
 #pragma unroll
-        for (int k = 0; k < EPT; ++k) {
-          const float e = e_val(v[k]);
-          if (pick < 0 && key_of(v[k], e) >= thresh_key) {
-            cum += fix_of(e);
-            if (cum > point) pick = (g0 + gb + lane) * EPT + k;
-          }
-        }
-        emit(pick);
+    for (int u = 0; u < AHEAD; ++u) t[u] = gb + 32 * u + lane < w1 ? group_mass(gb + 32 * u + lane, v) : 0;
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      u64 incl = t[u];
+      for (int o = 1; o < 32; o <<= 1) {
+        const u64 p = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += p;
       }
-      return;
+      const unsigned int hit = __ballot_sync(0xffffffffu, before + incl > point);
+      if (hit) {
+        if (lane == __ffs(hit) - 1) {
+          u64 cum = before + incl - t[u];
+          int pick = -1;
+          group(gb + 32 * u + lane, v);
+#pragma unroll
+          for (int k = 0; k < EPT; ++k) {
+            const float e = e_val(v[k]);
+            if (pick < 0 && key_of(v[k], e) >= thresh_key) {
+              cum += fix_of(e);
+              if (cum > point) pick = (g0 + gb + 32 * u + lane) * EPT + k;
+            }
+          }
+          emit(pick);
+        }
+        return;
+      }
+      before += __shfl_sync(0xffffffffu, incl, 31);
     }
-    before += __shfl_sync(0xffffffffu, incl, 31);
   }
 }
 
@@ -748,11 +765,11 @@ const char* logprob_rows_bwd(int dtype, void* logits, long long ld, const long l
 }
 
 namespace {
-template <typename T, bool VEC>
+template <typename T, bool VEC, bool CUT>
 const char* sample_launch(const void* logits, long long ld, const long long* global_rows, unsigned long long seed, const int* draw_dev,
                           int draw_host, long long* tok_out, float* lp_out, int rows, int V, float inv_t, float top_p, cudaStream_t s) {
   constexpr size_t kDyn = std::max(SEG * ST * sizeof(unsigned long long), (4 * KN + TINY) * sizeof(unsigned int));
-  if (!FERRL_ONCE_PER_DEVICE(cudaFuncSetAttribute(sample_rows_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (!FERRL_ONCE_PER_DEVICE(cudaFuncSetAttribute(sample_rows_kernel<T, VEC, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   static_cast<int>(kDyn)) == cudaSuccess))
     return "sample_rows: cannot reserve shared memory";
   // Clusters that give each SM two or three CTAs (one alone waits on its own barriers: 128 rows of 151936 bf16 logits take
@@ -770,7 +787,7 @@ const char* sample_launch(const void* logits, long long ld, const long long* glo
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, sample_rows_kernel<T, VEC>, static_cast<const T*>(logits), ld, global_rows,
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, sample_rows_kernel<T, VEC, CUT>, static_cast<const T*>(logits), ld, global_rows,
                                            static_cast<uint64_t>(seed), draw_dev, draw_host, tok_out, lp_out, V, inv_t, top_p);
   count_launch();
   return e == cudaSuccess ? nullptr : "sample_rows launch failed";
@@ -784,10 +801,15 @@ const char* sample_rows(int dtype, const void* logits, long long ld, const long 
   const float inv_t = 1.f / temperature;
   const int per = dtype == kF32 ? 4 : 8;
   const bool vec = V % per == 0 && ld % per == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
-#define FERRL_SAMPLE(T, VEC) \
-  sample_launch<T, VEC>(logits, ld, global_rows, seed, draw_dev, draw_host, tok_out, lp_out, rows, V, inv_t, top_p, s)
-  if (dtype == kF32) return vec ? FERRL_SAMPLE(float, true) : FERRL_SAMPLE(float, false);
-  return vec ? FERRL_SAMPLE(__nv_bfloat16, true) : FERRL_SAMPLE(__nv_bfloat16, false);
+  const bool cut = top_p > 0.f && top_p < 1.f;          // rows without a cut want no more than their sum
+#define FERRL_SAMPLE(T, VEC, CUT) \
+  sample_launch<T, VEC, CUT>(logits, ld, global_rows, seed, draw_dev, draw_host, tok_out, lp_out, rows, V, inv_t, top_p, s)
+  if (dtype == kF32) {
+    if (vec) return cut ? FERRL_SAMPLE(float, true, true) : FERRL_SAMPLE(float, true, false);
+    return cut ? FERRL_SAMPLE(float, false, true) : FERRL_SAMPLE(float, false, false);
+  }
+  if (vec) return cut ? FERRL_SAMPLE(__nv_bfloat16, true, true) : FERRL_SAMPLE(__nv_bfloat16, true, false);
+  return cut ? FERRL_SAMPLE(__nv_bfloat16, false, true) : FERRL_SAMPLE(__nv_bfloat16, false, false);
 #undef FERRL_SAMPLE
 }
 
