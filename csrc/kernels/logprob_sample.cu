@@ -302,6 +302,7 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
 
   auto e_val = [&](float xv) -> float { return __expf((xv - m) * inv_t); };   // exp(-inf) = 0 for padding
   auto fix_of = [&](float e) -> u64 { return static_cast<u64>(fmaxf(e, 0.f) * FIX); };    // NaN has no mass
+  constexpr float kLeast = 9.094947017729282e-13f;      // 2^-40, the least with a mass: masked entries cost no more than their load
   // The order of the cut: for 16-bit logits the sortable pattern of the logit itself (it orders as the probability
   // does), for 32-bit ones the pattern of the unnormalised probability.
   auto key_of = [&](float xv, float e) -> unsigned int {
@@ -492,8 +493,8 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
         group(g, v);
 #pragma unroll
         for (int k = 0; k < EPT; ++k) {
-          const float e = K16 ? 0.f : e_val(v[k]);
-          if (seg_of(v[k], e) == static_cast<unsigned int>(cut)) {
+          const float e = e_val(v[k]);
+          if (e >= kLeast && seg_of(v[k], e) == static_cast<unsigned int>(cut)) {
             const unsigned int key = key_of(v[k], e);
             lo = min(lo, key);
             hi = max(hi, key);
@@ -509,7 +510,10 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
       cluster.sync();
       lo = gather(&range_sh[0], [](unsigned int a, unsigned int b) { return min(a, b); });
       hi = gather(&range_sh[1], [](unsigned int a, unsigned int b) { return max(a, b); });
-      for (int it = 0;; ++it) {
+      if (lo == hi) {                         // a segment of one key, as in a flat row
+        kept_mass = above + gather(&segs[cut], plus);
+        mine += segs[cut];
+      } else for (int it = 0;; ++it) {
         const int shift = max(0, 24 - __clz(hi - lo));                       // BINS bins cover hi - lo
         for (int i = tid; i < 4 * BINS; i += ST) planes[0][i] = 0;
         __syncthreads();
@@ -523,6 +527,7 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
             if (at <= hi - lo) {
               if (K16) e = e_val(v[k]);
               const u64 f = fix_of(e);
+              if (f == 0) continue;
               const unsigned int b = at >> shift;
               atomicAdd(&planes[0][b], static_cast<unsigned int>(f & 0x7FFu));
               atomicAdd(&planes[1][b], static_cast<unsigned int>((f >> 11) & 0x3FFu));

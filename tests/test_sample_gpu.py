@@ -87,3 +87,13 @@ def test_rows_without_a_cut_cost_less(rows, V):
     """The sum of the masses is all that they want: 53 us before rows were counted, 71 with the counts, at 128 x 151936."""
     x = _plain(rows, V, torch.bfloat16)
     assert _us(x, None) < 0.75 * _us(x, 0.95)
+
+
+@pytest.mark.no_canary
+@pytest.mark.parametrize("kind", ["masked", "flat"])
+def test_32_bit_rows_of_one_key_or_with_finite_masks_cost_no_more(kind):
+    """Entries without a mass and segments of one key need no narrowing (128 x 151936: 311 and 419 us with it, 166 a plain row)."""
+    x = _plain(128, 151936, torch.float32)
+    plain = _us(x, 0.95)
+    x = x * 0 if kind == "flat" else x.index_fill(1, torch.arange(0, 151936, 2, device="cuda"), -1e4)
+    assert _us(x, 0.95) < 1.15 * plain
