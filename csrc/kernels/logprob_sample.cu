@@ -163,18 +163,19 @@ constexpr int SCL = 8;         // CTAs of a cluster at most
 constexpr int SEG = 8;         // segments of the general cut
 constexpr int BINS = 256;      // bins of a refinement
 constexpr int AHEAD = 4;       // groups of a lane in flight in the last walk
-constexpr int KLO = (127 - 9) << 7, KN = 18 * 128;   // 16-bit magnitudes from 2^-9 to 2^9: first pattern, how many
-constexpr int KPT = 2 * KN / ST;                     // counters of a thread
-constexpr int TINY = 1024;     // values below 2^-9 that a CTA lists
-static_assert(KPT * ST == 2 * KN && KPT * (ST / 2) == KN, "a thread's counters have one sign");
+constexpr int KN = 18 * 128;   // 16-bit magnitudes that have counters: 18 octaves
+constexpr int NC = 2 * KN + 2; // counters: negative values, -0, +0, positive values, in the order of their keys
+constexpr int TINY = 1024;     // values without a counter that a CTA lists
 
 // A cluster of CTAs draws a row's token, one contiguous slice of the vocabulary each.
 //
-// 16-bit logits have few distinct values, so one pass over HBM counts them (one shared atomic per element, and
+// 16-bit logits that are cut have few distinct values, so one pass over HBM counts them (one shared atomic per element, and
 // neighbouring bins are spread over the banks); masses, the total, the nucleus cut and each CTA's share of the kept
-// mass then come from the counts alone, and only the CTA that the draw falls into walks its slice again.
-// Values outside [2^-9, 2^9) have no counter: the small ones (a fraction of a percent of a row) are listed, and a row
-// with large ones, too many small ones, or its cut among the small ones takes the general path, as 32-bit rows do:
+// mass then come from the counts alone, and only the CTA that the draw falls into walks its slice again.  The 18 octaves that
+// have counters end an octave above the largest of 4096 sampled magnitudes, which every CTA finds for itself; the sample's
+// maximum also tells which values are too small to have a mass (masks, finite ones too), and those are skipped.  What else
+// lies outside the octaves is listed, and the cut may lie among it.  A row that overflows a list (many values of another
+// order of magnitude) takes the general path, as 32-bit rows and rows without a cut do:
 //
 //   1. maximum of the row
 //   2. masses of SEG segments of the row by distance from the maximum, in columns of shared memory that belong to
@@ -199,12 +200,12 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
   __shared__ unsigned int planes[4][BINS];
   __shared__ u64 bins[2][BINS];             // this CTA's masses of a refinement; two, read by the others in turn
   __shared__ u64 segs[SEG];
-  __shared__ u64 kept_sh, wmass[SW], sel_u64[2];
+  __shared__ u64 kept_sh, wmass[SW], wlist[SW][4], sel_u64[2];
   __shared__ float row_max, red[32];
-  __shared__ unsigned int range_sh[2], sel_u32, n_tiny, large;
-  unsigned int* counts = reinterpret_cast<unsigned int*>(priv);             // [2 * KN], ascending keys
-  unsigned int* tiny = counts + 2 * KN;                                     // [TINY]
-  unsigned int* merged = tiny + TINY;                                       // [2 * KN], the counts of the whole row
+  __shared__ unsigned int range_sh[2], sel_u32, n_tiny;
+  unsigned int* counts = reinterpret_cast<unsigned int*>(priv);             // [NC], ascending keys
+  unsigned int* tiny = counts + NC;                                     // [TINY]
+  unsigned int* merged = tiny + TINY;                                       // [NC], the counts of the whole row
   cg::cluster_group cluster = cg::this_cluster();
   const int CL = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
   const long long row = blockIdx.x / CL;
@@ -242,17 +243,40 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
   };
   auto plus = [](u64 a, u64 b) { return a + b; };
 
-  unsigned int *counts_top = counts + KN - 1, *counts_mid = counts + KN;    // of -2^-9 and 2^-9
+  unsigned int *counts_top = counts + KN - 1, *counts_mid = counts + KN + 2;     // of the least magnitudes that have counters
   constexpr bool counted = K16 && CUT;      // without a cut the sum of the masses is all that is wanted
 
   // 1. the row's maximum, and for 16-bit logits that are cut the counts of their values
+  unsigned int klo = 0;                     // the least magnitude with a counter
+  float least = -INFINITY;                  // the least value that may have a mass
   if (counted) {
-    for (int i = tid; i < 2 * KN; i += ST) counts[i] = 0;
-    if (tid == 0) n_tiny = large = 0;
-    __syncthreads();
+    float v[EPT], top = -INFINITY, mag = 0.f;
+    const uint4 sample = load(static_cast<int>(static_cast<long long>(tid) * Gt / ST) - g0);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)             // on their way meanwhile
+      if (VEC && tid + u * ST < G) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint4*>(x) + g0 + tid + u * ST));
+    for (int i = tid; i < NC; i += ST) counts[i] = 0;
+    if (tid == 0) n_tiny = 0;
+#pragma unroll
+    for (int k = 0; k < EPT; ++k) {
+      v[k] = to_f(reinterpret_cast<const T*>(&sample)[k]);
+      top = fmaxf(top, v[k]);
+    }
+    auto block = [&](float x, float* at) {
+      x = warp_max(x);
+      if (lane == 0) at[warp] = x;
+      __syncthreads();
+      return warp_max(at[lane % SW]);
+    };
+    least = block(top, red) - 28.f / inv_t;                 // e^-28 < 2^-40
+#pragma unroll
+    for (int k = 0; k < EPT; ++k)
+      if (v[k] >= least && fabsf(v[k]) < INFINITY) mag = fmaxf(mag, fabsf(v[k]));
+    const int octave = static_cast<int>(__float_as_uint(block(mag, red + SW)) >> 23);
+    klo = static_cast<unsigned int>(min(max(1, (octave - 16) * 128), 0x7F80 - KN));
   }
   float m = -INFINITY;
-  bool big = false;
+  unsigned int zeros = 0;                   // +0 in the lower half, -0 in the upper
   __nv_bfloat162 m2 = __float2bfloat162_rn(-INFINITY);
   for (int gb = tid; gb < G; gb += 4 * ST) {
     uint4 raw[4];
@@ -275,7 +299,7 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
         for (int k = 0; k < 8; ++k) {
           const unsigned int w = words[k >> 1];
           if (!(k & 1)) m2 = __hmax2(m2, *reinterpret_cast<const __nv_bfloat162*>(&w));
-          const unsigned int at = ((k & 1 ? w >> 16 : w) & 0x7FFFu) - KLO;
+          const unsigned int at = ((k & 1 ? w >> 16 : w) & 0x7FFFu) - klo;
           const bool neg = (k & 1 ? w : w << 16) & 0x80000000u;
           if (at < KN) atomicAdd(neg ? counts_top - at : counts_mid + at, 1u);
           odd |= at >= KN;
@@ -283,18 +307,21 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
         if (odd) {
           for (int k = 0; k < 8; ++k) {
             const unsigned int bits = (k & 1 ? words[k >> 1] >> 16 : words[k >> 1]) & 0xFFFFu, mag = bits & 0x7FFFu;
-            if (mag < KLO) {
+            if (mag == 0) {
+              zeros += bits ? 0x10000u : 1u;
+            } else if (mag - klo >= KN && mag < 0x7F80u && __uint_as_float(bits << 16) >= least) {
               const unsigned int i = atomicAdd(&n_tiny, 1u);
               if (i < TINY) tiny[i] = bits;
-            } else if (mag >= KLO + KN) {
-              big |= bits != 0xFF80u && mag <= 0x7F80u;   // masked entries and NaN carry no mass
             }
           }
         }
       }
   }
-  if (counted) m = fmaxf(__low2float(m2), __high2float(m2));
-  if (counted && big) large = 1;
+  if (counted) {
+    m = fmaxf(__low2float(m2), __high2float(m2));
+    if (zeros & 0xFFFFu) atomicAdd(&counts[KN + 1], zeros & 0xFFFFu);
+    if (zeros >> 16) atomicAdd(&counts[KN], zeros >> 16);
+  }
   m = block_max(m, red);
   if (tid == 0) row_max = m;
   cluster.sync();
@@ -328,48 +355,52 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
   u64 Z = 0, kept_mass = 0;
   u64 mine = 0;                             // kept mass of this CTA
   bool general = !counted;
+  // a cut to narrow down: keys lo .. hi, the masses above them and those to keep, of the listed values or of the row
+  bool narrow = false, listed = false;
+  unsigned int lo = 0, hi = 0;
+  u64 target = 0, above = 0;
+  auto value = [&](int s) {                 // of counter s
+    const unsigned int b = s >= KN + 2 ? s - (KN + 2) + klo : s >= KN ? (KN + 1 - s) << 15 : (0x8000u | (KN - 1 - s + klo));
+    return __uint_as_float(b << 16);
+  };
   if (counted) {
-    // a thread's KPT counters hold neighbouring values, highest first over the threads
-    auto slot = [&](int i) { return 2 * KN - 1 - (tid * KPT + i); };
-    auto value = [&](int s) {
-      const unsigned int b = s >= KN ? static_cast<unsigned int>(s - KN + KLO) : (0x8000u | (KN - 1 - s + KLO));
-      return __uint_as_float(b << 16);
-    };
-    auto block_u64 = [&](u64 v) -> u64 {    // the sum over the CTA
-      v = warp_total(v);
-      __syncthreads();
-      if (lane == 0) wmass[warp] = v;
-      __syncthreads();
-      u64 t = 0;
-#pragma unroll
-      for (int w = 0; w < SW; ++w) t += wmass[w];
-      return t;
-    };
-    const unsigned int worst = gather(&n_tiny, [](unsigned int a, unsigned int b) { return max(a, b); });
-    general = worst > TINY || gather(&large, [](unsigned int a, unsigned int b) { return a | b; }) != 0;
+    general = gather(&n_tiny, [](unsigned int a, unsigned int b) { return max(a, b); }) > TINY;
     if (!general) {
       // This CTA merges one part of the counters, in descending order of the values: other CTAs' shared memory is read
       // a warp's width at a time, and each counter by one CTA only (64 rows of
       // 50264: 35 us; 43 with all counters merged by every CTA, 117 with a thread's strided counters read one by one).
-      const int part = (2 * KN + CL - 1) / CL, per = (part + ST - 1) / ST;
-      const int p0 = min(2 * KN, rank * part), pn = min(2 * KN - p0, part);
+      const int part = (NC + CL - 1) / CL, per = (part + ST - 1) / ST;
+      const int p0 = min(NC, rank * part), pn = min(NC - p0, part);
       for (int i = tid; i < pn; i += ST)
-        merged[i] = gather(&counts[2 * KN - 1 - p0 - i], [](unsigned int a, unsigned int b) { return a + b; });
-      u64 few = 0, sum = 0;
-      for (unsigned int i = tid; i < n_tiny; i += ST) few += fix_of(e_val(__uint_as_float(tiny[i] << 16)));
+        merged[i] = gather(&counts[NC - 1 - p0 - i], [](unsigned int a, unsigned int b) { return a + b; });
+      // The listed values are of four classes, each between counters: large positive ones before them all, small positive
+      // ones before the zeros, small negative ones behind those, large negative ones behind all.
+      u64 sum = 0;
+      {
+        u64 f[4] = {};
+        for (unsigned int i = tid; i < n_tiny; i += ST) {
+          const unsigned int bits = tiny[i], far = (bits & 0x7FFFu) >= klo, c = bits & 0x8000u ? 2 + far : 1 - far;
+          const u64 t = fix_of(e_val(__uint_as_float(bits << 16)));
+#pragma unroll
+          for (int j = 0; j < 4; ++j) f[j] += c == j ? t : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const u64 t = warp_total(f[j]);
+          if (lane == 0) wlist[warp][j] = t;
+        }
+      }
       __syncthreads();
       const int i0 = min(pn, tid * per), i1 = min(pn, i0 + per);
       auto mass_at = [&](int i) -> u64 {
-        return merged[i] ? merged[i] * fix_of(e_val(value(2 * KN - 1 - p0 - i))) : 0;
+        return merged[i] ? merged[i] * fix_of(e_val(value(NC - 1 - p0 - i))) : 0;
       };
       for (int i = i0; i < i1; ++i) sum += mass_at(i);
-      few = block_u64(few);
       u64 incl = sum;
       for (int o = 1; o < 32; o <<= 1) {
         const u64 p = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += p;
       }
-      __syncthreads();
       if (lane == 31) wmass[warp] = incl;
       __syncthreads();
       u64 whole = 0;
@@ -378,49 +409,50 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
         if (w < warp) incl += wmass[w];
         whole += wmass[w];
       }
+      if (tid < 4) {
+        u64 t = 0;
+#pragma unroll
+        for (int w = 0; w < SW; ++w) t += wlist[w][tid];
+        segs[1 + tid] = t;
+      }
       if (tid == 0) {
         segs[0] = whole;
-        segs[1] = few;
         sel_u32 = 0;
         sel_u64[0] = 0;
       }
       cluster.sync();
       const u64 parts = lane < CL ? *cluster.map_shared_rank(&segs[0], lane) : 0;
-      const u64 small = warp_total(lane < CL ? *cluster.map_shared_rank(&segs[1], lane) : 0);
-      Z = warp_total(parts) + small;
-      const u64 target = static_cast<u64>(static_cast<double>(Z) * static_cast<double>(top_p));
-      u64 cum = warp_total(lane < rank ? parts : 0) + incl - sum;
-      if (cum + sum + small >= target)
+      u64 of_class = lane < 4 * CL ? *cluster.map_shared_rank(&segs[1 + (lane & 3)], lane >> 2) : 0;
+      for (int o = 4; o < 32; o <<= 1) of_class += __shfl_xor_sync(0xffffffffu, of_class, o);
+      u64 l[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) l[j] = __shfl_sync(0xffffffffu, of_class, j);
+      Z = warp_total(parts) + l[0] + l[1] + l[2] + l[3];
+      target = max(static_cast<u64>(static_cast<double>(Z) * static_cast<double>(top_p)), u64(1));
+      u64 cum = warp_total(lane < rank ? parts : 0) + incl - sum + l[0];
+      if (cum + sum + l[1] + l[2] >= target)
         for (int i = i0; i < i1; ++i) {
-          const u64 c = cum + (p0 + i >= KN ? small : 0), f = mass_at(i);        // the small values lie before the negative ones
-          if (c < target && c + f >= target) {                                  // in one thread of the cluster at most
-            sel_u64[0] = c + f;
-            sel_u32 = key_of(value(2 * KN - 1 - p0 - i), 0.f);
+          const int d = p0 + i;
+          const u64 c = cum + (d >= KN ? l[1] : 0) + (d >= KN + 2 ? l[2] : 0), f = mass_at(i);
+          const u64 before = d == KN ? l[1] : d == KN + 2 ? l[2] : 0;            // the listed class between counter d and the last
+          if (c < target ? c + f >= target : c - before < target && before) {    // in one thread of the cluster at most
+            sel_u64[0] = c < target ? c + f : c - before;
+            sel_u32 = c < target ? key_of(value(NC - 1 - d), 0.f) : d == KN ? 1 : 2;    // no key of a finite value is 1 or 2
           }
           cum += f;
         }
       cluster.sync();
       thresh_key = gather(&sel_u32, [](unsigned int a, unsigned int b) { return max(a, b); });
       kept_mass = gather(&sel_u64[0], [](u64 a, u64 b) { return max(a, b); });
-      general = thresh_key == 0;                         // among the small values (or nothing at all to cut)
-      if (!general) {
-#pragma unroll
-        for (int i = 0; i < KPT; ++i) {
-          const int s = slot(i);
-          const float xv = value(s);
-          if (counts[s] && key_of(xv, 0.f) >= thresh_key) mine += counts[s] * fix_of(e_val(xv));
-        }
-        for (unsigned int i = tid; i < n_tiny; i += ST) {
-          const float xv = __uint_as_float(tiny[i] << 16);
-          if (key_of(xv, 0.f) >= thresh_key) mine += fix_of(e_val(xv));
-        }
-        mine = block_u64(mine);
+      if (Z > 0 && (target <= l[0] || target > Z - l[3] || thresh_key < 3)) {
+        const unsigned int end = klo + KN;
+        narrow = listed = true;
+        above = target <= l[0] ? 0 : target > Z - l[3] ? Z - l[3] : kept_mass;
+        lo = target <= l[0] ? 0x8000u | end : target > Z - l[3] ? 0x0080u : thresh_key == 1 ? 0x8001u : 0x8000u - klo;
+        hi = target <= l[0] ? 0xFF7Fu : target > Z - l[3] ? 0x7FFFu - end : thresh_key == 1 ? 0x7FFFu + klo : 0x7FFEu;
       }
-    }
-    if (general) {
+    } else {
       cluster.sync();                       // the counters give way to the columns below
-      thresh_key = 0;
-      mine = 0;
     }
   }
   if (general) {
@@ -465,7 +497,6 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
     }
     if (tid < 2) range_sh[tid] = tid == 0 ? 0xFFFFFFFFu : 0u;
     cluster.sync();
-    u64 target = 0, above = 0;
     int cut = SEG;
     {
       const u64 t = lane < SEG ? gather(&segs[lane], plus) : 0;
@@ -487,7 +518,8 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
     // 3. the cut inside its segment
     kept_mass = Z;
     if (cut < SEG) {
-      unsigned int lo = 0xFFFFFFFFu, hi = 0;
+      lo = 0xFFFFFFFFu;
+      hi = 0;
       for (int g = w0 + lane; g < w1; g += 32) {
         float v[EPT];
         group(g, v);
@@ -510,86 +542,113 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
       cluster.sync();
       lo = gather(&range_sh[0], [](unsigned int a, unsigned int b) { return min(a, b); });
       hi = gather(&range_sh[1], [](unsigned int a, unsigned int b) { return max(a, b); });
-      if (lo == hi) {                         // a segment of one key, as in a flat row
+      thresh_key = lo;
+      narrow = lo < hi;
+      if (!narrow) {                          // a segment of one key, as in a flat row
         kept_mass = above + gather(&segs[cut], plus);
         mine += segs[cut];
-      } else for (int it = 0;; ++it) {
-        const int shift = max(0, 24 - __clz(hi - lo));                       // BINS bins cover hi - lo
-        for (int i = tid; i < 4 * BINS; i += ST) planes[0][i] = 0;
-        __syncthreads();
+      }
+    }
+  }
+  if (narrow) {
+    for (int it = 0;; ++it) {
+      const int shift = max(0, 24 - __clz(hi - lo));                         // BINS bins cover hi - lo
+      for (int i = tid; i < 4 * BINS; i += ST) planes[0][i] = 0;
+      __syncthreads();
+      auto add = [&](float xv) {
+        float e = K16 ? 0.f : e_val(xv);
+        const unsigned int at = key_of(xv, e) - lo;
+        if (at > hi - lo) return;
+        if (K16) e = e_val(xv);
+        const u64 f = fix_of(e);
+        if (f == 0) return;
+        const unsigned int b = at >> shift;
+        atomicAdd(&planes[0][b], static_cast<unsigned int>(f & 0x7FFu));
+        atomicAdd(&planes[1][b], static_cast<unsigned int>((f >> 11) & 0x3FFu));
+        atomicAdd(&planes[2][b], static_cast<unsigned int>((f >> 21) & 0x3FFu));
+        atomicAdd(&planes[3][b], static_cast<unsigned int>(f >> 31));
+      };
+      if (listed) {
+        for (unsigned int i = tid; i < n_tiny; i += ST) add(__uint_as_float(tiny[i] << 16));
+      } else {
         for (int g = w0 + lane; g < w1; g += 32) {
           float v[EPT];
           group(g, v);
 #pragma unroll
-          for (int k = 0; k < EPT; ++k) {
-            float e = K16 ? 0.f : e_val(v[k]);
-            const unsigned int at = key_of(v[k], e) - lo;
-            if (at <= hi - lo) {
-              if (K16) e = e_val(v[k]);
-              const u64 f = fix_of(e);
-              if (f == 0) continue;
-              const unsigned int b = at >> shift;
-              atomicAdd(&planes[0][b], static_cast<unsigned int>(f & 0x7FFu));
-              atomicAdd(&planes[1][b], static_cast<unsigned int>((f >> 11) & 0x3FFu));
-              atomicAdd(&planes[2][b], static_cast<unsigned int>((f >> 21) & 0x3FFu));
-              atomicAdd(&planes[3][b], static_cast<unsigned int>(f >> 31));
-            }
-          }
+          for (int k = 0; k < EPT; ++k) add(v[k]);
         }
-        __syncthreads();
-        u64* own = bins[it & 1];
-        if (tid < BINS)
-          own[tid] = static_cast<u64>(planes[0][tid]) + (static_cast<u64>(planes[1][tid]) << 11) +
-                     (static_cast<u64>(planes[2][tid]) << 21) + (static_cast<u64>(planes[3][tid]) << 31);
-        cluster.sync();
-        u64* total = priv;                    // the columns of the mass pass are done with
-        if (tid < BINS) total[tid] = gather(&own[tid], plus);
-        __syncthreads();
-        if (warp == 0) {                      // from the highest key down, eight bins to a lane
-          constexpr int PER = BINS / 32;
-          u64 t[PER], s = 0;
-#pragma unroll
-          for (int i = 0; i < PER; ++i) s += t[i] = total[BINS - 1 - lane * PER - i];
-          u64 incl = s;
-          for (int o = 1; o < 32; o <<= 1) {
-            const u64 p = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += p;
-          }
-          u64 cum = above + incl - s;
-          int b = -1;
-#pragma unroll
-          for (int i = 0; i < PER; ++i)
-            if (b < 0) {
-              if (t[i] > 0 && cum + t[i] >= target) b = BINS - 1 - lane * PER - i;
-              else cum += t[i];
-            }
-          const unsigned int hit = __ballot_sync(0xffffffffu, b >= 0);
-          const int src = hit ? __ffs(hit) - 1 : 31;
-          b = max(0, __shfl_sync(0xffffffffu, b, src));
-          u64 kept = 0;                       // of this CTA, above bin b
-          for (int i = b + 1 + lane; i < BINS; i += 32) kept += own[i];
-          kept = warp_total(kept);
-          if (lane == src) {
-            sel_u64[0] = cum;
-            sel_u32 = static_cast<unsigned int>(b);
-          }
-          if (lane == 0) sel_u64[1] = kept;
-        }
-        __syncthreads();
-        above = sel_u64[0];
-        mine += sel_u64[1];
-        const unsigned int b = sel_u32;
-        lo += b << shift;
-        if (shift == 0) {
-          kept_mass = above + total[b];
-          mine += own[b];
-          break;
-        }
-        hi = min(hi, lo + (1u << shift) - 1);
-        __syncthreads();
       }
-      thresh_key = lo;
+      __syncthreads();
+      u64* own = bins[it & 1];
+      if (tid < BINS)
+        own[tid] = static_cast<u64>(planes[0][tid]) + (static_cast<u64>(planes[1][tid]) << 11) +
+                   (static_cast<u64>(planes[2][tid]) << 21) + (static_cast<u64>(planes[3][tid]) << 31);
+      cluster.sync();
+      u64* total = reinterpret_cast<u64*>(merged);      // done with, as are the columns of the mass pass
+      if (tid < BINS) total[tid] = gather(&own[tid], plus);
+      __syncthreads();
+      if (warp == 0) {                      // from the highest key down, eight bins to a lane
+        constexpr int PER = BINS / 32;
+        u64 t[PER], s = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) s += t[i] = total[BINS - 1 - lane * PER - i];
+        u64 incl = s;
+        for (int o = 1; o < 32; o <<= 1) {
+          const u64 p = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += p;
+        }
+        u64 cum = above + incl - s;
+        int b = -1;
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+          if (b < 0) {
+            if (t[i] > 0 && cum + t[i] >= target) b = BINS - 1 - lane * PER - i;
+            else cum += t[i];
+          }
+        const unsigned int hit = __ballot_sync(0xffffffffu, b >= 0);
+        const int src = hit ? __ffs(hit) - 1 : 31;
+        b = max(0, __shfl_sync(0xffffffffu, b, src));
+        u64 kept = 0;                       // of this CTA, above bin b
+        for (int i = b + 1 + lane; i < BINS; i += 32) kept += own[i];
+        kept = warp_total(kept);
+        if (lane == src) {
+          sel_u64[0] = cum;
+          sel_u32 = static_cast<unsigned int>(b);
+        }
+        if (lane == 0) sel_u64[1] = kept;
+      }
+      __syncthreads();
+      above = sel_u64[0];
+      mine += sel_u64[1];
+      const unsigned int b = sel_u32;
+      lo += b << shift;
+      if (shift == 0) {
+        kept_mass = above + total[b];
+        mine += own[b];
+        break;
+      }
+      hi = min(hi, lo + (1u << shift) - 1);
+      __syncthreads();
     }
+    thresh_key = lo;
+  }
+  if (counted && !general) {                // from the counters and the list instead
+    mine = 0;
+    for (int s = tid; s < NC; s += ST) {
+      const float xv = value(s);
+      if (counts[s] && key_of(xv, 0.f) >= thresh_key) mine += counts[s] * fix_of(e_val(xv));
+    }
+    for (unsigned int i = tid; i < n_tiny; i += ST) {
+      const float xv = __uint_as_float(tiny[i] << 16);
+      if (key_of(xv, 0.f) >= thresh_key) mine += fix_of(e_val(xv));
+    }
+    mine = warp_total(mine);
+    __syncthreads();
+    if (lane == 0) wmass[warp] = mine;
+    __syncthreads();
+    mine = 0;
+#pragma unroll
+    for (int w = 0; w < SW; ++w) mine += wmass[w];
   }
 
   // 4. the draw
@@ -773,7 +832,7 @@ namespace {
 template <typename T, bool VEC, bool CUT>
 const char* sample_launch(const void* logits, long long ld, const long long* global_rows, unsigned long long seed, const int* draw_dev,
                           int draw_host, long long* tok_out, float* lp_out, int rows, int V, float inv_t, float top_p, cudaStream_t s) {
-  constexpr size_t kDyn = std::max(SEG * ST * sizeof(unsigned long long), (4 * KN + TINY) * sizeof(unsigned int));
+  constexpr size_t kDyn = std::max(SEG * ST * sizeof(unsigned long long), (2 * NC + TINY) * sizeof(unsigned int));
   if (!FERRL_ONCE_PER_DEVICE(cudaFuncSetAttribute(sample_rows_kernel<T, VEC, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   static_cast<int>(kDyn)) == cudaSuccess))
     return "sample_rows: cannot reserve shared memory";

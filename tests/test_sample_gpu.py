@@ -97,3 +97,48 @@ def test_32_bit_rows_of_one_key_or_with_finite_masks_cost_no_more(kind):
     plain = _us(x, 0.95)
     x = x * 0 if kind == "flat" else x.index_fill(1, torch.arange(0, 151936, 2, device="cuda"), -1e4)
     assert _us(x, 0.95) < 1.15 * plain
+
+
+def _kind(kind, rows, V):
+    """-> (bf16 logits, top-p, temperature) of rows whose values are not spread over a few octaves about one."""
+    x, even = _plain(rows, V, torch.float32), torch.arange(0, V, 2, device="cuda")
+    x, top_p, T = {"few masked": lambda: (x.index_fill(1, even[3:25], -1e4), 0.95, 1.0), "half masked": lambda: (x.index_fill(1, even, -1e4), 0.95, 1.0),
+                   "masked by the least value": lambda: (x.index_fill(1, even, torch.finfo(torch.bfloat16).min), 0.95, 1.0),
+                   "far up": lambda: (x + 600, 0.95, 1.0), "wide": lambda: (x * 120, 0.95, 1.0), "wide and hot": lambda: (x * 120, 0.95, 100.0),
+                   "nearly flat": lambda: (x * 4e-5, 0.95, 1.0), "cut about zero": lambda: (x * (1.645 / 2.5), 0.95, 1.0),
+                   "half zero": lambda: (x.index_fill(1, even, 0.0), 0.95, 1.0), "rectified": lambda: (x.clamp_min(0), 0.9, 1.0),
+                   "all zero": lambda: (torch.zeros_like(x), 0.5, 1.0), "one peak": lambda: (x.index_fill(1, even[7:8], 300.0), 0.95, 1.0),
+                   "two scales": lambda: ((x * 0.8 - 3).index_fill(1, even, 0.0) + (x * 8e-5).index_fill(1, torch.arange(1, V, 2, device="cuda"), 0.0), 0.7, 1.0),
+                   "tail below": lambda: (x.index_fill(1, even[4:8], -2000.0), 0.99999, 1000.0),
+                   "large outliers, hot": lambda: (x.index_fill(1, even[100:160], 5e4).index_fill(1, even[200:260], -5e4), 0.3, 1e5),
+                   "small cut, hot": lambda: (x.index_fill(1, even[100:160], 3e-6).index_fill(1, even[200:900], -3e-6), 0.5, 50.0)}[kind]()
+    return x.bfloat16(), top_p, T
+
+
+KINDS = ["few masked", "half masked", "masked by the least value", "far up", "wide", "wide and hot", "nearly flat", "cut about zero", "half zero",
+         "rectified", "all zero", "one peak", "two scales", "tail below", "large outliers, hot", "small cut, hot"]
+
+
+@pytest.mark.parametrize("rows,V", [(3, 20000), (40, 50257), (2, 262144)])
+@pytest.mark.parametrize("kind", KINDS)
+def test_16_bit_rows_draw_what_the_same_values_draw_in_32(kind, rows, V):
+    """The two paths share no counter, list or segment; the masses are the same integers.  Where neighbouring 16-bit values have one
+    32-bit probability (nearly flat rows) the 32-bit cut keeps both, so the log-prob moves by their share of the kept mass."""
+    from ferrl_b200.ops import cuda as Cc
+    x, top_p, T = _kind(kind, rows, V)
+    for seed in (1, 2, 3):
+        a, b = (Cc.sample_top_p(t, seed, torch.arange(rows, device="cuda"), 3, T, top_p, None) for t in (x, x.float()))
+        if kind in ("nearly flat", "cut about zero", "small cut, hot", "wide and hot", "large outliers, hot", "two scales"):
+            assert float((a[1] - b[1]).abs().max()) < 0.02
+        else:
+            assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+@pytest.mark.no_canary
+@pytest.mark.parametrize("rows,V", [(128, 151936), (512, 50264)])
+def test_values_outside_the_usual_octaves_cost_no_more(rows, V):
+    """Finite masks, large, small and repeated values are counted, skipped or listed.  128 x 151936, us: without that 120 to 180 as one
+    CTA a row, and 240 to 470 by the general path."""
+    plain = _us(_plain(rows, V, torch.bfloat16), 0.95)
+    slow = {k: _us(*_kind(k, rows, V)) / plain for k in KINDS if k != "large outliers, hot"}
+    assert all(r < (3.5 if k == "two scales" else 1.9 if k in ("half zero", "rectified", "all zero") else 1.4) for k, r in slow.items()), slow
