@@ -839,7 +839,8 @@ const char* sample_launch(const void* logits, long long ld, const long long* glo
   // Clusters that give each SM two or three CTAs (one alone waits on its own barriers: 128 rows of 151936 bf16 logits take
   // 107 us with one CTA, 76, 74, 80 and 90 with 2, 3, 4 and 8), down to slices of 16384 elements (256 rows of 32768: 48 us
   // with one CTA, 53 with two; 32 rows of 50264: 47 with one, 29 with three, 27 with six).
-  const int cl = std::max(1, std::min({SCL, (384 + rows - 1) / rows, V / 16384}));
+  // And enough of them that a CTA's slice stays within the 2^21 elements that its 32-bit histograms hold.
+  const int cl = std::max({1, std::min({SCL, (384 + rows - 1) / rows, V / 16384}), V > 1 << 21 ? std::min(SCL, (V >> 20) + 1) : 1});
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(rows) * cl);
   cfg.blockDim = dim3(ST);

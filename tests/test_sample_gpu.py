@@ -142,3 +142,18 @@ def test_values_outside_the_usual_octaves_cost_no_more(rows, V):
     plain = _us(_plain(rows, V, torch.bfloat16), 0.95)
     slow = {k: _us(*_kind(k, rows, V)) / plain for k in KINDS if k != "large outliers, hot"}
     assert all(r < (3.5 if k == "two scales" else 1.9 if k in ("half zero", "rectified", "all zero") else 1.4) for k, r in slow.items()), slow
+
+
+def test_many_rows_of_a_vast_vocabulary():
+    """One CTA a row would add more than 2^21 masses into a 32-bit histogram; alone, a row is shared by a whole cluster."""
+    from ferrl_b200.ops import cuda as Cc
+    rows, V = 384, 4300000
+    low = -13.9 - 0.001 * torch.arange(rows, device="cuda").float()[:, None]
+    x = low.expand(rows, V).contiguous()
+    x[:, ::2] -= 1e-4                                         # two keys of one segment
+    x[:, 7] = 0
+    ids = torch.arange(rows, device="cuda")
+    tok, lp = Cc.sample_top_p(x, 5, ids, 1, 1.0, 0.9, None)
+    for r in range(0, rows, 24):
+        t, l = Cc.sample_top_p(x[r:r + 1], 5, ids[r:r + 1], 1, 1.0, 0.9, None)
+        assert int(t) == int(tok[r]) and float(l) == float(lp[r])
