@@ -259,7 +259,6 @@ __global__ void __launch_bounds__(128) flash_bwd_dkv_kernel(FlashArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr int TILE = 64 * D * 2;
   constexpr int THREADS = 128;
-  constexpr int DW = D;  // accumulator width per warp
   uint8_t* sK = smem;
   uint8_t* sV = smem + TILE;
   uint8_t* sQ = smem + 2 * TILE;
@@ -269,16 +268,16 @@ __global__ void __launch_bounds__(128) flash_bwd_dkv_kernel(FlashArgs a) {
   const int n0 = blockIdx.x * BKV, hk = blockIdx.y, b = blockIdx.z;
   const int rep = a.Hq / a.Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int k0 = warp * 16, d0 = 0;
+  const int k0 = warp * 16;
   const __nv_bfloat16* kb = static_cast<const __nv_bfloat16*>(a.k) + b * a.k_bs + hk * D;
   const __nv_bfloat16* vb = static_cast<const __nv_bfloat16*>(a.v) + b * a.v_bs + hk * D;
   load_tile<D, THREADS>(sK, kb, a.k_ts, n0, a.Sk);
   load_tile<D, THREADS>(sV, vb, a.v_ts, n0, a.Sk);
   cp_commit();
 
-  float dk[DW / 8][4], dv[DW / 8][4];
+  float dk[D / 8][4], dv[D / 8][4];
 #pragma unroll
-  for (int i = 0; i < DW / 8; ++i) {
+  for (int i = 0; i < D / 8; ++i) {
     dk[i][0] = dk[i][1] = dk[i][2] = dk[i][3] = 0.f;
     dv[i][0] = dv[i][1] = dv[i][2] = dv[i][3] = 0.f;
   }
@@ -351,10 +350,10 @@ __global__ void __launch_bounds__(128) flash_bwd_dkv_kernel(FlashArgs a) {
 #pragma unroll
       for (int k2 = 0; k2 < 4; ++k2) {
 #pragma unroll
-        for (int dp = 0; dp < DW / 16; ++dp) {
+        for (int dp = 0; dp < D / 16; ++dp) {
           uint32_t bo[4], bq[4];
-          load_b_kn<D>(sdO, k2 * 16, d0 + dp * 16, bo);
-          load_b_kn<D>(sQ, k2 * 16, d0 + dp * 16, bq);
+          load_b_kn<D>(sdO, k2 * 16, dp * 16, bo);
+          load_b_kn<D>(sQ, k2 * 16, dp * 16, bq);
           mma16816(dv[2 * dp], pf[k2], bo[0], bo[1]);
           mma16816(dv[2 * dp + 1], pf[k2], bo[2], bo[3]);
           mma16816(dk[2 * dp], dsf[k2], bq[0], bq[1]);
@@ -364,14 +363,14 @@ __global__ void __launch_bounds__(128) flash_bwd_dkv_kernel(FlashArgs a) {
     }
   }
   cp_wait<0>();
-  __nv_bfloat16* dkb = static_cast<__nv_bfloat16*>(a.dk) + b * a.dk_bs + hk * D + d0;
-  __nv_bfloat16* dvb = static_cast<__nv_bfloat16*>(a.dv) + b * a.dv_bs + hk * D + d0;
+  __nv_bfloat16* dkb = static_cast<__nv_bfloat16*>(a.dk) + b * a.dk_bs + hk * D;
+  __nv_bfloat16* dvb = static_cast<__nv_bfloat16*>(a.dv) + b * a.dv_bs + hk * D;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     int key = n0 + k0 + g + r * 8;
     if (key >= a.Sk) continue;
 #pragma unroll
-    for (int i = 0; i < DW / 8; ++i) {
+    for (int i = 0; i < D / 8; ++i) {
       *reinterpret_cast<uint32_t*>(dkb + static_cast<long long>(key) * a.dk_ts + i * 8 + 2 * t) =
           pack_bf16(dk[i][2 * r] * a.scale, dk[i][2 * r + 1] * a.scale);
       *reinterpret_cast<uint32_t*>(dvb + static_cast<long long>(key) * a.dv_ts + i * 8 + 2 * t) =
