@@ -87,7 +87,9 @@ def test_experts_with_few_rows(T, E, k, H, I):
     gen = torch.Generator(device="cuda").manual_seed(T * E)
     x, gu, dn = _rnd(gen, T, H), _rnd(gen, E, 2 * I, H, std=H ** -0.5), _rnd(gen, E, H, I, std=I ** -0.5)
     logits = torch.randn(T, E, generator=gen, device="cuda") + 2 * torch.arange(E, device="cuda").float().cos()
-    torch.full((64 << 20,), float("nan"), device="cuda")                  # what padding rows find in memory
+    torch.full((64 << 20,), float("nan"), device="cuda")                  # what padding rows find in memory, in large buffers
+    small = [torch.full((1 << n,), float("nan"), device="cuda") for n in range(7, 18) for _ in range(12)]      # and in small ones
+    del small
     scores, idx, counts, _ = C.moe_route(logits, k, True)
     xs = x.clone().requires_grad_()
     y = C.moe_experts(xs, scores, idx, counts, gu, dn)
@@ -98,3 +100,21 @@ def test_experts_with_few_rows(T, E, k, H, I):
     yr.backward(dy.double())
     # bf16 activations between the products: 2^-9 of each, through two or three roundings
     assert float((y - yr).norm() / yr.norm()) < 0.01 and float((xs.grad - xr.grad).norm() / xr.grad.norm()) < 0.015
+
+
+def test_blocks_without_a_token_are_left_alone():
+    from ferrl_b200.ops import cuda as C
+    L, gen = C.lib(), torch.Generator(device="cuda").manual_seed(9)
+    x, w = _rnd(gen, 40, 64), _rnd(gen, 8, 128, 64)
+    _, sc, idx, counts = L.moe_route(torch.randn(40, 8, generator=gen, device="cuda"), 2, True, 0)
+    row_of, token_of, tile_expert, _ = L.moe_plan(idx, counts)
+    full = L.moe_gather(x, token_of, None, row_of)
+    out = L.moe_grouped_gemm(full, w, tile_expert, torch.full((full.shape[0], 128), float("nan"), device="cuda", dtype=torch.bfloat16), token_of=token_of)
+    used = tile_expert.repeat_interleave(128)[:full.shape[0]] >= 0
+    held = torch.zeros_like(used)
+    held[row_of.long()] = True
+    blocks = held.view(-1, 16).any(1).repeat_interleave(16)               # blocks of 16 rows with a token
+    assert bool(out[~blocks].isnan().all()) and not bool(out[blocks].isnan().any()) and int(blocks.sum()) < int(used.sum())
+    expert = tile_expert.clamp_min(0).repeat_interleave(128)[:full.shape[0]]
+    ref = torch.einsum("rk,rnk->rn", full[held].double(), w.double()[expert[held].long()])
+    _close(out[held], ref, torch.einsum("rk,rnk->rn", full[held].double().abs(), w.double().abs()[expert[held].long()]))

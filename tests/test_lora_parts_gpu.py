@@ -28,3 +28,27 @@ def test_parts_equal_stacks(M, K, outs, adapted, r):
     stacked = grads(lambda a, b: ops.lora_linear(a, m.weight, *m._stacks(), wt=m.weight_t, residual=b))
     for one, two in zip(grads(m.forward), stacked):
         assert one.shape == two.shape and one.dtype == two.dtype and torch.equal(one, two)
+
+
+def test_parts_inside_a_rematerialised_segment():
+    """The forward runs twice and its saved operands are of the second time: same bits as without."""
+    from ferrl_b200.models.lora import FusedLoraLinear, LoraSpec
+    from ferrl_b200.remat import remat_segment
+    torch.manual_seed(5)
+    m = FusedLoraLinear(128, [256, 64], ("a", "b"), (True, True), LoraSpec(16, 32.0), dtype=torch.bfloat16, device="cuda")
+    m.set_weight((torch.randn(320, 128, device="cuda") * 128 ** -0.5).bfloat16())
+    with torch.no_grad():
+        for p in (*m.lora_A, *m.lora_B):
+            p.copy_(torch.randn_like(p) * 0.1)
+    leaves = [*m.lora_A, *m.lora_B]
+    x, dy = torch.randn(3, 50, 128, device="cuda").bfloat16(), torch.randn(3, 50, 320, device="cuda").bfloat16()
+
+    def grads(f):
+        xs = x.clone().requires_grad_()
+        for p in leaves:
+            p.grad = None
+        y = f(xs)
+        y.backward(dy)
+        return [y, xs.grad, *(p.grad for p in leaves)]
+    for one, two in zip(grads(m), grads(lambda t: remat_segment(m, t, leaves))):
+        assert torch.equal(one, two)
