@@ -469,8 +469,7 @@ __global__ void qk_norm_rope_kernel(const T* __restrict__ q_in, long long ld_q, 
 // (partner lane = lane +- half/EPL).  Same arithmetic and rounding points as the kernel above.
 // What bounds it is instructions per entry: with a head of 128 to a warp (four entries a lane) shuffles, sums and the
 // angles, loaded again for each head, were most of them.
-// 8192 tokens x 40 heads of 128: forward 126 -> 74 us; 11384 tokens: 141 -> 91 us, backward 180 -> 157 us (the
-// bytes take 36 and 54 us).
+// 8192 tokens x 40 heads of 128: forward 95 -> 69 us, backward 135 -> 102 us (the bytes take 26 and 38 us).
 template <int EPL, bool BWD, int LPH, int U>
 __global__ void qk_norm_rope_vec_kernel(const __nv_bfloat16* __restrict__ q_in, long long ld_q,
                                         const __nv_bfloat16* __restrict__ k_in, long long ld_k, long long ld_dq,
@@ -781,13 +780,17 @@ static const char* qknr_t(const QkNormRopeArgs& a, cudaStream_t s) {
                     (!a.kc || (!BWD && al(a.kc, epl) && al(a.vc, epl) && al(a.v_in, a.ld_v) && a.kv_len));
     if (ok) {
       using B = __nv_bfloat16;
-      // many heads a warp where that still leaves every SM its 64 warps, one (a decode step's few tokens) where not;
       // heads of 128 in 16-byte pieces, where addresses and the rotated width allow it
       auto wide = [](const void* p, long long ld) { return (reinterpret_cast<uintptr_t>(p) % 16) == 0 && (ld % 8) == 0; };
       const bool eight = a.half % 8 == 0 && wide(a.q_in, a.ld_q) && wide(a.k_in, a.ld_k) && wide(a.q_out, BWD ? a.ld_dq : 8) &&
                          wide(a.k_out, BWD ? a.ld_dk : 8) && wide(a.qw, 8) && wide(a.kw, 8) && wide(a.dq, 8) && wide(a.dk, 8) &&
                          (!a.kc || (wide(a.kc, 8) && wide(a.vc, 8) && wide(a.v_in, a.ld_v)));
-      const int per = units < 148LL * 64 * 4 || !eight ? 1 : a.D == 128 ? 8 : 4;
+      // U head groups a warp: with one (a decode step's few tokens, U = 0 in pieces of EPL) latency counts, with two the loads of
+      // the second hide behind the first.  Four pay forward only, where no lane idles, for many heads: backward holds twice the
+      // registers (2048 tokens x 28 heads of 256: 42 us with one, 40 with two, 50 with four; 8192 x 10 of 128: 36, 31 and 45).
+      const int heads = a.Hq + a.Hkv, at_once = a.D == 128 ? 2 : 1;
+      const int U = units < 3000 || !eight ? 0 : units < 16000 ? 1 : BWD || units < 148LL * 64 * 4 || heads % (4 * at_once) ? 2 : 4;
+      const int per = U == 0 ? 1 : U * at_once;
       blocks = (a.n_tok * ((a.Hq + a.Hkv + per - 1) / per) + wpb - 1) / wpb;
 #define FERRL_QKV(EPLV, LPH, U)                                                                                     \
   launch_pdl(qk_norm_rope_vec_kernel<EPLV, BWD, LPH, U>, dim3(static_cast<unsigned>(blocks)), dim3(wpb * 32), 0, s,       \
@@ -796,10 +799,20 @@ static const char* qknr_t(const QkNormRopeArgs& a, cudaStream_t s) {
       static_cast<B*>(a.q_out), static_cast<B*>(a.k_out), static_cast<const B*>(a.dq), static_cast<const B*>(a.dk), \
       a.n_tok, a.Hq, a.Hkv, a.half, a.eps, a.zero_centered ? 1 : 0, static_cast<B*>(a.kc), static_cast<B*>(a.vc),      \
       static_cast<const B*>(a.v_in), a.ld_v, a.kv_len, a.table, a.bt_stride, a.page, a.smax)
-      if (per == 8) FERRL_QKV(8, 16, 4);
-      else if (per == 4) FERRL_QKV(8, 32, 4);
-      else if (epl == 4) FERRL_QKV(4, 32, 1);
-      else FERRL_QKV(8, 32, 1);
+      if (a.D == 128) {
+        switch (U) {
+          case 0: FERRL_QKV(4, 32, 1); break;
+          case 1: FERRL_QKV(8, 16, 1); break;
+          case 2: FERRL_QKV(8, 16, 2); break;
+          default: FERRL_QKV(8, 16, (BWD ? 2 : 4));
+        }
+      } else {
+        switch (U) {
+          case 2: FERRL_QKV(8, 32, 2); break;
+          case 4: FERRL_QKV(8, 32, (BWD ? 2 : 4)); break;
+          default: FERRL_QKV(8, 32, 1);
+        }
+      }
 #undef FERRL_QKV
       count_launch();
       return cudaGetLastError() == cudaSuccess ? nullptr : "qk_norm_rope launch failed";
