@@ -172,11 +172,11 @@ gdn_conv_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __
   }
 }
 
-// Tokens per thread: long runs re-read less context (K - 1 tokens a run); a short input takes shorter ones until the
-// chip has about 2048 threads an SM.
+// Tokens per thread: long runs re-read less context (K - 1 tokens a run).  Where a channel has a thread (V = 1: a short
+// input, whose time is the latency of a run) they shorten until there are 65536 threads, else until there are 2048 an SM.
 int conv_run(long long rows_of_tokens, int L, int C, int V) {
-  int run = 32;
-  while (run > 4 && rows_of_tokens * ((L + run - 1) / run) * (C / V) < 148LL * 2048) run /= 2;
+  int run = V == 1 ? 16 : 32;
+  while (run > (V == 1 ? 1 : 4) && rows_of_tokens * ((L + run - 1) / run) * (C / V) < (V == 1 ? 1LL << 16 : 148LL * 2048)) run /= 2;
   return run;
 }
 
@@ -365,7 +365,9 @@ bool conv_vec(int C, long long ldx, const void* x, const void* y, const void* z)
 template <int K>
 void conv_launch(bool bwd, const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, const __nv_bfloat16* left,
                  const __nv_bfloat16* dy, int B, int L, int C, int act, __nv_bfloat16* out, cudaStream_t stream) {
-  const bool vec = conv_vec(C, ldx, x, out, dy);
+  // eight channels and one a thread, us: one token of 3072 to 10240 channels 3.6 and 2.3, 40 of 3072 5.1 and 3.1, 5119 of 3072 46 and
+  // 35, 4 x 500 of 10240 47 and 45, 5119 of 6144 67 and 65, 5119 of 10240 94 and 102
+  const bool vec = conv_vec(C, ldx, x, out, dy) && static_cast<long long>(B) * L * C > 24000000;
   const int V = vec ? 8 : 1, run = conv_run(B, L, C, V), runs = (L + run - 1) / run;
   const dim3 grid(B * runs, (C / V + 127) / 128);
   if (!bwd && vec) gdn_conv_fwd_kernel<K, 8><<<grid, 128, 0, stream>>>(x, ldx, w, left, L, C, runs, run, act, out);
