@@ -185,9 +185,10 @@ constexpr int TINY = 1024;     // values without a counter that a CTA lists
 //      overflow one; a 64-bit shared atomic is a compare-and-swap loop)
 //
 // Every sum is an integer sum, so neither the cluster size, the path nor the order of the adds shows in the result.
-// 128 rows of 151936 bf16 logits, top-p 0.95: 171 -> 68 us (one CTA of 1024 threads per row, three shared atomics per
-// element and digit before; shared atomics still bound it, 17 cycles a warp, the bytes would take 6 us; without counters,
-// by the general path, 270 us).  float32: 339 -> 168 us.  One row of 151936: 168 -> 27 us.
+// 128 rows of 151936 bf16 logits, top-p 0.95: 178 -> 76 us (one CTA of 1024 threads per row, three shared atomics per
+// element and digit before; shared atomics still bound it, 17 cycles a warp, the bytes would take 6 us; half the row masked 120 ->
+// 74, half zeros 248 -> 76; a row of two scales by the general path 201 -> 193).  Without a cut 53 -> 38.  float32: 339 -> 165,
+// half masked 327 -> 150.  One row of 151936: 167 -> 30 us.
 template <typename T, bool VEC, bool CUT>
 __global__ void __launch_bounds__(ST, SRES)
 sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* __restrict__ global_rows,
@@ -634,9 +635,12 @@ sample_rows_kernel(const T* __restrict__ logits, long long ld, const long long* 
   }
   if (counted && !general) {                // from the counters and the list instead
     mine = 0;
-    for (int s = tid; s < NC; s += ST) {
+#pragma unroll
+    for (int i = 0; i < (NC + ST - 1) / ST; ++i) {
+      const int s = tid + i * ST;
+      const unsigned int n = s < NC ? counts[s] : 0;
       const float xv = value(s);
-      if (counts[s] && key_of(xv, 0.f) >= thresh_key) mine += counts[s] * fix_of(e_val(xv));
+      if (n && key_of(xv, 0.f) >= thresh_key) mine += n * fix_of(e_val(xv));
     }
     for (unsigned int i = tid; i < n_tiny; i += ST) {
       const float xv = __uint_as_float(tiny[i] << 16);
