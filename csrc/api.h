@@ -353,6 +353,10 @@ const char* flash_fwd_tc(const FlashArgs& a, void* vt_ws, int* status, cudaStrea
 bool flash_bwd_tc_supported(const FlashArgs& a);
 size_t flash_bwd_tc_scratch_floats(const FlashArgs& a);   // size of a.delta for flash_bwd_tc
 const char* flash_bwd_tc(const FlashArgs& a, int* status, cudaStream_t stream);
+// the same at head_dim 256 (csrc/kernels/flash_bwd256_tc.cu)
+bool flash_bwd256_tc_supported(const FlashArgs& a);
+size_t flash_bwd256_tc_scratch_floats(const FlashArgs& a);
+const char* flash_bwd256_tc(const FlashArgs& a, int* status, cudaStream_t stream);
 
 // ---- vocabulary rows ----
 // finish of the head GEMM's log-prob epilogue (GemmArgs::lp_mode 1): ws [n_tiles, M] float2, tl [M]

@@ -1766,6 +1766,12 @@ std::tuple<Tensor, Tensor, Tensor> flash_bwd(const Tensor& q, const Tensor& k, c
     FERRL_CHECK(ferrl::flash_bwd_tc(a, status_word(), stream()));
     return {dq, dk, dv};
   }
+  if (variant != 1 && ferrl::flash_bwd256_tc_supported(a)) {
+    Tensor stats = out_empty({static_cast<long long>(ferrl::flash_bwd256_tc_scratch_floats(a))}, lse.options());
+    a.delta = stats.data_ptr<float>();
+    FERRL_CHECK(ferrl::flash_bwd256_tc(a, status_word(), stream()));
+    return {dq, dk, dv};
+  }
   FERRL_CHECK(ferrl::flash_bwd(a, stream()));
   return {dq, dk, dv};
 }

@@ -498,7 +498,7 @@ const char* fwd_d(const FlashArgs& a, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? nullptr : "flash_fwd launch failed";
 }
 
-// ---- backward for head dim 256.  Eight warps form the score tiles once (16 rows x 32 columns each) and pass them on as
+// ---- backward for head dim 256 where flash_bwd256_tc.cu does not apply (no causal mask, an offset, keys of another length).  Eight warps form the score tiles once (16 rows x 32 columns each) and pass them on as
 // 16-bit operand fragments through shared memory; for the products with them a warp then has 32 rows and 64 of the 256
 // columns, so a fragment of the streamed tiles serves two row tiles.  The next pair of streamed tiles loads meanwhile.
 // What bounds it is reading fragments from shared memory (0.45 reads of 512 bytes per product).  With every warp forming
