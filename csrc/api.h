@@ -435,7 +435,7 @@ const char* gdn_tc_forward(const float* q, const float* k, const float* v, const
 const char* gdn_tc_backward(const float* q, const float* k, const float* v, const float* beta, const float* Gc, const float* gl,
                             const float* Tm, const float* Wn, const float* Kd, const float* Vn, const float* Sin,
                             const float* dO, const float* dS_final, int B, int T, int Hk, int Hv, float* X0, float* Y0,
-                            float* dVn, float* dSout, float* dW, float* dGpart, float* dq, float* dk, float* dv, float* dbeta,
+                            float* dVn, float* dSout, float* dq, float* dk, float* dv, float* dbeta,
                             float* dG, float* dS0, cudaStream_t stream);
 
 // ---- expert parallelism over the symmetric heap (csrc/moe/ep.cu)

@@ -645,14 +645,13 @@ std::vector<Tensor> gdn_tc_bwd(const Tensor& q, const Tensor& k, const Tensor& v
   c10::cuda::CUDAGuard guard(q.device());
   auto opt = q.options();
   Tensor X0 = out_empty_like(Vn), Y0 = out_empty_like(Sin), dVn = out_empty_like(Vn), dSout = out_empty_like(Sin);
-  Tensor dW = out_empty_like(Vn), dGpart = out_empty({2, B, T, Hv}, opt);
   Tensor dq = out_empty({B, T, Hv, 128}, opt), dk = out_empty({B, T, Hv, 128}, opt), dv = out_empty_like(v);
   Tensor dbeta = out_empty({B, T, Hv}, opt), dG = out_empty({B, T, Hv}, opt), dS0 = out_empty({B, Hv, 128, 128}, opt);
   FERRL_CHECK(ferrl::gdn_tc_backward(q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), beta.data_ptr<float>(),
                                      Gc.data_ptr<float>(), gl.data_ptr<float>(), Tm.data_ptr<float>(), Wn.data_ptr<float>(),
                                      Kd.data_ptr<float>(), Vn.data_ptr<float>(), Sin.data_ptr<float>(), dO.data_ptr<float>(), dsf,
                                      B, T, Hk, Hv, X0.data_ptr<float>(), Y0.data_ptr<float>(), dVn.data_ptr<float>(),
-                                     dSout.data_ptr<float>(), dW.data_ptr<float>(), dGpart.data_ptr<float>(), dq.data_ptr<float>(),
+                                     dSout.data_ptr<float>(), dq.data_ptr<float>(),
                                      dk.data_ptr<float>(), dv.data_ptr<float>(),
                                      dbeta.data_ptr<float>(), dG.data_ptr<float>(), dS0.data_ptr<float>(), stream()));
   return {dq, dk, dv, dbeta, dG, dS0};
