@@ -79,6 +79,8 @@ enum GemmRefuse { kNoPartials = 1, kNoCluster = 2, kNo32 = 4, kNo176 = 8 };
 constexpr int kStoredRows = kNo32 | kNo176;      // what B stored [K, N] refuses
 void gemm_plan(int M, int N, int K, int K2, int num_sms, int* bn_out, int* split_out, int* cluster_out,
                double* est_out = nullptr, int refuse = 0);
+// whether a grouped call of M rows (capacity of its plan) goes to pairs of SMs
+bool gemm_grouped_pairs(long long M, long long N, long long K, long long experts);
 const char* gemm_bf16(const GemmArgs& a, cudaStream_t stream);
 int gemm_pick_bn(int M, int N, int num_sms);
 

@@ -800,8 +800,9 @@ Tensor moe_gather(const Tensor& x, const Tensor& token_of, const optional<Tensor
 
 // ys[rows, N] = xs[rows, K] x W[e(row)]^T with W [E, N, K]; rows sorted by expert in 128-row segments
 // `nn`: W is [E,K,N] instead (the weight of the forward pass read by the backward one; K a multiple of 64).
+// `form`: 0 by size, for rows as `moe_plan` sizes them; 1 one SM a tile; 2 a pair of SMs for two row tiles of an expert.
 Tensor moe_grouped_gemm(const Tensor& xs, const Tensor& W, const Tensor& tile_expert, const optional<Tensor>& out_buf, bool nn,
-                        const optional<Tensor>& token_of) {
+                        const optional<Tensor>& token_of, int64_t form) {
   TORCH_CHECK(xs.is_cuda() && xs.scalar_type() == at::kBFloat16 && W.scalar_type() == at::kBFloat16, "moe_grouped_gemm: bf16");
   TORCH_CHECK(xs.dim() == 2 && W.dim() == 3 && W.is_contiguous() && xs.is_contiguous() && xs.size(1) == W.size(nn ? 1 : 2), "moe_grouped_gemm: xs [R,K], W [E,N,K]");
   TORCH_CHECK(xs.size(0) % 128 == 0 && tile_expert.numel() * 128 >= xs.size(0) && tile_expert.scalar_type() == at::kInt, "moe_grouped_gemm: rows in 128-row tiles with one expert id each");
@@ -826,6 +827,8 @@ Tensor moe_grouped_gemm(const Tensor& xs, const Tensor& W, const Tensor& tile_ex
   a.out = out.data_ptr(); a.ldo = a.N;
   a.status = status_word(); a.num_sms = num_sms();
   a.force_bn = a.N >= 256 ? 256 : (a.N >= 128 ? 128 : 64);
+  TORCH_CHECK(form >= 0 && form <= 2, "moe_grouped_gemm: form 0, 1 or 2");
+  if (form == 2 || (form == 0 && ferrl::gemm_grouped_pairs(a.M, a.N, a.K, W.size(0)))) a.two_cta = 256;
   FERRL_CHECK(ferrl::gemm_bf16(a, stream()));
   return out;
 }
@@ -2034,7 +2037,7 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("moe_route(Tensor logits, int k, bool renorm, int score=0) -> (Tensor, Tensor, Tensor, Tensor)", &moe_route);
   m.def("moe_plan(Tensor idx, Tensor counts) -> (Tensor, Tensor, Tensor, Tensor)", &moe_plan);
   m.def("moe_gather(Tensor x, Tensor token_of, Tensor? pair_w, Tensor row_of, bool sparse=False) -> Tensor", &moe_gather);
-  m.def("moe_grouped_gemm(Tensor xs, Tensor W, Tensor tile_expert, Tensor(a!)? out=None, bool nn=False, Tensor? token_of=None) -> Tensor(a!)", &moe_grouped_gemm);
+  m.def("moe_grouped_gemm(Tensor xs, Tensor W, Tensor tile_expert, Tensor(a!)? out=None, bool nn=False, Tensor? token_of=None, int form=1) -> Tensor(a!)", &moe_grouped_gemm);
   m.def("ep_dispatch(Tensor x, Tensor idx, Tensor? pair_w, Tensor counts, int[] counts_all, int[] xs, int[] flags, int rank, int world, int epoch, float limit_s, int cap_rows, Tensor(a!) dest_row, Tensor(b!) tile_expert, Tensor(c!) local_rows, bool reuse_plan, Tensor(d!) abort_word) -> ()", &ep_dispatch);
   m.def("ep_combine(int[] ys, Tensor idx, Tensor dest_row, Tensor? w, int H, int E_local, int[] flags, int rank, int world, int epoch, float limit_s, Tensor(a!)? keep_rows, Tensor(b!) abort_word) -> Tensor", &ep_combine);
   m.def("moe_combine(Tensor ys, Tensor row_of, Tensor? w, int T, int k) -> Tensor", &moe_combine);

@@ -989,8 +989,8 @@ def _grouped_input_grad(dy, w, wt, tile_expert, tok=None):
     64: a k-block must not reach into the next expert); ``wt`` is the optional resident transpose."""
     out = dy.new_empty(dy.shape[0], w.shape[2])
     if wt is None and w.shape[1] % 64 == 0:
-        return lib().moe_grouped_gemm(dy, w, tile_expert, out, True, tok)
-    return lib().moe_grouped_gemm(dy, w.transpose(1, 2).contiguous() if wt is None else wt, tile_expert, out, token_of=tok)
+        return lib().moe_grouped_gemm(dy, w, tile_expert, out, True, tok, 0)
+    return lib().moe_grouped_gemm(dy, w.transpose(1, 2).contiguous() if wt is None else wt, tile_expert, out, False, tok, 0)
 
 
 class _MoeExperts(torch.autograd.Function):
@@ -1010,10 +1010,10 @@ class _MoeExperts(torch.autograd.Function):
         xs = L.moe_gather(x.contiguous(), token_of, sc if weight_input else None, row_of, tok is not None)
         # rows of unused tiles are never written and never read back: the combine and the score gradient read routed rows
         # only, the grouped products skip those tiles in both directions
-        gu = L.moe_grouped_gemm(xs, gate_up, tile_expert, xs.new_empty(xs.shape[0], gate_up.shape[1]), token_of=tok)
+        gu = L.moe_grouped_gemm(xs, gate_up, tile_expert, xs.new_empty(xs.shape[0], gate_up.shape[1]), False, tok, 0)
         del xs
         h = L.glu_fwd(gu, act, token_of=tok)
-        ys = L.moe_grouped_gemm(h, down, tile_expert, h.new_empty(h.shape[0], down.shape[1]), token_of=tok)
+        ys = L.moe_grouped_gemm(h, down, tile_expert, h.new_empty(h.shape[0], down.shape[1]), False, tok, 0)
         del h
         out = L.moe_combine(ys, row_of, None if weight_input else sc, T, k)
         # kept rows: the outputs for the gradient of output weights, the tokens for that of input weights
