@@ -79,6 +79,10 @@ enum GemmRefuse { kNoPartials = 1, kNoCluster = 2, kNo32 = 4, kNo176 = 8 };
 constexpr int kStoredRows = kNo32 | kNo176;      // what B stored [K, N] refuses
 void gemm_plan(int M, int N, int K, int K2, int num_sms, int* bn_out, int* split_out, int* cluster_out,
                double* est_out = nullptr, int refuse = 0);
+// at most 16 rows (csrc/gemm/few_rows.cu); rows_of_w 8 or 16 a CTA, 0: its own choice
+bool gemm_few_rows_supported(const GemmArgs& a);
+bool gemm_few_rows_better(const GemmArgs& a);      // than the tiled kernels
+const char* gemm_few_rows(const GemmArgs& a, cudaStream_t stream, int rows_of_w = 0);
 // whether a grouped call of M rows (capacity of its plan) goes to pairs of SMs
 bool gemm_grouped_pairs(long long M, long long N, long long K, long long experts);
 const char* gemm_bf16(const GemmArgs& a, cudaStream_t stream);

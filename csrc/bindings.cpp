@@ -210,6 +210,10 @@ Tensor gemm(const Tensor& A, const Tensor& B, const optional<Tensor>& A2, const 
   // static_b: B (and B2) are weights that no kernel earlier in the stream writes, so a decode-shaped
   // call may start streaming them before its predecessor has finished (programmatic dependent launch)
   a.pdl = (static_b && a.M <= 256) ? 1 : 0;
+  if (force_bn == 0 && force_split == 0 && two_cta == 0 && cluster_k == 0 && stream_k == 0 && ferrl::gemm_few_rows_better(a)) {
+    FERRL_CHECK(ferrl::gemm_few_rows(a, stream()));
+    return out;
+  }
   if (two_cta > 0 && !out_f32) {   // forced
     TORCH_CHECK(two_cta == 128 || two_cta == 256, "gemm: two_cta must be 128 or 256");
     a.two_cta = static_cast<int>(two_cta);
@@ -324,6 +328,29 @@ std::vector<int64_t> gemm_plan(int64_t M, int64_t N, int64_t K, int64_t K2, int6
   return {bn, split, cluster};
 }
 
+// The kernel for at most 16 rows, which gemm() and gemm_glu() choose by themselves; act -1: none.
+Tensor gemm_few_rows(const Tensor& A, const Tensor& B, const optional<Tensor>& residual, int64_t act, double alpha, double limit, int64_t rows_of_w, bool static_b) {
+  TORCH_CHECK(A.is_cuda() && B.is_cuda() && A.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16 && A.dim() == 2 && B.dim() == 2 &&
+                  A.size(1) == B.size(1) && A.stride(1) == 1 && B.stride(1) == 1 && act >= -1 && act <= 2, "gemm_few_rows: A [M,K], B [N,K] bf16");
+  c10::cuda::CUDAGuard guard(A.device());
+  ferrl::GemmArgs a{};
+  a.A = A.data_ptr(); a.B = B.data_ptr(); a.lda = A.stride(0); a.ldb = B.stride(0);
+  a.M = A.size(0); a.N = B.size(0); a.K = A.size(1);
+  Tensor out = out_empty({A.size(0), act >= 0 ? B.size(0) / 2 : B.size(0)}, A.options());
+  a.out = out.data_ptr(); a.ldo = out.stride(0);
+  if (residual.has_value() && residual->defined()) {
+    TORCH_CHECK(residual->scalar_type() == at::kBFloat16 && residual->dim() == 2 && residual->size(0) == a.M && residual->size(1) == a.N &&
+                    residual->stride(1) == 1, "gemm_few_rows: residual bf16 [M,N]");
+    a.residual = residual->data_ptr(); a.ldr = residual->stride(0);
+  }
+  a.glu_act = static_cast<int>(act) + 1;
+  a.glu_alpha = alpha; a.glu_limit = limit;
+  a.num_sms = num_sms();
+  a.pdl = static_b ? 1 : 0;
+  FERRL_CHECK(ferrl::gemm_few_rows(a, stream(), static_cast<int>(rows_of_w)));
+  return out;
+}
+
 // act(x Wg^T) * (x Wu^T) in one kernel: W holds the gate and up rows interleaved in groups of 16
 // (8 gate rows, then the 8 up rows of the same features); returns [M, N/2].
 Tensor gemm_glu(const Tensor& A, const Tensor& B, int64_t act, bool static_b, double alpha, double limit) {
@@ -343,6 +370,10 @@ Tensor gemm_glu(const Tensor& A, const Tensor& B, int64_t act, bool static_b, do
   a.glu_act = static_cast<int>(act) + 1;
   a.glu_alpha = alpha; a.glu_limit = limit;
   a.pdl = (static_b && a.M <= 256) ? 1 : 0;
+  if (ferrl::gemm_few_rows_better(a)) {
+    FERRL_CHECK(ferrl::gemm_few_rows(a, stream()));
+    return out;
+  }
   int bn = 0, split = 1, cluster = 1;
   ferrl::gemm_plan(a.M, a.N, a.K, 0, a.num_sms, &bn, &split, &cluster, nullptr, ferrl::kNoPartials | ferrl::kNoCluster | ferrl::kNo32);
   a.force_bn = bn;                                         // the epilogue needs whole tiles in one CTA
@@ -2013,6 +2044,7 @@ void add_launches(int64_t n) { ferrl::count_launch(static_cast<int>(n)); }
 
 TORCH_LIBRARY(ferrl_b200, m) {
   m.def("gemm_plan(int M, int N, int K, int K2=0, int sms=148, bool nn=False) -> int[]", &gemm_plan);
+  m.def("gemm_few_rows(Tensor a, Tensor b, Tensor? residual=None, int act=-1, float alpha=0.0, float limit=0.0, int rows_of_w=0, bool static_b=True) -> Tensor", &gemm_few_rows);
   m.def("gemm_nn(Tensor a, Tensor b, Tensor? a2=None, Tensor? b2=None) -> Tensor", &gemm_nn);
   m.def("gemm(Tensor A, Tensor B, Tensor? A2, Tensor? B2, Tensor? residual, bool out_f32, int force_bn, int force_split, int two_cta=0, Tensor? debug=None, int cluster_k=0, int stream_k=0, bool static_b=False) -> Tensor", &gemm);  // two_cta: 0 auto, -1 never, 128/256 forced
   m.def("decode_gemm(Tensor A, Tensor B, Tensor? residual=None, int glu_act=-1, int max_clusters=0, bool static_b=False, Tensor? debug=None) -> Tensor", &decode_gemm);
