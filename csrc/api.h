@@ -213,7 +213,7 @@ struct DecodeAttnArgs {
 };
 const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s);
 size_t decode_attn_workspace_bytes(int B, int Hq, int D, int n_splits);
-int decode_attn_pick_splits(int B, int Hkv, int max_len, int num_sms);
+int decode_attn_pick_splits(int B, int Hkv, int max_len, int D, int num_sms);
 
 // ---- latent attention (csrc/kernels/latent_attn.cu; tcgen05 prefill form in flash_tc.cu) ----
 struct LatentPrepArgs {

@@ -1308,7 +1308,7 @@ Tensor decode_attn(const Tensor& q, const Tensor& kc, const Tensor& vc, const Te
     a.block_table = block_table->data_ptr<int>(); a.bt_stride = block_table->size(1); a.page = page;
   }
   a.scale = scale; a.window = window;
-  a.n_splits = n_splits > 0 ? n_splits : ferrl::decode_attn_pick_splits(a.B, a.Hkv, kc.size(1), num_sms());
+  a.n_splits = n_splits > 0 ? n_splits : ferrl::decode_attn_pick_splits(a.B, a.Hkv, kc.size(1), a.D, num_sms());
   Tensor out = out_empty_like(q);
   Tensor ws;
   if (prefix_len.has_value() && prefix_len->defined()) {

@@ -9,9 +9,12 @@
 // memory, kv-splits merged by a second tiny kernel through a caller-provided workspace.
 // Supports a sliding window (keys older than `window` are skipped without being read) and a
 // page table (`block_table[b, j / page]` gives the physical page of logical key j).
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "../api.h"
 #include "../common.cuh"
@@ -621,6 +624,7 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t& r0, uint32_t&
 // Three stages of 32 keys (48 KB at head_dim 128) let four CTAs share an SM: 592 CTA slots take the
 // 1024 (row, kv-head) items of a 128-row batch in two waves instead of three.
 constexpr int MSTAGES = 3;
+constexpr int MAX_CLUSTER = 8;     // splits of a row that merge through distributed shared memory
 
 template <int D, int REP>
 __global__ void __launch_bounds__(PWARPS * 32, (D <= 128 && REP <= 4) ? 4 : 1)
@@ -629,7 +633,7 @@ decode_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
                        const int* __restrict__ block_table, int bt_stride, int page,
                        __nv_bfloat16* __restrict__ out, float* __restrict__ ws, int Hq, int Hkv,
                        long long seq_stride, long long tok_stride, float scale, int window, int n_splits,
-                       const int* __restrict__ kv_start, int kv_start_div, int ws_off, int ws_total) {
+                       const int* __restrict__ kv_start, int kv_start_div, int ws_off, int ws_total, int clustered) {
   pdl_trigger();   // a dependent GEMM may start streaming its weights while this kernel runs
   pdl_wait();      // launched as a programmatic dependent itself: nothing is read before the predecessor is done
   static_assert(REP <= 8, "query heads of one KV head must fit rows 0..7 of the MMA tile");
@@ -767,17 +771,19 @@ decode_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < REP * D; i += blockDim.x) {
-    const int r = i / D, d = i - r * D;
-    float m = -INFINITY;
+  // o, m and l of one entry over all the warps
+  auto merged = [&](int r, int d, float& m, float& l, float& acc) {
+    m = -INFINITY;
+    l = acc = 0.f;
     for (int w = 0; w < PWARPS; ++w) m = fmaxf(m, m_s[w * REP + r]);
-    float l = 0.f, acc = 0.f;
     for (int w = 0; w < PWARPS; ++w) {
       const float mw = m_s[w * REP + r];
       const float c = (mw == -INFINITY) ? 0.f : __expf(mw - m);
       l += l_s[w * REP + r] * c;
       acc += o_s[(w * REP + r) * D + d] * c;
     }
+  };
+  auto finish = [&](int r, int d, float m, float l, float acc) {
     const long long head = static_cast<long long>(b) * Hq + hk * REP + r;
     if (ws_total > 0) {
       // shared-prefix mode: merge my keys with the prefix partials and write the final row
@@ -793,10 +799,62 @@ decode_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
         ot += base[sp * (D + 2) + d] * c;
       }
       out[head * D + d] = __float2bfloat16_rn((lt > 0.f && len > 0) ? ot / lt : 0.f);   // a retired row (length 0) stays zero
-    } else if (n_splits == 1) {
-      out[head * D + d] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
     } else {
-      float* w_ = ws + (head * n_splits + split) * (D + 2);
+      out[head * D + d] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
+    }
+  };
+  if (clustered) {
+    // the splits of a row are one cluster: each writes an equal share of the row from all the splits' sums, read out of their
+    // shared memory (in the order of the splits, as the second kernel reads them from the workspace)
+    float* p_m = o_s + PWARPS * REP * D;        // [REP]
+    float* p_l = p_m + REP;                     // [REP]
+    float* p_o = p_l + REP;                     // [REP][D]
+    for (int i = threadIdx.x; i < REP * D; i += blockDim.x) {
+      const int r = i / D, d = i - r * D;
+      float m, l, acc;
+      merged(r, d, m, l, acc);
+      p_o[i] = acc;
+      if (d == 0) {
+        p_m[r] = m;
+        p_l[r] = l;
+      }
+    }
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    const int share = (REP * D + n_splits - 1) / n_splits;
+    for (int i = split * share + threadIdx.x; i < min(REP * D, (split + 1) * share); i += blockDim.x) {
+      const int r = i / D, d = i - r * D;
+      float ms[MAX_CLUSTER], ls[MAX_CLUSTER], os[MAX_CLUSTER], m = -INFINITY, l = 0.f, acc = 0.f;
+#pragma unroll
+      for (int sp = 0; sp < MAX_CLUSTER; ++sp)
+        if (sp < n_splits) {
+          ms[sp] = *cluster.map_shared_rank(p_m + r, sp);
+          ls[sp] = *cluster.map_shared_rank(p_l + r, sp);
+          os[sp] = *cluster.map_shared_rank(p_o + i, sp);
+        }
+#pragma unroll
+      for (int sp = 0; sp < MAX_CLUSTER; ++sp)
+        if (sp < n_splits) m = fmaxf(m, ms[sp]);
+#pragma unroll
+      for (int sp = 0; sp < MAX_CLUSTER; ++sp)
+        if (sp < n_splits) {
+          const float c = (ms[sp] == -INFINITY) ? 0.f : __expf(ms[sp] - m);
+          l += ls[sp] * c;
+          acc += os[sp] * c;
+        }
+      finish(r, d, m, l, acc);
+    }
+    cluster.sync();                             // nobody leaves while its sums are read
+    return;
+  }
+  for (int i = threadIdx.x; i < REP * D; i += blockDim.x) {
+    const int r = i / D, d = i - r * D;
+    float m, l, acc;
+    merged(r, d, m, l, acc);
+    if (ws_total > 0 || n_splits == 1) {
+      finish(r, d, m, l, acc);
+    } else {
+      float* w_ = ws + ((static_cast<long long>(b) * Hq + hk * REP + r) * n_splits + split) * (D + 2);
       w_[d] = acc;
       if (d == 0) {
         w_[D] = m;
@@ -1311,15 +1369,40 @@ __global__ void decode_combine_kernel(const float* __restrict__ ws, __nv_bfloat1
 
 }  // namespace
 
+// The splits of a row are a cluster that merges by itself, or CTAs that do not know each other and a second kernel that merges them.
+// A cluster saves that kernel, but not all of the chip takes clusters (GPCs of 16 to 20 multiprocessors: 132 and 120 places for
+// clusters of 4 and 8), so with more than two CTAs to a place the free ones are faster (192 (row, head) pairs, 841 keys: 18.3
+// us free, 20.7 in clusters of two).
+static int cluster_share(long long ctas, int splits, int sms) {      // CTAs of clusters on a multiprocessor
+  const int places = splits <= 2 ? sms : sms * (splits <= 4 ? 132 : 120) / 148;
+  return static_cast<int>((ctas * splits + places - 1) / places);
+}
+static bool in_clusters(long long ctas, int splits, int sms) {
+  return splits > 1 && splits <= MAX_CLUSTER && cluster_share(ctas, splits, sms) <= 2;
+}
+// What a step takes with `splits`, in us at head dim 128: a tile of 32 keys passes in 0.61 alone, a multiprocessor moves one in 0.42;
+// fitted to 1 to 24 rows of 2 to 8 heads and 100 to 8000 keys.  841 keys: two pairs 11.3 -> 6.3 us, 32 pairs 12.3 -> 8.4, 128 pairs 19.6
+// -> 15.9; eight pairs of head dim 256 19.0 -> 10.8.
+static double split_time(long long ctas, int splits, int max_len, int D, int sms) {
+  const bool cl = in_clusters(ctas, splits, sms);
+  const double on_each = cl || splits == 1 ? cluster_share(ctas, splits, sms) : static_cast<double>(ctas * splits) / sms;
+  const int tiles = (max_len + 32 * splits - 1) / (32 * splits);
+  const double once = splits == 1 ? 1.0 : cl ? (splits <= 4 ? 3.2 : 3.9) : splits == 2 ? 3.5 : splits == 4 ? 5.0 : 6.0;
+  return (once + tiles * std::max(0.61, 0.42 * on_each)) * D / 128;
+}
+static int pick_splits(long long ctas, int max_len, int D, int sms, bool clusters_only) {
+  int best = 1;
+  for (int s = 2; s <= (clusters_only ? MAX_CLUSTER : 16); s *= 2)      // free CTAs: up to four a multiprocessor
+    if ((in_clusters(ctas, s, sms) || (!clusters_only && ctas * s < 4ll * sms)) && split_time(ctas, s, max_len, D, sms) <= split_time(ctas, best, max_len, D, sms)) best = s;
+  return best;
+}
+
 size_t decode_attn_workspace_bytes(int B, int Hq, int D, int n_splits) {
   return n_splits <= 1 ? 0 : static_cast<size_t>(B) * Hq * n_splits * (D + 2) * sizeof(float);
 }
 
-int decode_attn_pick_splits(int B, int Hkv, int max_len, int num_sms) {
-  long long ctas = static_cast<long long>(B) * Hkv;
-  int s = 1;
-  while (ctas * s < 2LL * num_sms && s < 16 && max_len / (s * 2) >= 256) s *= 2;
-  return s;
+int decode_attn_pick_splits(int B, int Hkv, int max_len, int D, int num_sms) {
+  return pick_splits(static_cast<long long>(B) * Hkv, max_len, D, num_sms, false);
 }
 
 const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s) {
@@ -1331,6 +1414,11 @@ const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s) {
   if (a.n_splits > 1 && !a.workspace) return "decode_attn: workspace required for split-kv";
   dim3 grid(a.B, a.Hkv, a.n_splits < 1 ? 1 : a.n_splits);
   bool launched = false;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long pairs = static_cast<long long>(a.B) * a.Hkv;
+  bool clustered = in_clusters(pairs, grid.z, sms), merged = false;      // splits that merge by themselves, if the tensor-core kernel runs
   // shared-prefix mode (grouped rollouts over a paged cache): see decode_attn_group_kernel
   const int* kv_start = nullptr;
   int kv_start_div = 1, ws_off = 0, ws_total = 0;
@@ -1379,7 +1467,12 @@ const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s) {
 #undef FERRL_DECODE_GROUP
     if (!ok) return "decode_attn: shared-prefix mode has no kernel for this (head_dim, heads per kv head, group) triple";
     count_launch();
+    grid.z = pick_splits(pairs, a.bt_stride * a.page, a.D, sms, true);      // of the private keys
+    clustered = grid.z > 1;
   }
+  // The CTAs of a cluster would sit together on as few multiprocessors as hold them: shared memory that nobody uses spreads them.
+  constexpr size_t kSpreadMax = 120 * 1024;
+  const size_t spread = !clustered ? 0 : cluster_share(pairs, grid.z, sms) == 1 ? kSpreadMax : 80 * 1024;
 #define FERRL_DECODE_FAST(DD, RR)                                                                                   \
   if (!launched && a.D == DD && rep == RR && !kv_start) {                                                                          \
     size_t fsm = (2 * WARPS * RR + static_cast<size_t>(WARPS) * RR * DD) * 4;                                         \
@@ -1409,15 +1502,30 @@ const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s) {
     constexpr size_t msm_bytes = static_cast<size_t>(MSTAGES) * 2 * PTK * DD * 2;                                     \
     auto mk = decode_attn_mma_kernel<DD, RR>;                                                                         \
     if (!FERRL_ONCE_PER_DEVICE(cudaFuncSetAttribute(mk, cudaFuncAttributeMaxDynamicSharedMemorySize,                  \
-                                                    static_cast<int>(msm_bytes)) == cudaSuccess &&                    \
+                                                    static_cast<int>(std::max(msm_bytes, kSpreadMax))) == cudaSuccess && \
                                cudaFuncSetAttribute(mk, cudaFuncAttributePreferredSharedMemoryCarveout,               \
                                                     cudaSharedmemCarveoutMaxShared) == cudaSuccess))                  \
       return "decode_attn: cannot reserve shared memory";                                                             \
-    launch_pdl(mk, grid, dim3(PWARPS * 32), msm_bytes, s,                                                             \
-        static_cast<const __nv_bfloat16*>(a.q), static_cast<const __nv_bfloat16*>(a.k),                               \
-        static_cast<const __nv_bfloat16*>(a.v), a.kv_len, a.block_table, a.bt_stride, a.page,                         \
-        static_cast<__nv_bfloat16*>(a.out), a.workspace, a.Hq, a.Hkv, a.seq_stride, a.tok_stride, a.scale, a.window,  \
-        grid.z, kv_start, kv_start_div, ws_off, ws_total);                                                            \
+    cudaLaunchConfig_t cfg{};                                                                                         \
+    cfg.gridDim = grid;                                                                                               \
+    cfg.blockDim = dim3(PWARPS * 32);                                                                                 \
+    cfg.dynamicSmemBytes = clustered ? std::max(msm_bytes, spread) : msm_bytes;                                       \
+    cfg.stream = s;                                                                                                   \
+    cudaLaunchAttribute at[2];                                                                                        \
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;                                                    \
+    at[0].val.programmaticStreamSerializationAllowed = 1;                                                             \
+    at[1].id = cudaLaunchAttributeClusterDimension;                                                                   \
+    at[1].val.clusterDim.x = at[1].val.clusterDim.y = 1;                                                              \
+    at[1].val.clusterDim.z = grid.z;                                                                                  \
+    cfg.attrs = at;                                                                                                   \
+    cfg.numAttrs = clustered ? 2 : 1;                                                                                 \
+    if (cudaLaunchKernelEx(&cfg, mk, static_cast<const __nv_bfloat16*>(a.q), static_cast<const __nv_bfloat16*>(a.k),  \
+                           static_cast<const __nv_bfloat16*>(a.v), a.kv_len, a.block_table, a.bt_stride, a.page,      \
+                           static_cast<__nv_bfloat16*>(a.out), a.workspace, a.Hq, a.Hkv, a.seq_stride, a.tok_stride,  \
+                           a.scale, a.window, static_cast<int>(grid.z), kv_start, kv_start_div, ws_off, ws_total,     \
+                           clustered ? 1 : 0) != cudaSuccess)                                                         \
+      return "decode_attn launch failed";                                                                             \
+    merged = clustered;                                                                                               \
     launched = true;                                                                                                  \
   }
   if ((a.tok_stride % 8) == 0 && (a.seq_stride % 8) == 0 && (reinterpret_cast<uintptr_t>(a.k) & 15) == 0 &&
@@ -1457,7 +1565,7 @@ const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s) {
                                         a.seq_stride, a.tok_stride, a.scale, a.window, grid.z);
   }
   count_launch();
-  if (grid.z > 1) {
+  if (grid.z > 1 && !merged) {
     launch_pdl(decode_combine_kernel, dim3(a.B * a.Hq), dim3(128), 0, s, a.workspace, static_cast<__nv_bfloat16*>(a.out), a.D,
                static_cast<int>(grid.z));
     count_launch();

@@ -577,8 +577,11 @@ def decode_attention(q, k_cache, v_cache, kv_len, *, scale, window=0, n_splits=0
         B = q.shape[0]
         if int(prefix_splits):
             ps = int(prefix_splits)
-        elif (q.shape[-1], q.shape[1] // k_cache.shape[2], group) == (128, 4, 8):
-            ps = 1          # the whole-group kernel: prefix and private keys in one launch
+        elif (q.shape[-1], q.shape[1] // k_cache.shape[2], group) == (128, 4, 8) and (B // group) * k_cache.shape[2] > 74:
+            # The whole-group kernel: prefix and private keys in one launch, one CTA a group and head.  With those on less than
+            # half the chip splits of both are faster (320 shared and 512 private keys, us: 8 pairs 57 and 19, 32 pairs 58
+            # and 44, 64 pairs 58 and 50, 96 pairs 58 and 80).
+            ps = 1
         else:
             ps = max(1, min(4, 296 // max(1, (B // group) * k_cache.shape[2])))   # about two prefix CTAs per SM
         return lib().decode_attn(q.contiguous(), k_cache, v_cache, kv_len.to(torch.int32), float(scale), 0, 1, block_table,
