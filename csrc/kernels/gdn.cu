@@ -31,38 +31,73 @@ __device__ __forceinline__ float dsilu_f(float x) {
 }
 
 // Causal depthwise convolution, forward and backward.  x [B, L, C] (row stride ldx), w [C, K], left [B, C, K-1] or null,
-// y, dy, dx [B, L, C] contiguous.  Bound by memory: every input is wanted once and every output written once.  A thread
-// owns V neighbouring channels (V = 8: one 16-byte access a token) and walks `run` tokens with the last K - 1 inputs in
-// registers, so a token is read once and not once per tap; the K - 1 tokens in front of a run are the only ones read
-// twice.  [5119, 10240] channels, K = 4: forward 371 us with one element a thread, K reads a token and an index division
-// each, 93 us so (210 MB; what is left is the SiLU's arithmetic as much as the traffic); backward 1043 us, which also
-// formed every output K times, 135 us so (315 MB).  The taps are added in the same order as before, so the results are
-// the same bits.
+// y, dy, dx [B, L, C] contiguous.  A thread owns V neighbouring channels and walks `run` tokens with the last K - 1 inputs
+// in registers, so a token is read once and not once per tap; the K - 1 tokens in front of a run are the only ones read
+// twice.  Bound by instruction issue, the SiLU's exponential and reciprocal before all, and not by its bytes (210 MB
+// forward, 315 MB backward at [5119, 10240], K = 4: 32 and 48 us).  So V = 4, one 8-byte access a token: eight channels
+// took 126 and 188 registers, which left too few warps to hide the exponentials (72 and 148 us); four take 70 and 93
+// (55 and 96 us).  The taps are read as whole words too: as V x K single values, a thread's own row apart from its
+// neighbour's, they cost more cache accesses than the tokens of a run (94 and 145 us together with the eight channels).
+// The next tokens are on their way while the present ones are worked on.  The taps are added in the order of the tap
+// number whatever V is, so the results are the same bits.
+template <int V> struct ConvRaw { using type = __nv_bfloat16; };      // V channels of a token as they lie
+template <> struct ConvRaw<4> { using type = uint2; };
 template <int V>
-__device__ __forceinline__ void conv_load(const __nv_bfloat16* p, float (&f)[V]) {
-  if constexpr (V == 8) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+__device__ __forceinline__ void conv_unpack(const typename ConvRaw<V>::type& u, float (&f)[V]) {
+  if constexpr (V > 1) {
+    const uint32_t* h = reinterpret_cast<const uint32_t*>(&u);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 t = __bfloat1622float2(h[e]);
-      f[2 * e] = t.x;
-      f[2 * e + 1] = t.y;
+    for (int e = 0; e < V / 2; ++e) {
+      f[2 * e] = __uint_as_float(h[e] << 16);
+      f[2 * e + 1] = __uint_as_float(h[e] & 0xffff0000u);
     }
   } else {
-    f[0] = __bfloat162float(p[0]);
+    f[0] = __bfloat162float(u);
   }
 }
 template <int V>
+__device__ __forceinline__ void conv_load(const __nv_bfloat16* p, float (&f)[V]) {
+  conv_unpack<V>(*reinterpret_cast<const typename ConvRaw<V>::type*>(p), f);
+}
+template <int V>
 __device__ __forceinline__ void conv_store(__nv_bfloat16* p, const float (&f)[V]) {
-  if constexpr (V == 8) {
-    uint4 u;
+  if constexpr (V > 1) {
+    typename ConvRaw<V>::type u;
     __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
-    *reinterpret_cast<uint4*>(p) = u;
+    for (int e = 0; e < V / 2; ++e) h[e] = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+    *reinterpret_cast<typename ConvRaw<V>::type*>(p) = u;
   } else {
     p[0] = __float2bfloat16_rn(f[0]);
+  }
+}
+// bf16 and back, two values a conversion
+template <int V>
+__device__ __forceinline__ void conv_round(float (&f)[V]) {
+  if constexpr (V > 1) {
+    typename ConvRaw<V>::type u;
+    conv_store<V>(reinterpret_cast<__nv_bfloat16*>(&u), f);
+    conv_unpack<V>(u, f);
+  } else {
+    f[0] = __bfloat162float(__float2bfloat16_rn(f[0]));
+  }
+}
+// the K taps of V channels: V x K neighbouring values
+template <int K, int V>
+__device__ __forceinline__ void conv_taps(const __nv_bfloat16* w, float (&wv)[K][V]) {
+  if constexpr (V > 1) {
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      float f[V];
+      conv_unpack<V>(reinterpret_cast<const typename ConvRaw<V>::type*>(w)[i], f);
+#pragma unroll
+      for (int e = 0; e < V; ++e) wv[(i * V + e) % K][(i * V + e) / K] = f[e];
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+#pragma unroll
+      for (int e = 0; e < V; ++e) wv[j][e] = __bfloat162float(w[e * K + j]);
   }
 }
 // channels c .. c+V-1 of x at token t of row b; the carried context where t < 0
@@ -86,30 +121,46 @@ gdn_conv_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __
   if (c >= C) return;
   const int b = blockIdx.x / runs, t0 = (blockIdx.x - b * runs) * run, t1 = min(L, t0 + run);
   float wv[K][V], win[K][V];            // win[j]: the input that tap j meets
-#pragma unroll
-  for (int j = 0; j < K; ++j)
-#pragma unroll
-    for (int e = 0; e < V; ++e) wv[j][e] = __bfloat162float(w[(c + e) * K + j]);
+  conv_taps<K, V>(w + static_cast<long long>(c) * K, wv);
 #pragma unroll
   for (int j = 1; j < K; ++j) conv_input<K, V>(x, ldx, left, b, t0 - K + j, c, L, C, win[j]);
-#pragma unroll 4
-  for (int t = t0; t < t1; ++t) {
+  // four tokens at a time, the next four on their way while these are worked on
+  using Raw = typename ConvRaw<V>::type;
+  constexpr int U = 4;
+  const __nv_bfloat16* xp = x + static_cast<long long>(b) * L * ldx + c;
+  __nv_bfloat16* yp = y + static_cast<long long>(b) * L * C + c;
+  Raw now[U], next[U];
 #pragma unroll
-    for (int j = 0; j + 1 < K; ++j)
+  for (int u = 0; u < U; ++u)
+    if (t0 + u < t1) now[u] = *reinterpret_cast<const Raw*>(xp + static_cast<long long>(t0 + u) * ldx);
+  for (int t = t0; t < t1; t += U) {
 #pragma unroll
-      for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
-    conv_load<V>(x + (static_cast<long long>(b) * L + t) * ldx + c, win[K - 1]);
-    float o[V];
+    for (int u = 0; u < U; ++u)
+      if (t + U + u < t1) next[u] = *reinterpret_cast<const Raw*>(xp + static_cast<long long>(t + U + u) * ldx);
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-      float acc = 0.f;
+    for (int u = 0; u < U; ++u) {
+      if (t + u >= t1) break;
 #pragma unroll
-      for (int j = 0; j < K; ++j) acc += wv[j][e] * win[j][e];
-      // the eager form rounds the conv output to the activation dtype before the SiLU
-      acc = __bfloat162float(__float2bfloat16_rn(acc));
-      o[e] = act ? silu_f(acc) : acc;
+      for (int j = 0; j + 1 < K; ++j)
+#pragma unroll
+        for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
+      conv_unpack<V>(now[u], win[K - 1]);
+      float o[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        o[e] = 0.f;
+#pragma unroll
+        for (int j = 0; j < K; ++j) o[e] += wv[j][e] * win[j][e];
+      }
+      if (act) {                         // the eager form rounds the conv output to the activation dtype before the SiLU
+        conv_round<V>(o);
+#pragma unroll
+        for (int e = 0; e < V; ++e) o[e] = silu_f(o[e]);
+      }
+      conv_store<V>(yp + static_cast<long long>(t + u) * C, o);
     }
-    conv_store<V>(y + (static_cast<long long>(b) * L + t) * C + c, o);
+#pragma unroll
+    for (int u = 0; u < U; ++u) now[u] = next[u];
   }
 }
 
@@ -123,17 +174,34 @@ gdn_conv_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __
   if (c >= C) return;
   const int b = blockIdx.x / runs, t0 = (blockIdx.x - b * runs) * run, t1 = min(L, t0 + run);
   float wv[K][V], win[K][V], d[K][V];   // d[j]: the gradient that tap j passes on, that of output t + K - 1 - j
+  conv_taps<K, V>(w + static_cast<long long>(c) * K, wv);
 #pragma unroll
   for (int j = 0; j < K; ++j)
 #pragma unroll
-    for (int e = 0; e < V; ++e) {
-      wv[j][e] = __bfloat162float(w[(c + e) * K + j]);
-      d[j][e] = 0.f;
-    }
+    for (int e = 0; e < V; ++e) d[j][e] = 0.f;
 #pragma unroll
   for (int j = 1; j < K; ++j) conv_input<K, V>(x, ldx, left, b, t0 - K + j, c, L, C, win[j]);
-#pragma unroll 4
-  for (int to = t0; to < t1 + K - 1; ++to) {
+  using Raw = typename ConvRaw<V>::type;
+  constexpr int U = 2;
+  const __nv_bfloat16* xp = x + static_cast<long long>(b) * L * ldx + c;
+  const __nv_bfloat16* gp = dy + static_cast<long long>(b) * L * C + c;
+  const int t2 = min(L, t1 + K - 1);
+  Raw now[2][U], next[2][U];
+  auto fetch = [&](Raw (&r)[2][U], int t) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (t + u < t2) {
+        r[0][u] = *reinterpret_cast<const Raw*>(xp + static_cast<long long>(t + u) * ldx);
+        r[1][u] = *reinterpret_cast<const Raw*>(gp + static_cast<long long>(t + u) * C);
+      }
+  };
+  fetch(now, t0);
+  for (int tb = t0; tb < t1 + K - 1; tb += U) {
+    fetch(next, tb + U);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int to = tb + u;
+    if (to >= t1 + K - 1) break;
 #pragma unroll
     for (int j = K - 1; j > 0; --j)
 #pragma unroll
@@ -143,16 +211,19 @@ gdn_conv_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __
       for (int j = 0; j + 1 < K; ++j)
 #pragma unroll
         for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
-      conv_load<V>(x + (static_cast<long long>(b) * L + to) * ldx + c, win[K - 1]);
-      conv_load<V>(dy + (static_cast<long long>(b) * L + to) * C + c, d[0]);
+      conv_unpack<V>(now[0][u], win[K - 1]);
+      conv_unpack<V>(now[1][u], d[0]);
       if (act) {
+        float pre[V];
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-          float pre = 0.f;
+          pre[e] = 0.f;
 #pragma unroll
-          for (int j = 0; j < K; ++j) pre += wv[j][e] * win[j][e];
-          d[0][e] *= dsilu_f(__bfloat162float(__float2bfloat16_rn(pre)));
+          for (int j = 0; j < K; ++j) pre[e] += wv[j][e] * win[j][e];
         }
+        conv_round<V>(pre);
+#pragma unroll
+        for (int e = 0; e < V; ++e) d[0][e] *= dsilu_f(pre[e]);
       }
     } else {
 #pragma unroll
@@ -170,13 +241,19 @@ gdn_conv_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __
       conv_store<V>(dx + (static_cast<long long>(b) * L + t) * C + c, o);
     }
   }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      now[0][u] = next[0][u];
+      now[1][u] = next[1][u];
+    }
+  }
 }
 
-// Tokens per thread: long runs re-read less context (K - 1 tokens a run).  Where a channel has a thread (V = 1: a short
-// input, whose time is the latency of a run) they shorten until there are 65536 threads, else until there are 2048 an SM.
+// Tokens per thread: long runs re-read less context (K - 1 tokens a run) and set out less often, but a short input wants
+// threads: they shorten until there are 32768, to eight tokens (one where a thread has one channel).
 int conv_run(long long rows_of_tokens, int L, int C, int V) {
   int run = V == 1 ? 16 : 32;
-  while (run > (V == 1 ? 1 : 4) && rows_of_tokens * ((L + run - 1) / run) * (C / V) < (V == 1 ? 1LL << 16 : 148LL * 2048)) run /= 2;
+  while (run > (V == 1 ? 1 : 8) && rows_of_tokens * ((L + run - 1) / run) * (C / V) < (V == 1 ? 1LL << 16 : 1LL << 15)) run /= 2;
   return run;
 }
 
@@ -356,23 +433,25 @@ gdn_decode_step_tile_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
 
 namespace {
 
-// 16-byte accesses want whole groups of eight channels on 16-byte boundaries; anything else goes channel by channel.
-bool conv_vec(int C, long long ldx, const void* x, const void* y, const void* z) {
-  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z);
-  return C % 8 == 0 && ldx % 8 == 0 && at % 16 == 0;
+constexpr int kConvV = 4;                // channels of a thread
+// 8-byte accesses want whole groups of four channels on 8-byte boundaries; anything else goes channel by channel.
+bool conv_vec(int C, long long ldx, const void* x, const void* w, const void* y, const void* z) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) |
+                       reinterpret_cast<uintptr_t>(z);
+  return C % kConvV == 0 && ldx % kConvV == 0 && at % 8 == 0;
 }
 
 template <int K>
 void conv_launch(bool bwd, const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, const __nv_bfloat16* left,
                  const __nv_bfloat16* dy, int B, int L, int C, int act, __nv_bfloat16* out, cudaStream_t stream) {
-  // eight channels and one a thread, us: one token of 3072 to 10240 channels 3.6 and 2.3, 40 of 3072 5.1 and 3.1, 5119 of 3072 46 and
-  // 35, 4 x 500 of 10240 47 and 45, 5119 of 6144 67 and 65, 5119 of 10240 94 and 102
-  const bool vec = conv_vec(C, ldx, x, out, dy) && static_cast<long long>(B) * L * C > 24000000;
-  const int V = vec ? 8 : 1, run = conv_run(B, L, C, V), runs = (L + run - 1) / run;
+  // four channels and one a thread, us forward / backward: 40 tokens of 3072 9 / 10 and 8 / 8, 300 of 8192 12 / 14 and
+  // 12 / 16, 1000 of 8192 17 / 25 and 25 / 35, 5119 of 10240 55 / 96 and 104 / 170
+  const bool vec = conv_vec(C, ldx, x, w, out, dy) && static_cast<long long>(B) * L * C >= 1LL << 20;
+  const int V = vec ? kConvV : 1, run = conv_run(B, L, C, V), runs = (L + run - 1) / run;
   const dim3 grid(B * runs, (C / V + 127) / 128);
-  if (!bwd && vec) gdn_conv_fwd_kernel<K, 8><<<grid, 128, 0, stream>>>(x, ldx, w, left, L, C, runs, run, act, out);
+  if (!bwd && vec) gdn_conv_fwd_kernel<K, kConvV><<<grid, 128, 0, stream>>>(x, ldx, w, left, L, C, runs, run, act, out);
   else if (!bwd) gdn_conv_fwd_kernel<K, 1><<<grid, 128, 0, stream>>>(x, ldx, w, left, L, C, runs, run, act, out);
-  else if (vec) gdn_conv_bwd_kernel<K, 8><<<grid, 128, 0, stream>>>(x, ldx, w, left, dy, L, C, runs, run, act, out);
+  else if (vec) gdn_conv_bwd_kernel<K, kConvV><<<grid, 128, 0, stream>>>(x, ldx, w, left, dy, L, C, runs, run, act, out);
   else gdn_conv_bwd_kernel<K, 1><<<grid, 128, 0, stream>>>(x, ldx, w, left, dy, L, C, runs, run, act, out);
 }
 
