@@ -407,7 +407,7 @@ const char* gdn_conv_step(const void* x, long long ldx, const void* w, void* sta
 const char* gdn_chunk_fwd(const void* q, const void* k, const void* v, long long q_bs, long long q_ts, long long k_bs,
                           long long k_ts, long long v_bs, long long v_ts, const float* g, const float* beta,
                           const float* S0, float* S_out, void* out, int B, int T, int Hk, int Hv, int KD, int VD,
-                          bool l2norm, float eps, void* workspace, cudaStream_t stream);
+                          bool l2norm, float eps, void* workspace, int* status, cudaStream_t stream);
 size_t gdn_chunk_workspace(int B, int T, int Hv);      // bytes that gdn_chunk_fwd takes
 // 16-bit activations <-> the 32-bit whole chunks of the training kernels (Tp = T rounded up to 64; heads packed, 8-byte aligned)
 const char* gdn_pack(const void* q, long long q_bs, long long q_ts, const void* k, long long k_bs, long long k_ts, const void* v,

@@ -769,7 +769,7 @@ std::tuple<Tensor, Tensor> gdn_chunk_fwd(const Tensor& q_, const Tensor& k_, con
   FERRL_CHECK(ferrl::gdn_chunk_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), q.stride(1), k.stride(0),
                                    k.stride(1), v.stride(0), v.stride(1), g.data_ptr<float>(), beta.data_ptr<float>(), s0,
                                    S.data_ptr<float>(), out.data_ptr(), B, T, Hk, Hv, KD, VD, l2norm,
-                                   static_cast<float>(eps), ws.data_ptr(), stream()));
+                                   static_cast<float>(eps), ws.data_ptr(), status_word(), stream()));
   return {out, S};
 }
 

@@ -30,6 +30,7 @@
 
 #include "../api.h"
 #include "../common.cuh"
+#include "../gemm/tc_common.cuh"
 #include "mma_sync.cuh"
 
 namespace ferrl {
@@ -41,17 +42,25 @@ constexpr int GD = 128;                      // key and value head dim
 constexpr int NTH = 256;
 constexpr int PIECE = GC * GC;               // entries of one piece of T or P
 constexpr int VEC = 5;                       // row factors: beta, beta gamma kn, gamma qn, kn exp(G_C - G), [gamma_C]
-constexpr int TILE = GC * GC * 2;            // bytes of a [64, 64] 16-bit tile
+constexpr uint32_t TILE = GC * GC * 2;       // bytes of a [64, 64] 16-bit tile
 
+// x - the upper or lower half of a pair of 16-bit values, in one instruction
+template <bool UPPER>
+__device__ __forceinline__ float less(uint32_t pair, float x) {
+  float d;
+  if constexpr (UPPER)
+    asm("{.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tfma.rn.f32.bf16 %0, hi, %2, %3;}" : "=f"(d) : "r"(pair), "h"(static_cast<unsigned short>(0xBF80)), "f"(x));
+  else
+    asm("{.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tfma.rn.f32.bf16 %0, lo, %2, %3;}" : "=f"(d) : "r"(pair), "h"(static_cast<unsigned short>(0xBF80)), "f"(x));
+  return d;
+}
 // pieces of two neighbouring entries: x = h + m + l
 __device__ __forceinline__ void split3(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
   h = pack_bf16(x, y);
-  x -= __uint_as_float(h << 16);
-  y -= __uint_as_float(h & 0xFFFF0000u);
+  x = less<false>(h, x);
+  y = less<true>(h, y);
   m = pack_bf16(x, y);
-  x -= __uint_as_float(m << 16);
-  y -= __uint_as_float(m & 0xFFFF0000u);
-  l = pack_bf16(x, y);
+  l = pack_bf16(less<false>(m, x), less<true>(m, y));
 }
 
 struct ChunkArgs {
@@ -59,9 +68,13 @@ struct ChunkArgs {
   long long q_bs, q_ts, k_bs, k_ts, v_bs, v_ts;
   const float *g, *beta;
   int T, Hk, Hv, c0, n;                      // chunks c0 .. c0 + n of every row
-  __nv_bfloat16* pieces;                     // [B * Hv, n, 6, 64, 64]: T then P
+  __nv_bfloat16* pieces;                     // [B * Hv, n, 6, 64, 64]: T then P, rows swizzled as the products read them
   float* vec;                                // [B * Hv, n, VEC, 64]
+  int* status;
 };
+
+// entry (i, c) of a piece: rows of 128 bytes, 16-byte chunks exchanged within groups of eight rows
+__device__ __forceinline__ int piece_at(int i, int c) { return i * GC + (((c >> 3) ^ (i & 7)) << 3) + (c & 7); }
 
 // Shared: k, q [64, 256 bytes] swizzled; A [64, 68]; T [64, 65]; G (two floats), kn, qn, beta [64].
 constexpr int LA = GC + 4, LT = GC + 1;
@@ -75,6 +88,7 @@ gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
   float* Ts = A + GC * LA;
   float *Gs = Ts + GC * LT, *Gl = Gs + GC, *kn = Gl + GC, *qn = kn + GC, *bs = qn + GC;
   const int ci = blockIdx.x % a.n, bh = blockIdx.x / a.n, b = bh / a.Hv, hv = bh % a.Hv;
+  pdl_trigger();                             // the scan sets up while the last of these run
   const int hk = hv / (a.Hv / a.Hk), t0 = (a.c0 + ci) * GC, n = min(GC, a.T - t0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int e = tid; e < 2 * GC * 16; e += NTH) {
@@ -148,7 +162,7 @@ gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
       uint32_t w[3];
       split3(p[0], p[1], w[0], w[1], w[2]);
 #pragma unroll
-      for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(pc + (3 + s) * PIECE + i * GC + c) = w[s];
+      for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(pc + (3 + s) * PIECE + piece_at(i, c)) = w[s];
     }
   const float glast = Gs[GC - 1], llast = Gl[GC - 1];
   if (tid < GC) {
@@ -187,236 +201,339 @@ gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
     uint32_t w[3];
     split3(Ts[i * LT + c], Ts[i * LT + c + 1], w[0], w[1], w[2]);
 #pragma unroll
-    for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(pc + s * PIECE + i * GC + c) = w[s];
+    for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(pc + s * PIECE + piece_at(i, c)) = w[s];
   }
 }
 
-// Shared: k and q of a chunk [128, 256 bytes], two buffers; three pieces each of T, P [64, 64], S [128, DV], R (later the
-// scaled Vn) and Vn [64, DV]; row factors, two buffers.  A warp has rows 16 mt of k and q, of R, Vn and O, rows 32 mt of the
-// state, and the columns of one half of DV.
-template <int DV>
-constexpr size_t scan_smem() {
-  return 2 * 2 * GC * GD * 2 + 6 * TILE + 3 * (GD + 2 * GC) * DV * 2 + 2 * VEC * GC * sizeof(float);
+// The scan.  Everything is transposed: a lane of tensor memory is a value column, so the state, R and Vn are operands that
+// the products read from tensor memory, written there by the threads that own the column, and k, q, T and P are the
+// operands in shared memory.  All 512 columns (32 bits each) are taken, X = 192 and Y = 320 changing places from chunk to
+// chunk; leading and small parts of a sum are 64 columns apart where nothing else is said:
+//   [0, 192) [448, 512)   pieces of the state; then Vn; then the state's increment, leading [0, 128), small [128, 192) [448, 512)
+//   X, 128 columns        k S; then pieces of R; then of the scaled Vn; then P Vn
+//   Y, 128 columns        q S; then pieces of Vn
+// A warp has 32 value columns and one half of the tokens (of the key dim, in the state): it alone reads and writes its
+// parts of these, so pieces may lie over the sums that they were made of.
+constexpr int CW = 8;                        // computing warps; one issues the products, three copy
+constexpr uint32_t KQ = 4 * TILE;            // k then q of a chunk, each as two tiles of 64 of the key dim
+constexpr uint32_t VT = GC * GD * 2;         // v of a chunk, rows as they are; then O
+constexpr uint32_t kScanTiles = 2 * KQ + 2 * 6 * TILE + 3 * VT;
+constexpr uint32_t kScanSmem = kScanTiles + 2 * VEC * GC * sizeof(float) + 20 * sizeof(uint64_t);
+constexpr uint32_t kMnMajorB = 1u << 16;     // operand B of a product lies with its columns, not its contraction, in rows
+constexpr uint32_t TM = 0;                   // tensor memory that is all of one block's starts at its first column
+
+__device__ __forceinline__ void tmem_st8(uint32_t at, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(at), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+// pieces of 32 entries of a lane: 16 columns each
+__device__ __forceinline__ void put_pieces(const float* x, uint32_t at_h, uint32_t at_m, uint32_t at_l) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    uint32_t h[8], m[8], l[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) split3(x[16 * i + 2 * e], x[16 * i + 2 * e + 1], h[e], m[e], l[e]);
+    tmem_st8(at_h + 8 * i, h);
+    tmem_st8(at_m + 8 * i, m);
+    tmem_st8(at_l + 8 * i, l);
+  }
+}
+// leading + small part of 32 columns
+__device__ __forceinline__ void read_sums(uint32_t hi, uint32_t lo, float* x) {
+  uint32_t c[32];
+  tc::tmem_ld32(hi, reinterpret_cast<uint32_t*>(x));
+  tc::tmem_ld32(lo, c);
+  tc::tmem_ld_wait();
+#pragma unroll
+  for (int e = 0; e < 32; ++e) x[e] += __uint_as_float(c[e]);
 }
 
-template <int DV>
-__global__ void __launch_bounds__(NTH, 1)
+__global__ void __launch_bounds__((CW + 4) * 32, 1)
 gdn_chunk_scan_kernel(ChunkArgs a, const float* S0, float* S_out, __nv_bfloat16* __restrict__ out) {
-  constexpr int NT = DV / 16;                // columns of a warp in eights
-  constexpr int RB = DV * 2;                 // bytes of a row of S, R, Vn
-  constexpr int KQ = 2 * GC * GD * 2;
-  extern __shared__ __align__(128) unsigned char sm8[];
-  const uint32_t kq = smem_addr(sm8), Ts = kq + 2 * KQ, Ps = Ts + 3 * TILE, Ss = Ps + 3 * TILE, Rs = Ss + 3 * GD * RB, Vs = Rs + 3 * GC * RB;
-  float* vec = reinterpret_cast<float*>(sm8 + 2 * KQ + 6 * TILE + 3 * (GD + 2 * GC) * RB);
-  constexpr int SL = GD / DV;
-  const int slice = blockIdx.x % SL, bh = blockIdx.x / SL, b = bh / a.Hv, hv = bh % a.Hv, hk = hv / (a.Hv / a.Hk);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mt = warp >> 1, nh = warp & 1;
-  const int col0 = slice * DV + nh * (DV / 2);         // the warp's columns in the head
-  const int g4 = lane >> 2, c2 = (lane & 3) * 2;
-  // 16-byte chunk of a [*, DV] tile, rows of RB bytes
-  auto at = [&](uint32_t base, int row, int chunk) {
-    if constexpr (RB == 128) return base + sw_off<128>(row, chunk);
-    else return base + static_cast<uint32_t>(row * RB + ((chunk ^ ((row >> 1) & 3)) << 4));
-  };
-  auto put = [&](uint32_t base, int rows, int row, int col, float x, float y) {      // pieces of two entries
-    uint32_t w[3];
-    split3(x, y, w[0], w[1], w[2]);
+  using namespace tc;
+  extern __shared__ __align__(1024) unsigned char scan_sm[];
+  unsigned char *kq = scan_sm, *tp = scan_sm + 2 * KQ, *vs = tp + 2 * 6 * TILE;
+  float* vec = reinterpret_cast<float*>(scan_sm + kScanTiles);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(vec + 2 * VEC * GC);
+  // T and P, and the rows and factors of a chunk, are here
+  uint64_t *tp_full = bars, *row_full = bars + 2;
+  // halves of the state's pieces, R's, the scaled Vn's, Vn's, O in v's place, O's sums read
+  uint64_t *s_full = bars + 4, *r_full = bars + 6, *w_full = bars + 7, *v_full = bars + 8, *o_full = bars + 9, *o_read = bars + 11;
+  uint64_t *ks_done = bars + 12, *qs_done = bars + 13, *vn_done = bars + 14, *inc_done = bars + 15, *o_done = bars + 16;
+  uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 18);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(slot + 1);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int bh = blockIdx.x, b = bh / a.Hv, hv = bh % a.Hv, hk = hv / (a.Hv / a.Hk);
+  if (smem_u32(scan_sm) & 1023) {            // the swizzled tiles start on a 1024-byte boundary, the same in every thread
+    if (tid == 0) atomicCAS(a.status, kStatusOk, kStatusBadShape);
+    return;
+  }
+  if (tid == 0) {
+    for (int i = 0; i < 18; ++i) mbar_init(&bars[i], i == 2 || i == 3 ? 3 : i >= 4 && i < 12 ? CW : 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == CW) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_wait();                                // the pieces and factors are written
+
+  // 168 registers a thread at launch: 56 for the last four warps and 224 for the others are the same sum
+  if (warp >= CW) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp == CW) {
+      const uint32_t base = smem_u32(scan_sm);
+      auto load_tp = [&](int ci) {
+        if (elect_one()) {
+          mbar_expect_tx(&tp_full[ci & 1], 6 * TILE);
+          bulk_load(tp + (ci & 1) * 6 * TILE, a.pieces + (static_cast<long long>(bh) * a.n + ci) * 6 * PIECE, 6 * TILE, &tp_full[ci & 1]);
+        }
+        __syncwarp();
+      };
+      constexpr uint32_t n64 = make_idesc_bf16(128, 64), inc64 = n64 | kMnMajorB, inc128 = make_idesc_bf16(128, 128) | kMnMajorB;
+      // 128 value columns x 64 tokens: the pieces of one half of each warp's part of the state with the rows of k or q
+      auto rows = [&](uint32_t to, uint64_t d, int half) {
 #pragma unroll
-    for (int s = 0; s < 3; ++s)
-      asm volatile("st.shared.b32 [%0], %1;" ::"r"(at(base + s * rows * RB, row, col >> 3) + (col & 7) * 2), "r"(w[s]) : "memory");
-  };
-  auto load_kq = [&](int ci, int buf) {
-    const int t0 = (a.c0 + ci) * GC, n = min(GC, a.T - t0);
-    for (int e = tid; e < 2 * GC * 16; e += NTH) {
-      const int which = e >> 10, r = (e >> 4) & 63, c = e & 15, t = t0 + min(r, n - 1);
-      const __nv_bfloat16* src = which ? a.q + b * a.q_bs + t * a.q_ts : a.k + b * a.k_bs + t * a.k_ts;
-      cp_async16(kq + buf * KQ + sw_off<256>(which * GC + r, c), src + hk * GD + c * 8, r < n);
-    }
-    const float* vp = a.vec + (static_cast<long long>(bh) * a.n + ci) * VEC * GC;
-    if (tid < VEC * GC / 4) cp_async16(smem_addr(vec + buf * VEC * GC) + tid * 16, vp + tid * 4, true);
-  };
-  auto load_tp = [&](int ci, int which) {    // 0: T, 1: P
-    const __nv_bfloat16* pc = a.pieces + (static_cast<long long>(bh) * a.n + ci) * 6 * PIECE + which * 3 * PIECE;
-    for (int e = tid; e < 3 * GC * 8; e += NTH) {
-      const int s = e >> 9, r = (e >> 3) & 63, c = e & 7;
-      cp_async16((which ? Ps : Ts) + s * TILE + sw_off<128>(r, c), pc + s * PIECE + r * GC + c * 8, true);
-    }
-  };
-  // three pieces of B fragments: rows k0 .. k0 + 16 of a [*, DV] tile, the warp's columns
-  auto load_b = [&](uint32_t base, int rows, int k0, uint32_t (*f)[NT][2]) {
+        for (int p = 2; p >= 0; --p)
 #pragma unroll
-    for (int s = 0; s < 3; ++s)
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t at = (i >> 1) ? (p == 2 ? 448u : 64u + 32u * p) : (p == 2 ? 128u : 32u * p);
+            umma_ts(TM + to + (p ? 64 : 0), TM + at + 16 * half + 8 * (i & 1), desc_adv(d, (i >> 1) * TILE + half * 64 + (i & 1) * 32), n64,
+                    p != 1 && half == 0 && i == 0 ? 0u : 1u);
+          }
+      };
+      // pieces of R or Vn with those of T or P, lower triangular: 16 tokens j reach the rows from j on
+      auto product6 = [&](uint32_t to, uint32_t from, uint64_t d, uint64_t* done) {
+        if (elect_one()) {
+          constexpr int pa[6] = {0, 1, 2, 0, 1, 0}, pb[6] = {2, 1, 0, 1, 0, 0};
 #pragma unroll
-      for (int j = 0; j < NT; j += 2)
-        ldsm4t(at(base + s * rows * RB, k0 + (lane & 15), nh * (DV / 16) + j + (lane >> 4)), f[s][j][0], f[s][j][1], f[s][j + 1][0], f[s][j + 1][1]);
-  };
-  // leading and small products of 32-bit [64, 64] pieces with a 32-bit [64, DV] tile; both lower triangular in blocks
-  auto product6 = [&](uint32_t base, uint32_t tile, float (*hi)[4], float (*lo)[4]) {
-    for (int s = 0; s <= mt; ++s) {
-      uint32_t fa[3][4], fb[3][NT][2];
+          for (int i = 0; i < 6; ++i)
 #pragma unroll
-      for (int p = 0; p < 3; ++p)
-        ldsm4(base + p * TILE + sw_off<128>(mt * 16 + (lane & 15), 2 * s + (lane >> 4)), fa[p][0], fa[p][1], fa[p][2], fa[p][3]);
-      load_b(tile, GC, s * 16, fb);
+            for (int s = 0; s < GC / 16; ++s)
+              umma_ts(TM + to + (i == 5 ? 0 : 64) + 16 * s, TM + from + (pa[i] == 2 ? 64u : 16u * pa[i]) + 32 * (s >> 1) + 8 * (s & 1),
+                      desc_adv(d, pb[i] * TILE + s * (16 * 128 + 32)), make_idesc_bf16(128, 64 - 16 * s), (i == 0 || i == 5) && s == 0 ? 0u : 1u);
+          umma_commit(done);
+        }
+        __syncwarp();
+      };
+      auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity, abort_flag, a.status, kStatusWaitTimeoutMma); };
+      auto chunk = [&](int ci) {
+        const uint32_t ph = ci & 1, X = 192 + 128 * ph, Y = 320 - 128 * ph;
+        const uint32_t twice = (ci >> 1) & 1;
+        const uint32_t at_k = base + (ci & 1) * KQ;
+        const uint64_t kd = make_smem_desc(at_k), td = make_smem_desc(base + 2 * KQ + (ci & 1) * 6 * TILE);
+        if ((ci > 0 && !wait(&o_done[ph ^ 1], ((ci - 1) >> 1) & 1)) || !wait(&s_full[0], ph)) return false;      // X held Vn
+        tc_fence_after();
+        if (elect_one()) rows(X, kd, 0);
+        __syncwarp();
+        if (!wait(&s_full[1], ph)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+          rows(X, kd, 1);
+          umma_commit(ks_done);
+        }
+        __syncwarp();
+        if (ci + 1 < a.n) load_tp(ci + 1);   // the last chunk's products have all retired: its buffer is free
+        if (ci > 0 && !wait(o_read, ph ^ 1)) return false;     // Y held O
+        tc_fence_after();
+        if (elect_one()) {
+          rows(Y, desc_adv(kd, 2 * TILE), 0);
+          rows(Y, desc_adv(kd, 2 * TILE), 1);
+          umma_commit(qs_done);
+        }
+        __syncwarp();
+        if (!wait(&tp_full[ph], twice) || !wait(qs_done, ph) || !wait(r_full, ph)) return false;
+        tc_fence_after();
+        product6(0, X, td, vn_done);
+        if (ci + 1 < a.n && !wait(&row_full[ph ^ 1], ((ci + 1) >> 1) & 1)) return false;       // here, where there is time
+        if (!wait(w_full, ph)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t kn = make_smem_desc_mn(at_k, TILE);
 #pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        mma16816(lo[j], fa[2], fb[0][j][0], fb[0][j][1]);
-        mma16816(lo[j], fa[1], fb[1][j][0], fb[1][j][1]);
-        mma16816(lo[j], fa[0], fb[2][j][0], fb[2][j][1]);
-        mma16816(lo[j], fa[1], fb[0][j][0], fb[0][j][1]);
-        mma16816(lo[j], fa[0], fb[1][j][0], fb[1][j][1]);
-        mma16816(hi[j], fa[0], fb[0][j][0], fb[0][j][1]);
+          for (int p = 2; p >= 0; --p)
+#pragma unroll
+            for (int s = 0; s < GC / 16; ++s) {
+              const uint32_t at = TM + X + (p == 2 ? 64u : 16u * p) + 32 * (s >> 1) + 8 * (s & 1);
+              if (p == 0) {
+                umma_ts(TM, at, desc_adv(kn, s * 16 * 128), inc128, s ? 1u : 0u);
+              } else {
+                umma_ts(TM + 128, at, desc_adv(kn, s * 16 * 128), inc64, p == 2 && s == 0 ? 0u : 1u);
+                umma_ts(TM + 448, at, desc_adv(kn, TILE + s * 16 * 128), inc64, p == 2 && s == 0 ? 0u : 1u);
+              }
+            }
+          umma_commit(inc_done);
+        }
+        __syncwarp();
+        if (!wait(v_full, ph) || !wait(inc_done, ph)) return false;      // P Vn goes where the scaled Vn was
+        tc_fence_after();
+        product6(X, Y, desc_adv(td, 3 * TILE), &o_done[ph]);
+        return true;
+      };
+      load_tp(0);
+      bool ok = wait(&row_full[0], 0);
+      for (int ci = 0; ci < a.n && ok; ++ci) ok = chunk(ci);
+    } else {
+      const int id = tid - (CW + 1) * 32;    // three warps: O to memory, the rows and factors of the chunk after the next from there
+      auto load = [&](int ci) {
+        const int t0 = (a.c0 + ci) * GC, n = min(GC, a.T - t0), buf = ci & 1;
+        const uint32_t dk = smem_u32(kq) + buf * KQ, dv = smem_u32(vs) + ci % 3 * VT;
+        const __nv_bfloat16 *kp = a.k + b * a.k_bs + t0 * a.k_ts + hk * GD, *qp = a.q + b * a.q_bs + t0 * a.q_ts + hk * GD;
+        const __nv_bfloat16* vp = a.v + b * a.v_bs + t0 * a.v_ts + hv * GD;
+#pragma unroll 2
+        for (int e = id; e < GC * 16; e += 96) {
+          const int r = e >> 4, c = e & 15, t = min(r, n - 1);
+          const uint32_t at = dk + (c >> 3) * TILE + sw_off<128>(r, c & 7);
+          cp_async16(at, kp + t * a.k_ts + c * 8, r < n);
+          cp_async16(at + 2 * TILE, qp + t * a.q_ts + c * 8, r < n);
+          cp_async16(dv + e * 16, vp + t * a.v_ts + c * 8, r < n);
+        }
+        const float* fp = a.vec + (static_cast<long long>(bh) * a.n + ci) * VEC * GC;
+        if (id < VEC * GC / 4) cp_async16(smem_u32(vec + buf * VEC * GC) + id * 16, fp + id * 4, true);
+        cp_commit();
+        cp_wait<0>();
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&row_full[buf]);
+      };
+      load(0);
+      if (a.n > 1) load(1);
+      auto wait = [&](uint64_t* bar, uint32_t parity) { return mbar_wait_warp(bar, parity, abort_flag, a.status, kStatusWaitTimeoutProducer); };
+      for (int ci = 0; ci <= a.n; ++ci) {
+        if (ci > 0) {
+          if (!wait(&o_full[(ci - 1) & 1], ((ci - 1) >> 1) & 1)) break;
+          const int t0 = (a.c0 + ci - 1) * GC;
+#pragma unroll 2
+          for (int e = id; e < GC * 16; e += 96) {
+            const int t = t0 + (e >> 4);
+            if (t < a.T)
+              *reinterpret_cast<uint4*>(out + ((static_cast<long long>(b) * a.T + t) * a.Hv + hv) * GD + (e & 15) * 8) =
+                  *reinterpret_cast<const uint4*>(vs + (ci - 1) % 3 * VT + e * 16);
+          }
+        }
+        if (ci + 2 < a.n) {
+          if (!wait(&o_done[ci & 1], (ci >> 1) & 1)) break;
+          // all of O is read before v takes its place (a warp that is here saw o_done, which the others see too)
+          asm volatile("bar.sync 1, 96;" ::: "memory");
+          load(ci + 2);
+        }
       }
     }
-  };
-
-  float S[2][NT][4];                         // rows 32 mt + 16 i + g4 (+ 8), columns col0 + 8 j + c2
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    const int w = warp >> 2;                 // half of the tokens; of the key dim in the state
+    const int col = (warp & 3) * 32 + lane;  // value column
+    const uint32_t tl = TM + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const uint32_t lo_s = tl + (w ? 448u : 128u);
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      const bool ok = mbar_wait_warp(bar, parity, abort_flag, a.status, kStatusWaitTimeoutEpilogue);
+      tc_fence_after();
+      return ok;
+    };
+    auto arrive = [&](uint64_t* bar) {       // what this warp stored in tensor memory is there
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    float S[64];                             // the state: row 64 w + e, this thread's column
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+    for (int e = 0; e < 64; ++e) S[e] = S0 ? S0[(static_cast<long long>(bh) * GD + 64 * w + e) * GD + col] : 0.f;
+    auto put_state = [&](int h) {
+      put_pieces(S + 32 * h, tl + 64 * w + 16 * h, tl + 64 * w + 32 + 16 * h, lo_s + 16 * h);
+      arrive(&s_full[h]);
+    };
+    put_state(0);
+    put_state(1);
+    float vv[32];                            // v of the chunk at hand, read while the state's increment of the last one is formed
+    uint32_t ob[16];                         // O of the last chunk, stored while Vn of the one at hand is formed
+    auto rows_of = [&](int ci) { return reinterpret_cast<unsigned short*>(vs + ci % 3 * VT) + 32 * w * GD + col; };
+    auto load_v = [&](int ci) {
+      if (!wait(&row_full[ci & 1], (ci >> 1) & 1)) return false;
+      const unsigned short* vr = rows_of(ci);
 #pragma unroll
-    for (int j = 0; j < NT; ++j)
+      for (int e = 0; e < 32; ++e) vv[e] = __uint_as_float(static_cast<uint32_t>(vr[e * GD]) << 16);
+      return true;
+    };
+    auto store_o = [&](int ci) {             // each where its thread read v
+      unsigned short* vr = rows_of(ci);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        vr[2 * e * GD] = static_cast<unsigned short>(ob[e]);
+        vr[(2 * e + 1) * GD] = static_cast<unsigned short>(ob[e] >> 16);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&o_full[ci & 1]);
+    };
+    bool ok = load_v(0);
+    for (int ci = 0; ci < a.n && ok; ++ci) {
+      const uint32_t ph = ci & 1, X = tl + (ph ? 320u : 192u) + 32 * w, Y = tl + (ph ? 192u : 320u) + 32 * w;
+      const float* vf = vec + ph * VEC * GC + 32 * w;
+      float x[32], q[32], f[32];
+      if (!(ok = wait(ks_done, ph))) break;
+      read_sums(X, X + 64, x);
+#pragma unroll
+      for (int e = 0; e < 32; e += 4) {
+        const float4 bt = *reinterpret_cast<const float4*>(vf + e), f1 = *reinterpret_cast<const float4*>(vf + GC + e);
+        x[e] = fmaf(bt.x, vv[e], -(f1.x * x[e]));              // the product with v is the large one: it does not round
+        x[e + 1] = fmaf(bt.y, vv[e + 1], -(f1.y * x[e + 1]));
+        x[e + 2] = fmaf(bt.z, vv[e + 2], -(f1.z * x[e + 2]));
+        x[e + 3] = fmaf(bt.w, vv[e + 3], -(f1.w * x[e + 3]));
+      }
+      put_pieces(x, X, X + 16, X + 64);
+      arrive(r_full);
+      if (ci > 0) store_o(ci - 1);
+      if (!(ok = wait(qs_done, ph))) break;
+      read_sums(Y, Y + 64, q);
+#pragma unroll
+      for (int e = 0; e < 32; e += 4) {
+        const float4 f2 = *reinterpret_cast<const float4*>(vf + 2 * GC + e);
+        q[e] *= f2.x;
+        q[e + 1] *= f2.y;
+        q[e + 2] *= f2.z;
+        q[e + 3] *= f2.w;
+        *reinterpret_cast<float4*>(f + e) = *reinterpret_cast<const float4*>(vf + 3 * GC + e);
+      }
+      const float gC = vec[ph * VEC * GC + 4 * GC];
+      if (!(ok = wait(vn_done, ph))) break;
+      read_sums(tl + 32 * w, tl + 64 + 32 * w, x);
+#pragma unroll
+      for (int e = 0; e < 32; ++e) f[e] *= x[e];
+      put_pieces(f, X, X + 16, X + 64);
+      arrive(w_full);
+      put_pieces(x, Y, Y + 16, Y + 64);
+      arrive(v_full);
+      if (ci + 1 < a.n && !(ok = load_v(ci + 1))) break;
+      if (!(ok = wait(inc_done, ph))) break;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int r = mt * 32 + i * 16 + g4 + 8 * h;
-        const float2 x = S0 ? *reinterpret_cast<const float2*>(S0 + static_cast<long long>(bh) * GD * GD + r * GD + col0 + j * 8 + c2)
-                            : make_float2(0.f, 0.f);
-        S[i][j][2 * h] = x.x;
-        S[i][j][2 * h + 1] = x.y;
-        put(Ss, GD, r, nh * (DV / 2) + j * 8 + c2, x.x, x.y);
-      }
-  load_kq(0, 0);
-  load_tp(0, 0);
-  cp_commit();
-  for (int ci = 0; ci < a.n; ++ci) {
-    const int buf = ci & 1, t0 = (a.c0 + ci) * GC, n = min(GC, a.T - t0);
-    const float* vf = vec + buf * VEC * GC;
-    const uint32_t kqb = kq + buf * KQ;
-    cp_wait<0>();
-    __syncthreads();                         // k, q, factors and T are here, the state's pieces are written, P and the other buffer are free
-    load_tp(ci, 1);
-    cp_commit();
-    if (ci + 1 < a.n) load_kq(ci + 1, buf ^ 1);
-    cp_commit();
-    uint32_t vv[2][NT];
+        read_sums(tl + 64 * w + 32 * h, lo_s + 32 * h, x);
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const int r = mt * 16 + g4 + 8 * h;
-        vv[h][j] = r < n ? *reinterpret_cast<const uint32_t*>(a.v + b * a.v_bs + (t0 + r) * a.v_ts + hv * GD + col0 + j * 8 + c2) : 0u;
+        for (int e = 0; e < 32; ++e) S[32 * h + e] = S[32 * h + e] * gC + x[e];
       }
-    // k S and q S
-    float xk[NT][4] = {}, xq[NT][4] = {}, lk[NT][4] = {}, lq[NT][4] = {};
-#pragma unroll 2
-    for (int s = 0; s < GD / 16; ++s) {
-      uint32_t fk[4], fq[4], fb[3][NT][2];
-      const int r = mt * 16 + (lane & 15), c = 2 * s + (lane >> 4);
-      ldsm4(kqb + sw_off<256>(r, c), fk[0], fk[1], fk[2], fk[3]);
-      ldsm4(kqb + sw_off<256>(GC + r, c), fq[0], fq[1], fq[2], fq[3]);
-      load_b(Ss, GD, s * 16, fb);
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        mma16816(lk[j], fk, fb[2][j][0], fb[2][j][1]);
-        mma16816(lq[j], fq, fb[2][j][0], fb[2][j][1]);
-        mma16816(lk[j], fk, fb[1][j][0], fb[1][j][1]);
-        mma16816(lq[j], fq, fb[1][j][0], fb[1][j][1]);
-        mma16816(xk[j], fk, fb[0][j][0], fb[0][j][1]);
-        mma16816(xq[j], fq, fb[0][j][0], fb[0][j][1]);
+      if (ci + 1 < a.n) {
+        put_state(0);
+        put_state(1);
       }
+      if (!(ok = wait(&o_done[ph], (ci >> 1) & 1))) break;
+      read_sums(X, X + 64, x);
+      arrive(o_read);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) ob[e] = pack_bf16(q[2 * e] + x[2 * e], q[2 * e + 1] + x[2 * e + 1]);
     }
+    if (ok) store_o(a.n - 1);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = mt * 16 + g4 + 8 * h;
-      const float bt = vf[r], f1 = vf[GC + r], f2 = vf[2 * GC + r];
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const float x = bt * __uint_as_float(vv[h][j] << 16) - f1 * (xk[j][2 * h] + lk[j][2 * h]);
-        const float y = bt * __uint_as_float(vv[h][j] & 0xFFFF0000u) - f1 * (xk[j][2 * h + 1] + lk[j][2 * h + 1]);
-        put(Rs, GC, r, nh * (DV / 2) + j * 8 + c2, x, y);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          xq[j][2 * h + e] = f2 * (xq[j][2 * h + e] + lq[j][2 * h + e]);
-          xk[j][2 * h + e] = lk[j][2 * h + e] = lq[j][2 * h + e] = 0.f;
-        }
-      }
-    }
-    __syncthreads();
-    product6(Ts, Rs, xk, lk);                // Vn
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) xk[j][e] += lk[j][e];
-    __syncthreads();                         // everyone has read R and T
-    if (ci + 1 < a.n) load_tp(ci + 1, 0);
-    cp_commit();
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = mt * 16 + g4 + 8 * h;
-      const float f3 = vf[3 * GC + r];
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const int c = nh * (DV / 2) + j * 8 + c2;
-        put(Vs, GC, r, c, xk[j][2 * h], xk[j][2 * h + 1]);
-        put(Rs, GC, r, c, f3 * xk[j][2 * h], f3 * xk[j][2 * h + 1]);
-      }
-    }
-    cp_wait<2>();                            // P; the next chunk's k, q and T may still be on their way
-    __syncthreads();
-    {                                        // the state: k^T (scaled Vn)
-      float hi[2][NT][4] = {}, lo[2][NT][4] = {};
-#pragma unroll
-      for (int s = 0; s < GC / 16; ++s) {
-        uint32_t fa[2][4], fb[3][NT][2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)          // stored [token, key dim]: rows and columns of the fragment change places
-          ldsm4t(kqb + sw_off<256>(s * 16 + (lane & 7) + ((lane >> 4) << 3), mt * 4 + 2 * i + ((lane >> 3) & 1)), fa[i][0], fa[i][1], fa[i][2], fa[i][3]);
-        load_b(Rs, GC, s * 16, fb);
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int j = 0; j < NT; ++j) {
-            mma16816(lo[i][j], fa[i], fb[2][j][0], fb[2][j][1]);
-            mma16816(lo[i][j], fa[i], fb[1][j][0], fb[1][j][1]);
-            mma16816(hi[i][j], fa[i], fb[0][j][0], fb[0][j][1]);
-          }
-      }
-      const float gC = vf[4 * GC];
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) S[i][j][e] = S[i][j][e] * gC + (hi[i][j][e] + lo[i][j][e]);
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-            put(Ss, GD, mt * 32 + i * 16 + g4 + 8 * h, nh * (DV / 2) + j * 8 + c2, S[i][j][2 * h], S[i][j][2 * h + 1]);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) xk[j][e] = 0.f;
-    product6(Ps, Vs, xk, lq);                // O
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = mt * 16 + g4 + 8 * h;
-      if (r < n) {
-        __nv_bfloat16* o = out + ((static_cast<long long>(b) * a.T + t0 + r) * a.Hv + hv) * GD + col0 + c2;
-#pragma unroll
-        for (int j = 0; j < NT; ++j)
-          *reinterpret_cast<uint32_t*>(o + j * 8) = pack_bf16(xq[j][2 * h] + (xk[j][2 * h] + lq[j][2 * h]),
-                                                              xq[j][2 * h + 1] + (xk[j][2 * h + 1] + lq[j][2 * h + 1]));
-      }
-    }
+    for (int e = 0; e < 64; ++e) S_out[(static_cast<long long>(bh) * GD + 64 * w + e) * GD + col] = S[e];
   }
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        *reinterpret_cast<float2*>(S_out + static_cast<long long>(bh) * GD * GD + (mt * 32 + i * 16 + g4 + 8 * h) * GD + col0 + j * 8 + c2) =
-            make_float2(S[i][j][2 * h], S[i][j][2 * h + 1]);
+  __syncthreads();
+  if (*abort_flag) {
+    for (int i = 0; i < 64; ++i) __nanosleep(10000);         // let a copy in flight land before shared memory goes away
+  }
+  if (warp == CW) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(TM), "r"(512));
 }
 
 constexpr size_t kChunkBytes = 6 * PIECE * 2 + VEC * GC * sizeof(float);      // workspace of one chunk of one head
@@ -437,28 +554,24 @@ size_t gdn_chunk_workspace(int B, int T, int Hv) {
 const char* gdn_chunk_fwd(const void* q, const void* k, const void* v, long long q_bs, long long q_ts, long long k_bs,
                           long long k_ts, long long v_bs, long long v_ts, const float* g, const float* beta,
                           const float* S0, float* S_out, void* out, int B, int T, int Hk, int Hv, int KD, int VD,
-                          bool l2norm, float eps, void* workspace, cudaStream_t stream) {
+                          bool l2norm, float eps, void* workspace, int* status, cudaStream_t stream) {
   if (KD != GD || VD != GD) return "gdn_chunk_fwd: key and value head dim must be 128";
   if (Hk <= 0 || Hv % Hk) return "gdn_chunk_fwd: value heads must be a multiple of key heads";
   if (B == 0 || T == 0) return nullptr;
   if (!FERRL_ONCE_PER_DEVICE(
           cudaFuncSetAttribute(gdn_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPrepSmem)) == cudaSuccess &&
-          cudaFuncSetAttribute(gdn_chunk_scan_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(scan_smem<64>())) == cudaSuccess &&
-          cudaFuncSetAttribute(gdn_chunk_scan_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(scan_smem<32>())) == cudaSuccess))
+          cudaFuncSetAttribute(gdn_chunk_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kScanSmem)) == cudaSuccess))
     return "gdn_chunk_fwd: cannot reserve shared memory";
   const int round = chunk_round(B, T, Hv), chunks = (T + GC - 1) / GC;
   ChunkArgs a{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v),
-              q_bs, q_ts, k_bs, k_ts, v_bs, v_ts, g, beta, T, Hk, Hv, 0, 0, static_cast<__nv_bfloat16*>(workspace), nullptr};
-  // One CTA fits an SM: narrow slices only where they all run at once.
-  const bool narrow = static_cast<long long>(B) * Hv * 4 <= 148;
+              q_bs, q_ts, k_bs, k_ts, v_bs, v_ts, g, beta, T, Hk, Hv, 0, 0, static_cast<__nv_bfloat16*>(workspace), nullptr, status};
   for (int c0 = 0; c0 < chunks; c0 += round) {
     a.c0 = c0;
     a.n = std::min(round, chunks - c0);
     a.vec = reinterpret_cast<float*>(a.pieces + static_cast<long long>(B) * Hv * a.n * 6 * PIECE);
     const float* from = c0 == 0 ? S0 : S_out;
     gdn_chunk_prep_kernel<<<a.n * B * Hv, NTH, kPrepSmem, stream>>>(a, l2norm ? 1 : 0, eps);
-    if (narrow) gdn_chunk_scan_kernel<32><<<B * Hv * 4, NTH, scan_smem<32>(), stream>>>(a, from, S_out, static_cast<__nv_bfloat16*>(out));
-    else gdn_chunk_scan_kernel<64><<<B * Hv * 2, NTH, scan_smem<64>(), stream>>>(a, from, S_out, static_cast<__nv_bfloat16*>(out));
+    launch_pdl(gdn_chunk_scan_kernel, dim3(B * Hv), dim3((CW + 4) * 32), kScanSmem, stream, a, from, S_out, static_cast<__nv_bfloat16*>(out));
     count_launch(2);
   }
   return cudaGetLastError() == cudaSuccess ? nullptr : "gdn_chunk_fwd launch failed";
