@@ -1169,6 +1169,30 @@ void kv_append_paged(const Tensor& k, const Tensor& v, Tensor kc, Tensor vc, con
                                      kc.size(2) * kc.size(3), stream()));
 }
 
+// k, v [P, L, Hkv, D] into pools [P * ppr + P * G * ppr, page, Hkv, D]; false: rows that are not whole 16-byte pieces of the
+// pools' type on 16-byte boundaries, and nothing done
+bool kv_prefill_paged(const Tensor& k, const Tensor& v, Tensor kc, Tensor vc, const Tensor& full, int64_t ppr, int64_t G) {
+  c10::cuda::CUDAGuard guard(k.device());
+  TORCH_CHECK(k.dim() == 4 && v.sizes() == k.sizes() && kc.dim() == 4 && vc.sizes() == kc.sizes() && kc.is_contiguous() && vc.is_contiguous() &&
+                  kc.size(2) == k.size(2) && kc.size(3) == k.size(3) && ppr >= 0 && G >= 1 && kc.size(0) == k.size(0) * ppr * (1 + G) &&
+                  full.scalar_type() == at::kLong && full.is_contiguous() && full.numel() == k.size(0) && full.is_cuda(),
+              "kv_prefill_paged: layout");
+  const int64_t e = k.element_size(), HD = k.size(2) * k.size(3);
+  auto pieces = [&](const Tensor& t) {
+    return t.is_cuda() && t.scalar_type() == kc.scalar_type() && (t.size(3) == 1 || t.stride(3) == 1) && (t.size(2) == 1 || t.stride(2) == t.size(3)) &&
+           t.stride(0) * e % 16 == 0 && t.stride(1) * e % 16 == 0 && t.stride(0) >= 0 && t.stride(1) >= 0 &&
+           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  };
+  if (vc.scalar_type() != kc.scalar_type() || !pieces(k) || !pieces(v) || HD * e % 16 || k.size(0) > 65535 ||
+      (reinterpret_cast<uintptr_t>(kc.data_ptr()) | reinterpret_cast<uintptr_t>(vc.data_ptr())) % 16)
+    return false;
+  const int64_t u = 16 / e;
+  FERRL_CHECK(ferrl::kv_prefill_paged(k.data_ptr(), v.data_ptr(), k.stride(0) / u, k.stride(1) / u, v.stride(0) / u, v.stride(1) / u,
+                                      kc.data_ptr(), vc.data_ptr(), reinterpret_cast<const long long*>(full.data_ptr<int64_t>()), k.size(0), k.size(1), ppr,
+                                      kc.size(1), G, HD / u, stream()));
+  return true;
+}
+
 static ferrl::GluAct glu_act(int64_t act, double alpha, double limit) {
   TORCH_CHECK(act >= ferrl::kActSilu && act <= ferrl::kActClipped && (act != ferrl::kActClipped || limit >= 0), "glu: unknown activation");
   return ferrl::GluAct{static_cast<int>(act), static_cast<float>(alpha), static_cast<float>(limit)};
@@ -2083,6 +2107,7 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("qk_norm_rope_fwd(Tensor q, Tensor k, Tensor? qw, Tensor? kw, Tensor cos, Tensor sin, Tensor pos, int pos_div, float eps, bool zc) -> (Tensor, Tensor)", &qk_norm_rope_fwd);
   m.def("qk_norm_rope_bwd(Tensor q, Tensor k, Tensor? qw, Tensor? kw, Tensor cos, Tensor sin, Tensor pos, int pos_div, float eps, bool zc, Tensor dq, Tensor dk, Tensor(a!) dq_in, Tensor(b!) dk_in) -> ()", &qk_norm_rope_bwd);
   m.def("kv_append(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor kv_len) -> ()", &kv_append);
+  m.def("kv_prefill_paged(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor full, int ppr, int G) -> bool", &kv_prefill_paged);
   m.def("kv_append_paged(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor kv_len, Tensor table) -> ()", &kv_append_paged);
   m.def("glu_fwd(Tensor gu, int act, float alpha=0.0, float limit=0.0, Tensor? token_of=None) -> Tensor", &glu_fwd);
   m.def("glu_bwd(Tensor gu, Tensor dout, int act, float alpha=0.0, float limit=0.0) -> Tensor", &glu_bwd);

@@ -132,7 +132,9 @@ class DenseLayer(nn.Module):
         k = k.reshape(B, S, self.hkv, self.D)
         v = v.reshape(B, S, self.hkv, self.D)
         q, k = ops.qk_norm_rope(q, k, self.q_norm, self.k_norm, self.eps, cos, sin, positions)
-        if kv_out is not None:
+        if callable(kv_out):
+            kv_out(k, v)
+        elif kv_out is not None:
             kv_out[0][:, :S].copy_(k)
             kv_out[1][:, :S].copy_(v)
         a = ops.attention(q, k, v, scale=self.scale, causal=True, softmax_fp32=True)
@@ -599,6 +601,23 @@ class DensePagedDecoder(DenseCachedDecoder):
     def _prefix(self):
         return (self.prefix_len, self.group) if self.share_prefix else None
 
+    def _store(self, i: int, k: torch.Tensor, v: torch.Tensor, full: torch.Tensor):
+        """Layer ``i``'s prompt rows ``[P, L, Hkv, D]`` into the shared pages; the tail of every prompt (< PAGE tokens past
+        its ``full`` pages) goes to the first private page of each of its rows."""
+        page, ppr = self.PAGE, self.pages_per_row
+        if ops.native(k):
+            from ..ops import cuda as _c
+            if _c.kv_prefill_paged(self.k[i], self.v[i], k, v, full, ppr, self.group):
+                return
+        P, L, hkv, D = k.shape
+        tail_idx = (full[:, None] * page + torch.arange(page, device=k.device)[None, :]).clamp(max=L - 1)     # [P, PAGE]
+        first_private = (self.shared_pages + torch.arange(self.batch, device=k.device) * ppr).long()
+        Lp = min(L, ppr * page)
+        for pool, src in ((self.k[i], k), (self.v[i], v)):
+            pool[:self.shared_pages].view(P, ppr * page, hkv, D)[:, :Lp] = src[:, :Lp]
+            tail = torch.gather(src, 1, tail_idx[:, :, None, None].expand(P, page, hkv, D)).to(pool.dtype)
+            pool[first_private] = tail.repeat_interleave(self.group, dim=0)
+
     @torch.no_grad()
     def prefill(self, ids: torch.Tensor, lens: torch.Tensor, rows: Optional[torch.Tensor] = None,
                 at: Optional[tuple] = None) -> torch.Tensor:
@@ -611,12 +630,10 @@ class DensePagedDecoder(DenseCachedDecoder):
         if P != self.prompts:
             raise ValueError(f"expected {self.prompts} prompts, got {P}")
         dev = ids.device
-        hkv, D = self.k[0].shape[2], self.k[0].shape[3]
-        tmp = [(torch.empty(P, L, hkv, D, dtype=m.dtype, device=dev), torch.empty(P, L, hkv, D, dtype=m.dtype, device=dev))
-               for _ in m.layers]
-        h = m.forward_hidden(ids, self.comm, merged=True, kv_out=tmp, detached=True, pick=_wanted(P, lens, at, ids.device))
         ppr = self.pages_per_row
         full = (lens // page).to(torch.int64)                                  # shared (full) pages per prompt
+        h = m.forward_hidden(ids, self.comm, merged=True, detached=True, pick=_wanted(P, lens, at, ids.device),
+                             kv_out=[lambda k, v, i=i: self._store(i, k, v, full) for i in range(len(m.layers))])
         # block table: shared page ids first, then the row's private pages
         j = torch.arange(ppr, device=dev)[None, :]
         p_of_row = torch.arange(P, device=dev).repeat_interleave(G)
@@ -625,15 +642,6 @@ class DensePagedDecoder(DenseCachedDecoder):
         private_id = self.shared_pages + torch.arange(self.batch, device=dev)[:, None] * ppr + (j - full_r).clamp(min=0)
         self.table.copy_(torch.where(j < full_r, shared_id, private_id).to(torch.int32))
         self.prefix_len.copy_((full * page).to(torch.int32))
-        # tail of every prompt (< PAGE tokens) goes to the first private page of each of its rows
-        tail_idx = (full[:, None] * page + torch.arange(page, device=dev)[None, :]).clamp(max=L - 1)     # [P, PAGE]
-        first_private = (self.shared_pages + torch.arange(self.batch, device=dev) * ppr).long()
-        Lp = min(L, ppr * page)
-        for i in range(len(m.layers)):
-            for pool, src in ((self.k[i], tmp[i][0]), (self.v[i], tmp[i][1])):
-                pool[:self.shared_pages].view(P, ppr * page, hkv, D)[:, :Lp] = src[:, :Lp]
-                tail = torch.gather(src, 1, tail_idx[:, :, None, None].expand(P, page, hkv, D))
-                pool[first_private] = tail.repeat_interleave(G, dim=0)
         self.kv_len.copy_(lens.to(torch.int32).repeat_interleave(G))
         last = ops.rmsnorm(h, m.final_norm, m.spec.rms_norm_eps)
         return ops.lora_linear(last, m.head_weight(), None, None).float()

@@ -601,6 +601,13 @@ def kv_append_paged(k_pool, v_pool, k, v, kv_len, table):
         (B, v.shape[-2] * v.shape[-1]), (v.stride(0), 1), v.storage_offset()), k_pool, v_pool, kv_len, table)
 
 
+def kv_prefill_paged(k_pool, v_pool, k, v, full, pages_per_row, group):
+    """Store the K/V ``[P, L, Hkv, D]`` of right-padded prompts in the paged pools: every row in its prompt's shared pages, and the
+    page that begins at ``full[p]`` whole pages in the first private page of each of the prompt's ``group`` rows.  False, and
+    nothing stored, where the rows are not whole 16-byte pieces of the pools' type."""
+    return lib().kv_prefill_paged(k, v, k_pool, v_pool, full, pages_per_row, group)
+
+
 def kv_append(k_cache, v_cache, k, v, kv_len):
     """Write one token's K/V per row at ``kv_len[b]`` (``k`` contiguous [B,Hkv,D], ``v`` may be a strided view)."""
     B = k.shape[0]
