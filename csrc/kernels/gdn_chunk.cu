@@ -15,13 +15,14 @@
 // the small ones have accumulators of their own, which keeps the chain that rounds at the leading size short.
 //
 //   gdn_chunk_prep_kernel   one CTA per (chunk, head): T and P as pieces, the row factors
-//   gdn_chunk_scan_kernel   one CTA per (head, DV value columns): chunks in order, the state in registers
+//   gdn_chunk_scan_kernel   one CTA per head: chunks in order, the state in registers and, as pieces, in tensor memory
 //
-// One CTA per head with everything in 32-bit multiply-adds was bound by them and by its serial chain, on 48 SMs for 48
-// heads: 5119 tokens x 48 heads 5057 -> 722 us, 4 x 2047 x 48 4053 -> 958 us, 1024 x 16 966 -> 95 us.  The state is now
-// 1.1e-7 to 1.8e-7 off float64 (2-norm), 1.7e-7 to 6.9e-7 before.  What bounds the scan is issuing the warp-level products
-// and their fragments (four barriers a chunk, 9 us a chunk for 64 columns); 16-bit pieces of a third the size would halve it and
-// lose the last eight bits of every sum.
+// The scan on warp-level products, two CTAs a head (four where they all ran at once), took 9 us a chunk, bound by issuing the
+// products and their fragments: 5119 tokens x 48 heads 549 us, 4 x 2047 x 48 677 (a round of 26 chunks), 1024 x 16 73.  On
+// tcgen05 with the state as an operand in tensor memory: 321, 295 and 69 us, 4 us a chunk.  A chunk is a chain of four
+// products, 3300 cycles of the tensor cores' time, with the threads' work between them: 5500 cycles, of which splitting an
+// entry into pieces takes 10 a pair of warps (28 with shifts and conversions of its own, 13 with cut-off pieces).  The state's
+// distance from float64 is 1.2e-7 to 1.7e-7 (2-norm), as it was.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -76,9 +77,14 @@ struct ChunkArgs {
 // entry (i, c) of a piece: rows of 128 bytes, 16-byte chunks exchanged within groups of eight rows
 __device__ __forceinline__ int piece_at(int i, int c) { return i * GC + (((c >> 3) ^ (i & 7)) << 3) + (c & 7); }
 
-// Shared: k, q [64, 256 bytes] swizzled; A [64, 68]; T [64, 65]; G (two floats), kn, qn, beta [64].
-constexpr int LA = GC + 4, LT = GC + 1;
-constexpr size_t kPrepSmem = 2 * GC * GD * 2 + (GC * LA + GC * LT + 5 * GC) * sizeof(float);
+// Shared: k, q [64, 256 bytes] swizzled, later the pieces of P, then of T; A, T [64, 68]; G (two floats), kn, qn, beta [64].
+//
+// T comes from its 16 x 16 diagonal blocks, each by substitution, a thread a column, and from products: with
+// [[T0, 0], [-T1 A10 T0, T1]] pairs of blocks become one, twice.  By substitution over all 64 rows, on 64 threads, it was 13 of
+// the block's 31 thousand cycles, the L2 factors (a warp a row) 7 thousand and stores of single words 6 thousand.
+// 5119 tokens x 48 heads: 167 -> 120 us, a chunk of one head 13 -> 8.
+constexpr int LA = GC + 4;
+constexpr size_t kPrepSmem = 2 * GC * GD * 2 + (2 * GC * LA + 5 * GC) * sizeof(float);
 
 __global__ void __launch_bounds__(NTH, 3)
 gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
@@ -86,7 +92,7 @@ gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
   const uint32_t ks = smem_addr(sm8), qs = ks + GC * GD * 2;
   float* A = reinterpret_cast<float*>(sm8 + 2 * GC * GD * 2);
   float* Ts = A + GC * LA;
-  float *Gs = Ts + GC * LT, *Gl = Gs + GC, *kn = Gl + GC, *qn = kn + GC, *bs = qn + GC;
+  float *Gs = Ts + GC * LA, *Gl = Gs + GC, *kn = Gl + GC, *qn = kn + GC, *bs = qn + GC;
   const int ci = blockIdx.x % a.n, bh = blockIdx.x / a.n, b = bh / a.Hv, hv = bh % a.Hv;
   pdl_trigger();                             // the scan sets up while the last of these run
   const int hk = hv / (a.Hv / a.Hk), t0 = (a.c0 + ci) * GC, n = min(GC, a.T - t0);
@@ -116,13 +122,24 @@ gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
   }
   cp_wait<0>();
   __syncthreads();
-  for (int r = warp; r < 2 * GC; r += 8) {   // L2 factors: a warp per row of k, then of q
-    const uint2 w = *reinterpret_cast<const uint2*>(sm8 + (r >> 6) * GC * GD * 2 + sw_off<256>(r & 63, lane >> 1) + (lane & 1) * 8);
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.x));
-    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.y));
-    const float s = warp_sum(x.x * x.x + x.y * x.y + y.x * y.x + y.y * y.y);
-    const float f = l2norm ? rsqrtf(s + eps) : 1.f;
-    if (lane == 0) (r < GC ? kn : qn)[r & 63] = r < GC ? f : f * rsqrtf(static_cast<float>(GD));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {              // L2 factors: eight threads a row of k, then of q
+    const int r = i * 32 + (tid >> 3);
+    float sum = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint4 w = *reinterpret_cast<const uint4*>(sm8 + (r >> 6) * GC * GD * 2 + sw_off<256>(r & 63, h * 8 + (tid & 7)));
+      const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float x = __uint_as_float(u[e] << 16), y = __uint_as_float(u[e] & 0xFFFF0000u);
+        sum += x * x + y * y;
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float f = l2norm ? rsqrtf(sum + eps) : 1.f;
+    if ((tid & 7) == 0) (r < GC ? kn : qn)[r & 63] = r < GC ? f : f * rsqrtf(static_cast<float>(GD));
   }
   // <k_i, k_j> and <q_i, k_j>: a warp has 16 rows and 32 columns of both
   const int mt = warp >> 1, nh = warp & 1;
@@ -144,9 +161,9 @@ gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
       mma16816(qk[j], fq, fb[j][0], fb[j][1]);
     }
   }
-  __syncthreads();                           // kn, qn
+  __syncthreads();                           // kn, qn; k and q are read
   const long long co = static_cast<long long>(bh) * a.n + ci;
-  __nv_bfloat16* pc = a.pieces + co * 6 * PIECE;
+  __nv_bfloat16 *pc = a.pieces + co * 6 * PIECE, *stage = reinterpret_cast<__nv_bfloat16*>(sm8);
 #pragma unroll
   for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -162,7 +179,7 @@ gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
       uint32_t w[3];
       split3(p[0], p[1], w[0], w[1], w[2]);
 #pragma unroll
-      for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(pc + (3 + s) * PIECE + piece_at(i, c)) = w[s];
+      for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(stage + s * PIECE + piece_at(i, c)) = w[s];
     }
   const float glast = Gs[GC - 1], llast = Gl[GC - 1];
   if (tid < GC) {
@@ -174,34 +191,98 @@ gdn_chunk_prep_kernel(ChunkArgs a, int l2norm, float eps) {
     vp[3 * GC] = kn[tid] * __expf((glast - Gs[tid]) + (llast - Gl[tid]));
     vp[4 * GC] = __expf(glast + llast);
   }
+  tc::fence_async_smem();
   __syncthreads();
-  if (tid < GC) {
-    // column tid of T: t[i] = [i == tid] - sum_{j<i} A[i][j] t[j]; a column depends on its own earlier rows only
-    float t[GC];
+  if (tid == 0) {
+    tc::bulk_store(pc + 3 * PIECE, stage, 3 * PIECE * 2);
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+  if (warp >= 4 && lane < 16) {              // column `lane` of a diagonal block: t[i] = [i == lane] - sum_{j<i} A[i][j] t[j]
+    const float* D = A + (warp - 4) * 16 * (LA + 1);
+    float t[16];
 #pragma unroll
-    for (int i = 0; i < GC; ++i) {
-      float a0 = (i == tid) ? 1.f : 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+    for (int i = 0; i < 16; ++i) {
+      float a0 = (i == lane) ? 1.f : 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
 #pragma unroll
       for (int j = 0; j + 3 < i; j += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(A + i * LA + j);
+        const float4 x = *reinterpret_cast<const float4*>(D + i * LA + j);
         a0 -= x.x * t[j];
         a1 -= x.y * t[j + 1];
         a2 -= x.z * t[j + 2];
         a3 -= x.w * t[j + 3];
       }
 #pragma unroll
-      for (int j = i & ~3; j < i; ++j) a0 -= A[i * LA + j] * t[j];
+      for (int j = i & ~3; j < i; ++j) a0 -= D[i * LA + j] * t[j];
       t[i] = (a0 + a1) + (a2 + a3);
-      Ts[i * LT + tid] = t[i];
+      Ts[(warp - 4) * 16 * (LA + 1) + i * LA + lane] = t[i];
     }
   }
   __syncthreads();
+  // a row of one operand with N columns of the other, k0 .. k1; the products on their way lie where T has its zeros
+  {                                          // blocks 0 and 1, 2 and 3: a thread has two columns
+    const int o = (tid >> 7) * 32 * (LA + 1), r = (tid >> 3) & 15, c = (tid & 7) * 2;
+    auto product = [&](const float* x, const float* y) {
+      float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 16; j += 4) {
+        const float4 u = *reinterpret_cast<const float4*>(x + j);
+        const float w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 z = *reinterpret_cast<const float2*>(y + (j + e) * LA);
+          acc.x += w[e] * z.x;
+          acc.y += w[e] * z.y;
+        }
+      }
+      return acc;
+    };
+    *reinterpret_cast<float2*>(Ts + o + r * LA + 16 + c) = product(A + o + (16 + r) * LA, Ts + o + c);
+    __syncthreads();
+    const float2 x = product(Ts + o + (16 + r) * LA + 16, Ts + o + 16 + c);
+    *reinterpret_cast<float2*>(Ts + o + (16 + r) * LA + c) = make_float2(-x.x, -x.y);
+  }
+  __syncthreads();
+  {                                          // rows 32 on, columns up to 32: a thread has four columns
+    const int r = tid >> 3, c = (tid & 7) * 4;
+    auto product = [&](const float* x, const float* y, int j0, int j1) {
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int j = j0; j < j1; j += 4) {
+        const float4 u = *reinterpret_cast<const float4*>(x + j);
+        const float w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float4 z = *reinterpret_cast<const float4*>(y + (j + e) * LA);
+          acc.x += w[e] * z.x;
+          acc.y += w[e] * z.y;
+          acc.z += w[e] * z.z;
+          acc.w += w[e] * z.w;
+        }
+      }
+      return acc;
+    };
+    // the columns from 16 on meet zeros above (products of the step before, not to be read), the rows below 16 likewise
+    *reinterpret_cast<float4*>(Ts + r * LA + 32 + c) = product(A + (32 + r) * LA, Ts + c, c & 16, 32);
+    __syncthreads();
+    const float4 x = product(Ts + (32 + r) * LA + 32, Ts + 32 + c, 0, (r & 16) + 16);
+    *reinterpret_cast<float4*>(Ts + (32 + r) * LA + c) = make_float4(-x.x, -x.y, -x.z, -x.w);
+  }
+  if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  __syncthreads();                           // T is whole, the pieces of P are on their way to memory
   for (int e = tid; e < PIECE / 2; e += NTH) {
     const int i = e >> 5, c = (e & 31) * 2;
+    const float2 x = c >> 4 <= i >> 4 ? *reinterpret_cast<const float2*>(Ts + i * LA + c) : make_float2(0.f, 0.f);
     uint32_t w[3];
-    split3(Ts[i * LT + c], Ts[i * LT + c + 1], w[0], w[1], w[2]);
+    split3(x.x, x.y, w[0], w[1], w[2]);
 #pragma unroll
-    for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(pc + s * PIECE + piece_at(i, c)) = w[s];
+    for (int s = 0; s < 3; ++s) *reinterpret_cast<uint32_t*>(stage + s * PIECE + piece_at(i, c)) = w[s];
+  }
+  tc::fence_async_smem();
+  __syncthreads();
+  if (tid == 0) {
+    tc::bulk_store(pc, stage, 3 * PIECE * 2);
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
 }
 
