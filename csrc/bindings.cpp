@@ -515,7 +515,7 @@ Tensor lora_grad(const Tensor& U, const Tensor& X) {
   const int64_t M = U.size(0), R = U.size(1), C = X.size(1);
   Tensor out = out_empty({R, C}, U.options().dtype(at::kFloat));
   if (M == 0) return out.zero_();
-  const int splits = ferrl::lora_grad_splits(M, C, num_sms());
+  const int splits = ferrl::lora_grad_splits(M, R, C, num_sms());
   Tensor partial = out_empty({static_cast<long long>(ferrl::lora_grad_workspace_floats(R, C, splits))}, out.options());
   // per-device counters, zero between calls (the kernel resets the ones it used)
   static std::vector<Tensor> counters(64);

@@ -29,10 +29,19 @@ using namespace mmah;
 constexpr int LG_COLS = 128;     // output columns per CTA
 constexpr int LG_ROWS = 64;      // tokens per stage
 constexpr int LG_STAGES = 3;
-constexpr int LG_TILE_BYTES = LG_ROWS * 256;   // both tiles use 256-byte rows (128 bf16)
+constexpr int LG_X_BYTES = LG_ROWS * 256;      // a stage's tile of X: rows of 128 bf16
+// a stage's tile of U: rows of 128 bytes up to rank 64, of 256 above
+template <int RT> constexpr int LG_U_ROW = RT <= 4 ? 128 : 256;
+template <int RT> constexpr int LG_STAGE_BYTES = LG_X_BYTES + LG_ROWS * LG_U_ROW<RT>;
+
+// Bound by reading X once.  11392 tokens, us (bytes' time), before and now: rank 16 x 4096 columns 35 and 32 (14), 32 x 24576 127 and
+// 107 (86), 48 x 6144 56 and 47 (22); 5119 tokens, 64 x 10240 60 and 39 (16); 4608 tokens, 32 x 43008 117 and 86 (61).  What the time was:
+// two CTAs an SM, because a tile of U took as much shared memory as one of X; an address computed anew for every 16 bytes;
+// the ranges' sums fetched one by one by the last CTA; ranges cut so that they filled waves and not so that they ended together.
+constexpr int LG_CHAIN = 8;      // stages whose products are summed by the tensor cores alone
 
 template <int RT>   // RT 16-row tiles of R (R <= 16*RT <= 128)
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, RT <= 4 ? 3 : 2)
 lora_grad_kernel(const __nv_bfloat16* __restrict__ U, long long ldu, int R, const __nv_bfloat16* __restrict__ X,
                  long long ldx, int C, int M, int rows_per_split, float* __restrict__ partial,
                  int* __restrict__ counters, float* __restrict__ out, long long ldo) {
@@ -43,23 +52,34 @@ lora_grad_kernel(const __nv_bfloat16* __restrict__ U, long long ldu, int R, cons
   const int c0 = ct * LG_COLS;
   const int m_begin = split * rows_per_split, m_end = min(M, m_begin + rows_per_split);
   const int n_stages = m_end > m_begin ? (m_end - m_begin + LG_ROWS - 1) / LG_ROWS : 0;
-  const int r_chunks = (R + 7) / 8;
+  constexpr int UR = LG_U_ROW<RT>;
+  // this thread's 16 bytes of every eighth row of X, and of U rows a stage's worth apart
+  const int xr = threadIdx.x >> 4, xc = threadIdx.x & 15;
+  const bool x_ok = c0 + xc * 8 < C;
+  const __nv_bfloat16* xp = X + static_cast<long long>(m_begin + xr) * ldx + (x_ok ? c0 + xc * 8 : 0);
+  constexpr int UC = 2 * RT <= 8 ? 8 : 16;     // threads a row of U, those past 2 RT idle
+  const int ur = threadIdx.x / UC, uc = threadIdx.x % UC;
+  const bool u_ok = uc * 8 < R;
+  const __nv_bfloat16* up = U + static_cast<long long>(m_begin + ur) * ldu + (u_ok ? uc * 8 : 0);
 
   auto issue = [&](int s) {
     if (s < n_stages) {
-      uint8_t* xt = lsm + (s % LG_STAGES) * 2 * LG_TILE_BYTES;
-      uint8_t* ut = xt + LG_TILE_BYTES;
-      const int m0 = m_begin + s * LG_ROWS;
-      for (int i = threadIdx.x; i < LG_ROWS * 16; i += 128) {
-        const int r = i >> 4, ch = i & 15;
-        const bool ok = (m0 + r) < m_end && (c0 + ch * 8) < C;
-        cp_async16(smem_addr(xt) + sw_off<256>(r, ch), X + static_cast<long long>(ok ? m0 + r : 0) * ldx + (ok ? c0 + ch * 8 : 0), ok);
+      const uint32_t xt = smem_addr(lsm + (s % LG_STAGES) * LG_STAGE_BYTES<RT>), ut = xt + LG_X_BYTES;
+      const int left = m_end - m_begin - s * LG_ROWS;          // rows of this stage that there are
+#pragma unroll
+      for (int i = 0; i < LG_ROWS / 8; ++i) {
+        const int r = i * 8 + xr;
+        cp_async16(xt + sw_off<256>(r, xc), r < left ? xp + static_cast<long long>(i) * 8 * ldx : X, x_ok && r < left);
       }
-      for (int i = threadIdx.x; i < LG_ROWS * 2 * RT; i += 128) {
-        const int r = i / (2 * RT), ch = i % (2 * RT);
-        const bool ok = (m0 + r) < m_end && ch < r_chunks;
-        cp_async16(smem_addr(ut) + sw_off<256>(r, ch), U + static_cast<long long>(ok ? m0 + r : 0) * ldu + (ok ? ch * 8 : 0), ok);
+      if (uc < 2 * RT) {
+#pragma unroll
+        for (int i = 0; i < LG_ROWS * UC / 128; ++i) {
+          const int r = i * (128 / UC) + ur;
+          cp_async16(ut + sw_off<UR>(r, uc), r < left ? up + static_cast<long long>(i) * (128 / UC) * ldu : U, u_ok && r < left);
+        }
       }
+      xp += LG_ROWS * ldx;
+      up += LG_ROWS * ldu;
     }
     cp_commit();
   };
@@ -72,14 +92,36 @@ lora_grad_kernel(const __nv_bfloat16* __restrict__ U, long long ldu, int R, cons
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[a][n][e] = 0.f;
 
+  // The tensor cores cut off where they add, so a long chain of sums drifts: up to rank 64 every LG_CHAIN stages join a total.
+  constexpr bool kTotal = RT <= 4;
+  float total[kTotal ? RT : 1][4][4];
+#pragma unroll
+  for (int a = 0; a < (kTotal ? RT : 1); ++a)
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) total[a][n][e] = 0.f;
+  auto join = [&]() {
+    if constexpr (kTotal) {
+#pragma unroll
+      for (int a = 0; a < RT; ++a)
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            total[a][n][e] += acc[a][n][e];
+            acc[a][n][e] = 0.f;
+          }
+    }
+  };
+
 #pragma unroll
   for (int s = 0; s < LG_STAGES - 1; ++s) issue(s);
   for (int s = 0; s < n_stages; ++s) {
     cp_wait<LG_STAGES - 2>();
     __syncthreads();
     issue(s + LG_STAGES - 1);
-    const uint8_t* xt = lsm + (s % LG_STAGES) * 2 * LG_TILE_BYTES;
-    const uint8_t* ut = xt + LG_TILE_BYTES;
+    const uint32_t xt = smem_addr(lsm + (s % LG_STAGES) * LG_STAGE_BYTES<RT>), ut = xt + LG_X_BYTES;
 #pragma unroll
     for (int ks = 0; ks < LG_ROWS / 16; ++ks) {
       // B fragments: X[k = token][n = column], 4 n-tiles of this warp's 32 columns
@@ -87,8 +129,8 @@ lora_grad_kernel(const __nv_bfloat16* __restrict__ U, long long ldu, int R, cons
       {
         const int row = ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
         const int chunk = warp * 4 + (lane >> 4);
-        ldsm4t(smem_addr(xt) + sw_off<256>(row, chunk), b[0], b[1], b[2], b[3]);
-        ldsm4t(smem_addr(xt) + sw_off<256>(row, chunk + 2), b[4], b[5], b[6], b[7]);
+        ldsm4t(xt + sw_off<256>(row, chunk), b[0], b[1], b[2], b[3]);
+        ldsm4t(xt + sw_off<256>(row, chunk + 2), b[4], b[5], b[6], b[7]);
       }
 #pragma unroll
       for (int rt = 0; rt < RT; ++rt) {
@@ -97,13 +139,23 @@ lora_grad_kernel(const __nv_bfloat16* __restrict__ U, long long ldu, int R, cons
         const int mat = lane >> 3;
         const int row = ks * 16 + (lane & 7) + (mat >> 1) * 8;
         const int chunk = rt * 2 + (mat & 1);
-        ldsm4t(smem_addr(ut) + sw_off<256>(row, chunk), a[0], a[1], a[2], a[3]);
+        ldsm4t(ut + sw_off<UR>(row, chunk), a[0], a[1], a[2], a[3]);
 #pragma unroll
         for (int n = 0; n < 4; ++n) mma16816(acc[rt][n], a, b[2 * n], b[2 * n + 1]);
       }
     }
+    if (s % LG_CHAIN == LG_CHAIN - 1) join();
   }
   cp_wait<0>();
+  if constexpr (kTotal) {
+    join();
+#pragma unroll
+    for (int a = 0; a < RT; ++a)
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[a][n][e] = total[a][n][e];
+  }
 
   // partial tile of this token range: [split][16*RT][C], fp32
   const int g = lane >> 2, t = lane & 3;
@@ -128,16 +180,37 @@ lora_grad_kernel(const __nv_bfloat16* __restrict__ U, long long ldu, int R, cons
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  // the last CTA of this column tile sums the ranges in order
-  for (int i = threadIdx.x; i < R * (LG_COLS / 4); i += 128) {
-    const int r = i / (LG_COLS / 4), c = c0 + (i % (LG_COLS / 4)) * 4;
-    if (c >= C) continue;
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < n_splits; ++s) {
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(partial + (static_cast<long long>(s) * (16 * RT) + r) * C + c));
-      sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+  // the last CTA of this column tile sums the ranges in order; two places of eight ranges are on their way at a time
+  for (int i = threadIdx.x; i < R * (LG_COLS / 4); i += 256) {
+    const float* src[2];
+    bool ok[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int at = i + 128 * h, r = at / (LG_COLS / 4), c = c0 + (at % (LG_COLS / 4)) * 4;
+      ok[h] = r < R && c < C;
+      src[h] = partial + (ok[h] ? static_cast<long long>(r) * C + c : 0);
     }
-    *reinterpret_cast<float4*>(out + static_cast<long long>(r) * ldo + c) = sum;
+    float4 sum[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    for (int s = 0; s < n_splits; s += 8) {
+      float4 v[2][8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (s + j < n_splits) v[h][j] = __ldcg(reinterpret_cast<const float4*>(src[h] + static_cast<long long>(s + j) * (16 * RT) * C));
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (s + j < n_splits) {
+            sum[h].x += v[h][j].x; sum[h].y += v[h][j].y; sum[h].z += v[h][j].z; sum[h].w += v[h][j].w;
+          }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int at = i + 128 * h;
+      if (ok[h]) *reinterpret_cast<float4*>(out + static_cast<long long>(at / (LG_COLS / 4)) * ldo + c0 + (at % (LG_COLS / 4)) * 4) = sum[h];
+    }
   }
 }
 
@@ -148,12 +221,15 @@ size_t lora_grad_workspace_floats(int R, int C, int n_splits) {
   return static_cast<size_t>(n_splits) * rt * 16 * C;
 }
 
-int lora_grad_splits(int M, int C, int num_sms) {
-  // Two CTAs fit on an SM.  The token split is chosen so that the grid fills whole waves of
-  // 2 * num_sms CTAs: a grid of 1.08 waves takes as long as one of two.
+int lora_grad_splits(int M, int R, int C, int num_sms) {
+  // Three CTAs fit on an SM up to rank 64, two above.  Up to rank 64 the token split is the largest whose CTAs all run at once:
+  // few long ranges, which end together (11392 tokens, us, and with the rule below: rank 32 x 24576 columns 107 and 117, 16 x 12288
+  // 64 and 68; 5119 tokens, 64 x 10240 39 and 50).  With more column tiles than that, and above rank 64, where a range is one chain
+  // of sums, the split is chosen so that the grid fills whole waves: a grid of 1.08 waves takes as long as one of two.
   const int col_tiles = (C + LG_COLS - 1) / LG_COLS;
-  const int slots = 2 * num_sms;
+  const int slots = (R <= 64 ? 3 : 2) * num_sms;
   const int max_s = std::min(64, std::max(1, (M + 4 * LG_ROWS - 1) / (4 * LG_ROWS)));   // at least four stages per CTA
+  if (R <= 64 && col_tiles <= slots) return std::min(max_s, slots / col_tiles);
   int best = 1;
   double best_eff = 0.0;
   for (int s = 1; s <= max_s; ++s) {
@@ -179,9 +255,9 @@ const char* lora_grad(const void* U, long long ldu, int R, const void* X, long l
   const int rt = (R + 15) / 16;
   const int rows_per_split = ((M + n_splits - 1) / n_splits + LG_ROWS - 1) / LG_ROWS * LG_ROWS;
   dim3 grid((C + LG_COLS - 1) / LG_COLS, n_splits);
-  constexpr int smem = LG_STAGES * 2 * LG_TILE_BYTES;
 #define FERRL_LG(RTV)                                                                                                 \
   case RTV: {                                                                                                         \
+    constexpr int smem = LG_STAGES * LG_STAGE_BYTES<RTV>;                                                             \
     if (!FERRL_ONCE_PER_DEVICE(cudaFuncSetAttribute(lora_grad_kernel<RTV>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                                     smem) == cudaSuccess))                                            \
       return "lora_grad: cannot reserve shared memory";                                                               \
