@@ -397,6 +397,9 @@ const char* moe_gather(const void* x, long long ldx, const int* token_of, const 
                        int n_pairs, float* row_scale, int rows, int H, void* xs, bool sparse, cudaStream_t stream);
 const char* moe_combine(const void* ys, const int* row_of, const float* w, int T, int k, int H, void* out,
                         cudaStream_t stream);
+// out = y + sigmoid(<x, w>) * sh over bf16 rows; gate [T]: the sigmoid.  Backward: dsh, and dx of the gate's logit.
+const char* moe_shared(const void* x, const void* w, const void* y, const void* sh, int T, int H, void* out, float* gate, cudaStream_t stream);
+const char* moe_shared_bwd(const void* dy, const void* sh, const float* gate, const void* w, int T, int H, void* dsh, void* dx, cudaStream_t stream);
 const char* moe_pair_dot(const void* dy, const void* ys, const int* row_of, int n_pairs, int k, int H, float* dw,
                          cudaStream_t stream);
 

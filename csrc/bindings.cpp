@@ -961,6 +961,28 @@ Tensor moe_combine(const Tensor& ys, const Tensor& row_of, const optional<Tensor
   return out;
 }
 
+// y + sigmoid(x w^T) * sh, rows of bf16; (out, the sigmoid [T])
+std::tuple<Tensor, Tensor> moe_shared(const Tensor& x, const Tensor& w, const Tensor& y, const Tensor& sh) {
+  auto ok = [](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous(); };
+  TORCH_CHECK(ok(x) && ok(w) && ok(y) && ok(sh) && x.dim() == 2 && y.sizes() == x.sizes() && sh.sizes() == x.sizes() && w.numel() == x.size(1),
+              "moe_shared: bf16 x, y, sh [T,H], w [H], contiguous");
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = out_empty({x.size(0), x.size(1)}, x.options()), gate = out_empty({x.size(0)}, x.options().dtype(at::kFloat));
+  FERRL_CHECK(ferrl::moe_shared(x.data_ptr(), w.data_ptr(), y.data_ptr(), sh.data_ptr(), x.size(0), x.size(1), out.data_ptr(), gate.data_ptr<float>(), stream()));
+  return {out, gate};
+}
+
+// (gradient of sh, gradient of x through the gate)
+std::tuple<Tensor, Tensor> moe_shared_bwd(const Tensor& dy, const Tensor& sh, const Tensor& gate, const Tensor& w) {
+  auto ok = [](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous(); };
+  TORCH_CHECK(ok(dy) && ok(sh) && ok(w) && dy.dim() == 2 && sh.sizes() == dy.sizes() && w.numel() == dy.size(1) && gate.is_cuda() &&
+                  gate.scalar_type() == at::kFloat && gate.is_contiguous() && gate.numel() == dy.size(0), "moe_shared_bwd: bf16 dy, sh [T,H], w [H], f32 gate [T]");
+  c10::cuda::CUDAGuard guard(dy.device());
+  Tensor dsh = out_empty({dy.size(0), dy.size(1)}, dy.options()), dx = out_empty({dy.size(0), dy.size(1)}, dy.options());
+  FERRL_CHECK(ferrl::moe_shared_bwd(dy.data_ptr(), sh.data_ptr(), gate.data_ptr<float>(), w.data_ptr(), dy.size(0), dy.size(1), dsh.data_ptr(), dx.data_ptr(), stream()));
+  return {dsh, dx};
+}
+
 // dw[t,j] = <dy[t], ys[row_of[t,j]]>
 Tensor moe_pair_dot(const Tensor& dy, const Tensor& ys, const Tensor& row_of, int64_t k) {
   TORCH_CHECK(dy.is_cuda() && dy.scalar_type() == at::kBFloat16 && dy.is_contiguous() && ys.is_contiguous() && dy.size(1) == ys.size(1), "moe_pair_dot: shapes");
@@ -2096,6 +2118,8 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("moe_grouped_gemm(Tensor xs, Tensor W, Tensor tile_expert, Tensor(a!)? out=None, bool nn=False, Tensor? token_of=None, int form=1) -> Tensor(a!)", &moe_grouped_gemm);
   m.def("ep_dispatch(Tensor x, Tensor idx, Tensor? pair_w, Tensor counts, int[] counts_all, int[] xs, int[] flags, int rank, int world, int epoch, float limit_s, int cap_rows, Tensor(a!) dest_row, Tensor(b!) tile_expert, Tensor(c!) local_rows, bool reuse_plan, Tensor(d!) abort_word) -> ()", &ep_dispatch);
   m.def("ep_combine(int[] ys, Tensor idx, Tensor dest_row, Tensor? w, int H, int E_local, int[] flags, int rank, int world, int epoch, float limit_s, Tensor(a!)? keep_rows, Tensor(b!) abort_word) -> Tensor", &ep_combine);
+  m.def("moe_shared(Tensor x, Tensor w, Tensor y, Tensor sh) -> (Tensor, Tensor)", &moe_shared);
+  m.def("moe_shared_bwd(Tensor dy, Tensor sh, Tensor gate, Tensor w) -> (Tensor, Tensor)", &moe_shared_bwd);
   m.def("moe_combine(Tensor ys, Tensor row_of, Tensor? w, int T, int k) -> Tensor", &moe_combine);
   m.def("moe_pair_dot(Tensor dy, Tensor ys, Tensor row_of, int k) -> Tensor", &moe_pair_dot);
   m.def("kernel_status() -> int", &kernel_status);

@@ -9,6 +9,7 @@
 //   moe_gather_kernel   xs[row] = scale(row) * x[token_of[row]]   (zero rows for padding)
 //   (grouped tcgen05 GEMM over the segments: csrc/gemm/tcgen05_gemm.cu, tile_expert mode)
 //   moe_combine_kernel  out[t] = sum_j w[t,j] * ys[row_of[t,j]]   (fixed order, fp32 accumulate)
+//   moe_shared_kernel   out = routed + sigmoid(<x, w>) * shared, and its gradient
 //   moe_pair_dot_kernel dw[t,j] = <dy[t], ys[row_of[t,j]]>        (router-weight gradient)
 //
 // The padded layout makes every 128-row m tile belong to exactly one expert, so the grouped GEMM
@@ -18,6 +19,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <initializer_list>
 
 #include "../api.h"
 #include "../common.cuh"
@@ -396,6 +398,110 @@ const char* moe_gather(const void* x, long long ldx, const int* token_of, const 
                                                 pair_w ? row_scale : nullptr, rows, H, static_cast<__nv_bfloat16*>(xs), sparse ? 1 : 0);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? nullptr : "moe_gather launch failed";
+}
+
+namespace {
+__device__ __forceinline__ void bf8(const uint4& u, float (&f)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    f[2 * e] = __uint_as_float(w[e] << 16);
+    f[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ uint4 to_bf8(const float (&f)[8]) {
+  uint4 u;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+  return u;
+}
+__device__ __forceinline__ float bf_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+
+// The gated shared expert, a warp per token; the gate's logit, the gate and its product round to the activations' type as
+// they would as tensors.  Bound by the bytes: a product with one column, a sigmoid, a broadcast product and a sum took 66 us at
+// 6140 tokens of 2048 forward, twice as many operators 79 us backward, now 25 and 23 (100 MB each: 15); 128 tokens 24 and 12 forward.
+__global__ void __launch_bounds__(256)
+moe_shared_kernel(const uint4* __restrict__ x, const uint4* __restrict__ w, const uint4* __restrict__ y, const uint4* __restrict__ sh, int T,
+                  int W, uint4* __restrict__ out, float* __restrict__ gate) {
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= T) return;
+  const long long row = static_cast<long long>(t) * W;
+  float dot = 0.f;
+#pragma unroll 4
+  for (int i = lane; i < W; i += 32) {
+    float a[8], b[8];
+    bf8(x[row + i], a);
+    bf8(w[i], b);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) dot += a[e] * b[e];
+  }
+  const float g = bf_round(1.f / (1.f + __expf(-bf_round(warp_sum(dot)))));
+  if (lane == 0) gate[t] = g;
+#pragma unroll 4
+  for (int i = lane; i < W; i += 32) {
+    float a[8], b[8];
+    bf8(sh[row + i], a);
+    bf8(y[row + i], b);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a[e] = b[e] + bf_round(g * a[e]);
+    out[row + i] = to_bf8(a);
+  }
+}
+// dsh = g dy, dx = <dy, sh> g (1 - g) w
+__global__ void __launch_bounds__(256)
+moe_shared_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ sh, const float* __restrict__ gate, const uint4* __restrict__ w, int T,
+                      int W, uint4* __restrict__ dsh, uint4* __restrict__ dx) {
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= T) return;
+  const long long row = static_cast<long long>(t) * W;
+  const float g = gate[t];
+  float dot = 0.f;
+#pragma unroll 4
+  for (int i = lane; i < W; i += 32) {
+    float a[8], b[8];
+    bf8(dy[row + i], a);
+    bf8(sh[row + i], b);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      dot += a[e] * b[e];
+      a[e] *= g;
+    }
+    dsh[row + i] = to_bf8(a);
+  }
+  const float dg = warp_sum(dot) * g * (1.f - g);
+#pragma unroll 4
+  for (int i = lane; i < W; i += 32) {
+    float a[8];
+    bf8(w[i], a);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a[e] *= dg;
+    dx[row + i] = to_bf8(a);
+  }
+}
+bool rows16(int H, std::initializer_list<const void*> ps) {
+  uintptr_t at = 0;
+  for (const void* p : ps) at |= reinterpret_cast<uintptr_t>(p);
+  return H % 8 == 0 && at % 16 == 0;
+}
+}  // namespace
+
+const char* moe_shared(const void* x, const void* w, const void* y, const void* sh, int T, int H, void* out, float* gate, cudaStream_t stream) {
+  if (!rows16(H, {x, w, y, sh, out})) return "moe_shared: rows of a multiple of 8, 16-byte aligned";
+  if (T == 0 || H == 0) return nullptr;
+  moe_shared_kernel<<<(T + 7) / 8, 256, 0, stream>>>(static_cast<const uint4*>(x), static_cast<const uint4*>(w), static_cast<const uint4*>(y),
+                                                     static_cast<const uint4*>(sh), T, H / 8, static_cast<uint4*>(out), gate);
+  count_launch();
+  return cudaGetLastError() == cudaSuccess ? nullptr : "moe_shared launch failed";
+}
+
+const char* moe_shared_bwd(const void* dy, const void* sh, const float* gate, const void* w, int T, int H, void* dsh, void* dx, cudaStream_t stream) {
+  if (!rows16(H, {dy, sh, w, dsh, dx})) return "moe_shared_bwd: rows of a multiple of 8, 16-byte aligned";
+  if (T == 0 || H == 0) return nullptr;
+  moe_shared_bwd_kernel<<<(T + 7) / 8, 256, 0, stream>>>(static_cast<const uint4*>(dy), static_cast<const uint4*>(sh), gate, static_cast<const uint4*>(w), T,
+                                                         H / 8, static_cast<uint4*>(dsh), static_cast<uint4*>(dx));
+  count_launch();
+  return cudaGetLastError() == cudaSuccess ? nullptr : "moe_shared_bwd launch failed";
 }
 
 const char* moe_combine(const void* ys, const int* row_of, const float* w, int T, int k, int H, void* out,

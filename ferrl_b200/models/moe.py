@@ -139,5 +139,14 @@ def sparse_moe_block(x: torch.Tensor, router_w, gate_up, down, top_k: int, share
         _, scores, idx = topk_router(x2, router_w, top_k)
         y = moe_experts(x2, idx, scores.to(x2.dtype), gate_up, down, act)
     if shared is not None:
-        y = y + torch.sigmoid(F.linear(x2, shared_gate_w)) * shared(x2)
+        y = add_shared(x2, shared_gate_w, y, shared(x2))
     return y.reshape(shape)
+
+
+def add_shared(x2, gate_w, y, sh):
+    """``y`` plus the shared expert's rows ``sh`` gated by ``sigmoid(x2 @ gate_w^T)``."""
+    out = None
+    if ops_native(x2):
+        from ..ops import cuda as C
+        out = C.moe_shared(x2, gate_w, y, sh)
+    return y + torch.sigmoid(F.linear(x2, gate_w)) * sh if out is None else out

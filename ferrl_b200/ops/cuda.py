@@ -1054,6 +1054,33 @@ class _MoeExperts(torch.autograd.Function):
         return dx, dsc, None, None, None, None, None, None, None, None
 
 
+class _MoeShared(torch.autograd.Function):
+    """``y + sigmoid(x w^T) * sh`` for a frozen gate ``w``."""
+
+    @staticmethod
+    def forward(ctx, x, w, y, sh):
+        out, gate = lib().moe_shared(x, w, y, sh)
+        ctx.save_for_backward(sh, gate, w)
+        return out
+
+    @staticmethod
+    def backward(ctx, dy):
+        dsh, dx = lib().moe_shared_bwd(dy.contiguous(), *ctx.saved_tensors)
+        return dx, None, dy, dsh
+
+
+def moe_shared(x, w, y, sh):
+    """The gated shared expert ``y + sigmoid(x w^T) * sh`` on rows ``[T,H]`` with ``w`` ``[1,H]``; ``None`` outside the kernel's
+    domain (bf16 rows of whole 16-byte pieces, a frozen gate)."""
+    ts = (x, w, y, sh)
+    if not all(_bf16(t) for t in ts) or w.requires_grad or x.dim() != 2 or w.numel() != x.shape[1] or not x.shape == y.shape == sh.shape or x.shape[1] % 8:
+        return None
+    ts = tuple(t.contiguous() for t in ts)
+    if any(t.data_ptr() % 16 for t in ts):
+        return None
+    return _MoeShared.apply(*ts)
+
+
 def moe_experts_any(x, scores, idx, counts, gate_up, down, act="silu", weight_input=False):
     """Grad-free routed experts for fp32 and for sizes outside ``moe_experts``'s domain, on the same device plan."""
     return lib().moe_experts_any(x if x.stride(1) == 1 else x.contiguous(), scores.float().contiguous(), idx.contiguous(), counts, gate_up, down,
