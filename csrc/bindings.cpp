@@ -1215,6 +1215,20 @@ bool kv_prefill_paged(const Tensor& k, const Tensor& v, Tensor kc, Tensor vc, co
   return true;
 }
 
+// a [.., W] contiguous times sigmoid(gate), gate [rows, W] with rows apart; with dy the gradients (da, dgate)
+std::tuple<Tensor, Tensor> gate_mul(const Tensor& a, const Tensor& gate, const optional<Tensor>& dy) {
+  auto ok = [](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16; };
+  const bool back = dy.has_value() && dy->defined();
+  TORCH_CHECK(ok(a) && ok(gate) && a.dim() == 2 && a.is_contiguous() && gate.sizes() == a.sizes() && (gate.size(1) == 1 || gate.stride(1) == 1) &&
+                  (!back || (ok(*dy) && dy->is_contiguous() && dy->sizes() == a.sizes())), "gate_mul: bf16 a, dy [R,W] contiguous, gate [R,W] rows");
+  c10::cuda::CUDAGuard guard(a.device());
+  Tensor out = out_empty({a.size(0), a.size(1)}, a.options()), dgate;
+  if (back) dgate = out_empty({a.size(0), a.size(1)}, a.options());
+  FERRL_CHECK(ferrl::gate_mul(a.data_ptr(), gate.data_ptr(), gate.stride(0), back ? dy->data_ptr() : nullptr, a.size(0), a.size(1), out.data_ptr(),
+                              back ? dgate.data_ptr() : nullptr, stream()));
+  return {out, dgate};
+}
+
 static ferrl::GluAct glu_act(int64_t act, double alpha, double limit) {
   TORCH_CHECK(act >= ferrl::kActSilu && act <= ferrl::kActClipped && (act != ferrl::kActClipped || limit >= 0), "glu: unknown activation");
   return ferrl::GluAct{static_cast<int>(act), static_cast<float>(alpha), static_cast<float>(limit)};
@@ -2131,6 +2145,7 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("qk_norm_rope_fwd(Tensor q, Tensor k, Tensor? qw, Tensor? kw, Tensor cos, Tensor sin, Tensor pos, int pos_div, float eps, bool zc) -> (Tensor, Tensor)", &qk_norm_rope_fwd);
   m.def("qk_norm_rope_bwd(Tensor q, Tensor k, Tensor? qw, Tensor? kw, Tensor cos, Tensor sin, Tensor pos, int pos_div, float eps, bool zc, Tensor dq, Tensor dk, Tensor(a!) dq_in, Tensor(b!) dk_in) -> ()", &qk_norm_rope_bwd);
   m.def("kv_append(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor kv_len) -> ()", &kv_append);
+  m.def("gate_mul(Tensor a, Tensor gate, Tensor? dy) -> (Tensor, Tensor)", &gate_mul);
   m.def("kv_prefill_paged(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor full, int ppr, int G) -> bool", &kv_prefill_paged);
   m.def("kv_append_paged(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor kv_len, Tensor table) -> ()", &kv_append_paged);
   m.def("glu_fwd(Tensor gu, int act, float alpha=0.0, float limit=0.0, Tensor? token_of=None) -> Tensor", &glu_fwd);

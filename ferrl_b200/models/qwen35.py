@@ -252,8 +252,12 @@ class Qwen35Layer(nn.Module):
             from .dense import ops_cache_write
             ops_cache_write(cache[0], cache[1], k[:, 0], v[:, 0], kv_len)
             a = ops.decode_attention(q[:, 0], cache[0], cache[1], kv_len + 1, scale=self.scale).unsqueeze(1)
-        a = a.reshape(B, S, hq * D) * torch.sigmoid(gate.float()).to(a.dtype)
-        return f(self.out, a)
+        a = a.reshape(B, S, hq * D)
+        gated = None
+        if ops.native(a):
+            from ..ops import cuda as C
+            gated = C.gate_mul(a, gate)
+        return f(self.out, a * torch.sigmoid(gate.float()).to(a.dtype) if gated is None else gated)
 
     def _gdn(self, x, merged, state=None, valid=None, decode=False):
         """``state`` = (conv_state [B,C,K-1], S [B,Hv,kd,vd]) or None. Returns (out, new_state)."""

@@ -1054,6 +1054,30 @@ class _MoeExperts(torch.autograd.Function):
         return dx, dsc, None, None, None, None, None, None, None, None
 
 
+class _GateMul(torch.autograd.Function):
+    """``a * sigmoid(gate)`` on rows; ``gate`` may be a slice of wider rows."""
+
+    @staticmethod
+    def forward(ctx, a, gate):
+        ctx.save_for_backward(a, gate)
+        return lib().gate_mul(a, gate, None)[0]
+
+    @staticmethod
+    def backward(ctx, dy):
+        return lib().gate_mul(*ctx.saved_tensors, dy.contiguous())
+
+
+def gate_mul(a, gate):
+    """``a * sigmoid(gate)`` for bf16 ``[..,W]``; ``None`` outside the kernel's domain (rows of whole 16-byte pieces)."""
+    W = a.shape[-1]
+    if not (_bf16(a) and _bf16(gate)) or a.shape != gate.shape or W % 8 or gate.stride(-1) != 1:
+        return None
+    a2, g2 = a.reshape(-1, W).contiguous(), gate.reshape(-1, W)
+    if g2.stride(1) != 1 or g2.stride(0) % 8 or a2.data_ptr() % 16 or g2.data_ptr() % 16:
+        return None
+    return _GateMul.apply(a2, g2).view(a.shape)
+
+
 class _MoeShared(torch.autograd.Function):
     """``y + sigmoid(x w^T) * sh`` for a frozen gate ``w``."""
 
