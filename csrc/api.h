@@ -161,6 +161,8 @@ const char* glu(int dtype, bool backward, const void* gu, const void* dout, void
                 const int* token_of = nullptr);
 const char* embedding(int dtype, const long long* ids, const void* table, void* out, long long n_tok, int H,
                       long long vocab, float scale, cudaStream_t s);
+// rows start[b] + i (at most S - 1) of x [B, S, width] bf16; backward: x is the gradient [B, L, width], out [B, S, width]
+const char* window_rows(const void* x, const long long* start, int B, int S, int L, int width, bool backward, void* out, int* status, cudaStream_t s);
 // out = a * sigmoid(gate), bf16 rows, gate rows ldg elements apart; with dy: out = da, and dgate
 const char* gate_mul(const void* a, const void* gate, long long ldg, const void* dy, long long rows, int width, void* out, void* dgate, cudaStream_t s);
 const char* lora_merge(int dtype, const void* w, const float* a, const float* b, void* out, int O, int I, int R,

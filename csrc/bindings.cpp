@@ -1215,6 +1215,17 @@ bool kv_prefill_paged(const Tensor& k, const Tensor& v, Tensor kc, Tensor vc, co
   return true;
 }
 
+// x [B, S, W] -> its rows start[b] .. start[b] + n - 1, the last one past the end; backward: x [B, L, W] their gradient, n = S
+Tensor window_rows(const Tensor& x, const Tensor& start, int64_t n, bool backward) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 3 && x.is_contiguous() && start.is_cuda() && start.scalar_type() == at::kLong &&
+                  start.is_contiguous() && start.numel() == x.size(0) && n >= 0 && (x.size(1) > 0 || backward || n == 0), "window_rows: bf16 [B,S,W], int64 [B]");
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = out_empty({x.size(0), n, x.size(2)}, x.options());
+  FERRL_CHECK(ferrl::window_rows(x.data_ptr(), reinterpret_cast<const long long*>(start.data_ptr<int64_t>()), x.size(0), backward ? n : x.size(1),
+                                 backward ? x.size(1) : n, x.size(2), backward, out.data_ptr(), status_word(), stream()));
+  return out;
+}
+
 // a [.., W] contiguous times sigmoid(gate), gate [rows, W] with rows apart; with dy the gradients (da, dgate)
 std::tuple<Tensor, Tensor> gate_mul(const Tensor& a, const Tensor& gate, const optional<Tensor>& dy) {
   auto ok = [](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kBFloat16; };
@@ -2145,6 +2156,7 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("qk_norm_rope_fwd(Tensor q, Tensor k, Tensor? qw, Tensor? kw, Tensor cos, Tensor sin, Tensor pos, int pos_div, float eps, bool zc) -> (Tensor, Tensor)", &qk_norm_rope_fwd);
   m.def("qk_norm_rope_bwd(Tensor q, Tensor k, Tensor? qw, Tensor? kw, Tensor cos, Tensor sin, Tensor pos, int pos_div, float eps, bool zc, Tensor dq, Tensor dk, Tensor(a!) dq_in, Tensor(b!) dk_in) -> ()", &qk_norm_rope_bwd);
   m.def("kv_append(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor kv_len) -> ()", &kv_append);
+  m.def("window_rows(Tensor x, Tensor start, int n, bool backward) -> Tensor", &window_rows);
   m.def("gate_mul(Tensor a, Tensor gate, Tensor? dy) -> (Tensor, Tensor)", &gate_mul);
   m.def("kv_prefill_paged(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor full, int ppr, int G) -> bool", &kv_prefill_paged);
   m.def("kv_append_paged(Tensor k, Tensor v, Tensor(a!) kc, Tensor(b!) vc, Tensor kv_len, Tensor table) -> ()", &kv_append_paged);

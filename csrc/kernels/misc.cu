@@ -365,6 +365,63 @@ const char* embedding(int dtype, const long long* ids, const void* table, void* 
 }
 
 namespace {
+// Rows start[b] .. start[b] + L - 1 of x [B, S, W pieces], the last row again past the end, a warp per row.  Backward: every
+// row's gradient is written, zeros outside the window; the last row's is a sum in the order of the window.  A negative start is
+// reported and gives zeros.  Bound by the bytes: a gather by an index per element took 120 us for 8 x 1024 rows of 4096 out of
+// 8 x 1423, its gradient a fill and an indexed sum 161; now 29 and 34 (134 and 160 MB: 20 and 24).
+template <bool BWD>
+__global__ void __launch_bounds__(256)
+window_rows_kernel(const uint4* __restrict__ x, const long long* __restrict__ start, int B, int S, int L, int W, uint4* __restrict__ out, int* status) {
+  const long long r = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, rows = BWD ? S : L;
+  if (r >= static_cast<long long>(B) * rows) return;
+  const int b = static_cast<int>(r / rows), i = static_cast<int>(r - static_cast<long long>(b) * rows);
+  const long long at = start[b];
+  if (at < 0 && lane == 0) atomicCAS(status, kStatusOk, kStatusBadShape);
+  const uint4* src = nullptr;
+  if (at >= 0) {
+    if (!BWD) src = x + (static_cast<long long>(b) * S + min(at + i, static_cast<long long>(S - 1))) * W;
+    else if (i >= at && i - at < L) src = x + (static_cast<long long>(b) * L + (i - at)) * W;
+  }
+  if (BWD && i == S - 1 && at >= 0 && at + L > S) {          // the windows' rows past the end are this one
+    for (int c = lane; c < W; c += 32) {
+      float sum[8] = {};
+      for (long long j = max(0LL, S - 1 - at); j < L; ++j) {
+        const uint4 u = x[(static_cast<long long>(b) * L + j) * W + c];
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          sum[2 * e] += __uint_as_float(w[e] << 16);
+          sum[2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u);
+        }
+      }
+      uint4 u;
+      __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(sum[2 * e], sum[2 * e + 1]);
+      out[r * W + c] = u;
+    }
+    return;
+  }
+#pragma unroll 4
+  for (int c = lane; c < W; c += 32) out[r * W + c] = src ? src[c] : make_uint4(0, 0, 0, 0);
+}
+}  // namespace
+
+const char* window_rows(const void* x, const long long* start, int B, int S, int L, int width, bool backward, void* out, int* status, cudaStream_t s) {
+  if (width % 8 || (reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) % 16) return "window_rows: bf16 rows of whole 16-byte pieces";
+  const long long rows = static_cast<long long>(B) * (backward ? S : L);
+  if (rows == 0 || width == 0) return nullptr;
+  const unsigned grid = static_cast<unsigned>((rows + 7) / 8);
+  if (backward)
+    window_rows_kernel<true><<<grid, 256, 0, s>>>(static_cast<const uint4*>(x), start, B, S, L, width / 8, static_cast<uint4*>(out), status);
+  else
+    window_rows_kernel<false><<<grid, 256, 0, s>>>(static_cast<const uint4*>(x), start, B, S, L, width / 8, static_cast<uint4*>(out), status);
+  count_launch();
+  return cudaGetLastError() == cudaSuccess ? nullptr : "window_rows launch failed";
+}
+
+namespace {
 // The sigmoid gate on an attention's output, bf16 rows of W pieces of eight, gate rows ldg pieces apart: out = a * s with s rounded
 // as a tensor of the same type would be; da = dy * s, dgate = dy * a * s (1 - s).  Bound by the bytes: a conversion to float32, a
 // sigmoid, a conversion back and a product took 220 us at 8188 rows of 4096 and their gradients 259; now 41 and 58 (201 and 335 MB:

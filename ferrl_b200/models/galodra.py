@@ -362,8 +362,7 @@ class GalodraGradModel(nn.Module):
     def token_logprobs(self, ids, win_start, targets, temperature: float = 1.0, comm: Optional[Comm] = None):
         x = self.forward_hidden(ids, comm, detached=not torch.is_grad_enabled())
         B, L = targets.shape
-        idx = (win_start.view(B, 1).long() + torch.arange(L, device=ids.device)[None, :]).clamp(max=ids.shape[1] - 1)
-        xw = torch.gather(x, 1, idx[:, :, None].expand(B, L, x.shape[-1]))
+        xw = ops.window_rows(x, win_start, L)
         h = self.final_hidden(xw.reshape(B * L, -1))
         return ops.logprob_gather(h, self.embed, targets.reshape(-1), temperature, 0.0, head_wt=self.head_t).view(B, L)
 

@@ -371,8 +371,7 @@ class Gemma4GradModel(nn.Module):
     def token_logprobs(self, ids, win_start, targets, temperature=1.0, comm: Optional[Comm] = None):
         h = self.forward_hidden(ids, comm, detached=not torch.is_grad_enabled())
         B, L = targets.shape
-        idx = (win_start.view(B, 1).long() + torch.arange(L, device=ids.device)[None, :]).clamp(max=ids.shape[1] - 1)
-        hw = torch.gather(h, 1, idx[:, :, None].expand(B, L, h.shape[-1]))
+        hw = ops.window_rows(h, win_start, L)
         hw = ops.rmsnorm(hw, self.final_norm, self.spec.rms_norm_eps)
         if comm is not None and comm.world_size > 1 and self.tp is not None and not self.full_ft:
             # tensor parallelism: every rank scores 1 / world of the (tied, replicated) vocabulary and the ranks

@@ -507,8 +507,7 @@ class Qwen35GradModel(nn.Module):
     def token_logprobs(self, ids, win_start, targets, temperature=1.0, comm: Optional[Comm] = None):
         h = self.forward_hidden(ids, detached=not torch.is_grad_enabled())
         B, L = targets.shape
-        idx = (win_start.view(B, 1).long() + torch.arange(L, device=ids.device)[None, :]).clamp(max=ids.shape[1] - 1)
-        hw = torch.gather(h, 1, idx[:, :, None].expand(B, L, h.shape[-1]))
+        hw = ops.window_rows(h, win_start, L)
         hw = ops.rmsnorm(hw, self.final_norm, self.spec.rms_norm_eps, True)
         return ops.logprob_gather(hw.reshape(B * L, -1), self.head_weight(), targets.reshape(-1), temperature, 0.0,
                                   head_wt=self.head_t).view(B, L)

@@ -45,6 +45,15 @@ def _on_gpu(*ts) -> bool:
     return native(*ts)
 
 
+def window_rows(x, start, n):
+    """Rows ``start[b] .. start[b] + n - 1`` of ``x`` ``[B,S,H]``; past the end the last row again."""
+    out = _cuda().window_rows(x, start, n) if _on_gpu(x) else None
+    if out is None:
+        idx = (start.view(-1, 1).long() + torch.arange(n, device=x.device)[None, :]).clamp(max=x.shape[1] - 1)
+        out = torch.gather(x, 1, idx[:, :, None].expand(x.shape[0], n, x.shape[-1]))
+    return out
+
+
 def rmsnorm(x, weight, eps, zero_centered=False):
     if _on_gpu(x):
         return _cuda().rmsnorm(x, weight, eps, zero_centered)

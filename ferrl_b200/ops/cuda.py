@@ -1054,6 +1054,28 @@ class _MoeExperts(torch.autograd.Function):
         return dx, dsc, None, None, None, None, None, None, None, None
 
 
+class _WindowRows(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, start, n):
+        ctx.save_for_backward(start)
+        ctx.rows = x.shape[1]
+        return lib().window_rows(x, start, n, False)
+
+    @staticmethod
+    def backward(ctx, dy):
+        return lib().window_rows(dy.contiguous(), ctx.saved_tensors[0], ctx.rows, True), None, None
+
+
+def window_rows(x, start, n):
+    """Rows ``start[b] .. start[b] + n - 1`` of bf16 ``x`` ``[B,S,W]``, the last one past the end; ``None`` outside the kernel's domain."""
+    if not _bf16(x) or x.dim() != 3 or x.shape[1] == 0 or x.shape[2] % 8 or not start.is_cuda or start.numel() != x.shape[0]:
+        return None
+    x = x.contiguous()
+    if x.data_ptr() % 16:
+        return None
+    return _WindowRows.apply(x, start.reshape(-1).long().contiguous(), int(n))
+
+
 class _GateMul(torch.autograd.Function):
     """``a * sigmoid(gate)`` on rows; ``gate`` may be a slice of wider rows."""
 
