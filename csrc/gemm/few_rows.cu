@@ -139,19 +139,20 @@ bool gemm_few_rows_supported(const GemmArgs& a) {
          !a.tile_expert && a.ar_world <= 1 && !a.ss_in && !a.ss_out && !a.lp_mode;
 }
 
-// Against the tiled kernels in a chain of dependent launches, weights from HBM (us, tiled and this one; 1 to 8 rows):
+// Against the tiled kernels in a chain of launches, weights from HBM (us, tiled and this one; 1 to 8 rows; launched early as below):
 // 256 x 1024 3.8, 1.7; 1536 x 1024 4.3, 1.9; 1024 x 3072 5.7, 3.4; 4096 x 4096 11.0, 8.1; 4096 x 12288 22.5, 19.0; 32768 x 1024 16.2,
 // 14.3.  The lines:
 //   * long sums of few columns leave multiprocessors idle, which the tiled kernels' k-splits do not (512 x 8192 7.5, 8.0; 1024 x 8192
 //     9.1, 8.8; 1024 x 16384 13.2, 15.8; 2560 x 9728 16.6, 13.5);
-//   * beyond 50 million entries the stream is all that counts and the tiled kernels' copies have the edge (24576 x 4096 36.2, 37.5), and
+//   * beyond 50 million entries, 34 of many short rows, the stream is all that counts and the tiled kernels' copies have the edge
+//     (24576 x 4096 36.2, 37.5; 24576 x 2048 20.8, 21.2; 49152 x 1024 21.0, 21.5; 16384 x 2048 15.4, 15.4; 4096 x 12288 22.4, 20.2), and
 //     from 20 million where the eight warps' shares of k do not come out even (32768 x 1280 17.9, 20.3);
 //   * 9 to 16 rows read X twice as often: up to 20 million entries (4096 x 4096 11.5, 8.8; 6144 x 4096 14.9, 15.5; 1344 x 5376 7.7, 8.5).
 bool gemm_few_rows_better(const GemmArgs& a) {
   if (!gemm_few_rows_supported(a)) return false;
   const long long entries = static_cast<long long>(a.N) * a.K, round = WARPS * KW;
   if (a.K > 4096 && a.N < (a.M <= 8 && a.K <= 8192 ? 1024 : 2048)) return false;
-  return entries <= 20000000 || (a.M <= 8 && entries <= 52000000 && a.K * 100ll >= (a.K + round - 1) / round * round * 85);
+  return entries <= 20000000 || (a.M <= 8 && entries <= (a.N <= 20480 ? 52000000 : 34000000) && a.K * 100ll >= (a.K + round - 1) / round * round * 85);
 }
 
 const char* gemm_few_rows(const GemmArgs& a, cudaStream_t stream, int rows_of_w) {
@@ -170,7 +171,11 @@ const char* gemm_few_rows(const GemmArgs& a, cudaStream_t stream, int rows_of_w)
   void (*kern)(FewArgs);
   if (a.M <= 8) kern = a.glu_act ? few_rows_kernel<2, 1, true> : wide ? few_rows_kernel<2, 1, false> : few_rows_kernel<1, 1, false>;
   else kern = a.glu_act ? few_rows_kernel<2, 2, true> : wide ? few_rows_kernel<2, 2, false> : few_rows_kernel<1, 2, false>;
-  if (a.pdl) launch_pdl(kern, grid, dim3(WARPS * 32), 0, stream, f);
+  // CTAs that are resident early share the chip with whatever runs there: with more of them than its left-over places the rest
+  // waits for a second wave (a decode step of 8 rows, 3712 wide, 522 us, and 410 with such grids launched in stream order).  The line
+  // lies where one on every multiprocessor still has a place (12 rows, 2176 wide, 136 CTAs: 213 and 175 us; 1024 wide, up to 128: 236 and
+  // 252 without any early launch).
+  if (a.pdl && static_cast<int>(grid.x) <= a.num_sms * 7 / 8) launch_pdl(kern, grid, dim3(WARPS * 32), 0, stream, f);
   else kern<<<grid, WARPS * 32, 0, stream>>>(f);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? nullptr : "few rows: launch failed";

@@ -6,7 +6,8 @@
 // K rows are consumed lane-per-key (each lane streams one 2*D-byte row with 16-byte loads, q is
 // broadcast from shared memory); V rows are consumed warp-per-key (coalesced) with the key's
 // probabilities broadcast by shuffle.  Online softmax per warp, warps merged through shared
-// memory, kv-splits merged by a second tiny kernel through a caller-provided workspace.
+// memory; kv-splits are merged in a cluster through distributed shared memory (the tensor-core form) or by a
+// second tiny kernel through a caller-provided workspace.
 // Supports a sliding window (keys older than `window` are skipped without being read) and a
 // page table (`block_table[b, j / page]` gives the physical page of logical key j).
 #include <cooperative_groups.h>
