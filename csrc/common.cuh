@@ -16,6 +16,7 @@ enum : int {
   kStatusWaitTimeoutEpilogue = 3,
   kStatusPeerWaitTimeout = 4,
   kStatusBadShape = 5,
+  kStatusBadIndex = 6,       // an index in front of its sequence, known on the device only
 };
 
 #ifdef __CUDACC__

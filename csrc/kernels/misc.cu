@@ -367,7 +367,7 @@ const char* embedding(int dtype, const long long* ids, const void* table, void* 
 namespace {
 // Rows start[b] .. start[b] + L - 1 of x [B, S, W pieces], the last row again past the end, a warp per row.  Backward: every
 // row's gradient is written, zeros outside the window; the last row's is a sum in the order of the window.  A negative start is
-// reported and gives zeros.  Bound by the bytes: a gather by an index per element took 120 us for 8 x 1024 rows of 4096 out of
+// reported and its sequence becomes NaNs in both directions, so that no result comes out of it.  Bound by the bytes: a gather by an index per element took 120 us for 8 x 1024 rows of 4096 out of
 // 8 x 1423, its gradient a fill and an indexed sum 161; now 29 and 34 (134 and 160 MB: 20 and 24).
 template <bool BWD>
 __global__ void __launch_bounds__(256)
@@ -377,7 +377,8 @@ window_rows_kernel(const uint4* __restrict__ x, const long long* __restrict__ st
   if (r >= static_cast<long long>(B) * rows) return;
   const int b = static_cast<int>(r / rows), i = static_cast<int>(r - static_cast<long long>(b) * rows);
   const long long at = start[b];
-  if (at < 0 && lane == 0) atomicCAS(status, kStatusOk, kStatusBadShape);
+  if (at < 0 && lane == 0) atomicCAS(status, kStatusOk, kStatusBadIndex);
+  const uint32_t fill = at < 0 ? 0x7FFF7FFFu : 0u;
   const uint4* src = nullptr;
   if (at >= 0) {
     if (!BWD) src = x + (static_cast<long long>(b) * S + min(at + i, static_cast<long long>(S - 1))) * W;
@@ -404,7 +405,7 @@ window_rows_kernel(const uint4* __restrict__ x, const long long* __restrict__ st
     return;
   }
 #pragma unroll 4
-  for (int c = lane; c < W; c += 32) out[r * W + c] = src ? src[c] : make_uint4(0, 0, 0, 0);
+  for (int c = lane; c < W; c += 32) out[r * W + c] = src ? src[c] : make_uint4(fill, fill, fill, fill);
 }
 }  // namespace
 

@@ -170,6 +170,8 @@ class LmPolicy(Policy):
         N = rollouts[0].width
         if any(r.width != N for r in rollouts):
             raise ValueError("rollouts of one scoring call must share max_new_tokens")
+        if any(len(r) > 0 and r.prompt_len < 1 for r in rollouts):
+            raise ValueError("empty prompt: its first completion token has no position that predicts it")
         W = max(r.token_ids.shape[1] for r in rollouts)
         R = sum(len(r) for r in rollouts)
         ids = torch.full((R, W), self.pad_token_id, dtype=torch.int64)

@@ -42,6 +42,17 @@ def kernel_status() -> int:
     return int(lib().kernel_status())
 
 
+STATUS_BAD_INDEX = 6      # the codes of csrc/common.cuh
+
+
+def status_message(code: int) -> str:
+    if code == STATUS_BAD_INDEX:
+        return "a kernel met an index in front of its sequence (a window start or a prompt length below zero)"
+    if code == 5:
+        return "a kernel refused the sizes that it was given"
+    return f"a kernel reported a bounded-wait timeout (status {code})"
+
+
 def _bf16(t):
     return t is not None and t.dtype == torch.bfloat16
 

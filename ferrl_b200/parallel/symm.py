@@ -99,6 +99,8 @@ class SymmHeap:
         st = self.C.kernel_status()
         if st != 0:
             self.C.lib().reset_status()
+            if st == self.C.STATUS_BAD_INDEX:       # an argument of some call before, and nothing that a peer did
+                raise ValueError(f"{what}: {self.C.status_message(st)}")
             self.poisoned = f"{what}: kernel reported status {st} (peer wait timed out)"
             raise CommTimeout(self.poisoned)
 

@@ -80,8 +80,9 @@ class TraceReplay:
             out = out.float().cpu()
         if self.policy.device().type == "cuda":
             from .ops import cuda as C
-            if C.kernel_status() != 0:
-                raise RuntimeError("a kernel reported a bounded-wait timeout")
+            status = C.kernel_status()
+            if status != 0:
+                raise RuntimeError(C.status_message(status))
         return out
 
     def _decoder(self, batch: int, longest: int):
