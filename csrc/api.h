@@ -220,7 +220,8 @@ struct DecodeAttnArgs {
 };
 const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s);
 size_t decode_attn_workspace_bytes(int B, int Hq, int D, int n_splits);
-int decode_attn_pick_splits(int B, int Hkv, int max_len, int D, int num_sms);
+// room: keys that a row may have; tensor_cores: the variant that may merge in clusters
+int decode_attn_pick_splits(int B, int Hq, int Hkv, int D, int room, int num_sms, bool tensor_cores);
 
 // ---- latent attention (csrc/kernels/latent_attn.cu; tcgen05 prefill form in flash_tc.cu) ----
 struct LatentPrepArgs {

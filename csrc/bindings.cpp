@@ -1363,6 +1363,12 @@ void grpo_scale_rows(Tensor dlogp, const Tensor& row_scale) {
   FERRL_CHECK(ferrl::grpo_scale_rows(dlogp.data_ptr<float>(), row_scale.data_ptr<float>(), dlogp.size(0), dlogp.size(1), stream()));
 }
 
+// the number of splits that decode_attn chooses
+int64_t decode_attn_splits(int64_t B, int64_t Hq, int64_t Hkv, int64_t D, int64_t room, int64_t window, int64_t variant, int64_t sms) {
+  TORCH_CHECK(B >= 0 && Hkv > 0 && Hq % Hkv == 0 && sms > 0, "decode_attn_splits: sizes");
+  return ferrl::decode_attn_pick_splits(B, Hq, Hkv, D, window > 0 ? std::min(window, room) : room, sms, variant == 0);
+}
+
 Tensor decode_attn(const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& kv_len, double scale,
                    int64_t window, int64_t n_splits, const optional<Tensor>& block_table, int64_t page, int64_t variant,
                    const optional<Tensor>& prefix_len, int64_t group, int64_t prefix_splits) {
@@ -1379,7 +1385,7 @@ Tensor decode_attn(const Tensor& q, const Tensor& kc, const Tensor& vc, const Te
     a.block_table = block_table->data_ptr<int>(); a.bt_stride = block_table->size(1); a.page = page;
   }
   a.scale = scale; a.window = window;
-  a.n_splits = n_splits > 0 ? n_splits : ferrl::decode_attn_pick_splits(a.B, a.Hkv, kc.size(1), a.D, num_sms());
+  a.n_splits = n_splits > 0 ? n_splits : decode_attn_splits(a.B, a.Hq, a.Hkv, a.D, kc.size(1), window, variant, num_sms());
   Tensor out = out_empty_like(q);
   Tensor ws;
   if (prefix_len.has_value() && prefix_len->defined()) {
@@ -2167,6 +2173,7 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("adamw_step(Tensor[] params, Tensor[] grads, Tensor[] m, Tensor[] v, float lr, float b1, float b2, float eps, float wd, int step, float max_norm, float pre_scale, bool compute_norm) -> Tensor", &adamw_step);
   m.def("grpo_loss_rows(Tensor logp, Tensor logp_old, Tensor? logp_ref, Tensor adv, Tensor mask, Tensor? tis, float eps_lo, float eps_hi, float beta, bool seq_level, bool want_grad) -> (Tensor, Tensor, Tensor)", &grpo_loss_rows);
   m.def("grpo_scale_rows(Tensor(a!) dlogp, Tensor row_scale) -> ()", &grpo_scale_rows);
+  m.def("decode_attn_splits(int B, int Hq, int Hkv, int D, int room, int window=0, int variant=0, int sms=148) -> int", &decode_attn_splits);
   m.def("decode_attn(Tensor q, Tensor kc, Tensor vc, Tensor kv_len, float scale, int window, int n_splits, Tensor? block_table, int page, int variant=0, Tensor? prefix_len=None, int group=1, int prefix_splits=1) -> Tensor", &decode_attn);
   m.def("latent_prep(Tensor(a!) q, Tensor dkv, Tensor norm_w, float eps, Tensor cos_t, Tensor sin_t, Tensor pos, int dim, int rank, int width) -> Tensor", &latent_prep);
   m.def("latent_append(Tensor(a!) q, Tensor dkv, Tensor norm_w, float eps, Tensor cos_t, Tensor sin_t, Tensor kv_len, Tensor(b!) cache, int dim, int rank) -> ()", &latent_append);

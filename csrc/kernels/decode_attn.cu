@@ -626,15 +626,16 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t& r0, uint32_t&
 // 1024 (row, kv-head) items of a 128-row batch in two waves instead of three.
 constexpr int MSTAGES = 3;
 constexpr int MAX_CLUSTER = 8;     // splits of a row that merge through distributed shared memory
+constexpr int ALONE = 64;          // keys that one CTA of a cluster takes by itself: the merge takes longer than they do
 
-template <int D, int REP>
-__global__ void __launch_bounds__(PWARPS * 32, (D <= 128 && REP <= 4) ? 4 : 1)
+template <int D, int REP, bool CLUSTERED>
+__global__ void __launch_bounds__(PWARPS * 32, D <= 128 && REP <= 4 ? 4 : 1)
 decode_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc,
                        const __nv_bfloat16* __restrict__ vc, const int* __restrict__ kv_len,
                        const int* __restrict__ block_table, int bt_stride, int page,
                        __nv_bfloat16* __restrict__ out, float* __restrict__ ws, int Hq, int Hkv,
                        long long seq_stride, long long tok_stride, float scale, int window, int n_splits,
-                       const int* __restrict__ kv_start, int kv_start_div, int ws_off, int ws_total, int clustered) {
+                       const int* __restrict__ kv_start, int kv_start_div, int ws_off, int ws_total) {
   pdl_trigger();   // a dependent GEMM may start streaming its weights while this kernel runs
   pdl_wait();      // launched as a programmatic dependent itself: nothing is read before the predecessor is done
   static_assert(REP <= 8, "query heads of one KV head must fit rows 0..7 of the MMA tile");
@@ -666,7 +667,9 @@ decode_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
   // keys below kv_start[b / kv_start_div] belong to a prefix that another kernel covers (see the group kernel)
   if (kv_start) lo = max(lo, kv_start[b / kv_start_div]);
   const int span = max(len - lo, 0);
-  const int per = (span + n_splits - 1) / n_splits;
+  const bool alone = CLUSTERED && ws_total == 0 && span <= ALONE;      // the same for the whole cluster; prefix partials are better shared
+  if (alone && split > 0) return;
+  const int per = alone ? span : (span + n_splits - 1) / n_splits;
   const int s0 = lo + split * per;
   const int s1 = min(len, s0 + per);
   const int n_tiles = s1 > s0 ? (s1 - s0 + PTK - 1) / PTK : 0;
@@ -804,7 +807,7 @@ decode_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
       out[head * D + d] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
     }
   };
-  if (clustered) {
+  if (CLUSTERED && !alone) {
     // the splits of a row are one cluster: each writes an equal share of the row from all the splits' sums, read out of their
     // shared memory (in the order of the splits, as the second kernel reads them from the workspace)
     float* p_m = o_s + PWARPS * REP * D;        // [REP]
@@ -852,7 +855,7 @@ decode_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16*
     const int r = i / D, d = i - r * D;
     float m, l, acc;
     merged(r, d, m, l, acc);
-    if (ws_total > 0 || n_splits == 1) {
+    if (CLUSTERED || ws_total > 0 || n_splits == 1) {
       finish(r, d, m, l, acc);
     } else {
       float* w_ = ws + ((static_cast<long long>(b) * Hq + hk * REP + r) * n_splits + split) * (D + 2);
@@ -1381,29 +1384,59 @@ static int cluster_share(long long ctas, int splits, int sms) {      // CTAs of 
 static bool in_clusters(long long ctas, int splits, int sms) {
   return splits > 1 && splits <= MAX_CLUSTER && cluster_share(ctas, splits, sms) <= 2;
 }
-// What a step takes with `splits`, in us at head dim 128: a tile of 32 keys passes in 0.61 alone, a multiprocessor moves one in 0.42;
-// fitted to 1 to 24 rows of 2 to 8 heads and 100 to 8000 keys.  841 keys: two pairs 11.3 -> 6.3 us, 32 pairs 12.3 -> 8.4, 128 pairs 19.6
-// -> 15.9; eight pairs of head dim 256 19.0 -> 10.8.
-static double split_time(long long ctas, int splits, int max_len, int D, int sms) {
-  const bool cl = in_clusters(ctas, splits, sms);
-  const double on_each = cl || splits == 1 ? cluster_share(ctas, splits, sms) : static_cast<double>(ctas * splits) / sms;
-  const int tiles = (max_len + 32 * splits - 1) / (32 * splits);
-  const double once = splits == 1 ? 1.0 : cl ? (splits <= 4 ? 3.2 : 3.9) : splits == 2 ? 3.5 : splits == 4 ? 5.0 : 6.0;
-  return (once + tiles * std::max(0.61, 0.42 * on_each)) * D / 128;
+// Splits of a row by the room of its cache (or the window, where that is shorter), which is all that the host knows: a cache fills up
+// from its first key to its last one, so a number is taken where the mean over all lengths is lower, and ALONE keeps the short ones
+// cheap.  Times in us with caches out of memory, head dim 128: one split, clusters, free ones (the number):
+//    16 pairs   room  300: 8 keys 2.2, 2.5 (4), 4.5 (2)   all keys  7.5,  4.9, 7.9       room  600: all keys 13.1,  6.4 (8),  9.9 (2)
+//               room 2048: 8 keys 2.3, 3.0 (8), 5.4 (8)   all keys 39.4, 10.1, 9.9       room 8192: all keys  152, 27.6 (8), 22.2 (16)
+//    64 pairs   room  300: 8 keys 2.2, 2.9 (4), 4.5 (2)   all keys  8.2,  6.9, 7.4       room 2048: all keys 39.9, 16.8 (4), 16.6 (8)
+//    80 pairs   room  600: all keys 13.3, 10.9 (2), 8.9 (4)
+//   128 pairs   room  600: 8 keys 2.8, 3.4 (2), 6.2 (2)   all keys 17.7, 14.7, 18.5      room 2048: all keys 52, 25 (2), 23 (4)
+static int cluster_splits(long long pairs, int room, int D, int sms) {
+  const bool eight = pairs * 8 <= 120ll * sms / 148 || (D <= 128 && room >= 768 && pairs * 8 <= 128ll * sms / 148);
+  if (room < 256 || room >= 4096) return 1;
+  if (room < 384) return pairs * 4 <= 132ll * sms / 148 ? 4 : 1;
+  if (eight) return 8;
+  if (pairs * 4 <= 264ll * sms / 148) {
+    if (room >= 2048) return pairs * 4 > 132ll * sms / 148 ? 4 : 1;
+    return D > 128 && room >= 1024 && pairs * 6 <= sms ? 1 : 4;
+  }
+  if (pairs > sms || room >= 2048) return 1;
+  return D > 128 ? (room >= 1024 ? 2 : 1) : (room < 512 || pairs * 4 >= 3ll * sms ? 2 : 1);
 }
-static int pick_splits(long long ctas, int max_len, int D, int sms, bool clusters_only) {
-  int best = 1;
-  for (int s = 2; s <= (clusters_only ? MAX_CLUSTER : 16); s *= 2)      // free CTAs: up to four a multiprocessor
-    if ((in_clusters(ctas, s, sms) || (!clusters_only && ctas * s < 4ll * sms)) && split_time(ctas, s, max_len, D, sms) <= split_time(ctas, best, max_len, D, sms)) best = s;
-  return best;
+// Of a row whose splits cannot be anything but clusters: as many as fit, where there is room to share.
+static int prefix_splits_of_rest(long long pairs, int room, int sms) {
+  if (room < 512) return 1;
+  return pairs * 8 <= 128ll * sms / 148 ? 8 : pairs * 4 <= 264ll * sms / 148 ? 4 : pairs <= sms ? 2 : 1;
+}
+// CTAs that do not know each other.  Two to a multiprocessor with at least 256 keys each (three or four where twice as few leave some
+// idle; at head dim 256 no more than two fit).  The forms without tensor cores take eight times as long for a key, so they go on to
+// shorter splits (two pairs of 900 keys, three heads each: four splits 83 us, sixteen 25).
+static int free_splits(long long pairs, int room, int D, int sms, bool tensor_cores) {
+  int s = 1;
+  if (!tensor_cores) {
+    while (s < 16 && pairs * s * 2 <= 4ll * sms && room / (s * 2) >= (pairs * s * 2 <= 2ll * sms ? 32 : 100)) s *= 2;
+    return s;
+  }
+  if (D <= 64 && pairs > sms && room < 1024) return 1;
+  if (D <= 128 && room >= 512)
+    while (s < 4 && room / (s * 2) >= 128 && pairs * s * 2 <= 3ll * sms) s *= 2;
+  while (s < 16 && room / (s * 2) >= 256 && (D > 128 ? pairs * s * 2 <= 2ll * sms : pairs * s < 2ll * sms)) s *= 2;
+  return s;
+}
+static bool tensor_core_form(int D, int rep) {
+  return (D == 64 || D == 128 || D == 256) && (rep == 1 || rep == 2 || rep == 4 || rep == 8 || (D == 256 && rep == 6));
 }
 
 size_t decode_attn_workspace_bytes(int B, int Hq, int D, int n_splits) {
   return n_splits <= 1 ? 0 : static_cast<size_t>(B) * Hq * n_splits * (D + 2) * sizeof(float);
 }
 
-int decode_attn_pick_splits(int B, int Hkv, int max_len, int D, int num_sms) {
-  return pick_splits(static_cast<long long>(B) * Hkv, max_len, D, num_sms, false);
+int decode_attn_pick_splits(int B, int Hq, int Hkv, int D, int room, int num_sms, bool tensor_cores) {
+  const long long pairs = static_cast<long long>(B) * Hkv;
+  tensor_cores = tensor_cores && Hkv > 0 && tensor_core_form(D, Hq / Hkv);
+  const int s = tensor_cores ? cluster_splits(pairs, room, D, num_sms) : 1;
+  return s > 1 ? s : free_splits(pairs, room, D, num_sms, tensor_cores);
 }
 
 const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s) {
@@ -1468,7 +1501,7 @@ const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s) {
 #undef FERRL_DECODE_GROUP
     if (!ok) return "decode_attn: shared-prefix mode has no kernel for this (head_dim, heads per kv head, group) triple";
     count_launch();
-    grid.z = pick_splits(pairs, a.bt_stride * a.page, a.D, sms, true);      // of the private keys
+    grid.z = prefix_splits_of_rest(pairs, a.bt_stride * a.page, sms);      // of the private keys
     clustered = grid.z > 1;
   }
   // The CTAs of a cluster would sit together on as few multiprocessors as hold them: shared memory that nobody uses spreads them.
@@ -1501,10 +1534,15 @@ const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s) {
 #define FERRL_DECODE_MMA(DD, RR)                                                                                    \
   if (!launched && a.D == DD && rep == RR && a.no_pipe == 0) {                                                        \
     constexpr size_t msm_bytes = static_cast<size_t>(MSTAGES) * 2 * PTK * DD * 2;                                     \
-    auto mk = decode_attn_mma_kernel<DD, RR>;                                                                         \
-    if (!FERRL_ONCE_PER_DEVICE(cudaFuncSetAttribute(mk, cudaFuncAttributeMaxDynamicSharedMemorySize,                  \
+    auto one = decode_attn_mma_kernel<DD, RR, false>;                                                                 \
+    auto many = decode_attn_mma_kernel<DD, RR, true>;                                                                 \
+    if (!FERRL_ONCE_PER_DEVICE(cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize,                 \
+                                                    static_cast<int>(msm_bytes)) == cudaSuccess &&                    \
+                               cudaFuncSetAttribute(many, cudaFuncAttributeMaxDynamicSharedMemorySize,                \
                                                     static_cast<int>(std::max(msm_bytes, kSpreadMax))) == cudaSuccess && \
-                               cudaFuncSetAttribute(mk, cudaFuncAttributePreferredSharedMemoryCarveout,               \
+                               cudaFuncSetAttribute(one, cudaFuncAttributePreferredSharedMemoryCarveout,              \
+                                                    cudaSharedmemCarveoutMaxShared) == cudaSuccess &&                 \
+                               cudaFuncSetAttribute(many, cudaFuncAttributePreferredSharedMemoryCarveout,             \
                                                     cudaSharedmemCarveoutMaxShared) == cudaSuccess))                  \
       return "decode_attn: cannot reserve shared memory";                                                             \
     cudaLaunchConfig_t cfg{};                                                                                         \
@@ -1520,11 +1558,10 @@ const char* decode_attn(const DecodeAttnArgs& a, cudaStream_t s) {
     at[1].val.clusterDim.z = grid.z;                                                                                  \
     cfg.attrs = at;                                                                                                   \
     cfg.numAttrs = clustered ? 2 : 1;                                                                                 \
-    if (cudaLaunchKernelEx(&cfg, mk, static_cast<const __nv_bfloat16*>(a.q), static_cast<const __nv_bfloat16*>(a.k),  \
+    if (cudaLaunchKernelEx(&cfg, clustered ? many : one, static_cast<const __nv_bfloat16*>(a.q), static_cast<const __nv_bfloat16*>(a.k),  \
                            static_cast<const __nv_bfloat16*>(a.v), a.kv_len, a.block_table, a.bt_stride, a.page,      \
                            static_cast<__nv_bfloat16*>(a.out), a.workspace, a.Hq, a.Hkv, a.seq_stride, a.tok_stride,  \
-                           a.scale, a.window, static_cast<int>(grid.z), kv_start, kv_start_div, ws_off, ws_total,     \
-                           clustered ? 1 : 0) != cudaSuccess)                                                         \
+                           a.scale, a.window, static_cast<int>(grid.z), kv_start, kv_start_div, ws_off, ws_total) != cudaSuccess) \
       return "decode_attn launch failed";                                                                             \
     merged = clustered;                                                                                               \
     launched = true;                                                                                                  \

@@ -588,10 +588,13 @@ def decode_attention(q, k_cache, v_cache, kv_len, *, scale, window=0, n_splits=0
         B = q.shape[0]
         if int(prefix_splits):
             ps = int(prefix_splits)
-        elif (q.shape[-1], q.shape[1] // k_cache.shape[2], group) == (128, 4, 8) and (B // group) * k_cache.shape[2] > 74:
-            # The whole-group kernel: prefix and private keys in one launch, one CTA a group and head.  With those on less than
-            # half the chip splits of both are faster (320 shared and 512 private keys, us: 8 pairs 57 and 19, 32 pairs 58
-            # and 44, 64 pairs 58 and 50, 96 pairs 58 and 80).
+        elif ((q.shape[-1], q.shape[1] // k_cache.shape[2], group) == (128, 4, 8) and
+              ((B // group) * k_cache.shape[2] > 74 or
+               ((B // group) * k_cache.shape[2] > 16 and block_table.shape[1] * k_cache.shape[1] < 1024))):
+            # The whole-group kernel: prefix and private keys in one launch, one CTA a group and head.  Splits of both are slower
+            # while the rows have few keys of their own and much faster later (320 shared keys, us, 1 / 128 / 760 private ones: 8 pairs
+            # 15.0 / 24.3 / 77 and 15.8 / 14.8 / 21; 16 pairs 15.4 / 24.6 / 77 and 19 / 20 / 32; 32 pairs 15.4 / 24.7 / 78 and
+            # 20 / 25 / 60; 64 pairs 15.4 / 25.1 / 78 and 21 / 26 / 63), so more than 16 pairs want room for that.
             ps = 1
         else:
             ps = max(1, min(4, 296 // max(1, (B // group) * k_cache.shape[2])))   # about two prefix CTAs per SM
