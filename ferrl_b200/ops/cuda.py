@@ -1068,6 +1068,12 @@ class _MoeExperts(torch.autograd.Function):
         return dx, dsc, None, None, None, None, None, None, None, None
 
 
+def _pieces(t):
+    """Whole 16-byte pieces: packed, and moved where a view starts off such a boundary."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _WindowRows(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, start, n):
@@ -1077,7 +1083,7 @@ class _WindowRows(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        return lib().window_rows(dy.contiguous(), ctx.saved_tensors[0], ctx.rows, True), None, None
+        return lib().window_rows(_pieces(dy), ctx.saved_tensors[0], ctx.rows, True), None, None
 
 
 def window_rows(x, start, n):
@@ -1100,7 +1106,7 @@ class _GateMul(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        return lib().gate_mul(*ctx.saved_tensors, dy.contiguous())
+        return lib().gate_mul(*ctx.saved_tensors, _pieces(dy))
 
 
 def gate_mul(a, gate):
@@ -1125,7 +1131,7 @@ class _MoeShared(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        dsh, dx = lib().moe_shared_bwd(dy.contiguous(), *ctx.saved_tensors)
+        dsh, dx = lib().moe_shared_bwd(_pieces(dy), *ctx.saved_tensors)
         return dx, None, dy, dsh
 
 
