@@ -341,7 +341,8 @@ gdn_chunk_scan_kernel(ChunkArgs a, const float* S0, float* S_out, __nv_bfloat16*
   // halves of the state's pieces, R's, the scaled Vn's, Vn's, O in v's place, O's sums read
   uint64_t *s_full = bars + 4, *r_full = bars + 6, *w_full = bars + 7, *v_full = bars + 8, *o_full = bars + 9, *o_read = bars + 11;
   uint64_t *ks_done = bars + 12, *qs_done = bars + 13, *vn_done = bars + 14, *inc_done = bars + 15, *o_done = bars + 16;
-  uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 18);
+  uint64_t* o_taken = bars + 18;             // the copying warps have read O out of v's place
+  uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 19);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(slot + 1);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int bh = blockIdx.x, b = bh / a.Hv, hv = bh % a.Hv, hk = hv / (a.Hv / a.Hk);
@@ -350,7 +351,7 @@ gdn_chunk_scan_kernel(ChunkArgs a, const float* S0, float* S_out, __nv_bfloat16*
     return;
   }
   if (tid == 0) {
-    for (int i = 0; i < 18; ++i) mbar_init(&bars[i], i == 2 || i == 3 ? 3 : i >= 4 && i < 12 ? CW : 1);
+    for (int i = 0; i < 19; ++i) mbar_init(&bars[i], i == 2 || i == 3 || i == 18 ? 3 : i >= 4 && i < 12 ? CW : 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -498,8 +499,9 @@ gdn_chunk_scan_kernel(ChunkArgs a, const float* S0, float* S_out, __nv_bfloat16*
         }
         if (ci + 2 < a.n) {
           if (!wait(&o_done[ci & 1], (ci >> 1) & 1)) break;
-          // all of O is read before v takes its place (a warp that is here saw o_done, which the others see too)
-          asm volatile("bar.sync 1, 96;" ::: "memory");
+          __syncwarp();                      // all of O is read before v takes its place
+          if (lane == 0) mbar_arrive(o_taken);
+          if (!wait(o_taken, ci & 1)) break;
           load(ci + 2);
         }
       }
