@@ -150,7 +150,7 @@ const char* kv_append_paged(const void* k, const void* v, long long ldv, void* k
                             const int* table, int bt_stride, int page, int batch, int HD, cudaStream_t s);
 // strides and W (a row of all heads) in 16-byte pieces; full: whole pages of each prompt
 const char* kv_prefill_paged(const void* k, const void* v, long long k_bs, long long k_ts, long long v_bs, long long v_ts, void* kc,
-                             void* vc, const long long* full, int P, int L, int ppr, int page, int G, int W, cudaStream_t s);
+                             void* vc, const long long* full, int P, int L, int ppr, int page, int G, int W, int* status, cudaStream_t s);
 const char* kv_append(int dtype, const void* k, const void* v, long long ldv, void* kc, void* vc, const int* kv_len,
                       int batch, int smax, int HD, cudaStream_t s);
 

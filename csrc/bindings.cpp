@@ -1196,7 +1196,7 @@ void kv_append_paged(const Tensor& k, const Tensor& v, Tensor kc, Tensor vc, con
 bool kv_prefill_paged(const Tensor& k, const Tensor& v, Tensor kc, Tensor vc, const Tensor& full, int64_t ppr, int64_t G) {
   c10::cuda::CUDAGuard guard(k.device());
   TORCH_CHECK(k.dim() == 4 && v.sizes() == k.sizes() && kc.dim() == 4 && vc.sizes() == kc.sizes() && kc.is_contiguous() && vc.is_contiguous() &&
-                  kc.size(2) == k.size(2) && kc.size(3) == k.size(3) && ppr >= 0 && G >= 1 && kc.size(0) == k.size(0) * ppr * (1 + G) &&
+                  kc.size(2) == k.size(2) && kc.size(3) == k.size(3) && ppr >= 1 && G >= 1 && kc.size(0) == k.size(0) * ppr * (1 + G) &&
                   full.scalar_type() == at::kLong && full.is_contiguous() && full.numel() == k.size(0) && full.is_cuda(),
               "kv_prefill_paged: layout");
   const int64_t e = k.element_size(), HD = k.size(2) * k.size(3);
@@ -1211,7 +1211,7 @@ bool kv_prefill_paged(const Tensor& k, const Tensor& v, Tensor kc, Tensor vc, co
   const int64_t u = 16 / e;
   FERRL_CHECK(ferrl::kv_prefill_paged(k.data_ptr(), v.data_ptr(), k.stride(0) / u, k.stride(1) / u, v.stride(0) / u, v.stride(1) / u,
                                       kc.data_ptr(), vc.data_ptr(), reinterpret_cast<const long long*>(full.data_ptr<int64_t>()), k.size(0), k.size(1), ppr,
-                                      kc.size(1), G, HD / u, stream()));
+                                      kc.size(1), G, HD / u, status_word(), stream()));
   return true;
 }
 

@@ -877,16 +877,18 @@ __global__ void kv_append_paged_kernel(const __nv_bfloat16* __restrict__ k, cons
 
 // A prompt batch's K and V into the pool: row [p, u] goes to the u-th slot of prompt p's shared pages, and the page of rows
 // that begins at the prompt's last whole page goes to the first private page of each of its G rows too (past the end: the last
-// row again).  A warp per row, blockIdx.z: K or V.  Bound by the bytes: 16 prompts of 512 tokens, 8 heads of 128, groups of 8
+// row again; a negative number of pages is reported, and the page becomes NaNs).  A warp per row, blockIdx.z: K or V.  Bound by the bytes: 16 prompts of 512 tokens, 8 heads of 128, groups of 8
 // took ten copies, gathers and indexed stores, 230 us a layer; now 18 us (101 MB: 15).
 __global__ void __launch_bounds__(256)
 kv_prefill_paged_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, long long k_bs, long long k_ts, long long v_bs,
                         long long v_ts, uint4* __restrict__ kc, uint4* __restrict__ vc, const long long* __restrict__ full, int L, int Lp,
-                        int ppr, int page, int P, int G, int W) {
+                        int ppr, int page, int P, int G, int W, int* status) {
   const int p = blockIdx.y, u = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (u >= Lp + page) return;
   const bool tail = u >= Lp;
-  const long long t = tail ? min(full[p] * page + (u - Lp), static_cast<long long>(L - 1)) : u;
+  const long long whole = tail ? full[p] : 0;
+  if (whole < 0 && lane == 0) atomicCAS(status, kStatusOk, kStatusBadIndex);
+  const long long t = tail ? min(whole * page + (u - Lp), static_cast<long long>(L - 1)) : u;
   const uint4* src = blockIdx.z ? v + p * v_bs + t * v_ts : k + p * k_bs + t * k_ts;
   uint4* pool = blockIdx.z ? vc : kc;
   // slots are a row of pieces wide; a prompt's shared pages are ppr, then come ppr private ones for every row
@@ -897,7 +899,7 @@ kv_prefill_paged_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v
     uint4 x[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      if (i0 + j * 32 + lane < W) x[j] = src[i0 + j * 32 + lane];
+      if (i0 + j * 32 + lane < W) x[j] = whole < 0 ? make_uint4(~0u, ~0u, ~0u, ~0u) : src[i0 + j * 32 + lane];
     for (int g = 0; g < copies; ++g)
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -907,15 +909,16 @@ kv_prefill_paged_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v
 }  // namespace
 
 const char* kv_prefill_paged(const void* k, const void* v, long long k_bs, long long k_ts, long long v_bs, long long v_ts, void* kc,
-                             void* vc, const long long* full, int P, int L, int ppr, int page, int G, int W, cudaStream_t s) {
+                             void* vc, const long long* full, int P, int L, int ppr, int page, int G, int W, int* status, cudaStream_t s) {
   if (P == 0 || L == 0 || W == 0) return nullptr;
+  if (ppr < 1 || page < 1 || G < 1) return "kv_prefill_paged: at least one page and one row";
   if ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15)
     return "kv_prefill_paged: 16-byte aligned rows required";
   if (P > 65535) return "kv_prefill_paged: at most 65535 prompts";
   const int Lp = static_cast<int>(std::min<long long>(L, static_cast<long long>(ppr) * page));
   kv_prefill_paged_kernel<<<dim3((Lp + page + 7) / 8, P, 2), 256, 0, s>>>(static_cast<const uint4*>(k), static_cast<const uint4*>(v), k_bs, k_ts,
                                                                           v_bs, v_ts, static_cast<uint4*>(kc), static_cast<uint4*>(vc), full, L,
-                                                                          Lp, ppr, page, P, G, W);
+                                                                          Lp, ppr, page, P, G, W, status);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? nullptr : "kv_prefill_paged launch failed";
 }

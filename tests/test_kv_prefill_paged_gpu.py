@@ -37,3 +37,26 @@ def test_pools_are_the_same_bytes(P, L, ppr, G, hkv, D, dtype):
     finally:
         ops.native = native
     assert torch.equal(a.k[0], b.k[0]) and torch.equal(a.v[0], b.v[0])
+
+
+def test_pools_without_pages_and_negative_lengths():
+    """A layout without a page is refused before anything is written; a prompt whose length the device finds below zero gets NaNs."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from ferrl_b200.ops import cuda as C
+    k, v = (torch.randn(2, 70, 2, 64, device="cuda").bfloat16() for _ in range(2))
+    empty = torch.zeros(0, 64, 2, 64, device="cuda", dtype=torch.bfloat16)
+    for ppr in (0, -1):
+        with pytest.raises(RuntimeError, match="layout"):
+            C.kv_prefill_paged(empty, empty.clone(), k, v, torch.tensor([1, 1], device="cuda"), ppr, 2)
+    kc, vc = (torch.zeros(2 * 2 * 3, 64, 2, 64, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    assert C.kernel_status() == 0
+    assert C.kv_prefill_paged(kc, vc, k, v, torch.tensor([1, -1], device="cuda"), 2, 2)
+    try:
+        assert C.kernel_status() == C.STATUS_BAD_INDEX
+    finally:
+        C.lib().reset_status()
+    for pool, src in ((kc, k), (vc, v)):
+        first = pool[4::2]                                  # first private pages of the four rows
+        assert torch.equal(first[0, :6], src[0, 64:]) and torch.equal(first[0], first[1])
+        assert first[2:].isnan().all() and not pool[:4].isnan().any()
