@@ -1088,7 +1088,7 @@ class _WindowRows(torch.autograd.Function):
 
 def window_rows(x, start, n):
     """Rows ``start[b] .. start[b] + n - 1`` of bf16 ``x`` ``[B,S,W]``, the last one past the end; ``None`` outside the kernel's domain."""
-    if not _bf16(x) or x.dim() != 3 or x.shape[1] == 0 or x.shape[2] % 8 or not start.is_cuda or start.numel() != x.shape[0]:
+    if not _bf16(x) or x.dim() != 3 or x.shape[1] == 0 or x.shape[2] % 8 or start.device != x.device or start.numel() != x.shape[0]:
         return None
     x = x.contiguous()
     if x.data_ptr() % 16:
@@ -1112,7 +1112,7 @@ class _GateMul(torch.autograd.Function):
 def gate_mul(a, gate):
     """``a * sigmoid(gate)`` for bf16 ``[..,W]``; ``None`` outside the kernel's domain (rows of whole 16-byte pieces)."""
     W = a.shape[-1]
-    if not (_bf16(a) and _bf16(gate)) or a.shape != gate.shape or W % 8 or gate.stride(-1) != 1:
+    if not (_bf16(a) and _bf16(gate)) or a.shape != gate.shape or a.device != gate.device or W % 8 or gate.stride(-1) != 1:
         return None
     a2, g2 = a.reshape(-1, W).contiguous(), gate.reshape(-1, W)
     if g2.stride(1) != 1 or g2.stride(0) % 8 or a2.data_ptr() % 16 or g2.data_ptr() % 16:
@@ -1139,7 +1139,7 @@ def moe_shared(x, w, y, sh):
     """The gated shared expert ``y + sigmoid(x w^T) * sh`` on rows ``[T,H]`` with ``w`` ``[1,H]``; ``None`` outside the kernel's
     domain (bf16 rows of whole 16-byte pieces, a frozen gate)."""
     ts = (x, w, y, sh)
-    if not all(_bf16(t) for t in ts) or w.requires_grad or x.dim() != 2 or w.numel() != x.shape[1] or not x.shape == y.shape == sh.shape or x.shape[1] % 8:
+    if not all(_bf16(t) and t.device == x.device for t in ts) or w.requires_grad or x.dim() != 2 or w.numel() != x.shape[1] or not x.shape == y.shape == sh.shape or x.shape[1] % 8:
         return None
     ts = tuple(t.contiguous() for t in ts)
     if any(t.data_ptr() % 16 for t in ts):
