@@ -124,43 +124,51 @@ gdn_conv_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __
   conv_taps<K, V>(w + static_cast<long long>(c) * K, wv);
 #pragma unroll
   for (int j = 1; j < K; ++j) conv_input<K, V>(x, ldx, left, b, t0 - K + j, c, L, C, win[j]);
-  // four tokens at a time, the next four on their way while these are worked on
   using Raw = typename ConvRaw<V>::type;
-  constexpr int U = 4;
   const __nv_bfloat16* xp = x + static_cast<long long>(b) * L * ldx + c;
   __nv_bfloat16* yp = y + static_cast<long long>(b) * L * C + c;
-  Raw now[U], next[U];
+  auto read = [&](int t) { return *reinterpret_cast<const Raw*>(xp + static_cast<long long>(t) * ldx); };
+  auto token = [&](int t, const Raw& in) {
 #pragma unroll
-  for (int u = 0; u < U; ++u)
-    if (t0 + u < t1) now[u] = *reinterpret_cast<const Raw*>(xp + static_cast<long long>(t0 + u) * ldx);
-  for (int t = t0; t < t1; t += U) {
+    for (int j = 0; j + 1 < K; ++j)
+#pragma unroll
+      for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
+    conv_unpack<V>(in, win[K - 1]);
+    float o[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      o[e] = 0.f;
+#pragma unroll
+      for (int j = 0; j < K; ++j) o[e] += wv[j][e] * win[j][e];
+    }
+    if (act) {                           // the eager form rounds the conv output to the activation dtype before the SiLU
+      conv_round<V>(o);
+#pragma unroll
+      for (int e = 0; e < V; ++e) o[e] = silu_f(o[e]);
+    }
+    conv_store<V>(yp + static_cast<long long>(t) * C, o);
+  };
+  if constexpr (V == 1) {                // short runs and many threads: nothing ahead (40 x 3072 2.8 us with, 2.5 without; 6000 x 1001 13.3, 11.5)
+#pragma unroll 4
+    for (int t = t0; t < t1; ++t) token(t, read(t));
+  } else {                               // four tokens at a time, the next four on their way while these are worked on
+    constexpr int U = 4;
+    Raw now[U], next[U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (t + U + u < t1) next[u] = *reinterpret_cast<const Raw*>(xp + static_cast<long long>(t + U + u) * ldx);
+      if (t0 + u < t1) now[u] = read(t0 + u);
+    for (int t = t0; t < t1; t += U) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (t + u >= t1) break;
+      for (int u = 0; u < U; ++u)
+        if (t + U + u < t1) next[u] = read(t + U + u);
 #pragma unroll
-      for (int j = 0; j + 1 < K; ++j)
-#pragma unroll
-        for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
-      conv_unpack<V>(now[u], win[K - 1]);
-      float o[V];
-#pragma unroll
-      for (int e = 0; e < V; ++e) {
-        o[e] = 0.f;
-#pragma unroll
-        for (int j = 0; j < K; ++j) o[e] += wv[j][e] * win[j][e];
+      for (int u = 0; u < U; ++u) {
+        if (t + u >= t1) break;
+        token(t + u, now[u]);
       }
-      if (act) {                         // the eager form rounds the conv output to the activation dtype before the SiLU
-        conv_round<V>(o);
 #pragma unroll
-        for (int e = 0; e < V; ++e) o[e] = silu_f(o[e]);
-      }
-      conv_store<V>(yp + static_cast<long long>(t + u) * C, o);
+      for (int u = 0; u < U; ++u) now[u] = next[u];
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u) now[u] = next[u];
   }
 }
 
@@ -182,26 +190,13 @@ gdn_conv_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __
 #pragma unroll
   for (int j = 1; j < K; ++j) conv_input<K, V>(x, ldx, left, b, t0 - K + j, c, L, C, win[j]);
   using Raw = typename ConvRaw<V>::type;
-  constexpr int U = 2;
   const __nv_bfloat16* xp = x + static_cast<long long>(b) * L * ldx + c;
   const __nv_bfloat16* gp = dy + static_cast<long long>(b) * L * C + c;
-  const int t2 = min(L, t1 + K - 1);
-  Raw now[2][U], next[2][U];
-  auto fetch = [&](Raw (&r)[2][U], int t) {
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (t + u < t2) {
-        r[0][u] = *reinterpret_cast<const Raw*>(xp + static_cast<long long>(t + u) * ldx);
-        r[1][u] = *reinterpret_cast<const Raw*>(gp + static_cast<long long>(t + u) * C);
-      }
+  auto read = [&](Raw& in, Raw& grad, int t) {
+    in = *reinterpret_cast<const Raw*>(xp + static_cast<long long>(t) * ldx);
+    grad = *reinterpret_cast<const Raw*>(gp + static_cast<long long>(t) * C);
   };
-  fetch(now, t0);
-  for (int tb = t0; tb < t1 + K - 1; tb += U) {
-    fetch(next, tb + U);
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const int to = tb + u;
-    if (to >= t1 + K - 1) break;
+  auto token = [&](int to, const Raw& in, const Raw& grad) {
 #pragma unroll
     for (int j = K - 1; j > 0; --j)
 #pragma unroll
@@ -211,8 +206,8 @@ gdn_conv_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __
       for (int j = 0; j + 1 < K; ++j)
 #pragma unroll
         for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
-      conv_unpack<V>(now[0][u], win[K - 1]);
-      conv_unpack<V>(now[1][u], d[0]);
+      conv_unpack<V>(in, win[K - 1]);
+      conv_unpack<V>(grad, d[0]);
       if (act) {
         float pre[V];
 #pragma unroll
@@ -240,7 +235,23 @@ gdn_conv_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __
       }
       conv_store<V>(dx + (static_cast<long long>(b) * L + t) * C + c, o);
     }
-  }
+  };
+  const int t2 = min(L, t1 + K - 1);
+  constexpr int U = 2;
+  Raw now[2][U], next[2][U];
+  auto fetch = [&](Raw (&r)[2][U], int t) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (t + u < t2) read(r[0][u], r[1][u], t + u);
+  };
+  fetch(now, t0);
+  for (int tb = t0; tb < t1 + K - 1; tb += U) {
+    fetch(next, tb + U);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (tb + u >= t1 + K - 1) break;
+      token(tb + u, now[0][u], now[1][u]);
+    }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       now[0][u] = next[0][u];
@@ -444,8 +455,8 @@ bool conv_vec(int C, long long ldx, const void* x, const void* w, const void* y,
 template <int K>
 void conv_launch(bool bwd, const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, const __nv_bfloat16* left,
                  const __nv_bfloat16* dy, int B, int L, int C, int act, __nv_bfloat16* out, cudaStream_t stream) {
-  // four channels and one a thread, us forward / backward: 40 tokens of 3072 9 / 10 and 8 / 8, 300 of 8192 12 / 14 and
-  // 12 / 16, 1000 of 8192 17 / 25 and 25 / 35, 5119 of 10240 55 / 96 and 104 / 170
+  // one channel and four a thread, us forward / backward: 130 tokens of 10240 5.0 / 7.9 and 4.1 / 6.0, 1000 of 3072 7.4 / 12.3
+  // and 5.8 / 8.9, 5000 of 10240 86 / 136 and 48 / 89; below a million values one is as fast or faster
   const bool vec = conv_vec(C, ldx, x, w, out, dy) && static_cast<long long>(B) * L * C >= 1LL << 20;
   const int V = vec ? kConvV : 1, run = conv_run(B, L, C, V), runs = (L + run - 1) / run;
   const dim3 grid(B * runs, (C / V + 127) / 128);
