@@ -369,6 +369,7 @@ size_t flash_bwd_tc_scratch_floats(const FlashArgs& a);   // size of a.delta for
 const char* flash_bwd_tc(const FlashArgs& a, int* status, cudaStream_t stream);
 // the same at head_dim 256 (csrc/kernels/flash_bwd256_tc.cu)
 bool flash_bwd256_tc_supported(const FlashArgs& a);
+bool flash_bwd256_tc_better(int B, int S, int Hq, int Hkv, int num_sms);      // than flash_bwd
 size_t flash_bwd256_tc_scratch_floats(const FlashArgs& a);
 const char* flash_bwd256_tc(const FlashArgs& a, int* status, cudaStream_t stream);
 

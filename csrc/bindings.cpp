@@ -1847,6 +1847,9 @@ std::tuple<Tensor, Tensor> flash_fwd(const Tensor& q, const Tensor& k, const Ten
   return {o, lse};
 }
 
+// which kernels take the backward at head dim 256
+bool flash_bwd256_better(int64_t B, int64_t S, int64_t Hq, int64_t Hkv, int64_t sms) { return ferrl::flash_bwd256_tc_better(B, S, Hq, Hkv, sms); }
+
 std::tuple<Tensor, Tensor, Tensor> flash_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o,
                                              const Tensor& lse, const Tensor& d_o, double scale, bool causal,
                                              int64_t window, int64_t q_offset, int64_t variant,
@@ -1876,7 +1879,7 @@ std::tuple<Tensor, Tensor, Tensor> flash_bwd(const Tensor& q, const Tensor& k, c
     FERRL_CHECK(ferrl::flash_bwd_tc(a, status_word(), stream()));
     return {dq, dk, dv};
   }
-  if (variant != 1 && ferrl::flash_bwd256_tc_supported(a)) {
+  if (variant != 1 && ferrl::flash_bwd256_tc_supported(a) && ferrl::flash_bwd256_tc_better(a.B, a.Sq, a.Hq, a.Hkv, num_sms())) {
     Tensor stats = out_empty({static_cast<long long>(ferrl::flash_bwd256_tc_scratch_floats(a))}, lse.options());
     a.delta = stats.data_ptr<float>();
     FERRL_CHECK(ferrl::flash_bwd256_tc(a, status_word(), stream()));
@@ -2194,6 +2197,7 @@ TORCH_LIBRARY(ferrl_b200, m) {
   m.def("gemm_glu(Tensor A, Tensor B, int act, bool static_b=False, float alpha=0.0, float limit=0.0) -> Tensor", &gemm_glu);
   m.def("qk_norm_rope_append(Tensor q, Tensor k, Tensor v, Tensor? qw, Tensor? kw, Tensor cos_t, Tensor sin_t, Tensor pos, float eps, bool zc, Tensor(a!) kc, Tensor(b!) vc, Tensor kv_len, Tensor? table) -> Tensor", &qk_norm_rope_append);
   m.def("flash_fwd(Tensor q, Tensor k, Tensor v, float scale, bool causal, int window, int q_offset, int variant=0) -> (Tensor, Tensor)", &flash_fwd);
+  m.def("flash_bwd256_tc_better(int B, int S, int Hq, int Hkv, int sms=148) -> bool", &flash_bwd256_better);
   m.def("flash_bwd(Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor d_o, float scale, bool causal, int window, int q_offset, int variant=0, Tensor? debug=None) -> (Tensor, Tensor, Tensor)", &flash_bwd);
   m.def("logprob_head_fwd(Tensor hidden, Tensor w, Tensor targets, float temperature, float softcap) -> (Tensor, Tensor)", &logprob_head_fwd);
   m.def("logprob_head_shard_stats(Tensor hidden, Tensor w, Tensor targets, float temperature, float softcap, int col0) -> Tensor", &logprob_head_shard_stats);

@@ -16,8 +16,8 @@
 // What bounds it: a streamed tile of TA stays from its load through scores, softmax and last product, and two slots are all
 // that fits, so a step takes about half of that life; the tensor cores need 1536 of its cycles.  All three kernels with the
 // tensor maps' host time, against the warp-level kernels of flash_attn.cu: 5119 tokens, 24 and 4 heads 5974 -> 1523 us (529
-// TFLOP/s, 32 % of measured); 4 x 1535, 16 and 2 heads 1732 -> 515; 1000, 8 and 2 heads 392 -> 95; 64, 8 and 2 heads 46 -> 44, so
-// no length is left to them.
+// TFLOP/s, 32 % of measured); 4 x 1535, 16 and 2 heads 1732 -> 515; 1000, 8 and 2 heads 392 -> 95; 64, 8 and 2 heads 34 -> 22.
+// Many rows of a tile or less are left to them (flash_bwd256_tc_better).
 //
 // dK and dV walk every query head of the group.  The first key tile sees all queries, so where key tiles are few a cluster
 // of 2 or 4 CTAs takes the heads of a key tile in shares and adds the shares through distributed shared memory in rank order.
@@ -461,6 +461,24 @@ flash_bwd256_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid
 
 }  // namespace
 
+// as many as it takes for about three CTAs a multiprocessor, since the first key tile is twice the mean
+static int pick_shares(long long ctas, int G, int sms) {
+  int shares = 1;
+  while (2 * shares <= G && 2 * shares <= kMaxShares && ctas * shares < 3ll * sms) shares *= 2;
+  return shares;
+}
+
+// Not where there are many short rows: a wave of these CTAs takes 10 us, whatever little it has to do, and the warp-level kernels take 6
+// for each query head of a key head and one for 10 tokens or so (us, these and those, waves 3, 4, 6, 7: 4 rows of 8 tokens, 32 and 8
+// heads 35, 29; 8 of 16, 24 and 4 43, 46; 8 of 64, 32 and 8 66, 45; 16 of 64, 24 and 4 80, 65; 16 of 96, 32 and 8 114, 174).
+bool flash_bwd256_tc_better(int B, int S, int Hq, int Hkv, int sms) {
+  if (S > 64 || Hkv < 1) return true;
+  const int G = Hq / Hkv;
+  const long long dq = static_cast<long long>(B) * Hq, dkv = 2ll * B * Hkv * pick_shares(2ll * B * Hkv, G, sms);
+  const long long waves = (dq + sms - 1) / sms + (dkv + sms - 1) / sms;
+  return waves < 3 || 64 * waves < 58 + 31 * G + S;
+}
+
 size_t flash_bwd256_tc_scratch_floats(const FlashArgs& a) {
   return static_cast<size_t>(a.B) * a.Hq * ((a.Sq + RT - 1) / RT * RT) * 2;
 }
@@ -504,13 +522,10 @@ const char* flash_bwd256_tc(const FlashArgs& a, int* status, cudaStream_t stream
     return "flash_bwd256_tc: cannot reserve shared memory";
   flash_bwd256_dq_tc_kernel<<<dim3(a.Hq, a.B, n_t), THREADS, SMEM, stream>>>(mQ, mdO, mKt, mVt, p);
   count_launch();
-  // shares: as many as it takes for about three CTAs a multiprocessor, since the first key tile is twice the mean
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long ctas = 2ll * a.B * a.Hkv * n_t;
-  p.shares = 1;
-  while (2 * p.shares <= G && 2 * p.shares <= kMaxShares && ctas * p.shares < 3ll * sms) p.shares *= 2;
+  p.shares = pick_shares(2ll * a.B * a.Hkv * n_t, G, sms);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(p.shares, 2 * a.B * a.Hkv, n_t);
   cfg.blockDim = dim3(THREADS);
