@@ -139,15 +139,17 @@ bool gemm_few_rows_supported(const GemmArgs& a) {
          !a.tile_expert && a.ar_world <= 1 && !a.ss_in && !a.ss_out && !a.lp_mode;
 }
 
-// Against the tiled kernels in a chain of launches, weights from HBM (us, tiled and this one; 1 to 8 rows; launched early as below):
-// 256 x 1024 3.8, 1.7; 1536 x 1024 4.3, 1.9; 1024 x 3072 5.7, 3.4; 4096 x 4096 11.0, 8.1; 4096 x 12288 22.5, 19.0; 32768 x 1024 16.2,
-// 14.3.  The lines:
-//   * long sums of few columns leave multiprocessors idle, which the tiled kernels' k-splits do not (512 x 8192 7.5, 8.0; 1024 x 8192
-//     9.1, 8.8; 1024 x 16384 13.2, 15.8; 2560 x 9728 16.6, 13.5);
-//   * beyond 50 million entries, 34 of many short rows, the stream is all that counts and the tiled kernels' copies have the edge
-//     (24576 x 4096 36.2, 37.5; 24576 x 2048 20.8, 21.2; 49152 x 1024 21.0, 21.5; 16384 x 2048 15.4, 15.4; 4096 x 12288 22.4, 20.2), and
-//     from 20 million where the eight warps' shares of k do not come out even (32768 x 1280 17.9, 20.3);
-//   * 9 to 16 rows read X twice as often: up to 20 million entries (4096 x 4096 11.5, 8.8; 6144 x 4096 14.9, 15.5; 1344 x 5376 7.7, 8.5).
+// Against the tiled kernels in a chain of launches, weights from HBM, as both are launched (us, tiled and this one; 1 to 8 rows; * this
+// one early, see below): 256 x 1024* 3.6, 1.5; 1536 x 1024* 4.2, 1.9; 1024 x 3072* 5.3, 4.0; 4096 x 1024 5.7, 3.5; 4096 x 4096 9.8, 8.5;
+// 6144 x 4096 13.8, 12.7; 4096 x 12288 20.5, 18.5; 12288 x 4096 23.4, 20.6.  The lines:
+//   * long sums of few columns leave multiprocessors idle, which the tiled kernels' k-splits do not (512 x 8192* 7.3, 8.0; 1024 x 8192*
+//     8.9, 8.7; 1536 x 8192 9.3, 9.8; 1024 x 16384* 12.7, 15.7; 2560 x 9728 15.2, 13.4);
+//   * beyond 52 million entries, 34 where rows are short and many, the stream is all that counts and the tiled kernels' copies have
+//     the edge (24576 x 4096 34.2, 37.1; 24576 x 2048 19.0, 19.7; 49152 x 1024 19.3, 20.0; a tie at 32768 x 1024 14.3, 14.1 and 16384 x
+//     2048 13.7, 13.9), and from 20 million where the eight warps' shares of k do not come out even (32768 x 1280 16.4, 19.8; 16384 x
+//     1280 9.9, 11.5);
+//   * 9 to 16 rows read X twice as often: up to 20 million entries (4096 x 4096 9.9, 9.0; 2048 x 8192 11.2, 11.1; 16384 x 2048 13.8, 15.6;
+//     1344 x 5376 7.4, 8.2).
 bool gemm_few_rows_better(const GemmArgs& a) {
   if (!gemm_few_rows_supported(a)) return false;
   const long long entries = static_cast<long long>(a.N) * a.K, round = WARPS * KW;
@@ -162,9 +164,11 @@ const char* gemm_few_rows(const GemmArgs& a, cudaStream_t stream, int rows_of_w)
   f.out = static_cast<__nv_bfloat16*>(a.out);
   f.ldx = a.lda; f.ldw = a.ldb; f.ldr = a.ldr; f.ldo = a.ldo;
   f.M = a.M; f.N = a.N; f.K = a.K; f.act = a.glu_act - 1; f.alpha = a.glu_alpha; f.limit = a.glu_limit;
-  // Tiles of 8 rows of W while each has a place of its own on the chip and enough columns to share out (2048 x 4096 6.2 -> 5.5 us,
-  // 1024 x 3072 3.8 -> 3.4; 2496 x 1664, 312 tiles for 296 places, 3.2 -> 4.6; 1536 x 1024 1.9 -> 2.0).
-  const bool narrow = a.N <= 16 * a.num_sms && a.K >= 2048 && a.M <= 8;
+  // Tiles of 8 rows of W while each has a place of its own on the chip and enough columns to share out, but not where only tiles of 16
+  // are few enough to be launched early (us, 8 and 16: 1024 x 3072 3.6, 4.0; 1024 x 8192 8.4, 9.2; 2048 x 2048 3.8, 3.2; 2048 x 4096 6.3,
+  // 5.9; 2368 x 4096 6.4, 6.8; 2496 x 1664 5.2, 4.0).
+  const int early = a.num_sms * 7 / 8;
+  const bool narrow = a.N <= 16 * a.num_sms && a.K >= 2048 && a.M <= 8 && !(a.pdl && a.N > 8 * early && a.N <= 16 * early);
   const bool wide = a.glu_act || (rows_of_w ? rows_of_w == 16 : !narrow);
   const int tiles = (a.N + (wide ? 15 : 7)) / (wide ? 16 : 8);
   const dim3 grid(std::min(tiles, 2 * a.num_sms));
@@ -175,7 +179,7 @@ const char* gemm_few_rows(const GemmArgs& a, cudaStream_t stream, int rows_of_w)
   // waits for a second wave (a decode step of 8 rows, 3712 wide, 522 us, and 410 with such grids launched in stream order).  The line
   // lies where one on every multiprocessor still has a place (12 rows, 2176 wide, 136 CTAs: 213 and 175 us; 1024 wide, up to 128: 236 and
   // 252 without any early launch).
-  if (a.pdl && static_cast<int>(grid.x) <= a.num_sms * 7 / 8) launch_pdl(kern, grid, dim3(WARPS * 32), 0, stream, f);
+  if (a.pdl && static_cast<int>(grid.x) <= early) launch_pdl(kern, grid, dim3(WARPS * 32), 0, stream, f);
   else kern<<<grid, WARPS * 32, 0, stream>>>(f);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? nullptr : "few rows: launch failed";
