@@ -34,8 +34,9 @@ constexpr int LG_X_BYTES = LG_ROWS * 256;      // a stage's tile of X: rows of 1
 template <int RT> constexpr int LG_U_ROW = RT <= 4 ? 128 : 256;
 template <int RT> constexpr int LG_STAGE_BYTES = LG_X_BYTES + LG_ROWS * LG_U_ROW<RT>;
 
-// Bound by reading X once.  11392 tokens, us (bytes' time), before and now: rank 16 x 4096 columns 35 and 32 (14), 32 x 24576 127 and
-// 107 (86), 48 x 6144 56 and 47 (22); 5119 tokens, 64 x 10240 60 and 39 (16); 4608 tokens, 32 x 43008 117 and 86 (61).  What the time was:
+// Bound by reading X once.  In a chain of calls, us (bytes' time), before and now: 11392 tokens, rank 16 x 4096 columns 25 and 22 (14),
+// 32 x 24576 114 and 90 (86), 48 x 6144 50 and 34 (22); 5119 tokens, 64 x 10240 54 and 32 (16); 4608 tokens, 32 x 43008 106 and 70 (61).  What
+// the time was:
 // two CTAs an SM, because a tile of U took as much shared memory as one of X; an address computed anew for every 16 bytes;
 // the ranges' sums fetched one by one by the last CTA; ranges cut so that they filled waves and not so that they ended together.
 constexpr int LG_CHAIN = 8;      // stages whose products are summed by the tensor cores alone
@@ -232,8 +233,8 @@ size_t lora_grad_workspace_floats(int R, int C, int n_splits) {
 
 int lora_grad_splits(int M, int R, int C, int num_sms) {
   // Three CTAs fit on an SM up to rank 64, two above.  Up to rank 64 the token split is the largest whose CTAs all run at once:
-  // few long ranges, which end together (11392 tokens, us, and with the rule below: rank 32 x 24576 columns 107 and 117, 16 x 12288
-  // 64 and 68; 5119 tokens, 64 x 10240 39 and 50).  With more column tiles than that, and above rank 64, where a range is one chain
+  // few long ranges, which end together (us by single calls, and with the rule below: 11392 tokens, rank 32 x 24576 columns 107 and 117,
+  // 16 x 12288 64 and 68; 5119 tokens, 64 x 10240 39 and 50).  With more column tiles than that, and above rank 64, where a range is one chain
   // of sums, the split is chosen so that the grid fills whole waves: a grid of 1.08 waves takes as long as one of two.
   const int col_tiles = (C + LG_COLS - 1) / LG_COLS;
   const int slots = (R <= 64 ? 3 : 2) * num_sms;

@@ -467,9 +467,10 @@ __global__ void qk_norm_rope_kernel(const T* __restrict__ q_in, long long ld_q, 
 // bf16 vector form for D = LPH*EPL (128 or 256): LPH lanes hold a head, EPL consecutive channels each in one 8- or
 // 16-byte access, and a warp takes U times 32/LPH heads of one token; rotation partners are fetched with a warp shuffle
 // (partner lane = lane +- half/EPL).  Same arithmetic and rounding points as the kernel above.
-// What bounds it is instructions per entry: with a head of 128 to a warp (four entries a lane) shuffles, sums and the
-// angles, loaded again for each head, were most of them.
-// 8192 tokens x 40 heads of 128: forward 95 -> 69 us, backward 135 -> 102 us (the bytes take 26 and 38 us).
+// What bounds it is instructions per entry, not the bytes.  With a head of 128 to a warp (four entries a lane) shuffles, sums and the
+// angles, loaded again for each head, were most of them; then unpacking, shuffles of single values and addresses, so everything
+// stays in words of two 16-bit values.  Us, values and words (bytes' time), in a chain of calls: 11384 tokens, 32 and 8 heads of 128
+// forward 90, 57 (36), backward 130, 81 (53); 5119 tokens, 24 and 4 heads of 256 62, 40 and 88, 54.
 template <int EPL, bool BWD, int LPH, int U>
 __global__ void qk_norm_rope_vec_kernel(const __nv_bfloat16* __restrict__ q_in, long long ld_q,
                                         const __nv_bfloat16* __restrict__ k_in, long long ld_k, long long ld_dq,
@@ -499,9 +500,7 @@ __global__ void qk_norm_rope_vec_kernel(const __nv_bfloat16* __restrict__ q_in, 
   const bool in_rot = i0 < rot, lower = i0 < half;
   const int partner = in_rot ? (lower ? lane + shift : lane - shift) : lane;
 
-  // Everything in words of two 16-bit values: what instruction issue costs (it bounds this kernel, not the bytes) is unpacking,
-  // shuffles and addresses.  11384 tokens, 32 and 8 heads of 128: 98 -> 64 us forward, 137 -> 88 backward (bytes 36 and 53);
-  // 5119 tokens, 24 and 4 heads of 256: 71 -> 45, 94 -> 57.  Angles 16 bytes at a time change nothing.
+  // angles 16 bytes at a time change nothing
   constexpr int NW = EPL / 2;
   auto load = [&](const __nv_bfloat16* ptr, uint32_t* w) {
     if (EPL == 4) {
